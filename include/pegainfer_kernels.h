@@ -179,6 +179,9 @@ const char* pk_b200_version(void);
 /* Number of kernels launched by this library on the calling thread since the last
  * reset (bench.py's gpu_launches; counts launches recorded into a capture too). */
 int64_t pk_b200_launch_count(int reset);
+/* Waits inside this thread's kernels that ran into their iteration limit since cublas_init (0 in a sound run; the launch's results are then
+ * not valid).  Synchronises; -1: the device could not be read. */
+int pk_b200_wait_errors(void);
 /* Enable (1) / disable (0) programmatic dependent launch on this thread's launches. */
 void pk_b200_set_pdl(int enable);
 

@@ -25,10 +25,9 @@ struct ThreadState {
   size_t scratch_bytes = 0;
   int sm_count = 0;
   int device = -1;
-  // split-K workspace of the skinny tensor-core GEMM (gemm.cu): fp32 partial tiles + per-tile tickets
-  float* gemm_part = nullptr;
-  unsigned int* gemm_cnt = nullptr;
-  size_t gemm_part_bytes = 0;
+  float* work = nullptr;  // workspace of the delta rule over a sequence (qwen35_ops.cu)
+  size_t work_bytes = 0;
+  unsigned int* wait_err = nullptr;  // device word: bounded waits that ran out (pk_b200_wait_errors)
 };
 ThreadState& tls();
 int sm_count();
@@ -154,6 +153,16 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
   while (!mbar_try_wait(bar, parity)) {
   }
+}
+// Bounded wait: a barrier that never completes (a fault of the kernel) ends the CTA's work instead of hanging the GPU.  *dead (shared memory) is
+// set and seen by the CTA's other waits; the kernel counts it in ThreadState::wait_err and returns in order.
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* dead) {
+  for (uint32_t spins = 0; !mbar_try_wait(bar, parity); ++spins)
+    if (spins > (1u << 24) || *dead) {
+      *dead = 1;
+      return false;
+    }
+  return true;
 }
 __device__ __forceinline__ uint64_t l2_evict_first_policy() {
   uint64_t pol;

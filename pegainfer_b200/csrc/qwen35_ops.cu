@@ -441,11 +441,11 @@ int pk_b200_gated_delta_rule_prefill_recurrent(const pk_bf16* qkv_seq, const pk_
   ThreadState& ts = tls();
   static const bool use_v1 = [] { const char* e = getenv("PK_GDR_SEQ"); return e && atoi(e) == 1; }();
   const size_t per_tok = ((size_t)2 * num_key_heads * GK + 2 * num_value_heads) * sizeof(float);
-  if (!use_v1 && ts.gemm_part && ts.gemm_part_bytes >= per_tok * 64) {
-    const int max_t = (int)std::min<size_t>(ts.gemm_part_bytes / per_tok, 1 << 20);
+  if (!use_v1 && ts.work && ts.work_bytes >= per_tok * 64) {
+    const int max_t = (int)std::min<size_t>(ts.work_bytes / per_tok, 1 << 20);
     for (int t0 = 0; t0 < seq_len; t0 += max_t) {
       const int n = std::min(max_t, seq_len - t0);
-      float* qn = ts.gemm_part;
+      float* qn = ts.work;
       float* kn = qn + (size_t)n * num_key_heads * GK;
       float* dec = kn + (size_t)n * num_key_heads * GK;
       float* bet = dec + (size_t)n * num_value_heads;

@@ -43,17 +43,20 @@ void cublas_init() {
       ts.scratch_bytes = 0;
     }
   }
-  if (ts.gemm_part == nullptr) {  // split-K partial tiles: up to one 128 x 256 fp32 tile per SM, + tickets
-    const size_t bytes = (size_t)160 * 128 * 256 * 4;
-    void* p = nullptr;
-    void* c = nullptr;
-    if (cudaMalloc(&p, bytes) == cudaSuccess && cudaMalloc(&c, 4096) == cudaSuccess) {
-      cudaMemset(c, 0, 4096);
-      ts.gemm_part = static_cast<float*>(p);
-      ts.gemm_cnt = static_cast<unsigned int*>(c);
-      ts.gemm_part_bytes = bytes;
+  if (ts.wait_err == nullptr) {
+    if (cudaMalloc(&ts.wait_err, 256) == cudaSuccess) {
+      cudaMemset(ts.wait_err, 0, 256);
     } else {
-      if (p) cudaFree(p);
+      ts.wait_err = nullptr;
+      cudaGetLastError();
+    }
+  }
+  if (ts.work == nullptr) {
+    const size_t bytes = (size_t)20 << 20;
+    if (cudaMalloc(&ts.work, bytes) == cudaSuccess) {
+      ts.work_bytes = bytes;
+    } else {
+      ts.work = nullptr;
       cudaGetLastError();
     }
   }
@@ -67,12 +70,14 @@ void cublas_destroy() {
     ts.scratch = nullptr;
     ts.scratch_bytes = 0;
   }
-  if (ts.gemm_part != nullptr) {
-    cudaFree(ts.gemm_part);
-    cudaFree(ts.gemm_cnt);
-    ts.gemm_part = nullptr;
-    ts.gemm_cnt = nullptr;
-    ts.gemm_part_bytes = 0;
+  if (ts.wait_err != nullptr) {
+    cudaFree(ts.wait_err);
+    ts.wait_err = nullptr;
+  }
+  if (ts.work != nullptr) {
+    cudaFree(ts.work);
+    ts.work = nullptr;
+    ts.work_bytes = 0;
   }
 }
 
@@ -85,6 +90,14 @@ int64_t pk_b200_launch_count(int reset) {
   int64_t v = ts.launches;
   if (reset) ts.launches = 0;
   return v;
+}
+
+int pk_b200_wait_errors(void) {
+  pk::ThreadState& ts = pk::tls();
+  unsigned int n = 0;
+  if (ts.wait_err == nullptr) return 0;
+  if (cudaMemcpy(&n, ts.wait_err, sizeof n, cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
+  return (int)n;
 }
 
 void pk_b200_set_pdl(int enable) { pk::tls().pdl = enable != 0; }
