@@ -25,8 +25,6 @@ struct ThreadState {
   size_t scratch_bytes = 0;
   int sm_count = 0;
   int device = -1;
-  float* work = nullptr;  // workspace of the delta rule over a sequence (qwen35_ops.cu)
-  size_t work_bytes = 0;
   unsigned int* wait_err = nullptr;  // device word: bounded waits that ran out (pk_b200_wait_errors)
 };
 ThreadState& tls();

@@ -1,0 +1,409 @@
+// Gated delta rule over a sequence in chunks of 16 tokens, fp32 throughout, for bf16 q / k / v and one decay per head (recurrent_mixers.cu,
+// qwen35_ops.cu).  The recurrence  S <- g_t S;  u_t = beta_t (v_t - S^T k_t);  S <- S + k_t u_t^T;  o_t = S^T q_t  unrolled over a chunk that
+// starts with state S0, with r(t, s) = g_(s+1) ... g_t and c_t = g_1 ... g_t:
+//   w_t = beta_t (v_t - c_t S0^T k_t)                         u = (I + A)^-1 w,   A[t][s] = beta_t r(t, s) (k_t . k_s),  s < t
+//   o_t = c_t S0^T q_t + sum_(s <= t) B[t][s] u_s             B[t][s] = r(t, s) (q_t . k_s)
+//   S  <- c_16 S0 + sum_s r(16, s) k_s u_s^T
+// so that the long products (S0 with 32 vectors, the update with 16) have no dependency from token to token, and what is left of the chain is a
+// 16 x 16 triangle per chunk.  Factors r and c are products of decays, never quotients: nothing can overflow.
+//
+// CTA = (entry, head, COLS value columns).  Warps 0-3 hold S in fp32 registers, warp w the rows [w DK/4, (w+1) DK/4), as accumulators of
+// S^T tiles (m16n8k16: m = column, n = row).  In that layout the state is also the B operand of the products with k and q, so it never moves.  The
+// products run on the tensor cores without giving up fp32: k and q are bf16 rows, taken as they are (their unit factors are applied to the results),
+// and an fp32 operand (S, u) enters as the sum of three bf16 parts, which hold all of its 24 bits, each part with an accumulator of its own or added
+// smallest first; every product is exact and the sums are fp32.  What a chunk adds to S is summed from zero and added with one rounding.
+// The other warps each prepare every kDcPrep-th chunk by themselves, start to end (rows by cp.async, Gram matrices, decay products, the triangle's
+// inverse by forward substitution with a lane per column), so that their latency is spread over kDcPrep chunks; they hand it over in a ring of stages.
+// Bound by the chain products -> sum over the warps -> triangle -> update (three barriers of the four warps a chunk); the figures stand where it is launched.
+// Sums over s <= t leave the later tokens out by selection, not by a factor of zero: a NaN or an infinity reaches the same tokens as token by token.
+#pragma once
+#include "common.cuh"
+#include "mma.cuh"
+
+namespace pk {
+
+struct F2 {  // a packed pair of floats
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_pack(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 f2_unpack(F2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+
+constexpr int kDcT = 16;    // tokens per chunk
+constexpr int kDcPrep = 8;  // preparing warps = stages
+constexpr int kDcThreads = 128 + 32 * kDcPrep;
+
+struct DeltaRows {      // what one (entry, head) of the step works on
+  const bf16 *q, *k, *v;  // first token's row of the head's q, k and (from the CTA's first column on) v; rows `ld` elements apart
+  int ld, n;            // tokens
+  bool vec;             // rows of q and k start on 16-byte boundaries
+  float* state;         // [DK][vdim]
+  int vdim, col0;       // first column of this CTA
+  float unit_eps, q_scale;
+  unsigned int* err;    // counts waits that ran out (null: not counted)
+};
+
+// shared-memory layout, in floats
+template <int DK, int COLS>
+struct DcSmem {
+  static constexpr int LDR = DK + 8, PLD = COLS + 8, UBLD = 24;  // strides that keep fragment loads and partial stores free of bank conflicts
+  // a stage
+  static constexpr int RAW = 0;                        // bf16 [32][LDR]: k of 16 tokens, then q
+  static constexpr int TM = RAW + 2 * kDcT * LDR / 2;  // [16][16]: (I + A)^-1
+  static constexpr int BM = TM + 256;                  // [16][16]
+  static constexpr int VB = BM + 256;                  // [16][COLS]: beta v
+  static constexpr int CK = VB + kDcT * COLS;          // beta_t c_t kf_t
+  static constexpr int CQ = CK + kDcT;                 // c_t qf_t
+  static constexpr int CS = CQ + kDcT;                 // r(16, s) kf_s
+  static constexpr int GC = CS + kDcT;                 // c_16 (4 floats)
+  static constexpr int GM = GC + 4;                    // scratch: [2][16][17] k . k and q . k, then A [16][16]
+  static constexpr int FT = GM + 2 * kDcT * 17;        // scratch: beta_t kf_t, qf_t, decays
+  static constexpr int STAGE = FT + 3 * kDcT;
+  // the four state warps
+  static constexpr int PART = kDcPrep * STAGE;         // [4][32][PLD]
+  static constexpr int W = PART + 4 * 2 * kDcT * PLD;  // [16][COLS]
+  static constexpr int U = W + kDcT * COLS;            // [16][COLS]
+  static constexpr int UB = U + kDcT * COLS;           // bf16 [3][COLS][UBLD]: the parts of u_s r(16, s) kf_s, transposed
+  static constexpr int BARS = UB + 3 * COLS * UBLD / 2;
+  static constexpr int FLOATS = BARS + 4 * kDcPrep + 4;
+  static constexpr size_t BYTES = (size_t)FLOATS * 4;
+  static_assert(STAGE % 4 == 0 && PART % 4 == 0 && UB % 4 == 0 && BARS % 2 == 0, "alignment");
+};
+
+// x = hi + mid + lo, bf16 each (exact for finite x that does not underflow)
+__device__ __forceinline__ void dc_split(float x, float y, uint32_t (&p)[3]) {
+  p[0] = pack_bf16(x, y);
+  x -= bf16_lo(p[0]);
+  y -= bf16_hi(p[0]);
+  p[1] = pack_bf16(x, y);
+  x -= bf16_lo(p[1]);
+  y -= bf16_hi(p[1]);
+  p[2] = pack_bf16(x, y);
+}
+
+// `gates(t, g, beta)`: decay and write strength of token t (t < n).  `store(t, col, value)`: the read-out of token t.  All kDcThreads threads call.
+template <int DK, int COLS, typename Gates, typename Store>
+__device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates gates, Store store) {
+  using L = DcSmem<DK, COLS>;
+  constexpr int LDR = L::LDR, RW = DK / 4, RB = RW / 8, KS = RB / 2, MT = COLS / 16;  // rows, row blocks, k steps per warp; column tiles
+  constexpr int NTK = COLS / 8;                                                      // (token, column) pairs per thread in the triangle
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n = a.n, n_chunks = (n + kDcT - 1) / kDcT;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sm + L::BARS);
+  uint64_t* empty = full + kDcPrep;
+  volatile int* dead = reinterpret_cast<volatile int*>(empty + kDcPrep);
+  if (tid == 0) {
+    for (int i = 0; i < kDcPrep; ++i) {
+      mbar_init(full + i, 32);
+      mbar_init(empty + i, 4);
+    }
+    *dead = 0;
+    mbar_fence_init();
+  }
+  __syncthreads();
+  const int fr = (lane & 7) + ((lane >> 3) & 1) * 8, fc = ((lane >> 4) & 1) * 8;  // this lane's row and column in a 16 x 16 ldmatrix.x4
+  if (warp >= 4) {
+    // ---- preparation
+    constexpr int PR = DK / 8, NVL = kDcT * COLS / 32;  // 16-byte pieces per row; values per lane
+    const int pw = warp - 4, half = lane >> 4, s = lane & 15;
+    float* st = sm + pw * L::STAGE;
+    bf16* raw = reinterpret_cast<bf16*>(st + L::RAW);
+    uint32_t ph = 1;
+    for (int b = pw; b < n_chunks; b += kDcPrep, ph ^= 1u) {
+      const int t0 = b * kDcT, nb = min(kDcT, n - t0);  // tokens past the end: zero rows, decay 1, write strength 0
+      mbar_wait_bounded(empty + pw, ph, dead);
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < PR; ++i) {
+        const int p = lane + 32 * i, row = p / PR, c = (p % PR) * 8, t = row & (kDcT - 1);
+        const bf16* src = (row < kDcT ? a.k : a.q) + (size_t)(t0 + t) * a.ld + c;
+        bf16* dst = raw + row * LDR + c;
+        if (t >= nb) {
+          *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+        } else if (a.vec) {
+          cp_async16(dst, src);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) dst[j] = src[j];
+        }
+      }
+      cp_async_commit();
+      float g = 1.f, beta = 0.f;
+      if (half == 0 && s < nb) gates(t0 + s, g, beta);
+      bf16 vr[NVL];
+#pragma unroll
+      for (int i = 0; i < NVL; ++i) {
+        const int at = lane + 32 * i, t = at / COLS, c = at % COLS;
+        vr[i] = t < nb && a.col0 + c < a.vdim ? a.v[(size_t)(t0 + t) * a.ld + c] : f2bf(0.f);
+      }
+      cp_async_wait_all();
+      __syncwarp();
+      // unit factors: lane = row
+      float d[4] = {};
+#pragma unroll
+      for (int i = 0; i < PR; ++i) {
+        const uint4 u = *reinterpret_cast<const uint4*>(raw + lane * LDR + i * 8);
+        d[0] = fmaf(bf16_lo(u.x), bf16_lo(u.x), d[0]);
+        d[1] = fmaf(bf16_hi(u.x), bf16_hi(u.x), d[1]);
+        d[2] = fmaf(bf16_lo(u.y), bf16_lo(u.y), d[2]);
+        d[3] = fmaf(bf16_hi(u.y), bf16_hi(u.y), d[3]);
+        d[0] = fmaf(bf16_lo(u.z), bf16_lo(u.z), d[0]);
+        d[1] = fmaf(bf16_hi(u.z), bf16_hi(u.z), d[1]);
+        d[2] = fmaf(bf16_lo(u.w), bf16_lo(u.w), d[2]);
+        d[3] = fmaf(bf16_hi(u.w), bf16_hi(u.w), d[3]);
+      }
+      const float unit = (half ? a.q_scale : 1.f) / sqrtf((d[0] + d[1]) + (d[2] + d[3]) + a.unit_eps);
+      const float kf = __shfl_sync(0xffffffffu, unit, s), ft = half ? unit : beta * unit;
+      st[L::FT + lane] = ft;
+      if (half == 0) st[L::FT + 2 * kDcT + s] = g;
+      // Gram matrices k . k and q . k.  A fragments are rows of k (q); as B operand (its columns are rows of k) the same registers serve: tokens
+      // 0-7 in registers 0 and 2, 8-15 in 1 and 3.  Odd and even k steps add up apart.
+      float kk[2][2][4] = {}, qk[2][2][4] = {};
+#pragma unroll
+      for (int k0 = 0; k0 < DK / 16; ++k0) {
+        uint32_t fk[4], fq[4];
+        ldsm_x4(fk, raw + fr * LDR + k0 * 16 + fc);
+        ldsm_x4(fq, raw + (kDcT + fr) * LDR + k0 * 16 + fc);
+        mma_bf16_16816(kk[k0 & 1][0], fk, fk[0], fk[2]);
+        mma_bf16_16816(kk[k0 & 1][1], fk, fk[1], fk[3]);
+        mma_bf16_16816(qk[k0 & 1][0], fq, fk[0], fk[2]);
+        mma_bf16_16816(qk[k0 & 1][1], fq, fk[1], fk[3]);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int at = ((lane >> 2) + (e >> 1) * 8) * 17 + j * 8 + (lane & 3) * 2 + (e & 1);
+          st[L::GM + at] = kk[0][j][e] + kk[1][j][e];
+          st[L::GM + kDcT * 17 + at] = qk[0][j][e] + qk[1][j][e];
+        }
+      __syncwarp();
+      // lanes 0-15: column s of A;  16-31: column s of B
+      float gt[kDcT], f[kDcT], gm[kDcT];
+#pragma unroll
+      for (int t = 0; t < kDcT; t += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(st + L::FT + 2 * kDcT + t), y = *reinterpret_cast<const float4*>(st + L::FT + half * kDcT + t);
+        gt[t] = x.x; gt[t + 1] = x.y; gt[t + 2] = x.z; gt[t + 3] = x.w;
+        f[t] = y.x; f[t + 1] = y.y; f[t + 2] = y.z; f[t + 3] = y.w;
+      }
+#pragma unroll
+      for (int t = 0; t < kDcT; ++t) gm[t] = st[L::GM + half * kDcT * 17 + t * 17 + s];
+      float r = 1.f, c = 1.f, cs = 1.f;
+#pragma unroll
+      for (int t = 0; t < kDcT; ++t) {
+        r = t > s ? r * gt[t] : r;
+        c *= gt[t];
+        cs = t == s ? c : cs;
+        gm[t] = t > s || (half && t == s) ? (f[t] * kf) * r * gm[t] : 0.f;
+      }
+      __syncwarp();  // the Gram matrices have been read
+      float* to = half ? st + L::BM : st + L::GM;
+#pragma unroll
+      for (int t = 0; t < kDcT; ++t) to[t * kDcT + s] = gm[t];
+      st[(half ? L::CQ : L::CK) + s] = ft * cs;
+      if (half == 0) st[L::CS + s] = r * kf;
+      if (lane == 0) st[L::GC] = c;
+#pragma unroll
+      for (int i = 0; i < NVL; ++i) {
+        const int at = lane + 32 * i;
+        st[L::VB + at] = __shfl_sync(0xffffffffu, beta, at / COLS) * bf2f(vr[i]);
+      }
+      __syncwarp();
+      float T[kDcT];  // column s of (I + A)^-1
+#pragma unroll
+      for (int t = 0; t < kDcT; ++t) {
+        float acc = t == s ? 1.f : 0.f;
+#pragma unroll
+        for (int s4 = 0; s4 < t; s4 += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(st + L::GM + t * kDcT + s4);
+          acc = fmaf(-x.x, T[s4], acc);
+          if (s4 + 1 < t) acc = fmaf(-x.y, T[s4 + 1], acc);
+          if (s4 + 2 < t) acc = fmaf(-x.z, T[s4 + 2], acc);
+          if (s4 + 3 < t) acc = fmaf(-x.w, T[s4 + 3], acc);
+        }
+        T[t] = acc;
+      }
+      if (half == 0) {
+#pragma unroll
+        for (int t = 0; t < kDcT; ++t) st[L::TM + t * kDcT + s] = T[t];
+      }
+      mbar_arrive(full + pw);
+    }
+    return;
+  }
+  // ---- state and products
+  const int g = lane >> 2, tq = lane & 3, row0 = warp * RW;
+  float S[MT][RB][4];  // [..][e]: column 16 mt + g + 8 (e >> 1), row row0 + 8 j + 2 tq + (e & 1)
+  auto each_state = [&](auto body) {
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int j = 0; j < RB; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int col = a.col0 + mt * 16 + g + (e >> 1) * 8;
+          body(S[mt][j][e], a.state + (size_t)(row0 + j * 8 + 2 * tq + (e & 1)) * a.vdim + col, col < a.vdim);
+        }
+  };
+  each_state([](float& x, const float* p, bool on) { x = on ? *p : 0.f; });
+  auto bar = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
+  const int pc = tid % COLS, pt0 = tid / COLS * NTK;  // triangle: column pc, tokens pt0 .. pt0 + NTK - 1
+  bf16* ub = reinterpret_cast<bf16*>(sm + L::UB);
+  int slot = 0;
+  uint32_t ph = 0;
+  for (int b = 0; b < n_chunks; ++b) {
+    const float* st = sm + slot * L::STAGE;
+    const bf16* raw = reinterpret_cast<const bf16*>(st + L::RAW);
+    // the state's parts as B operand: k step ks, columns 8 nt ..
+    uint32_t sp[KS][2 * MT][2][3];
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+      for (int nt = 0; nt < 2 * MT; ++nt)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) dc_split(S[nt >> 1][2 * ks + i][(nt & 1) * 2], S[nt >> 1][2 * ks + i][(nt & 1) * 2 + 1], sp[ks][nt][i]);
+    mbar_wait_bounded(full + slot, ph, dead);
+    __syncwarp();
+    // ---- S0^T k and S0^T q over this warp's rows
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      float p[2 * MT][3][4] = {};
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks) {
+        uint32_t f[4];
+        ldsm_x4(f, raw + (x * kDcT + fr) * LDR + row0 + ks * 16 + fc);
+#pragma unroll
+        for (int part = 0; part < 3; ++part)
+#pragma unroll
+          for (int nt = 0; nt < 2 * MT; ++nt) mma_bf16_16816(p[nt][part], f, sp[ks][nt][0][part], sp[ks][nt][1][part]);
+      }
+      float* to = sm + L::PART + (warp * 2 * kDcT + x * kDcT + g) * L::PLD + 2 * tq;
+#pragma unroll
+      for (int nt = 0; nt < 2 * MT; ++nt) {
+        float v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = p[nt][0][e] + (p[nt][1][e] + p[nt][2][e]);
+        *reinterpret_cast<float2*>(to + nt * 8) = make_float2(v[0], v[1]);
+        *reinterpret_cast<float2*>(to + 8 * L::PLD + nt * 8) = make_float2(v[2], v[3]);
+      }
+    }
+    bar();
+    float po[NTK];
+#pragma unroll
+    for (int i = 0; i < NTK; ++i) {
+      const int t = pt0 + i;
+      float pk[4], pq[4];
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        pk[w] = sm[L::PART + (w * 2 * kDcT + t) * L::PLD + pc];
+        pq[w] = sm[L::PART + (w * 2 * kDcT + kDcT + t) * L::PLD + pc];
+      }
+      sm[L::W + t * COLS + pc] = fmaf(-st[L::CK + t], (pk[0] + pk[1]) + (pk[2] + pk[3]), st[L::VB + t * COLS + pc]);
+      po[i] = st[L::CQ + t] * ((pq[0] + pq[1]) + (pq[2] + pq[3]));
+    }
+    bar();
+    float u[NTK];
+#pragma unroll
+    for (int i = 0; i < NTK; ++i) u[i] = 0.f;
+#pragma unroll
+    for (int s4 = 0; s4 < kDcT; s4 += 4) {
+      float w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = sm[L::W + (s4 + j) * COLS + pc];
+#pragma unroll
+      for (int i = 0; i < NTK; ++i) {
+        const int t = pt0 + i;
+        const float4 m = *reinterpret_cast<const float4*>(st + L::TM + t * kDcT + s4);
+        u[i] = fmaf(m.x, s4 <= t ? w[0] : 0.f, u[i]);
+        u[i] = fmaf(m.y, s4 + 1 <= t ? w[1] : 0.f, u[i]);
+        u[i] = fmaf(m.z, s4 + 2 <= t ? w[2] : 0.f, u[i]);
+        u[i] = fmaf(m.w, s4 + 3 <= t ? w[3] : 0.f, u[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NTK; i += 2) {
+      sm[L::U + (pt0 + i) * COLS + pc] = u[i];
+      sm[L::U + (pt0 + i + 1) * COLS + pc] = u[i + 1];
+      uint32_t q[3];
+      dc_split(u[i] * st[L::CS + pt0 + i], u[i + 1] * st[L::CS + pt0 + i + 1], q);
+#pragma unroll
+      for (int part = 0; part < 3; ++part) *reinterpret_cast<uint32_t*>(ub + (part * COLS + pc) * L::UBLD + pt0 + i) = q[part];
+    }
+    bar();
+    // ---- state update: S^T = c S^T + U^T K
+    const float gc = st[L::GC];
+    uint32_t fu[MT][3][4];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int part = 0; part < 3; ++part) ldsm_x4(fu[mt][part], ub + (part * COLS + mt * 16 + fr) * L::UBLD + fc);
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      uint32_t fk[4];
+      ldsm_x4_trans(fk, raw + fr * LDR + row0 + ks * 16 + fc);
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          float add[4] = {};
+#pragma unroll
+          for (int part = 2; part >= 0; --part) mma_bf16_16816(add, fu[mt][part], fk[2 * i], fk[2 * i + 1]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) S[mt][2 * ks + i][e] = fmaf(S[mt][2 * ks + i][e], gc, add[e]);
+        }
+    }
+    // ---- read-out
+#pragma unroll
+    for (int s4 = 0; s4 < kDcT; s4 += 4) {
+      float w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = sm[L::U + (s4 + j) * COLS + pc];
+#pragma unroll
+      for (int i = 0; i < NTK; ++i) {
+        const int t = pt0 + i;
+        const float4 m = *reinterpret_cast<const float4*>(st + L::BM + t * kDcT + s4);
+        po[i] = fmaf(m.x, s4 <= t ? w[0] : 0.f, po[i]);
+        po[i] = fmaf(m.y, s4 + 1 <= t ? w[1] : 0.f, po[i]);
+        po[i] = fmaf(m.z, s4 + 2 <= t ? w[2] : 0.f, po[i]);
+        po[i] = fmaf(m.w, s4 + 3 <= t ? w[3] : 0.f, po[i]);
+      }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty + slot);  // this warp has read all of the stage
+#pragma unroll
+    for (int i = 0; i < NTK; ++i)
+      if (b * kDcT + pt0 + i < n && a.col0 + pc < a.vdim) store(b * kDcT + pt0 + i, pc, po[i]);
+    if (++slot == kDcPrep) {
+      slot = 0;
+      ph ^= 1u;
+    }
+  }
+  each_state([](float& x, float* p, bool on) {
+    if (on) *p = x;
+  });
+  if (tid == 0 && *dead && a.err) atomicAdd(a.err, 1u);
+}
+
+}  // namespace pk

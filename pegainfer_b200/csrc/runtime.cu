@@ -51,15 +51,6 @@ void cublas_init() {
       cudaGetLastError();
     }
   }
-  if (ts.work == nullptr) {
-    const size_t bytes = (size_t)20 << 20;
-    if (cudaMalloc(&ts.work, bytes) == cudaSuccess) {
-      ts.work_bytes = bytes;
-    } else {
-      ts.work = nullptr;
-      cudaGetLastError();
-    }
-  }
   (void)pk::sm_count();
 }
 
@@ -73,11 +64,6 @@ void cublas_destroy() {
   if (ts.wait_err != nullptr) {
     cudaFree(ts.wait_err);
     ts.wait_err = nullptr;
-  }
-  if (ts.work != nullptr) {
-    cudaFree(ts.work);
-    ts.work = nullptr;
-    ts.work_bytes = 0;
   }
 }
 
