@@ -12,6 +12,7 @@
 // products run on the tensor cores without giving up fp32: k and q are bf16 rows, taken as they are (their unit factors are applied to the results),
 // and an fp32 operand (S, u) enters as the sum of three bf16 parts, which hold all of its 24 bits, each part with an accumulator of its own or added
 // smallest first; every product is exact and the sums are fp32.  What a chunk adds to S is summed from zero and added with one rounding.
+// Warps 4-7 read out, a chunk behind: q . S0 of the four warps, and B u.
 // The other warps each prepare every kDcPrep-th chunk by themselves, start to end (rows by cp.async, Gram matrices, decay products, the triangle's
 // inverse by forward substitution with a lane per column), so that their latency is spread over kDcPrep chunks; they hand it over in a ring of stages.
 // Bound by the chain products -> sum over the warps -> triangle -> update (three barriers of the four warps a chunk); the figures stand where it is launched.
@@ -52,8 +53,8 @@ __device__ __forceinline__ float2 f2_unpack(F2 a) {
 }
 
 constexpr int kDcT = 16;    // tokens per chunk
-constexpr int kDcPrep = 8;  // preparing warps = stages
-constexpr int kDcThreads = 128 + 32 * kDcPrep;
+constexpr int kDcPrep = 4;  // preparing warps = stages; with 12 warps a thread may hold 168 registers (four of them were enough to keep the state warps busy)
+constexpr int kDcThreads = 256 + 32 * kDcPrep;
 
 struct DeltaRows {      // what one (entry, head) of the step works on
   const bf16 *q, *k, *v;  // first token's row of the head's q, k and (from the CTA's first column on) v; rows `ld` elements apart
@@ -82,25 +83,27 @@ struct DcSmem {
   static constexpr int FT = GM + 2 * kDcT * 17;        // scratch: beta_t kf_t, qf_t, decays
   static constexpr int STAGE = FT + 3 * kDcT;
   // the four state warps
-  static constexpr int PART = kDcPrep * STAGE;         // [4][32][PLD]
-  static constexpr int W = PART + 4 * 2 * kDcT * PLD;  // [16][COLS]
-  static constexpr int U = W + kDcT * COLS;            // [16][COLS]
-  static constexpr int UB = U + kDcT * COLS;           // bf16 [3][COLS][UBLD]: the parts of u_s r(16, s) kf_s, transposed
+  static constexpr int WLD = kDcT + 4;                 // a column's 16 tokens, 16-byte reads without conflicts
+  static constexpr int PK = kDcPrep * STAGE;           // [4][16][PLD]: S0^T k over each warp's rows
+  static constexpr int PQ = PK + 4 * kDcT * PLD;       // two of [4][16][PLD]: S0^T q
+  static constexpr int W = PQ + 2 * 4 * kDcT * PLD;    // [COLS][WLD]
+  static constexpr int U = W + COLS * WLD;             // two of [COLS][WLD]
+  static constexpr int UB = U + 2 * COLS * WLD;        // bf16 [3][COLS][UBLD]: the parts of u_s r(16, s) kf_s, transposed
   static constexpr int BARS = UB + 3 * COLS * UBLD / 2;
   static constexpr int FLOATS = BARS + 4 * kDcPrep + 4;
   static constexpr size_t BYTES = (size_t)FLOATS * 4;
-  static_assert(STAGE % 4 == 0 && PART % 4 == 0 && UB % 4 == 0 && BARS % 2 == 0, "alignment");
+  static_assert(STAGE % 4 == 0 && PK % 4 == 0 && W % 4 == 0 && UB % 4 == 0 && BARS % 2 == 0, "alignment");
 };
 
-// x = hi + mid + lo, bf16 each (exact for finite x that does not underflow)
+// x = hi + mid + lo, bf16 each: cut off after 8 and 16 of the 24 bits, so the sum is exact (for finite x that does not underflow)
 __device__ __forceinline__ void dc_split(float x, float y, uint32_t (&p)[3]) {
-  p[0] = pack_bf16(x, y);
-  x -= bf16_lo(p[0]);
-  y -= bf16_hi(p[0]);
-  p[1] = pack_bf16(x, y);
-  x -= bf16_lo(p[1]);
-  y -= bf16_hi(p[1]);
-  p[2] = pack_bf16(x, y);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const uint32_t ux = __float_as_uint(x), uy = __float_as_uint(y);
+    p[i] = __byte_perm(ux, uy, 0x7632);
+    x -= __uint_as_float(ux & 0xffff0000u);
+    y -= __uint_as_float(uy & 0xffff0000u);
+  }
 }
 
 // `gates(t, g, beta)`: decay and write strength of token t (t < n).  `store(t, col, value)`: the read-out of token t.  All kDcThreads threads call.
@@ -117,17 +120,17 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
   if (tid == 0) {
     for (int i = 0; i < kDcPrep; ++i) {
       mbar_init(full + i, 32);
-      mbar_init(empty + i, 4);
+      mbar_init(empty + i, 8);
     }
     *dead = 0;
     mbar_fence_init();
   }
   __syncthreads();
   const int fr = (lane & 7) + ((lane >> 3) & 1) * 8, fc = ((lane >> 4) & 1) * 8;  // this lane's row and column in a 16 x 16 ldmatrix.x4
-  if (warp >= 4) {
+  if (warp >= 8) {
     // ---- preparation
     constexpr int PR = DK / 8, NVL = kDcT * COLS / 32;  // 16-byte pieces per row; values per lane
-    const int pw = warp - 4, half = lane >> 4, s = lane & 15;
+    const int pw = warp - 8, half = lane >> 4, s = lane & 15;
     float* st = sm + pw * L::STAGE;
     bf16* raw = reinterpret_cast<bf16*>(st + L::RAW);
     uint32_t ph = 1;
@@ -150,6 +153,15 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
         }
       }
       cp_async_commit();
+      {  // this warp's next chunk on its way to L2: a lane per row, two lines each
+        const int t = t0 + kDcPrep * kDcT + s;
+        if (t < n) {
+          const bf16* src = (half ? a.q : a.k) + (size_t)t * a.ld;
+          prefetch_l2(src);
+          if (DK > 64) prefetch_l2(src + 64);
+          if (half) prefetch_l2(a.v + (size_t)t * a.ld);
+        }
+      }
       float g = 1.f, beta = 0.f;
       if (half == 0 && s < nb) gates(t0 + s, g, beta);
       bf16 vr[NVL];
@@ -253,6 +265,63 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
     }
     return;
   }
+  const int pc = (tid & 127) % COLS, pt0 = (tid & 127) / COLS * NTK;  // triangle and read-out: column pc, tokens pt0 .. pt0 + NTK - 1
+  // sum over s <= t of m[t][s] x[s] for this thread's tokens
+  auto lower = [&](const float* m, const float* x, float (&acc)[NTK]) {
+    float4 v[kDcT / 4], w[NTK][kDcT / 4];
+#pragma unroll
+    for (int j = 0; j < kDcT / 4; ++j) v[j] = *reinterpret_cast<const float4*>(x + pc * L::WLD + 4 * j);
+#pragma unroll
+    for (int i = 0; i < NTK; ++i)
+#pragma unroll
+      for (int j = 0; j < kDcT / 4; ++j) w[i][j] = *reinterpret_cast<const float4*>(m + (pt0 + i) * kDcT + 4 * j);
+#pragma unroll
+    for (int i = 0; i < NTK; ++i) {
+      const int t = pt0 + i;
+      float a1 = 0.f;  // two chains
+#pragma unroll
+      for (int j = 0; j < kDcT / 4; ++j) {
+        acc[i] = fmaf(w[i][j].x, 4 * j <= t ? v[j].x : 0.f, acc[i]);
+        a1 = fmaf(w[i][j].y, 4 * j + 1 <= t ? v[j].y : 0.f, a1);
+        acc[i] = fmaf(w[i][j].z, 4 * j + 2 <= t ? v[j].z : 0.f, acc[i]);
+        a1 = fmaf(w[i][j].w, 4 * j + 3 <= t ? v[j].w : 0.f, a1);
+      }
+      acc[i] += a1;
+    }
+  };
+  // Named barriers: 1 the state warps, 4 / 5 u and S0^T q of an even / odd chunk are there, 6 / 7 they have been read
+  if (warp >= 4) {
+    // ---- read-out
+    int slot = 0;
+    uint32_t ph = 0;
+    for (int b = 0; b < n_chunks; ++b) {
+      const float* st = sm + slot * L::STAGE;
+      mbar_wait_bounded(full + slot, ph, dead);
+      __syncwarp();
+      if (b & 1) asm volatile("bar.sync 5, 256;" ::: "memory");
+      else asm volatile("bar.sync 4, 256;" ::: "memory");
+      float o[NTK];
+      const float* pq = sm + L::PQ + (b & 1) * 4 * kDcT * L::PLD + pc;
+#pragma unroll
+      for (int i = 0; i < NTK; ++i) {
+        const int t = pt0 + i;
+        o[i] = st[L::CQ + t] * ((pq[t * L::PLD] + pq[(kDcT + t) * L::PLD]) + (pq[(2 * kDcT + t) * L::PLD] + pq[(3 * kDcT + t) * L::PLD]));
+      }
+      lower(st + L::BM, sm + L::U + (b & 1) * COLS * L::WLD, o);
+      if (b & 1) asm volatile("bar.arrive 7, 256;" ::: "memory");
+      else asm volatile("bar.arrive 6, 256;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty + slot);
+#pragma unroll
+      for (int i = 0; i < NTK; ++i)
+        if (b * kDcT + pt0 + i < n && a.col0 + pc < a.vdim) store(b * kDcT + pt0 + i, pc, o[i]);
+      if (++slot == kDcPrep) {
+        slot = 0;
+        ph ^= 1u;
+      }
+    }
+    return;
+  }
   // ---- state and products
   const int g = lane >> 2, tq = lane & 3, row0 = warp * RW;
   float S[MT][RB][4];  // [..][e]: column 16 mt + g + 8 (e >> 1), row row0 + 8 j + 2 tq + (e & 1)
@@ -269,7 +338,6 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
   };
   each_state([](float& x, const float* p, bool on) { x = on ? *p : 0.f; });
   auto bar = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
-  const int pc = tid % COLS, pt0 = tid / COLS * NTK;  // triangle: column pc, tokens pt0 .. pt0 + NTK - 1
   bf16* ub = reinterpret_cast<bf16*>(sm + L::UB);
   int slot = 0;
   uint32_t ph = 0;
@@ -286,10 +354,12 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
         for (int i = 0; i < 2; ++i) dc_split(S[nt >> 1][2 * ks + i][(nt & 1) * 2], S[nt >> 1][2 * ks + i][(nt & 1) * 2 + 1], sp[ks][nt][i]);
     mbar_wait_bounded(full + slot, ph, dead);
     __syncwarp();
-    // ---- S0^T k and S0^T q over this warp's rows
+    // S0^T x over this warp's rows, x = k (0) or q (1)
+    auto products = [&](int x, float (&p)[2 * MT][3][4]) {
 #pragma unroll
-    for (int x = 0; x < 2; ++x) {
-      float p[2 * MT][3][4] = {};
+      for (int nt = 0; nt < 2 * MT; ++nt)
+#pragma unroll
+        for (int part = 0; part < 3; ++part) p[nt][part][0] = p[nt][part][1] = p[nt][part][2] = p[nt][part][3] = 0.f;
 #pragma unroll
       for (int ks = 0; ks < KS; ++ks) {
         uint32_t f[4];
@@ -299,7 +369,9 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
 #pragma unroll
           for (int nt = 0; nt < 2 * MT; ++nt) mma_bf16_16816(p[nt][part], f, sp[ks][nt][0][part], sp[ks][nt][1][part]);
       }
-      float* to = sm + L::PART + (warp * 2 * kDcT + x * kDcT + g) * L::PLD + 2 * tq;
+    };
+    auto put = [&](float* to, const float (&p)[2 * MT][3][4]) {
+      to += (warp * kDcT + g) * L::PLD + 2 * tq;
 #pragma unroll
       for (int nt = 0; nt < 2 * MT; ++nt) {
         float v[4];
@@ -308,52 +380,49 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
         *reinterpret_cast<float2*>(to + nt * 8) = make_float2(v[0], v[1]);
         *reinterpret_cast<float2*>(to + 8 * L::PLD + nt * 8) = make_float2(v[2], v[3]);
       }
+    };
+    float p[2 * MT][3][4];
+    products(0, p);
+    put(sm + L::PK, p);
+    float ck[NTK], vb[NTK], cs[NTK];  // on their way before the barrier
+#pragma unroll
+    for (int i = 0; i < NTK; ++i) {
+      ck[i] = st[L::CK + pt0 + i];
+      cs[i] = st[L::CS + pt0 + i];
+      vb[i] = st[L::VB + (pt0 + i) * COLS + pc];
     }
+    const float gc = st[L::GC];
     bar();
-    float po[NTK];
+    const float* pk = sm + L::PK + pc;
 #pragma unroll
     for (int i = 0; i < NTK; ++i) {
       const int t = pt0 + i;
-      float pk[4], pq[4];
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        pk[w] = sm[L::PART + (w * 2 * kDcT + t) * L::PLD + pc];
-        pq[w] = sm[L::PART + (w * 2 * kDcT + kDcT + t) * L::PLD + pc];
-      }
-      sm[L::W + t * COLS + pc] = fmaf(-st[L::CK + t], (pk[0] + pk[1]) + (pk[2] + pk[3]), st[L::VB + t * COLS + pc]);
-      po[i] = st[L::CQ + t] * ((pq[0] + pq[1]) + (pq[2] + pq[3]));
+      const float x = (pk[t * L::PLD] + pk[(kDcT + t) * L::PLD]) + (pk[(2 * kDcT + t) * L::PLD] + pk[(3 * kDcT + t) * L::PLD]);
+      sm[L::W + pc * L::WLD + t] = fmaf(-ck[i], x, vb[i]);
     }
+    products(1, p);  // under the barrier and the triangle
     bar();
     float u[NTK];
 #pragma unroll
     for (int i = 0; i < NTK; ++i) u[i] = 0.f;
-#pragma unroll
-    for (int s4 = 0; s4 < kDcT; s4 += 4) {
-      float w[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = sm[L::W + (s4 + j) * COLS + pc];
-#pragma unroll
-      for (int i = 0; i < NTK; ++i) {
-        const int t = pt0 + i;
-        const float4 m = *reinterpret_cast<const float4*>(st + L::TM + t * kDcT + s4);
-        u[i] = fmaf(m.x, s4 <= t ? w[0] : 0.f, u[i]);
-        u[i] = fmaf(m.y, s4 + 1 <= t ? w[1] : 0.f, u[i]);
-        u[i] = fmaf(m.z, s4 + 2 <= t ? w[2] : 0.f, u[i]);
-        u[i] = fmaf(m.w, s4 + 3 <= t ? w[3] : 0.f, u[i]);
-      }
+    lower(st + L::TM, sm + L::W, u);
+    if (b >= 2) {  // the read-out warps are done with this buffer's last contents
+      if (b & 1) asm volatile("bar.sync 7, 256;" ::: "memory");
+      else asm volatile("bar.sync 6, 256;" ::: "memory");
     }
 #pragma unroll
     for (int i = 0; i < NTK; i += 2) {
-      sm[L::U + (pt0 + i) * COLS + pc] = u[i];
-      sm[L::U + (pt0 + i + 1) * COLS + pc] = u[i + 1];
+      *reinterpret_cast<float2*>(sm + L::U + ((b & 1) * COLS + pc) * L::WLD + pt0 + i) = make_float2(u[i], u[i + 1]);
       uint32_t q[3];
-      dc_split(u[i] * st[L::CS + pt0 + i], u[i + 1] * st[L::CS + pt0 + i + 1], q);
+      dc_split(u[i] * cs[i], u[i + 1] * cs[i + 1], q);
 #pragma unroll
       for (int part = 0; part < 3; ++part) *reinterpret_cast<uint32_t*>(ub + (part * COLS + pc) * L::UBLD + pt0 + i) = q[part];
     }
     bar();
+    put(sm + L::PQ + (b & 1) * 4 * kDcT * L::PLD, p);
+    if (b & 1) asm volatile("bar.arrive 5, 256;" ::: "memory");
+    else asm volatile("bar.arrive 4, 256;" ::: "memory");
     // ---- state update: S^T = c S^T + U^T K
-    const float gc = st[L::GC];
     uint32_t fu[MT][3][4];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
@@ -374,27 +443,8 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
           for (int e = 0; e < 4; ++e) S[mt][2 * ks + i][e] = fmaf(S[mt][2 * ks + i][e], gc, add[e]);
         }
     }
-    // ---- read-out
-#pragma unroll
-    for (int s4 = 0; s4 < kDcT; s4 += 4) {
-      float w[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = sm[L::U + (s4 + j) * COLS + pc];
-#pragma unroll
-      for (int i = 0; i < NTK; ++i) {
-        const int t = pt0 + i;
-        const float4 m = *reinterpret_cast<const float4*>(st + L::BM + t * kDcT + s4);
-        po[i] = fmaf(m.x, s4 <= t ? w[0] : 0.f, po[i]);
-        po[i] = fmaf(m.y, s4 + 1 <= t ? w[1] : 0.f, po[i]);
-        po[i] = fmaf(m.z, s4 + 2 <= t ? w[2] : 0.f, po[i]);
-        po[i] = fmaf(m.w, s4 + 3 <= t ? w[3] : 0.f, po[i]);
-      }
-    }
     __syncwarp();
     if (lane == 0) mbar_arrive(empty + slot);  // this warp has read all of the stage
-#pragma unroll
-    for (int i = 0; i < NTK; ++i)
-      if (b * kDcT + pt0 + i < n && a.col0 + pc < a.vdim) store(b * kDcT + pt0 + i, pc, po[i]);
     if (++slot == kDcPrep) {
       slot = 0;
       ph ^= 1u;
