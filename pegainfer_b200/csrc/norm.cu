@@ -6,6 +6,7 @@
 // Unlike the reference there is no residual->out staging memcpy.  One CTA per token; the row is
 // read from HBM once (16-B vectors) and parked in shared memory as fp32 between the two passes.
 #include "common.cuh"
+#include "norm_rows.cuh"
 
 namespace pk {
 
@@ -78,6 +79,10 @@ static void launch_norm(const pk_bf16* x, pk_bf16* hidden, const pk_bf16* residu
                         pk_stream stream) {
   if (dim <= 0 || rows <= 0) return;
   const bool vec = dim % 8 == 0 && al16(x) && al16(hidden) && al16(residual) && al16(w) && al16(out);
+  if (vec && rms_rows_fit(dim, rows)) {
+    launch_rms_rows<kFusedAdd ? 1 : 0>((const bf16*)x, (bf16*)hidden, (const bf16*)residual, (const bf16*)w, (bf16*)out, dim, rows, eps, stream);
+    return;
+  }
   int threads = vec ? (dim / 8) : dim;
   threads = ((threads + 31) / 32) * 32;
   if (threads > 1024) threads = 1024;
