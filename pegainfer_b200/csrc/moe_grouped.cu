@@ -1,171 +1,378 @@
 // Mixture-of-experts feed-forward for many tokens at once (prompt portions): the (token, choice) pairs are bucketed by
 // expert, and each expert's rows run as one tensor-core GEMM over that expert's weights, so a weight tile is read once
-// per 64 rows instead of once per token (moe.cu is the per-token form for a few tokens).
-//   1. moe_bucket_kernel     one CTA: histogram of the routed ids, offsets per expert, a slot for every pair, and the list
-//                            of 64-row tiles (expert, first slot).  Which slot a pair gets inside its expert's run may
-//                            vary from run to run; every row's result is independent of its slot, so outputs do not.
-//   2. moe_grouped_gemm<0>   hid[slot] = relu(W_up[e] x[token(slot)])^2          (rows gathered through the slot list)
+// per 256 rows instead of once per token (moe.cu is the per-token form for a few tokens).
+//   1. moe_bucket_kernel     one CTA: histogram of the routed ids, offsets per expert, a slot for every pair, and the list of row tiles: an
+//                            expert's rows in as few tiles of at most 256 as they need, of equal size.  Which slot a pair gets inside its
+//                            expert's run may vary from run to run; every row's result is independent of its slot, so outputs do not.
+//   2. moe_gather_kernel     xs[slot] = x[token(slot)]  (TMA then reads an expert's rows as a block)
+//   3. moe_grouped_gemm<0>   hid[slot] = relu(W_up[e] xs[slot])^2
 //      moe_grouped_gemm<2>   hid[slot] = silu(W_gate[e] x) * (W_up[e] x)            (gated experts, gate / up rows interleaved)
 //      moe_grouped_gemm<3>   hid[slot] = g logistic(p1 g) (u + 1), g = min(W_gate[e] x, p0), u = clamp(W_up[e] x, -p0, p0)
-//   3. moe_grouped_gemm<1>   part[slot] = weight(pair) * W_down[e] hid[slot]     (fp32)
-//   4. moe_combine_kernel    y[t] = sum_k part[slot(t, k)] (+ logistic(g_t) * shared[t]), summed in the order of k
-// GEMM tiles: 64 rows x 64 outputs x 64 deep, 4 warps of 32 x 32, mma.sync m16n8k16 bf16 with fp32 accumulation, operands
-// through a two-stage cp.async ring.  Tensor-bound: 4 * pairs * ff * width flop per layer.
+//   4. moe_grouped_gemm<1>   part[slot] = weight(pair) * W_down[e] hid[slot]     (fp32)
+//   5. moe_combine_kernel    y[t] = sum_k part[slot(t, k)] (+ logistic(g_t) * shared[t]), summed in the order of k
+// GEMM: tcgen05, persistent CTAs.  The weights are the M axis (128 features, TMEM lane = feature) and the rows the N axis (TMEM column = row), so that
+// a tile costs MMAs for its own rows (to the next 16) and not for a full tile of 128; an expert of the usual 100-250 rows reads its weights once.
+//   warp 0 TMA (4 stages of 64 deep) | warp 1 MMA | warps 2-5 epilogue from the other of two accumulators.
+// Bound: HBM for few rows per expert (all weights are read once), the tensor pipe and the operand traffic out of L2 for many.  2048 tokens, 64 experts
+// of 2048 x 1408, top 6 (B200, whole call): 1028 us with 64 x 64 tiles of mma.sync, 377 us so.
+#include <cuda.h>
+
 #include "common.cuh"
 #include "mma.cuh"
+#include "tcgen05.cuh"
 
 namespace pk {
 
-constexpr int kGT = 64, kGK = 64, kGLd = kGK + 8, kGPieces = kGT * kGK / 8 / 128;  // 16-byte pieces per thread, operand and k tile
+constexpr int kMoeTile = 256;   // rows per tile at most (UMMA N)
+constexpr int kMoeSlack = 64;   // the workspace has room for a tile per so many pairs
 
 // meta layout (ints): [0] number of row tiles, [1 .. E+1] offsets (exclusive scan, E + 1 entries), then tile_expert[max_tiles],
-// tile_row0[max_tiles]; slot_pair[pairs] and pair_slot[pairs] are separate arrays.
-__global__ void moe_bucket_kernel(const int* __restrict__ ids, int pairs, int experts, int max_tiles, int* __restrict__ meta,
-                                  int* __restrict__ slot_pair, int* __restrict__ pair_slot) {
-  extern __shared__ int sh[];  // [experts] counts, then [experts] cursors
+// tile_row0[max_tiles] (one entry more than tiles: the end); slot_pair[pairs] and pair_slot[pairs] are separate arrays.
+constexpr int kBucketThreads = 1024, kBucketIds = 16;  // ids a thread keeps in registers
+__global__ void __launch_bounds__(kBucketThreads) moe_bucket_kernel(const int* __restrict__ ids, int pairs, int experts, int max_tiles,
+                                                                    int* __restrict__ meta, int* __restrict__ slot_pair, int* __restrict__ pair_slot) {
+  extern __shared__ int sh[];  // [experts] counts, then [experts] cursors, then [2 * 33] sums per warp
   pdl_wait();
   pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
   int* cnt = sh;
   int* cur = sh + experts;
-  for (int e = threadIdx.x; e < experts; e += blockDim.x) cnt[e] = 0;
+  int* wsum = sh + 2 * experts;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int e = tid; e < experts; e += kBucketThreads) cnt[e] = 0;
+  int mine[kBucketIds];  // all loads on their way before the first is used
+#pragma unroll
+  for (int i = 0; i < kBucketIds; ++i) mine[i] = tid + i * kBucketThreads < pairs ? ids[tid + i * kBucketThreads] : -1;
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) atomicAdd(&cnt[ids[p]], 1);
+#pragma unroll
+  for (int i = 0; i < kBucketIds; ++i)
+    if (mine[i] >= 0) atomicAdd(&cnt[mine[i]], 1);
+  for (int p = tid + kBucketIds * kBucketThreads; p < pairs; p += kBucketThreads) atomicAdd(&cnt[ids[p]], 1);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int* off = meta + 1;
-    int* te = meta + 2 + experts;
-    int* tr = te + max_tiles;
-    int run = 0, nt = 0;
-    for (int e = 0; e < experts; ++e) {
-      off[e] = run;
-      cur[e] = run;
-      for (int r = 0; r < cnt[e]; r += kGT) {
-        te[nt] = e;
-        tr[nt] = run + r;
-        ++nt;
+  // exclusive scans of the row and the tile counts over the experts, kBucketThreads experts at a time
+  int* off = meta + 1;
+  int* te = meta + 2 + experts;
+  int* tr = te + max_tiles;
+  int rows0 = 0, tiles0 = 0;
+  for (int e0 = 0; e0 < experts; e0 += kBucketThreads) {
+    const int e = e0 + tid, c = e < experts ? cnt[e] : 0, nt = (c + kMoeTile - 1) / kMoeTile;
+    int rc = c, rt = nt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, rc, o), b = __shfl_up_sync(0xffffffffu, rt, o);
+      if (lane >= o) {
+        rc += a;
+        rt += b;
       }
-      run += cnt[e];
     }
-    off[experts] = run;
-    meta[0] = nt;
+    if (lane == 31) {
+      wsum[warp] = rc;
+      wsum[33 + warp] = rt;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      int a = wsum[lane], b = wsum[33 + lane];
+      const int a0 = a, b0 = b;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, a, o), y = __shfl_up_sync(0xffffffffu, b, o);
+        if (lane >= o) {
+          a += x;
+          b += y;
+        }
+      }
+      wsum[lane] = a - a0;
+      wsum[33 + lane] = b - b0;
+      if (lane == 31) {
+        wsum[32] = a;
+        wsum[65] = b;
+      }
+    }
+    __syncthreads();
+    if (e < experts) {
+      const int row = rows0 + wsum[warp] + rc - c, tile = tiles0 + wsum[33 + warp] + rt - nt;
+      off[e] = row;
+      cur[e] = row;
+      const int size = nt ? ((c + nt - 1) / nt + 15) / 16 * 16 : 0;
+      for (int i = 0; i < nt; ++i) {
+        te[tile + i] = e;
+        tr[tile + i] = row + i * size;
+      }
+    }
+    rows0 += wsum[32];
+    tiles0 += wsum[65];
+    __syncthreads();
   }
-  __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
+  if (tid == 0) {
+    off[experts] = rows0;
+    tr[tiles0] = rows0;
+    meta[0] = tiles0;
+  }
+#pragma unroll
+  for (int i = 0; i < kBucketIds; ++i) {
+    if (mine[i] < 0) continue;
+    const int p = tid + i * kBucketThreads, s = atomicAdd(&cur[mine[i]], 1);
+    slot_pair[s] = p;
+    pair_slot[p] = s;
+  }
+  for (int p = tid + kBucketIds * kBucketThreads; p < pairs; p += kBucketThreads) {
     const int s = atomicAdd(&cur[ids[p]], 1);
     slot_pair[s] = p;
     pair_slot[p] = s;
   }
 }
 
+// xs[slot] = x[slot_pair[slot] / top], 16-byte pieces
+__global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict__ x, const int* __restrict__ slot_pair, bf16* __restrict__ xs, int width,
+                                                         int top) {
+  pdl_wait();
+  pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
+  const int s = blockIdx.x, nv = width >> 3;
+  const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(slot_pair[s] / top) * width);
+  uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)s * width);
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) dst[i] = src[i];
+}
+
+constexpr int kMgStages = 4, kMgThreads = 192, kMgChunk = 32;  // chunk: rows of an epilogue step
+constexpr int kMgA = 128 * 64 * 2, kMgBox = 64 * 64 * 2, kMgStage = kMgA + kMoeTile * 64 * 2;
+constexpr size_t kMgSmem = (size_t)kMgStages * kMgStage + 1024 + kMgChunk * 128 * 2 + (2 * kMgStages + 4) * 8 + 16;
+
+__device__ __forceinline__ void mg_tma_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
+      "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
+      : "memory");
+}
+
+struct MgArgs {
+  void* out;
+  const int* meta;
+  const int* slot_pair;
+  const float* weights;
+  int experts, max_tiles, N, K;  // N: weight rows per expert
+  float p0, p1;
+  unsigned int* err;
+};
+
 // EPI 0: out bf16 [slots][N] = relu(acc)^2.   EPI 1: out fp32 [slots][N] = acc * weights[pair of the slot].
 // EPI 2: W rows interleaved (2f = gate f, 2f + 1 = up f): out bf16 [slots][N / 2] = silu(acc[2f]) * acc[2f + 1].
 // EPI 3: the same rows with clamped pre-activations: g = min(acc[2f], p0), u = clamp(acc[2f + 1], -p0, p0), out = g logistic(p1 g) (u + 1).
-// A row of slot s: A + (gather_div ? slot_pair[s] / gather_div : s) * K.
 template <int EPI>
-__global__ void __launch_bounds__(128) moe_grouped_gemm_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, void* __restrict__ out,
-                                                              const int* __restrict__ meta, const int* __restrict__ slot_pair,
-                                                              const float* __restrict__ weights, int experts, int max_tiles, int N, int K,
-                                                              int gather_div, float p0, float p1) {
-  __shared__ __align__(16) bf16 As[2][kGT * kGLd];
-  __shared__ __align__(16) bf16 Bs[2][kGT * kGLd];
+__global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                                                                        const MgArgs a) {
+  extern __shared__ uint8_t mg_smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(mg_smem_raw) + 1023) & ~(uintptr_t)1023);
+  bf16* tile = reinterpret_cast<bf16*>(smem + (size_t)kMgStages * kMgStage);  // epilogue: [32 rows][64 or 128 outputs]
+  uint64_t* full = reinterpret_cast<uint64_t*>(tile + kMgChunk * 128);
+  uint64_t* empty = full + kMgStages;
+  uint64_t* tfull = empty + kMgStages;
+  uint64_t* tempty = tfull + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+  volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kMgStages; ++s) {
+      mbar_init(full + s, 1);
+      mbar_init(empty + s, 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(tfull + s, 1);
+      mbar_init(tempty + s, 4);
+    }
+    *dead = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();  // after the allocation: a dependent that came first would hold the TMEM while it waits for this grid
   pdl_wait();
-  pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
-  if ((int)blockIdx.y >= meta[0]) return;
-  const int* off = meta + 1;
-  const int e = meta[2 + experts + blockIdx.y], m0 = meta[2 + experts + max_tiles + blockIdx.y];
-  const int m_end = off[e + 1], n0 = blockIdx.x * kGT;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tq = lane & 3, wm = warp >> 1, wn = warp & 1;
-  const bf16* We = W + (size_t)e * N * K;
-  // each thread copies kGPieces 16-byte pieces of A and of B per k tile
-  const bf16* a_src[kGPieces];
-  const bf16* b_src[kGPieces];
-  int kc[kGPieces], sm_off[kGPieces];
-#pragma unroll
-  for (int i = 0; i < kGPieces; ++i) {
-    const int c = tid + i * 128, r = c / (kGK / 8);
-    kc[i] = (c % (kGK / 8)) * 8;
-    sm_off[i] = r * kGLd + kc[i];
-    const int s = m0 + r;
-    a_src[i] = s < m_end ? A + (size_t)(gather_div ? slot_pair[s] / gather_div : s) * K : nullptr;
-    b_src[i] = n0 + r < N ? We + (size_t)(n0 + r) * K : nullptr;
-  }
-  auto load = [&](int kt, int buf) {
-#pragma unroll
-    for (int i = 0; i < kGPieces; ++i) {
-      const int k = kt * kGK + kc[i];
-      if (a_src[i] && k < K) cp_async16(&As[buf][sm_off[i]], a_src[i] + k);
-      else *reinterpret_cast<uint4*>(&As[buf][sm_off[i]]) = make_uint4(0, 0, 0, 0);
-      if (b_src[i] && k < K) cp_async16(&Bs[buf][sm_off[i]], b_src[i] + k);
-      else *reinterpret_cast<uint4*>(&Bs[buf][sm_off[i]]) = make_uint4(0, 0, 0, 0);
-    }
-    cp_async_commit();
-  };
-  float acc[2][4][4] = {};
-  const int nk = (K + kGK - 1) / kGK;
-  load(0, 0);
-  for (int kt = 0; kt < nk; ++kt) {
-    const int buf = kt & 1;
-    cp_async_wait_all();
-    __syncthreads();
-    if (kt + 1 < nk) load(kt + 1, buf ^ 1);
-#pragma unroll
-    for (int kk = 0; kk < kGK; kk += 16) {
-      uint32_t a[2][4], b[2][4];
-#pragma unroll
-      for (int mi = 0; mi < 2; ++mi)
-        ldsm_x4(a[mi], &As[buf][(wm * 32 + mi * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * kGLd + kk + ((lane >> 4) & 1) * 8]);
-#pragma unroll
-      for (int np = 0; np < 2; ++np)
-        ldsm_x4(b[np], &Bs[buf][(wn * 32 + np * 16 + (lane & 7) + ((lane >> 4) & 1) * 8) * kGLd + kk + ((lane >> 3) & 1) * 8]);
-#pragma unroll
-      for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) mma_bf16_16816(acc[mi][ni], a[mi], b[ni >> 1][(ni & 1) * 2], b[ni >> 1][(ni & 1) * 2 + 1]);
-    }
-  }
-#pragma unroll
-  for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-    for (int hf = 0; hf < 2; ++hf) {
-      const int s = m0 + wm * 32 + mi * 16 + g + hf * 8;
-      if (s >= m_end) continue;
-      const float wgt = EPI == 1 ? weights[slot_pair[s]] : 1.f;
-#pragma unroll
-      for (int ni = 0; ni < 4; ++ni) {
-        const int n = n0 + wn * 32 + ni * 8 + 2 * tq;
-        float v0 = acc[mi][ni][hf * 2], v1 = acc[mi][ni][hf * 2 + 1];
-        if (EPI == 0) {
-          v0 = fmaxf(v0, 0.f);
-          v1 = fmaxf(v1, 0.f);
-          bf16* o = static_cast<bf16*>(out) + (size_t)s * N + n;
-          if (n + 1 < N) *reinterpret_cast<uint32_t*>(o) = pack_bf16(v0 * v0, v1 * v1);
-          else if (n < N) o[0] = f2bf(v0 * v0);
-        } else if (EPI == 2) {
-          if (n + 1 < N) static_cast<bf16*>(out)[(size_t)s * (N / 2) + n / 2] = f2bf(v0 / (1.f + expf(-v0)) * v1);
-        } else if (EPI == 3) {
-          v0 = fminf(v0, p0);
-          v1 = fminf(fmaxf(v1, -p0), p0);
-          if (n + 1 < N) static_cast<bf16*>(out)[(size_t)s * (N / 2) + n / 2] = f2bf(v0 / (1.f + expf(-p1 * v0)) * (v1 + 1.f));
-        } else {
-          float* o = static_cast<float*>(out) + (size_t)s * N + n;
-          if (n + 1 < N) *reinterpret_cast<float2*>(o) = make_float2(v0 * wgt, v1 * wgt);
-          else if (n < N) o[0] = v0 * wgt;
+  const int* te = a.meta + 2 + a.experts;
+  const int* tr = te + a.max_tiles;
+  const int n_ft = (a.N + 127) / 128, tiles = a.meta[0] * n_ft, k_blocks = (a.K + 63) / 64;
+  // neighbouring CTAs share an expert's rows
+  if (warp == 0) {
+    if (lane == 0) {
+      int s = 0;
+      uint32_t ph = 1;
+      for (int t = blockIdx.x; t < tiles && !*dead; t += gridDim.x) {
+        const int rt = t / n_ft, m0 = tr[rt], rows = tr[rt + 1] - m0, w0 = te[rt] * a.N + (t - rt * n_ft) * 128, boxes = (rows + 63) / 64;
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          if (!mbar_wait_bounded(empty + s, ph, dead)) break;
+          mbar_expect_tx(full + s, kMgA + boxes * kMgBox);
+          uint8_t* st = smem + (size_t)s * kMgStage;
+          mg_tma_2d(st, &map_w, kb * 64, w0, full + s);
+          for (int b = 0; b < boxes; ++b) mg_tma_2d(st + kMgA + b * kMgBox, &map_x, kb * 64, m0 + b * 64, full + s);
+          if (++s == kMgStages) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
       }
     }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int s = 0, lt = 0;
+      uint32_t ph = 0;
+      for (int t = blockIdx.x; t < tiles && !*dead; t += gridDim.x, ++lt) {
+        const int rt = t / n_ft, n16 = (tr[rt + 1] - tr[rt] + 15) / 16, as = lt & 1;
+        // instruction descriptor: D = f32 [4,6) = 1, A = bf16 [7,10) = 1, B = bf16 [10,13) = 1, both K-major, N >> 3 at [17,23), M >> 4 at [24,29)
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n16 * 2) << 17) | ((uint32_t)(128 >> 4) << 24);
+        if (!mbar_wait_bounded(tempty + as, (uint32_t)(((lt >> 1) & 1) ^ 1), dead)) break;
+        tc_fence_after();
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          if (!mbar_wait_bounded(full + s, ph, dead)) break;
+          tc_fence_after();
+          const uint32_t a_addr = smem_u32(smem + (size_t)s * kMgStage);
+          const uint64_t ad = make_sw128_desc(a_addr), bd = make_sw128_desc(a_addr + kMgA);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            umma_bf16(tmem_base + (uint32_t)(as * kMoeTile), ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          umma_commit(empty + s);
+          if (++s == kMgStages) {
+            s = 0;
+            ph ^= 1u;
+          }
+        }
+        umma_commit(tfull + as);
+      }
+    }
+  } else {
+    const int q = warp & 3, et = threadIdx.x & 127;  // TMEM lane quarter this warp may read; thread of the four epilogue warps (2, 3, 4, 5 -> 64 .. 191)
+    const int out_n = EPI >= 2 ? a.N / 2 : a.N;
+    int lt = 0;
+    for (int t = blockIdx.x; t < tiles && !*dead; t += gridDim.x, ++lt) {
+      const int rt = t / n_ft, m0 = tr[rt], rows = tr[rt + 1] - m0, f0 = (t - rt * n_ft) * 128, as = lt & 1;
+      mbar_wait_bounded(tfull + as, (uint32_t)((lt >> 1) & 1), dead);
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * kMoeTile);
+      for (int c = 0; c < rows; c += kMgChunk) {
+        uint32_t v[32];
+        tmem_ld32(t_row + (uint32_t)c, v);
+        const int n = min(kMgChunk, rows - c);
+        if (EPI == 1) {  // fp32: a row's 32 features of a warp are 128 contiguous bytes
+          const int f = f0 + q * 32 + lane;
+          const float wl = lane < n ? a.weights[a.slot_pair[m0 + c + lane]] : 0.f;
+          float* o = static_cast<float*>(a.out) + (size_t)(m0 + c) * a.N + f;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const float w = __shfl_sync(0xffffffffu, wl, j);
+            if (j < n && f < a.N) o[(size_t)j * a.N] = __uint_as_float(v[j]) * w;
+          }
+          continue;
+        }
+        // bf16: through shared memory, [row][output], so that a row leaves in 16-byte pieces
+        constexpr int OW = EPI >= 2 ? 64 : 128;
+        asm volatile("bar.sync 1, 128;" ::: "memory");  // the last chunk has left
+        if (EPI == 0) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const float z = fmaxf(__uint_as_float(v[j]), 0.f);
+            tile[j * OW + q * 32 + lane] = f2bf(z * z);
+          }
+        } else {
+          // gate in the even lane, up in the odd one: of two rows the even lane takes the first, the odd lane the second
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const float give = __uint_as_float(lane & 1 ? v[j] : v[j + 1]), keep = __uint_as_float(lane & 1 ? v[j + 1] : v[j]);
+            const float got = __shfl_xor_sync(0xffffffffu, give, 1);
+            float gt = lane & 1 ? got : keep, up = lane & 1 ? keep : got, y;
+            if (EPI == 2) {
+              y = gt / (1.f + expf(-gt)) * up;
+            } else {
+              gt = fminf(gt, a.p0);
+              up = fminf(fmaxf(up, -a.p0), a.p0);
+              y = gt / (1.f + expf(-a.p1 * gt)) * (up + 1.f);
+            }
+            tile[(j + (lane & 1)) * OW + q * 16 + (lane >> 1)] = f2bf(y);
+          }
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        const int o0 = EPI >= 2 ? f0 / 2 : f0;
+        for (int i = et; i < kMgChunk * OW / 8; i += 128) {
+          const int r = i / (OW / 8), p = (i % (OW / 8)) * 8;
+          if (r < n && o0 + p < out_n)
+            *reinterpret_cast<uint4*>(static_cast<bf16*>(a.out) + (size_t)(m0 + c + r) * out_n + o0 + p) = *reinterpret_cast<const uint4*>(tile + r * OW + p);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tempty + as);
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0 && *dead && a.err) atomicAdd(a.err, 1u);
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
 }
 
-__global__ void moe_combine_kernel(const float* __restrict__ part, const int* __restrict__ pair_slot, const bf16* __restrict__ shared,
-                                   const float* __restrict__ sg, float* __restrict__ y, int width, int top) {
+// y[t] = sum over k of part[slot(t, k)], in the order of k; float4 pieces (width is a multiple of 8)
+__global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ part, const int* __restrict__ pair_slot, const bf16* __restrict__ shared,
+                                                          const float* __restrict__ sg, float* __restrict__ y, int width, int top) {
   pdl_wait();
   pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
-  const int t = blockIdx.x;
+  const int t = blockIdx.x, nv = width >> 2;
   const float g = shared ? (sg ? 1.f / (1.f + expf(-sg[t])) : 1.f) : 0.f;
-  for (int i = threadIdx.x; i < width; i += blockDim.x) {
-    float acc = 0.f;
-    for (int k = 0; k < top; ++k) acc += part[(size_t)pair_slot[(size_t)t * top + k] * width + i];
-    y[(size_t)t * width + i] = acc + (shared ? g * bf2f(shared[(size_t)t * width + i]) : 0.f);
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) {
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int k = 0; k < top; ++k) {
+      const float4 p = reinterpret_cast<const float4*>(part + (size_t)pair_slot[(size_t)t * top + k] * width)[i];
+      acc.x += p.x;
+      acc.y += p.y;
+      acc.z += p.z;
+      acc.w += p.w;
+    }
+    if (shared) {
+      const bf16* s = shared + (size_t)t * width + i * 4;
+      acc.x += g * bf2f(s[0]);
+      acc.y += g * bf2f(s[1]);
+      acc.z += g * bf2f(s[2]);
+      acc.w += g * bf2f(s[3]);
+    }
+    float* o = y + (size_t)t * width + i * 4;
+    if ((reinterpret_cast<uintptr_t>(y) & 15) == 0) {
+      *reinterpret_cast<float4*>(o) = acc;
+    } else {
+      o[0] = acc.x;
+      o[1] = acc.y;
+      o[2] = acc.z;
+      o[3] = acc.w;
+    }
   }
+}
+
+static bool mg_map(CUtensorMap* map, const void* base, long rows, int K, int box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+  cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int EPI>
+static cudaError_t mg_launch(const void* rows, long n_rows, const void* w, const MgArgs& a, cudaStream_t st) {
+  CUtensorMap mx, mw;
+  if (!mg_map(&mx, rows, n_rows, a.K, 64) || !mg_map(&mw, w, (long)a.experts * a.N, a.K, 128)) return cudaErrorInvalidValue;
+  auto kern = moe_grouped_gemm_kernel<EPI>;
+  static thread_local bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMgSmem);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  // as many CTAs as there can be tiles, one per SM at most
+  const long tiles = (n_rows / kMoeTile + (n_rows < a.experts ? n_rows : a.experts)) * ((a.N + 127) / 128);
+  return launch(kern, dim3((unsigned)(tiles < sm_count() ? tiles : sm_count())), dim3(kMgThreads), kMgSmem, st, true, mx, mw, a);
 }
 
 }  // namespace pk
@@ -173,11 +380,11 @@ __global__ void moe_combine_kernel(const float* __restrict__ part, const int* __
 using namespace pk;
 
 extern "C" long pk_moe_grouped_workspace_bytes(int tokens, int top, int experts, int width, int ff) {
-  const long pairs = (long)tokens * top, max_tiles = pairs / kGT + experts + 1;
+  const long pairs = (long)tokens * top, max_tiles = pairs / kMoeSlack + experts + 1;
   long b = (2 + experts + 2 * max_tiles + 2 * pairs) * 4;  // meta, slot_pair, pair_slot
   b = (b + 255) / 256 * 256;
   b += (pairs * ff * 2 + 255) / 256 * 256;  // hid
-  b += pairs * width * 4;                   // part
+  b += pairs * width * 4;                   // part; before that, the gathered rows
   return b + 256;
 }
 
@@ -200,7 +407,7 @@ extern "C" int pk_moe_grouped_act_p(const void* xa, const void* w_up, const void
       (reinterpret_cast<uintptr_t>(w_down) & 15) || (reinterpret_cast<uintptr_t>(workspace) & 255))
     return -2;
   const long pairs = (long)tokens * top;
-  const int max_tiles = (int)(pairs / kGT) + experts + 1;
+  const int max_tiles = (int)(pairs / kMoeSlack) + experts + 1;
   char* ws = static_cast<char*>(workspace);
   int* meta = reinterpret_cast<int*>(ws);
   int* slot_pair = meta + 2 + experts + 2 * max_tiles;
@@ -209,19 +416,17 @@ extern "C" int pk_moe_grouped_act_p(const void* xa, const void* w_up, const void
   bf16* hid = reinterpret_cast<bf16*>(ws + o);
   o += (pairs * ff * 2 + 255) / 256 * 256;
   float* part = reinterpret_cast<float*>(ws + o);
-  launch(moe_bucket_kernel, dim3(1), dim3(1024), (size_t)2 * experts * sizeof(int), st, true, ids, (int)pairs, experts, max_tiles, meta, slot_pair,
-         pair_slot);
-  if (act == 2)
-    launch(moe_grouped_gemm_kernel<3>, dim3((2 * ff + kGT - 1) / kGT, max_tiles), dim3(128), 0, st, true, (const bf16*)xa, (const bf16*)w_up, (void*)hid,
-           (const int*)meta, (const int*)slot_pair, weights, experts, max_tiles, 2 * ff, width, top, p0, p1);
-  else if (act == 1)
-    launch(moe_grouped_gemm_kernel<2>, dim3((2 * ff + kGT - 1) / kGT, max_tiles), dim3(128), 0, st, true, (const bf16*)xa, (const bf16*)w_up, (void*)hid,
-           (const int*)meta, (const int*)slot_pair, weights, experts, max_tiles, 2 * ff, width, top, 0.f, 0.f);
-  else
-    launch(moe_grouped_gemm_kernel<0>, dim3((ff + kGT - 1) / kGT, max_tiles), dim3(128), 0, st, true, (const bf16*)xa, (const bf16*)w_up, (void*)hid,
-           (const int*)meta, (const int*)slot_pair, weights, experts, max_tiles, ff, width, top, 0.f, 0.f);
-  launch(moe_grouped_gemm_kernel<1>, dim3((width + kGT - 1) / kGT, max_tiles), dim3(128), 0, st, true, (const bf16*)hid, (const bf16*)w_down,
-         (void*)part, (const int*)meta, (const int*)slot_pair, weights, experts, max_tiles, width, ff, 0, 0.f, 0.f);
+  bf16* xs = reinterpret_cast<bf16*>(part);  // done with when `part` is written
+  launch(moe_bucket_kernel, dim3(1), dim3(kBucketThreads), (size_t)(2 * experts + 66) * sizeof(int), st, true, ids, (int)pairs, experts, max_tiles, meta,
+         slot_pair, pair_slot);
+  launch(moe_gather_kernel, dim3((unsigned)pairs), dim3(width >= 2048 ? 256 : 128), 0, st, true, (const bf16*)xa, (const int*)slot_pair, xs, width, top);
+  MgArgs a{hid, meta, slot_pair, weights, experts, max_tiles, act ? 2 * ff : ff, width, p0, p1, tls().wait_err};
+  cudaError_t e = act == 2 ? mg_launch<3>(xs, pairs, w_up, a, st) : act == 1 ? mg_launch<2>(xs, pairs, w_up, a, st) : mg_launch<0>(xs, pairs, w_up, a, st);
+  if (e != cudaSuccess) return (int)e;
+  a.out = part;
+  a.N = width;
+  a.K = ff;
+  if ((e = mg_launch<1>(hid, pairs, w_down, a, st)) != cudaSuccess) return (int)e;
   launch(moe_combine_kernel, dim3(tokens), dim3(256), 0, st, true, (const float*)part, (const int*)pair_slot, (const bf16*)shared, shared_gate, y, width,
          top);
   return (int)cudaGetLastError();
