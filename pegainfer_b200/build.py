@@ -43,16 +43,16 @@ def _run(cmd: list[str]) -> None:
 # What one design needs when nothing is built yet (a fresh checkout asked to serve that design compiles these files and no
 # others): kernel sources, host sources.  A later full build adds the rest and links both libraries again.
 PARTS_OF = {
-    "Vamadra": (("runtime.cu", "gemm.cu", "gemm2.cu", "gemm_skinny.cu", "gemv.cu", "sampling.cu", "residual32_ops.cu", "gemm_batched_mma.cu", "latent_attention.cu", "latent_attention_mma.cu", "moe.cu", "moe_grouped.cu"),
+    "Vamadra": (("runtime.cu", "gemm.cu", "gemm2.cu", "gemm_skinny.cu", "gemv.cu", "sampling.cu", "residual32_ops.cu", "gemm_batched_mma.cu", "latent_attention.cu", "latent_attention_mma.cu", "latent_attention_tc.cu", "moe.cu", "moe_grouped.cu"),
                 ("qwen3_host.cpp", "layered_host.cpp")),
     "Risolorn": (("runtime.cu", "gemm.cu", "gemm2.cu", "gemm_skinny.cu", "gemv.cu", "sampling.cu", "residual32_ops.cu", "gemm_batched_mma.cu", "gqa_attention.cu", "recurrent_mixers.cu", "moe.cu", "moe_grouped.cu"),
                  ("qwen3_host.cpp", "layered_host.cpp")),
-    "Nagosun": (("runtime.cu", "gemm.cu", "gemm2.cu", "gemm_skinny.cu", "gemv.cu", "sampling.cu", "residual32_ops.cu", "gemm_batched_mma.cu", "gqa_attention.cu", "latent_attention.cu", "latent_attention_mma.cu"),
+    "Nagosun": (("runtime.cu", "gemm.cu", "gemm2.cu", "gemm_skinny.cu", "gemv.cu", "sampling.cu", "residual32_ops.cu", "gemm_batched_mma.cu", "gqa_attention.cu", "latent_attention.cu", "latent_attention_mma.cu", "latent_attention_tc.cu"),
                 ("qwen3_host.cpp", "layered_host.cpp")),
 }
 PARTS_OF["Rilonex"] = (("runtime.cu", "gemm.cu", "gemm2.cu", "gemm_skinny.cu", "gemv.cu", "sampling.cu", "residual32_ops.cu", "gemm_batched_mma.cu", "gqa_attention.cu", "gqa_mixed_attention.cu", "recurrent_mixers.cu"),
                        ("qwen3_host.cpp", "layered_host.cpp"))
-PARTS_OF["Vegodra"] = (("runtime.cu", "gemm.cu", "gemm2.cu", "gemm_skinny.cu", "gemv.cu", "sampling.cu", "residual32_ops.cu", "gemm_batched_mma.cu", "gqa_attention.cu", "latent_attention.cu", "latent_attention_mma.cu", "recurrent_mixers.cu"),
+PARTS_OF["Vegodra"] = (("runtime.cu", "gemm.cu", "gemm2.cu", "gemm_skinny.cu", "gemv.cu", "sampling.cu", "residual32_ops.cu", "gemm_batched_mma.cu", "gqa_attention.cu", "latent_attention.cu", "latent_attention_mma.cu", "latent_attention_tc.cu", "recurrent_mixers.cu"),
                        ("qwen3_host.cpp", "layered_host.cpp"))
 PARTS_OF["Goguzen"] = PARTS_OF["Risolorn"]  # the same files: attention, recurrent mixers, experts on the fp32 residual stream
 MANIFEST = os.path.join(OBJ, "linked.txt")

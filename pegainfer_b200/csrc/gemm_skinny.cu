@@ -121,7 +121,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (tc_elect_one()) {
       // instruction descriptor: D = f32 [4,6) = 1, A = bf16 [7,10) = 1, B = bf16 [10,13) = 1, both K-major, N >> 3 at [17,23), M >> 4 at [24,29)
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(SK_BM >> 4) << 24);
       int s = 0;

@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (tc_elect_one()) {
       int s = 0, lt = 0;
       uint32_t ph = 0;
       for (int t = blockIdx.x; t < tiles && !*dead; t += gridDim.x, ++lt) {

@@ -1,0 +1,67 @@
+"""The latent attention of prompt portions on tcgen05 (csrc/latent_attention_tc.cu): tiles that several requests share, windows, contexts carried over,
+page sizes on both sides of a key block, feature counts off its 64-wide chunks, and caches whose unused slots hold NaN."""
+import pytest
+import torch
+
+from pegainfer_b200 import ffi
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def lib():
+    l = ffi.lib()
+    l.cuda_set_device(0)
+    l.cublas_init()
+    return l
+
+
+@pytest.mark.parametrize("rank,rot", [(512, 64), (256, 32), (64, 8), (320, 0)])
+@pytest.mark.parametrize("starts,lens,H,window,ps,sink", [
+    ([0], [700], 16, 0, 16, False), ([0, 130, 5], [300, 333, 67], 16, 0, 16, True), ([500, 0], [400, 301], 16, 150, 8, True),
+    ([40], [1300], 8, 64, 32, False), ([0] * 40, [17 + i for i in range(40)], 10, 0, 128, True), ([3, 900], [640, 1], 16, 1000, 64, False)])
+def test_against_64_bits(lib, starts, lens, H, window, ps, sink, rank, rot):
+    D, T = rank + rot, sum(lens)
+    g = torch.Generator(device="cuda").manual_seed(T + rank)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    need = [(s + n + ps - 1) // ps for s, n in zip(starts, lens)]
+    order = torch.randperm(sum(need) + 3, generator=g, device="cuda").tolist()
+    stride = ps * D + 24
+    cache = torch.full((sum(need) + 3, stride), float("nan"), device="cuda").bfloat16()
+    off, k = [], 0
+    ctx = []
+    for s, n, m in zip(starts, lens, need):
+        rows = rn(s + n, D).bfloat16()
+        rows[:, 0] += 1.0
+        ctx.append(rows)
+        for p in range(m):
+            part = rows[p * ps:(p + 1) * ps]
+            cache[order[k + p], :len(part) * D] = part.reshape(-1)
+        off.append(k)
+        k += m
+    qa, sk = (1.5 * rn(T, H, D)).bfloat16(), rn(H).bfloat16()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    pos = i32([s + j for s, n in zip(starts, lens) for j in range(n)])
+    req = i32([r for r, n in enumerate(lens) for _ in range(n)])
+    out = torch.full((T + 1, H, rank), 9.0, device="cuda").bfloat16()
+    off_d, pages_d, scale = i32(off), i32(order), 1.3 * D ** -0.5
+    assert lib.pk_latent_attention_ex(qa.data_ptr(), cache.data_ptr(), sk.data_ptr() if sink else None, pos.data_ptr(), req.data_ptr(), off_d.data_ptr(),
+                                      pages_d.data_ptr(), out.data_ptr(), stride, ps, T, H, rank, rot, scale, window,
+                                      max(s + n for s, n in zip(starts, lens)), 0, None) == 0
+    torch.cuda.synchronize()
+    assert (out[T] == 9.0).all() and lib.pk_b200_wait_errors() == 0
+    row = 0
+    for s, n, keys in zip(starts, lens, ctx):
+        kd = keys.double()
+        at, j = torch.arange(s, s + n, device="cuda")[:, None], torch.arange(s + n, device="cuda")[None]
+        hidden = (j > at) | ((j <= at - window) if window else (j < 0))
+        for h in range(H):
+            sc = (qa[row:row + n, h].double() @ kd.T * scale).masked_fill(hidden, -float("inf"))
+            if sink:
+                sc = torch.cat([sc, sk[h].double().expand(n, 1)], 1)
+            p = torch.softmax(sc, -1)[:, :s + n]
+            want, got = p @ kd[:, :rank], out[row:row + n, h].double()
+            # weights and result are rounded to bf16 once each; a row's weights are positive, so the first rounding stays below 2^-8 of |v| weighed
+            bound = 2 ** -8 * (p @ kd[:, :rank].abs()) + 2 ** -8 * want.abs() + 1e-4
+            assert ((got - want).abs() <= bound).all(), (h, (got - want).abs().max().item())
+        row += n
