@@ -99,8 +99,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // not before this CTA holds its TMEM: a dependent that came first would hold it while it waits for this grid
-  pdl_launch_dependents();
+  // no early trigger: gemv.cu streams its weights before it waits for its predecessor, and they may be this kernel's output
   pdl_wait();
 
   if (warp == 0) {

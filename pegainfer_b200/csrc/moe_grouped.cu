@@ -186,8 +186,8 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_launch_dependents();  // after the allocation: a dependent that came first would hold the TMEM while it waits for this grid
   pdl_wait();
+  pdl_launch_dependents();  // after the allocation: a dependent that came first would hold the TMEM while it waits for this grid
   const int* te = a.meta + 2 + a.experts;
   const int* tr = te + a.max_tiles;
   const int n_ft = (a.N + 127) / 128, tiles = a.meta[0] * n_ft, k_blocks = (a.K + 63) / 64;

@@ -57,3 +57,27 @@ def test_three_outputs(lib, segs, N):
     assert rc == 0
     torch.cuda.synchronize()
     check(torch.cat([o for o, s in zip(outs, segs) if s], 1), W, X)
+
+
+@pytest.mark.parametrize("N,M,K", [(64, 4096, 2560), (128, 2560, 512), (200, 1024, 4096)])
+def test_product_as_the_weights_of_a_gemv(lib, N, M, K):
+    """The kernel for one row streams its weights before it waits for its predecessor: a product that is used as weights has to be complete by then."""
+    g = torch.Generator(device="cuda").manual_seed(N)
+    W = [torch.randn(M, K, generator=g, device="cuda").mul_(0.1).bfloat16() for _ in range(4)]
+    X = torch.randn(N, K, generator=g, device="cuda").bfloat16()
+    v = torch.randn(M, generator=g, device="cuda").bfloat16()
+    Y, out = torch.zeros(N, M, device="cuda").bfloat16(), torch.zeros(len(W), N, device="cuda").bfloat16()
+    st = torch.cuda.current_stream().cuda_stream
+    lib.pk_b200_set_pdl(1)
+    try:
+        for i, w in enumerate(W):
+            lib.gemm_cuda(w.data_ptr(), X.data_ptr(), Y.data_ptr(), M, N, K, st)
+            lib.gemm_cuda(Y.data_ptr(), v.data_ptr(), out[i].data_ptr(), N, 1, M, st)
+    finally:
+        lib.pk_b200_set_pdl(0)
+    torch.cuda.synchronize()
+    check(Y, W[-1], X)
+    for i, w in enumerate(W):  # the products of this run, rounded once
+        lib.gemm_cuda(w.data_ptr(), X.data_ptr(), Y.data_ptr(), M, N, K, st)
+        torch.cuda.synchronize()
+        check(out[i:i + 1], Y, v[None])
