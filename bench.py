@@ -720,7 +720,7 @@ def config4_leg(device):
         return {"workload": "Qwen3.5-4B hybrid bf16 random-init, 1024-token prompt + 128 greedy decode steps, bs 1, CUDA Graph on",
                 "ttft_ms": ttft, "tpot_ms": tpot, "decode_tok_s": 1000.0 / tpot, "launches_per_step": launches,
                 "step_hbm_frac": (wbytes + state_bytes) / (tpot * 1e-3) / 1e9 / peak, "bytes_per_token": wbytes + state_bytes,
-                "prefill": "tensor-core GEMMs + conv1d + delta-rule SEQUENCE kernel (recurrent, not chunk-wise) + HD-256 paged FA kernel",
+                "prefill": "tensor-core GEMMs + conv1d + delta rule in chunks of 16 tokens + HD-256 paged FA kernel",
                 "model_load_s": round(load_s, 1)}
     except Exception as e:
         return {"available": False, "why": f"{type(e).__name__}: {e}"[:300]}

@@ -197,7 +197,7 @@ int pk_b200_gemm_segments(const pk_bf16* W, const pk_bf16* X, pk_bf16* const* Y,
 int pk_b200_gemm_swiglu(const pk_bf16* W, const pk_bf16* X, pk_bf16* Y, int M, int N, int K, pk_stream stream);
 /* Which prefill GEMM kernel a [M features] x [N tokens] x [K] problem gets on a GPU with `sms` SMs (the choice gemm_cuda /
  * pk_b200_gemm_segments / pk_b200_gemm_swiglu make internally): 256 / 320 / 128 = tile width of the CTA-pair tcgen05 kernel
- * (gemm2.cu), -2 = the single-CTA kernel (gemm.cu, split-K when skinny).  Pure host arithmetic, no CUDA call: the wave-count
+ * (gemm2.cu), -2 = another one (gemm_skinny.cu, gemm.cu).  Shapes of few output tiles beyond 128 tokens go to gemm_skinny.cu whatever this says.  Pure host arithmetic, no CUDA call: the wave-count
  * cost model calibrated on B200 measurements (profiles/README.md round 2) is pinned by a CPU test. */
 int pk_b200_gemm_plan(int M, int N, int K, int swiglu, int sms);
 
@@ -315,9 +315,9 @@ int pk_b200_decode_attention_fused_prefetch(
 int pk_b200_gemv_grid(int M, int epi);
 
 /* ---- Qwen3.5 hybrid-layer ops (next scope row; ffi.rs:181-226,981-1039) --------
- * Memory-bound pieces of the gated-delta-net / gated HD-256 attention layers behind the reference's names
- * (csrc/{flashinfer_norm,norm,conv1d,gated_delta_rule,prefill_attention_hd256}.cu).  HD-256 attention and the
- * chunk-wise prefill of the delta rule are not provided yet.  Arithmetic: oracle/qwen35_oracle.py. */
+ * Pieces of the gated-delta-net / gated HD-256 attention layers behind the reference's names
+ * (csrc/{flashinfer_norm,norm,conv1d,gated_delta_rule,prefill_attention_hd256}.cu).
+ * Arithmetic: oracle/qwen35_oracle.py. */
 void rms_norm_batched_offset_cuda(const pk_bf16* x, const pk_bf16* weight, pk_bf16* out, int hidden_dim,
                                   int seq_len, float eps, pk_stream stream); /* out = x*rsqrt(mean+eps)*(1+w) */
 void rms_norm_offset_cuda(const pk_bf16* x, const pk_bf16* weight, pk_bf16* out, int n, float eps,
@@ -329,7 +329,7 @@ void gated_delta_rule_decode_cuda(const pk_bf16* qkv, const pk_bf16* b_proj, con
                                   pk_bf16* output, int num_key_heads, int num_value_heads, int key_dim,
                                   int val_dim, pk_stream stream); /* key_dim == val_dim == 128 */
 /* B200 extension: the same recurrence over a whole sequence (qkv_seq [T, 2*nk*128 + nv*128], b_seq / a_seq [T, nv],
- * out_seq [T, nv*128]) with the state held in registers -- correctness-first prefill until the chunk-wise kernel exists. */
+ * out_seq [T, nv*128]) in chunks of 16 tokens, state held in registers. */
 int pk_b200_gated_delta_rule_prefill_recurrent(const pk_bf16* qkv_seq, const pk_bf16* b_seq, const pk_bf16* a_seq,
                                                const pk_bf16* dt_bias, const float* A_log, float* state,
                                                pk_bf16* out_seq, int num_key_heads, int num_value_heads,

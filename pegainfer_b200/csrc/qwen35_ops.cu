@@ -1,11 +1,8 @@
-// Qwen3.5 hybrid-layer ops behind the reference's ABI names (the next scope row).
-// Covered here: the memory-bound pieces -- (1+w) RMSNorm, gated per-head RMSNorm, causal depthwise conv1d + SiLU, the
-// recurrent gated-delta-rule decode step, the HD-256 QK-norm + partial-RoPE preparation (prefill and batched decode)
-// and the sigmoid output gate.  NOT yet here: HD-256 attention and the chunk-wise prefill of the delta rule
-// (oracle/qwen35_chunkwise.py is its specification).  Arithmetic and rounding points follow the reference kernels
-// cited per function; oracle/qwen35_oracle.py restates them and is pinned to HF.
-// STATUS: compiled for sm_100a and exported; the GPU parity tests (tests/test_qwen35_ops_gpu.py) are opt-in
-// (PK_TEST_QWEN35=1) until they have run on hardware.
+// Qwen3.5 hybrid-layer ops behind the reference's ABI names.
+// Covered here: (1+w) RMSNorm, gated per-head RMSNorm, causal depthwise conv1d + SiLU, the gated-delta-rule decode step
+// and its prefill in chunks (delta_chunk.cuh), the HD-256 QK-norm + partial-RoPE preparation (prefill and batched
+// decode) and the sigmoid output gate.  Arithmetic and rounding points follow the reference kernels cited per function;
+// oracle/qwen35_oracle.py restates them and is pinned to HF.
 #include <algorithm>
 
 #include "common.cuh"
@@ -237,7 +234,6 @@ gated_delta_rule_seq_kernel(const bf16* __restrict__ qkv_seq, const bf16* __rest
                             bf16* __restrict__ out_seq, int nk, int nv, int T, unsigned int* err) {
   extern __shared__ __align__(16) float gdr_sm[];
   pdl_wait();
-  pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
   const int vh = blockIdx.x, col0 = blockIdx.y * GC, kh = vh * nk / nv, ld = 2 * nk * GK + nv * GV;
   const DeltaRows rows{qkv_seq + (size_t)kh * GK, qkv_seq + (size_t)(nk + kh) * GK, qkv_seq + (size_t)2 * nk * GK + (size_t)vh * GV + col0, ld, T,
                        (reinterpret_cast<uintptr_t>(qkv_seq) & 15) == 0, state + (size_t)vh * GK * GV, GV, col0, 1e-12f, rsqrtf((float)GK), err};
