@@ -121,7 +121,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   pdl_wait();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc_elect_one()) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
       int it = 0;
@@ -138,34 +138,29 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    // instruction descriptor: D=f32 [4,6)=1, A=bf16 [7,10)=1, B=bf16 [10,13)=1, K-major both,
-    // N>>3 at [17,23), M>>4 at [24,29)
-    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                               ((uint32_t)(BM >> 4) << 24);
-    int it = 0, lt = 0;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++lt) {
-      const int as = lt & 1;
-      mbar_wait(tempty + as, (uint32_t)(((lt >> 1) & 1) ^ 1));
-      tc_fence_after();
-      const uint32_t d_tmem = tmem_base + (uint32_t)(as * BN);
-      for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-        const int s = it % STAGES;
-        mbar_wait(full + s, (uint32_t)((it / STAGES) & 1));
+    // by elect.sync, not by `lane == 0`: the descriptors are uniform registers, which a thread picked by its lane fills through a vote per instruction
+    if (tc_elect_one()) {
+      // instruction descriptor: D=f32 [4,6)=1, A=bf16 [7,10)=1, B=bf16 [10,13)=1, K-major both, N>>3 at [17,23), M>>4 at [24,29)
+      constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+      int it = 0, lt = 0;
+      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++lt) {
+        const int as = lt & 1;
+        mbar_wait(tempty + as, (uint32_t)(((lt >> 1) & 1) ^ 1));
         tc_fence_after();
-        if (lane == 0) {
+        const uint32_t d_tmem = tmem_base + (uint32_t)(as * BN);
+        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+          const int s = it % STAGES;
+          mbar_wait(full + s, (uint32_t)((it / STAGES) & 1));
+          tc_fence_after();
           const uint32_t a_addr = smem_u32(smem + (size_t)s * STAGE_BYTES);
           const uint64_t adesc = make_sw128_desc(a_addr);
           const uint64_t bdesc = make_sw128_desc(a_addr + A_BYTES);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            // advance the start address by k*32 bytes inside the 128-byte swizzle span
-            umma_bf16(d_tmem, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc,
-                      (kb > 0 || k > 0) ? 1u : 0u);
-          }
-          umma_commit(empty + s);                       // smem stage free once these MMAs retire
-          if (kb == k_blocks - 1) umma_commit(tfull + as);  // accumulator ready for the epilogue
+          for (int k = 0; k < BK / UMMA_K; ++k)  // advance the start address by k * 32 bytes inside the 128-byte swizzle span
+            umma_bf16(d_tmem, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          umma_commit(empty + s);  // smem stage free once these MMAs retire
         }
-        __syncwarp();
+        umma_commit(tfull + as);  // accumulator ready for the epilogue
       }
     }
   } else {

@@ -13,12 +13,17 @@
 //           (cp.async.bulk.tensor ... .cta_group::2); the leader arms it with the bytes of both CTAs
 //   warp 1  MMA issuer (leader only): tcgen05.mma.cta_group::2 M256 x BN x K16, tcgen05.commit ... multicast::cluster
 //           frees the stage in BOTH CTAs / publishes the accumulator to BOTH epilogues
-//   warps 2-5 epilogue (both CTAs): tcgen05.ld 32x32b.x32 -> bf16 -> 64-byte row stores; tmem-empty arrives on the
+//   warps 2-9 epilogue (both CTAs): tcgen05.ld 32x32b.x32 -> bf16 -> 64-byte row stores; tmem-empty arrives on the
 //           leader's barrier (remote mbarrier arrive for the peer)
 // SwiGLU mode (gate_up projection): the pair's B halves are the SAME 128 features of the gate block (leader CTA) and
 // of the up block (peer CTA) of the stacked [gate; up] weight, so columns [0,128) / [128,256) of every accumulator row
 // are gate / up of one feature: the epilogue writes bf16(silu(bf16(g)) * bf16(u)) (csrc/fused_proj.cu:44-63 rounding)
 // and the separate SiLU-mul pass over 2*I*T elements disappears.
+// The MMA issuer and the producer are threads chosen by elect.sync: picked by `lane == 0` they filled the descriptors' uniform registers through a vote
+// per instruction, and a K block took 0.42 us whatever the tile's width.  B200, us a launch over cold weights, before -> after (2048 tokens):
+// 6144 x 2560 59.5 -> 48.4, 2560 x 4096 45.6 -> 37.5, 2560 x 9728 88.8 -> 74.3, 4096 x 12288 160.6 -> 144.1.
+// The gated epilogue evaluates its 32 columns side by side, on two warps per lane quarter; one after the other (a branch on the activation per
+// element) a tile's epilogue took 26 us and set the pace: 9728 x 2560 gated 253 -> 154, 12288 x 4096 gated (3001 tokens) 557 -> 433.
 // Every barrier wait is bounded (trap instead of hang).
 #include <cuda.h>
 
@@ -34,7 +39,8 @@ namespace {
 
 constexpr int G2_BM = 128;       // tokens per CTA (UMMA M = 256 per pair)
 constexpr int G2_BK = 64;        // K elements per stage (one 128-byte swizzle span)
-constexpr int G2_THREADS = 192;  // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
+constexpr int G2_EPI = 8;        // epilogue warps: two for each quarter of the TMEM lanes, taking turns at blocks of 32 columns
+constexpr int G2_THREADS = 64 + 32 * G2_EPI;  // warp 0 TMA, warp 1 MMA, then the epilogue
 
 __device__ __forceinline__ uint32_t g2_rank() {
   uint32_t r;
@@ -113,7 +119,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)STAGES * STAGE_BYTES);  // used in the leader
   uint64_t* empty = full + STAGES;   // one per CTA (multicast commit)
   uint64_t* tfull = empty + STAGES;  // [2] one per CTA
-  uint64_t* tempty = tfull + 2;      // [2] used in the leader (8 arrivals: 4 epilogue warps x 2 CTAs)
+  uint64_t* tempty = tfull + 2;      // [2] used in the leader (an arrival per epilogue warp of both CTAs)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -133,7 +139,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(tfull + s, 1);
-      mbar_init(tempty + s, 8);
+      mbar_init(tempty + s, 2 * G2_EPI);
     }
     mbar_fence_init();
   }
@@ -146,7 +152,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
   pdl_wait();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc_elect_one()) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
       int it = 0;
@@ -168,7 +174,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    if (leader) {
+    // by elect.sync, not by `lane == 0`: the descriptors are uniform registers, which a thread picked by its lane fills through a vote per instruction
+    if (leader && tc_elect_one()) {
       // instruction descriptor: D=f32 [4,6)=1, A=bf16 [7,10)=1, B=bf16 [10,13)=1, K-major both, N>>3 at [17,23), M>>4 at [24,29)
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
       int it = 0, lt = 0;
@@ -181,24 +188,21 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
           const int s = it % STAGES;
           g2_wait(full + s, (uint32_t)((it / STAGES) & 1));
           tc_fence_after();
-          if (lane == 0) {
-            const uint32_t a_addr = smem_u32(smem + (size_t)s * STAGE_BYTES);
-            const uint64_t adesc = make_sw128_desc(a_addr);
+          const uint32_t a_addr = smem_u32(smem + (size_t)s * STAGE_BYTES);
+          const uint64_t adesc = make_sw128_desc(a_addr);
 #pragma unroll
-            for (int k = 0; k < G2_BK / 16; ++k)
+          for (int k = 0; k < G2_BK / 16; ++k)
 #pragma unroll
-              for (int j = 0; j < NSUB; ++j)
-                g2_umma(d_tmem + (uint32_t)(j * BN), adesc + (uint64_t)(k * 2),
-                        make_sw128_desc(a_addr + A_BYTES + j * B_SUB) + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-            g2_commit_both(empty + s);
-            if (kb == k_blocks - 1) g2_commit_both(tfull + as);
-          }
-          __syncwarp();
+            for (int j = 0; j < NSUB; ++j)
+              g2_umma(d_tmem + (uint32_t)(j * BN), adesc + (uint64_t)(k * 2),
+                      make_sw128_desc(a_addr + A_BYTES + j * B_SUB) + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          g2_commit_both(empty + s);
         }
+        g2_commit_both(tfull + as);
       }
     }
   } else {
-    const int q = warp & 3;  // TMEM lane quarter this warp may access
+    const int q = warp & 3, c0 = (warp - 2) / 4 * 32;  // TMEM lane quarter this warp may access, its first column
     const bool vec_ok = (a.e0 % 32 == 0) && (a.e1 % 32 == 0) && (M % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.Y) & 15) == 0) &&
                         ((reinterpret_cast<uintptr_t>(a.Y1) & 15) == 0) && ((reinterpret_cast<uintptr_t>(a.Y2) & 15) == 0);
     const uint32_t tempty_leader0 = g2_map(smem_u32(tempty), 0);
@@ -213,19 +217,31 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
       if (a.swiglu) {
         // columns [0, HB) = gate, [HB, BN) = up of features nb*HB + c
 #pragma unroll 1
-        for (int c = 0; c < HB; c += 32) {
+        for (int c = c0; c < HB; c += 8 * G2_EPI) {
           uint32_t gv[32], uv[32];
           tmem_ld32_nowait(t_row + (uint32_t)c, gv);
           tmem_ld32(t_row + (uint32_t)(HB + c), uv);
           const int f0 = nb * HB + c;
           if (tok < N && f0 < M) {
             bf16* dst = a.Y + (size_t)tok * a.ldy + f0;
-            float r[32];
+            // one loop per activation and step: a branch per element would leave the elements' long chains one behind the other
+            float g[32], u[32], r[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
-              const float g = round_bf16(__uint_as_float(gv[j]));  // gate_up_out is bf16 in the reference
-              const float u = round_bf16(__uint_as_float(uv[j]));
-              r[j] = (a.swiglu == 2 ? fmaxf(g, 0.f) : a.swiglu == 3 ? gelu_tanh_gate(g) : g / (1.0f + expf(-g))) * u;
+              g[j] = round_bf16(__uint_as_float(gv[j]));  // gate_up_out is bf16 in the reference
+              u[j] = round_bf16(__uint_as_float(uv[j]));
+            }
+            if (a.swiglu == 2) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) r[j] = fmaxf(g[j], 0.f) * u[j];
+            } else if (a.swiglu == 3) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) r[j] = gelu_tanh_gate(g[j]) * u[j];
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) r[j] = 1.0f + expf(-g[j]);
+#pragma unroll
+              for (int j = 0; j < 32; ++j) r[j] = g[j] / r[j] * u[j];
             }
             if (M % 8 == 0 && a.ldy % 8 == 0 && f0 + 32 <= M && (reinterpret_cast<uintptr_t>(a.Y) & 15) == 0) {
 #pragma unroll
@@ -238,13 +254,15 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 reinterpret_cast<uint4*>(dst)[j] = o;
               }
             } else {
-              for (int j = 0; j < 32 && f0 + j < M; ++j) dst[j] = f2bf(r[j]);
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (f0 + j < M) dst[j] = f2bf(r[j]);
             }
           }
         }
       } else {
 #pragma unroll 1
-        for (int c = 0; c < TN; c += 32) {
+        for (int c = c0; c < TN; c += 8 * G2_EPI) {
           uint32_t v[32];
           tmem_ld32(t_row + (uint32_t)c, v);
           const int f0 = nb * TN + c;
@@ -264,8 +282,10 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 reinterpret_cast<uint4*>(dst)[j] = o;
               }
             } else {
-              for (int j = 0; j < 32 && f0 + j < M; ++j) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
                 const int f = f0 + j;
+                if (f >= M) break;
                 bf16* d1 = f < a.e0 ? a.Y + (size_t)tok * a.e0 + f
                                     : (f < a.e1 ? a.Y1 + (size_t)tok * (a.e1 - a.e0) + (f - a.e0) : a.Y2 + (size_t)tok * (M - a.e1) + (f - a.e1));
                 *d1 = f2bf(__uint_as_float(v[j]));
@@ -319,25 +339,42 @@ cudaError_t g2_launch(const CUtensorMap& mx, const CUtensorMap& mw, const G2Args
 
 }  // namespace
 
-// Tile choice by wave count (cost ~ waves x (tile width + epilogue)), in the units of gemm.cu's model: a pair tile of 256
-// tokens on sms/2 pairs costs what a 128-token tile of the same width costs on sms single CTAs.  Returns the candidate
-// index (0: 256-wide, 1: 2 x 160-wide, 2: 128-wide) or -2 when the single-CTA kernel of gemm.cu should take the shape.
+// Tile choice by wave count: a wave of tiles takes as long as its width + 32 columns (M = 6144, K = 2560, B200: 9.2 us a wave at 128 columns, 10.5 at
+// 160, 12.9 at 192, 14.8 at 224, 16.8 at 256, beside 6 us once), so the width whose last wave is fullest wins:
+//   M x K, tokens           256     224     192     160     128     us a launch over cold weights
+//   6144 x 2560,  400       23.3    21.2    19.1    25.2    23.1
+//   6144 x 2560, 1024       34.0    31.4    28.0    33.4    29.4
+//   2560 x 4096, 1024       33.9    29.2    27.0    23.5    32.9
+//   2560 x 9728, 1024       55.1    49.8    43.6    39.5    58.9
+//   2560 x 9728, 3001      111.2   105.2   129.8   112.4   124.0
+//   9728 x 2560,  400       57.9            53.9            53.5    (gated)
+//   4096 x 12288, 4096     305.2   378.3   332.9   336.4   331.9
+// Beyond three waves of 256 the last one matters less than what narrower tiles read more often, and 256 columns stand.
+// In the units of gemm.cu's model: a pair tile of 256 tokens on sms/2 pairs costs what a 128-token tile of the same width costs on sms single CTAs.
+// Returns the index into g2_widths, or -2 when the single-CTA kernel of gemm.cu should take the shape.
 // Pure host arithmetic (exported as pk_b200_gemm_plan so the calibration is pinned by a CPU test).
+struct G2Width {
+  int bn, nsub;  // columns per accumulator, accumulators per tile
+  bool gated;    // halves of 32 columns each: a gated tile's epilogue reads gate and up 32 columns at a time
+};
+constexpr int kG2Widths = 6;
+constexpr G2Width g2_widths[kG2Widths] = {{256, 1, true}, {160, 2, false}, {128, 1, true}, {192, 1, true}, {160, 1, false}, {224, 1, false}};
+
 static int g2_plan(int M, int N, int K, int swiglu, int sms) {
   if (K % 8 != 0 || M <= 0 || sms < 2) return -2;
   if (N <= G2_BM) return -2;  // one token tile: nothing for the second CTA of a pair to do
   const int pairs = sms / 2;
   const long m_tiles = (N + 2 * G2_BM - 1) / (2 * G2_BM);
-  const int bn[3] = {256, 160, 128}, nsub[3] = {1, 2, 1};
   int best = -1;
   long best_cost = -1;
-  for (int ci = 0; ci < (swiglu ? 1 : 3); ++ci) {
-    const int tn = bn[ci] * nsub[ci];
-    const long nt = swiglu ? (M + bn[ci] / 2 - 1) / (bn[ci] / 2) : (M + tn - 1) / tn;
+  for (int ci = 0; ci < kG2Widths; ++ci) {
+    if (swiglu && !g2_widths[ci].gated) continue;
+    const int bn = g2_widths[ci].bn, nsub = g2_widths[ci].nsub, tn = bn * nsub;
+    const long nt = swiglu ? (M + bn / 2 - 1) / (bn / 2) : (M + tn - 1) / tn;
     const long waves = (m_tiles * nt + pairs - 1) / pairs;
-    // a 320-wide tile has ONE accumulator buffer in TMEM: its epilogue is not hidden behind the next tile's MMAs
-    // (measured: gate_up 209 us with 320-wide vs 165 us with 256-wide tiles), so it only pays as a single wave
-    const long cost = waves * (nsub[ci] == 2 ? tn + tn / 3 + 32 : tn + 32);
+    if (ci >= 2 && m_tiles * (swiglu ? (M + 127) / 128 : (M + 255) / 256) > 3 * pairs) continue;
+    // a 320-wide tile has ONE accumulator buffer in TMEM: its epilogue is not hidden behind the next tile's MMAs, so it only pays as a single wave
+    const long cost = waves * (nsub == 2 ? tn + 64 + (waves > 1 ? tn / 3 : 0) : tn + 32);
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
       best = ci;
@@ -367,22 +404,25 @@ int launch_gemm_pair(const bf16* W, const bf16* X, bf16* Y, bf16* Y1, bf16* Y2, 
   G2Args a{Y, Y1, Y2, e0, e1, M, N, K, swiglu, ldy};
   CUtensorMap mx, mw;
   if (!g2_make_map(&mx, X, N, K, G2_BM)) return -2;
-  const int bn[3] = {256, 160, 128};
   const int rows_w = swiglu ? 2 * M : M;
-  if (!g2_make_map(&mw, W, rows_w, K, bn[best] / 2)) return -2;
+  if (!g2_make_map(&mw, W, rows_w, K, g2_widths[best].bn / 2)) return -2;
   cudaError_t e;
-  if (best == 0) e = g2_launch<256, 1, 6>(mx, mw, a, stream);
-  else if (best == 1) e = g2_launch<160, 2, 5>(mx, mw, a, stream);
-  else e = g2_launch<128, 1, 8>(mx, mw, a, stream);
+  switch (best) {
+    case 0: e = g2_launch<256, 1, 6>(mx, mw, a, stream); break;
+    case 1: e = g2_launch<160, 2, 5>(mx, mw, a, stream); break;
+    case 2: e = g2_launch<128, 1, 8>(mx, mw, a, stream); break;
+    case 3: e = g2_launch<192, 1, 7>(mx, mw, a, stream); break;
+    case 4: e = g2_launch<160, 1, 8>(mx, mw, a, stream); break;
+    default: e = g2_launch<224, 1, 7>(mx, mw, a, stream); break;
+  }
   return e == cudaSuccess ? 0 : (int)e;
 }
 
 }  // namespace pk
 
-// Which prefill GEMM kernel a [M features] x [N tokens] x [K] problem gets on a GPU with `sms` SMs: 256 / 320 / 128 = tile
-// width of the CTA-pair kernel, -2 = the single-CTA kernel (gemm.cu; split-K when skinny).  No CUDA call.
+// Which prefill GEMM kernel a [M features] x [N tokens] x [K] problem gets on a GPU with `sms` SMs: 128 .. 320 = tile
+// width of the CTA-pair kernel, -2 = another kernel (gemm_skinny.cu, gemm.cu).  No CUDA call.
 extern "C" int pk_b200_gemm_plan(int M, int N, int K, int swiglu, int sms) {
-  const int widths[3] = {256, 320, 128};
   const int best = pk::g2_plan(M, N, K, swiglu, sms);
-  return best < 0 ? -2 : widths[best];
+  return best < 0 ? -2 : pk::g2_widths[best].bn * pk::g2_widths[best].nsub;
 }
