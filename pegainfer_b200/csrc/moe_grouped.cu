@@ -14,7 +14,7 @@
 // a tile costs MMAs for its own rows (to the next 16) and not for a full tile of 128; an expert of the usual 100-250 rows reads its weights once.
 //   warp 0 TMA (4 stages of 64 deep) | warp 1 MMA | warps 2-5 epilogue from the other of two accumulators.
 // Bound: HBM for few rows per expert (all weights are read once), the tensor pipe and the operand traffic out of L2 for many.  2048 tokens, 64 experts
-// of 2048 x 1408, top 6 (B200, whole call): 1028 us with 64 x 64 tiles of mma.sync, 377 us so.
+// of 2048 x 1408, top 6 (B200, whole call): 1025 us with 64 x 64 tiles of mma.sync, 363 us so.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
   const int n_ft = (a.N + 127) / 128, tiles = a.meta[0] * n_ft, k_blocks = (a.K + 63) / 64;
   // neighbouring CTAs share an expert's rows
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc_elect_one()) {
       int s = 0;
       uint32_t ph = 1;
       for (int t = blockIdx.x; t < tiles && !*dead; t += gridDim.x) {
@@ -274,20 +274,23 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
           }
         } else {
           // gate in the even lane, up in the odd one: of two rows the even lane takes the first, the odd lane the second
+          // (exponentials, then divisions: side by side, where one loop would run an element's chain after the other's)
+          float gt[16], up[16], den[16];
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float give = __uint_as_float(lane & 1 ? v[j] : v[j + 1]), keep = __uint_as_float(lane & 1 ? v[j + 1] : v[j]);
+          for (int j = 0; j < 16; ++j) {
+            const float give = __uint_as_float(lane & 1 ? v[2 * j] : v[2 * j + 1]), keep = __uint_as_float(lane & 1 ? v[2 * j + 1] : v[2 * j]);
             const float got = __shfl_xor_sync(0xffffffffu, give, 1);
-            float gt = lane & 1 ? got : keep, up = lane & 1 ? keep : got, y;
-            if (EPI == 2) {
-              y = gt / (1.f + expf(-gt)) * up;
-            } else {
-              gt = fminf(gt, a.p0);
-              up = fminf(fmaxf(up, -a.p0), a.p0);
-              y = gt / (1.f + expf(-a.p1 * gt)) * (up + 1.f);
+            gt[j] = lane & 1 ? got : keep;
+            up[j] = lane & 1 ? keep : got;
+            if (EPI == 3) {
+              gt[j] = fminf(gt[j], a.p0);
+              up[j] = fminf(fmaxf(up[j], -a.p0), a.p0) + 1.f;
             }
-            tile[(j + (lane & 1)) * OW + q * 16 + (lane >> 1)] = f2bf(y);
           }
+#pragma unroll
+          for (int j = 0; j < 16; ++j) den[j] = 1.f + expf(EPI == 3 ? -a.p1 * gt[j] : -gt[j]);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) tile[(2 * j + (lane & 1)) * OW + q * 16 + (lane >> 1)] = f2bf(gt[j] / den[j] * up[j]);
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");
         const int o0 = EPI >= 2 ? f0 / 2 : f0;
