@@ -3,7 +3,7 @@
     python -m pegainfer_b200.build            # build everything that is stale
     python -m pegainfer_b200.build --force
 
-Outputs (git-ignored, shipped to the GPU box by gpurun):
+Outputs (git-ignored):
     pegainfer_b200/libpegainfer_kernels_b200.so   -- the C-ABI kernel library (include/pegainfer_kernels.h)
     pegainfer_b200/libpegainfer_qwen3_host.so     -- C++ mirror of the reference's Rust host side
 """
