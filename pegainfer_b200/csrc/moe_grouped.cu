@@ -242,7 +242,8 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
     const int q = warp & 3, et = threadIdx.x & 127;  // TMEM lane quarter this warp may read; thread of the four epilogue warps (2, 3, 4, 5 -> 64 .. 191)
     const int out_n = EPI >= 2 ? a.N / 2 : a.N;
     int lt = 0;
-    for (int t = blockIdx.x; t < tiles && !*dead; t += gridDim.x, ++lt) {
+    // (to the last tile even when a wait ran out: a warp that left on its own reading of *dead would leave the others at barrier 1)
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++lt) {
       const int rt = t / n_ft, m0 = tr[rt], rows = tr[rt + 1] - m0, f0 = (t - rt * n_ft) * 128, as = lt & 1;
       mbar_wait_bounded(tfull + as, (uint32_t)((lt >> 1) & 1), dead);
       __syncwarp();
