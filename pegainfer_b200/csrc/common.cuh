@@ -152,15 +152,33 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
   while (!mbar_try_wait(bar, parity)) {
   }
 }
-// Bounded wait: a barrier that never completes (a fault of the kernel) ends the CTA's work instead of hanging the GPU.  *dead (shared memory) is
-// set and seen by the CTA's other waits; the kernel counts it in ThreadState::wait_err and returns in order.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* dead) {
-  for (uint32_t spins = 0; !mbar_try_wait(bar, parity); ++spins)
-    if (spins > (1u << 24) || *dead) {
-      *dead = 1;
+// Waits with a limit: a barrier that never completes (a fault of the kernel) ends the CTA's work instead of hanging the GPU.  The first wait of a CTA
+// that runs out sets *dead (shared memory), which ends the CTA's other waits, and counts in *err there and then, whatever its role does afterwards.
+// The kernel goes on in order: it waits for its copies and MMAs in flight (mbar_drain), frees its TMEM and returns.
+constexpr uint32_t kWaitSpins = 1u << 24;
+struct WaitFlag {
+  int* dead;          // shared memory, zero at the start
+  unsigned int* err;  // wait_err_word(); null: not counted
+};
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, const WaitFlag& f, uint32_t limit = kWaitSpins) {
+  for (uint32_t spins = 0; !mbar_try_wait(bar, parity); ++spins) {
+    if (*static_cast<volatile int*>(f.dead)) return false;
+    if (spins >= limit) {
+      if (atomicExch(f.dead, 1) == 0 && f.err) atomicAdd(f.err, 1u);
       return false;
     }
+  }
   return true;
+}
+__device__ __forceinline__ bool wait_failed(const WaitFlag& f) { return *static_cast<volatile int*>(f.dead) != 0; }
+// What a role that gave up still has in flight lands in shared or tensor memory: waited for before the CTA ends, with a limit of its own
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+  for (uint32_t spins = 0; spins < kWaitSpins && !mbar_try_wait(bar, parity); ++spins) {
+  }
+}
+// the copies of a ring whose fill j went to stage j % stages, `fills` of them started
+__device__ __forceinline__ void ring_drain(uint64_t* full, int stages, int fills) {
+  for (int j = fills > stages ? fills - stages : 0; j < fills; ++j) mbar_drain(full + j % stages, (uint32_t)((j / stages) & 1));
 }
 __device__ __forceinline__ uint64_t l2_evict_first_policy() {
   uint64_t pol;

@@ -59,7 +59,7 @@ __device__ __forceinline__ float lt_exp2(float x) {
 }
 
 struct LtSmem {  // behind Q and the key chunks
-  uint64_t q_full, k_full[LT_MAXC], k_empty[LT_MAXC], s_full[2], p_ready[2], pv_done;
+  uint64_t q_full, k_full[LT_MAXC], k_empty[LT_MAXC], s_full[2], p_ready[2], pv_done, done;
   uint32_t tmem_slot;
   int dead, n_runs;
   int tok_req[LT_ROWS], tok_pos[LT_ROWS];
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
   uint8_t* Qs = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(lt_smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* Ks = Qs + (size_t)a.nc * LT_QC;
   LtSmem& m = *reinterpret_cast<LtSmem*>(Ks + (size_t)a.nc * LT_KC);
-  volatile int* dead = &m.dead;
+  const WaitFlag wf{&m.dead, a.err};
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int half = blockIdx.x % a.halves, tile = gridDim.x / a.halves - 1 - blockIdx.x / a.halves;  // late tokens (long contexts) first
   const int R0 = tile * LT_ROWS, total = a.tokens * a.heads;
@@ -89,7 +89,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
       mbar_init(m.p_ready + i, LT_ROWS);
     }
     mbar_init(&m.pv_done, 1);
-    *dead = 0;
+    mbar_init(&m.done, 1);
+    m.dead = 0;
     mbar_fence_init();
   }
   if (warp == 4) tmem_alloc(&m.tmem_slot, 512);
@@ -132,23 +133,30 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
     // lane j copies the j-th piece (a page, or 64 slots of one) of every chunk; its page number is looked up once per block, a block ahead
     const int box = min(a.page_size, LT_KEYS), pieces = LT_KEYS / box;
     uint32_t n = 0;
-    for (int i = 0; i < n_runs; ++i) {
+    int fills = 0;  // of the key chunks, in the order in which they are loaded
+    bool on = true;
+    for (int i = 0; i < n_runs && on; ++i) {
       const LtRun r = m.runs[i];
       const int* pg = a.pages + r.pages;
       const int nb = blocks_of(r), last = (r.end - 1) / a.page_size;
       auto page_of = [&](int b) { return pg[min((r.k0 + b * LT_KEYS + lane * box) / a.page_size, last)]; };  // behind the end: the last page again (masked)
       int next = lane < pieces ? page_of(0) : 0;
-      for (int b = 0; b < nb; ++b, ++n) {
+      for (int b = 0; b < nb && on; ++b, ++n) {
         const int page = next, slot = (r.k0 + b * LT_KEYS + lane * box) % a.page_size;
         if (lane < pieces && b + 1 < nb) next = page_of(b + 1);
-        for (int x = 0; x < a.nc; ++x) {
+        for (int x = 0; x < a.nc; ++x, ++fills) {
           const int c = (x + vc0 + nvc) % a.nc;  // the value chunks last
-          mbar_wait_bounded(m.k_empty + c, (n & 1) ^ 1, dead);
+          on = __all_sync(0xffffffffu, mbar_wait_bounded(m.k_empty + c, (n & 1) ^ 1, wf));
+          if (!on) break;
           if (lane == 0) mbar_expect_tx(m.k_full + c, LT_KC);
           __syncwarp();
           if (lane < pieces) lt_tma_3d(Ks + (size_t)c * LT_KC + lane * box * 128, &map_k, c * 64, slot, page, m.k_full + c);
         }
       }
+    }
+    if (!on) {
+      mbar_drain(&m.q_full, 0);
+      for (int j = max(0, fills - a.nc); j < fills; ++j) mbar_drain(m.k_full + (j % a.nc + vc0 + nvc) % a.nc, (uint32_t)((j / a.nc) & 1));
     }
     __syncwarp();
   } else if (warp == 4) {
@@ -164,7 +172,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
       auto issue_s = [&](uint32_t n, int x0, int x1) {
         for (int x = x0; x < x1; ++x) {
           const int c = (x + vc0 + nvc) % a.nc;
-          mbar_wait_bounded(m.k_full + c, n & 1, dead);
+          mbar_wait_bounded(m.k_full + c, n & 1, wf);
           tc_fence_after();
           const uint64_t qd = make_sw128_desc(smem_u32(Qs + (size_t)c * LT_QC)), kd = make_sw128_desc(smem_u32(Ks + (size_t)c * LT_KC));
 #pragma unroll
@@ -174,12 +182,12 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         }
         if (x1 == a.nc) umma_commit(m.s_full + (n & 1));
       };
-      mbar_wait_bounded(&m.q_full, 0, dead);
+      mbar_wait_bounded(&m.q_full, 0, wf);
       issue_s(0, 0, a.nc);
       const uint64_t vd = make_sw128_mn_desc(smem_u32(Ks + (size_t)vc0 * LT_KC), LT_KC, 1024);
       for (uint32_t n = 0; n < total_blocks; ++n) {
         if (n + 1 < total_blocks) issue_s(n + 1, 0, n_other);
-        mbar_wait_bounded(m.p_ready + (n & 1), (n >> 1) & 1, dead);
+        mbar_wait_bounded(m.p_ready + (n & 1), (n >> 1) & 1, wf);
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < LT_KEYS / 16; ++k)
@@ -187,6 +195,10 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         for (int c = vc0; c < vc0 + nvc; ++c) umma_commit(m.k_empty + c);
         umma_commit(&m.pv_done);
         if (n + 1 < total_blocks) issue_s(n + 1, n_other, a.nc);
+      }
+      if (wait_failed(wf)) {
+        umma_commit(&m.done);
+        mbar_drain(&m.done, 0);
       }
     }
     __syncwarp();
@@ -203,7 +215,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
       const int nb = blocks_of(r);
       for (int b = 0; b < nb; ++b, ++n) {
         const int j0 = r.k0 + b * LT_KEYS;
-        mbar_wait_bounded(m.s_full + (n & 1), (n >> 1) & 1, dead);
+        mbar_wait_bounded(m.s_full + (n & 1), (n >> 1) & 1, wf);
         __syncwarp();
         tc_fence_after();
         const uint32_t t_s = t_lane + (n & 1) * LT_KEYS;
@@ -231,7 +243,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
           mx = to;
           l *= corr;
           if (n > 0) {  // O holds the blocks before this one
-            mbar_wait_bounded(&m.pv_done, (n - 1) & 1, dead);
+            mbar_wait_bounded(&m.pv_done, (n - 1) & 1, wf);
             __syncwarp();
             tc_fence_after();
             for (int c = 0; c < nvc * 64; c += 64) {
@@ -275,7 +287,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
       }
     }
     // ---- O / l -> bf16
-    mbar_wait_bounded(&m.pv_done, (n - 1) & 1, dead);
+    mbar_wait_bounded(&m.pv_done, (n - 1) & 1, wf);
     __syncwarp();
     tc_fence_after();
     const float sk = a.sink && tok >= 0 ? bf2f(a.sink[R % a.heads]) * 1.4426950408889634f : -INFINITY;
@@ -299,7 +311,6 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
   }
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && *dead && a.err) atomicAdd(a.err, 1u);
   if (warp == 4) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);

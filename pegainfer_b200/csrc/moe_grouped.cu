@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict_
 
 constexpr int kMgStages = 4, kMgThreads = 192, kMgChunk = 32;  // chunk: rows of an epilogue step
 constexpr int kMgA = 128 * 64 * 2, kMgBox = 64 * 64 * 2, kMgStage = kMgA + kMoeTile * 64 * 2;
-constexpr size_t kMgSmem = (size_t)kMgStages * kMgStage + 1024 + kMgChunk * 128 * 2 + (2 * kMgStages + 4) * 8 + 16;
+constexpr size_t kMgSmem = (size_t)kMgStages * kMgStage + 1024 + kMgChunk * 128 * 2 + (2 * kMgStages + 5) * 8 + 16;
 
 __device__ __forceinline__ void mg_tma_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
   asm volatile(
@@ -166,8 +166,9 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
   uint64_t* empty = full + kMgStages;
   uint64_t* tfull = empty + kMgStages;
   uint64_t* tempty = tfull + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
-  volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* done = tempty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  const WaitFlag wf{reinterpret_cast<int*>(tmem_slot + 1), a.err};
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMgStages; ++s) {
@@ -178,7 +179,8 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
       mbar_init(tfull + s, 1);
       mbar_init(tempty + s, 4);
     }
-    *dead = 0;
+    mbar_init(done, 1);
+    *wf.dead = 0;
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
@@ -194,12 +196,13 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
   // neighbouring CTAs share an expert's rows
   if (warp == 0) {
     if (tc_elect_one()) {
-      int s = 0;
+      int s = 0, fills = 0;
       uint32_t ph = 1;
-      for (int t = blockIdx.x; t < tiles && !*dead; t += gridDim.x) {
+      for (int t = blockIdx.x; t < tiles && !wait_failed(wf); t += gridDim.x) {
         const int rt = t / n_ft, m0 = tr[rt], rows = tr[rt + 1] - m0, w0 = te[rt] * a.N + (t - rt * n_ft) * 128, boxes = (rows + 63) / 64;
         for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait_bounded(empty + s, ph, dead)) break;
+          if (!mbar_wait_bounded(empty + s, ph, wf)) break;
+          ++fills;
           mbar_expect_tx(full + s, kMgA + boxes * kMgBox);
           uint8_t* st = smem + (size_t)s * kMgStage;
           mg_tma_2d(st, &map_w, kb * 64, w0, full + s);
@@ -210,19 +213,20 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
           }
         }
       }
+      if (wait_failed(wf)) ring_drain(full, kMgStages, fills);
     }
   } else if (warp == 1) {
     if (tc_elect_one()) {
       int s = 0, lt = 0;
       uint32_t ph = 0;
-      for (int t = blockIdx.x; t < tiles && !*dead; t += gridDim.x, ++lt) {
+      for (int t = blockIdx.x; t < tiles && !wait_failed(wf); t += gridDim.x, ++lt) {
         const int rt = t / n_ft, n16 = (tr[rt + 1] - tr[rt] + 15) / 16, as = lt & 1;
         // instruction descriptor: D = f32 [4,6) = 1, A = bf16 [7,10) = 1, B = bf16 [10,13) = 1, both K-major, N >> 3 at [17,23), M >> 4 at [24,29)
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n16 * 2) << 17) | ((uint32_t)(128 >> 4) << 24);
-        if (!mbar_wait_bounded(tempty + as, (uint32_t)(((lt >> 1) & 1) ^ 1), dead)) break;
+        if (!mbar_wait_bounded(tempty + as, (uint32_t)(((lt >> 1) & 1) ^ 1), wf)) break;
         tc_fence_after();
         for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait_bounded(full + s, ph, dead)) break;
+          if (!mbar_wait_bounded(full + s, ph, wf)) break;
           tc_fence_after();
           const uint32_t a_addr = smem_u32(smem + (size_t)s * kMgStage);
           const uint64_t ad = make_sw128_desc(a_addr), bd = make_sw128_desc(a_addr + kMgA);
@@ -237,15 +241,19 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
         }
         umma_commit(tfull + as);
       }
+      if (wait_failed(wf)) {
+        umma_commit(done);
+        mbar_drain(done, 0);
+      }
     }
   } else {
     const int q = warp & 3, et = threadIdx.x & 127;  // TMEM lane quarter this warp may read; thread of the four epilogue warps (2, 3, 4, 5 -> 64 .. 191)
     const int out_n = EPI >= 2 ? a.N / 2 : a.N;
     int lt = 0;
-    // (to the last tile even when a wait ran out: a warp that left on its own reading of *dead would leave the others at barrier 1)
+    // (to the last tile even when a wait ran out: a warp that left on its own reading of the flag would leave the others at barrier 1)
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++lt) {
       const int rt = t / n_ft, m0 = tr[rt], rows = tr[rt + 1] - m0, f0 = (t - rt * n_ft) * 128, as = lt & 1;
-      mbar_wait_bounded(tfull + as, (uint32_t)((lt >> 1) & 1), dead);
+      mbar_wait_bounded(tfull + as, (uint32_t)((lt >> 1) & 1), wf);
       __syncwarp();
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * kMoeTile);
@@ -309,7 +317,6 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && *dead && a.err) atomicAdd(a.err, 1u);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
