@@ -64,9 +64,25 @@ def test_prefill_gemm_plan_matches_the_measured_calibration():
     H, I, QKV, Q = 2560, 9728, 6144, 4096  # Qwen3-4B
     assert plan(Q, 2048, H, 0, 148) == 256 and plan(QKV, 2048, H, 0, 148) == 256   # q / fused qkv
     assert plan(H, 2048, Q, 0, 148) == 320 and plan(H, 2048, I, 0, 148) == 320       # o_proj, down_proj
-    assert plan(I, 2048, H, 1, 148) == 256                                            # gate_up + SwiGLU: 256-wide only
+    assert plan(I, 2048, H, 1, 148) == 256                                            # gate_up + SwiGLU: full tiles
     assert plan(2 * I, 2048, H, 0, 148) == 256                                        # plain gate_up: never the single-buffered 320
     for m, k in ((Q, H), (H, Q), (H, I), (2 * I, H)):
-        assert plan(m, 128, k, 0, 148) == -2                                          # one token tile: single-CTA kernel (split-K)
+        assert plan(m, 128, k, 0, 148) == -2                                          # one token tile: gemm_skinny.cu or gemm.cu
     assert plan(I, 128, H, 1, 148) == -2 and plan(Q, 2048, H + 4, 0, 148) == -2       # SwiGLU at 128 tokens, K % 8 != 0
     assert plan(4096, 2048, 4096, 0, 148) in (256, 320, 128)                          # Qwen3-8B q: some pair tile
+    # the fullest last wave of up to three (the table at g2_plan): the fastest width of each row there
+    assert [plan(QKV, t, H, 0, 148) for t in (400, 1024)] == [192, 192]
+    assert plan(H, 1024, Q, 0, 148) == 160 and plan(H, 1024, I, 0, 148) == 160
+    assert plan(H, 3001, I, 0, 148) == 224 and plan(4096, 4096, 12288, 0, 148) == 256
+    assert plan(I, 400, H, 1, 148) == 192 and plan(1000, 400, H, 1, 148) == 128       # gated
+
+
+def test_the_pair_gemms_shapes_cover_every_width():
+    from pegainfer_b200 import ffi
+    from tests import test_gemm_pair_gpu as t
+    plan = ffi.lib().pk_b200_gemm_plan
+    marks = {f.__name__: {m.args[0]: m.args[1] for m in f.pytestmark if m.name == "parametrize"} for f in (t.test_against_64_bits, t.test_every_width, t.test_gated)}
+    plain = {plan(m, n, 200, 0, 148) for m, n in marks["test_every_width"]["M,N"]}
+    plain |= {plan(m, n, 264, 0, 148) for m in marks["test_against_64_bits"]["M"] for n in marks["test_against_64_bits"]["N"]}
+    assert plain >= {128, 160, 192, 224, 256, 320}
+    assert {plan(m, n, 264, 1, 148) for m in marks["test_gated"]["M"] for n in marks["test_gated"]["N"]} == {128, 192, 256}

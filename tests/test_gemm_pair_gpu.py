@@ -1,4 +1,4 @@
-"""The CTA-pair GEMM (csrc/gemm2.cu) at every tile width that its plan may choose: tokens and features around the tiles, K with a ragged last
+"""The CTA-pair GEMM (csrc/gemm2.cu) at every tile width that its plan may choose (test_abi.py holds the shapes to that): tokens and features around the tiles, K with a ragged last
 block, outputs split at odd places, gated and plain."""
 import ctypes as C
 

@@ -225,14 +225,14 @@ def test_gemm_swiglu_epilogue(inter, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(2560, 8, 2560), (2560, 64, 9728), (1024, 33, 2560)])
-def test_gemm_graphsafe_batch_bucket(lib, M, N, K):  # decode bucket > 4 goes to the tensor-core path (split-K when skinny)
+def test_gemm_graphsafe_batch_bucket(lib, M, N, K):  # decode bucket > 4 goes to the tensor-core path (gemm_skinny.cu)
     W, X = rnd((M, K), 19, 0.02), rnd((N, K), 20, 1.0)
     W_d, X_d = dev(W), dev(X)
     Y = torch.zeros((N, M), dtype=torch.bfloat16, device="cuda")
     lib.gemm_graphsafe_cuda(p(W_d), p(X_d), p(Y), M, N, K, stream())
     want = O.gemm(bits(W), bits(X))
     assert_bf16_close(bits(Y), want, 1, floor=float(np.abs(f32(want)).max()) / 64, frac_exact=0.9)
-    # the split-K reduction sums the partial tiles in a fixed order: repeated launches are bit-identical
+    # the parts of K are added up in a fixed order: repeated launches are bit-identical
     Y2 = torch.zeros_like(Y)
     for _ in range(3):
         lib.gemm_graphsafe_cuda(p(W_d), p(X_d), p(Y2), M, N, K, stream())
