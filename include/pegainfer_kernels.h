@@ -179,9 +179,14 @@ const char* pk_b200_version(void);
 /* Number of kernels launched by this library on the calling thread since the last
  * reset (bench.py's gpu_launches; counts launches recorded into a capture too). */
 int64_t pk_b200_launch_count(int reset);
-/* Waits inside this thread's kernels that ran into their iteration limit since cublas_init (0 in a sound run; the launch's results are then
- * not valid).  Synchronises; -1: the device could not be read. */
+/* Kernels of this process with a wait that ran into its iteration limit since the first cublas_init (0 in a sound run; the results of such a
+ * launch are not valid).  Synchronises the device; -1: no cublas_init yet, or the device reports an error.  _seen does not synchronise (0 before
+ * the first cublas_init): for a caller that has just waited for its stream.  The hosts read it behind every synchronisation and refuse all steps
+ * of a model from the first run-out on. */
 int pk_b200_wait_errors(void);
+unsigned int pk_b200_wait_errors_seen(void);
+/* Launches a kernel whose one wait runs out after `spins` (1 .. 1024) tries: what a run-out does can be tried without a fault. */
+int pk_b200_wait_probe(int spins, pk_stream stream);
 /* Enable (1) / disable (0) programmatic dependent launch on this thread's launches. */
 void pk_b200_set_pdl(int enable);
 

@@ -25,10 +25,12 @@ struct ThreadState {
   size_t scratch_bytes = 0;
   int sm_count = 0;
   int device = -1;
-  unsigned int* wait_err = nullptr;  // device word: bounded waits that ran out (pk_b200_wait_errors)
 };
 ThreadState& tls();
 int sm_count();
+// The word that counts waits that ran out (mbar_wait_bounded), in mapped host memory: one per process, made by the first cublas_init and kept, so that a
+// captured graph may hold it and any thread may read it after a synchronisation of its own.  Null before that.
+unsigned int* wait_err_word();
 
 // Launch with optional programmatic dependent launch (PDL).  Kernels that opt in call
 // pdl_wait() before touching data produced by the previous kernel in the stream.

@@ -302,7 +302,7 @@ int sk_run(const bf16* W, const bf16* X, bf16* Y, bf16* Y1, bf16* Y2, int e0, in
   const int n_tiles = (N + NT - 1) / NT, tiles = ((M + p.rows - 1) / p.rows) * n_tiles;
   CUtensorMap mx, mw;
   if (!sk_make_map(&mx, X, N, K, NT) || !sk_make_map(&mw, W, M, K, p.rows)) return -2;
-  const SkArgs a{Y, Y1, Y2, e0, e1, M, N, K, n_tiles, p.rows, p.stages, tls().wait_err};
+  const SkArgs a{Y, Y1, Y2, e0, e1, M, N, K, n_tiles, p.rows, p.stages, wait_err_word()};
   return (int)sk_launch<NT>(mx, mw, a, tiles, p.splits, stream);
 }
 

@@ -122,6 +122,7 @@ struct Lib {
   // every design / the block forms that route to experts / the ones with a dense feed-forward / one block form each
 #define PV_COMMON(X)                                                                                                                       \
   X(cuda_set_device) X(cublas_init) X(cublas_destroy) X(gemm_cuda) X(flashinfer_top1_cuda) X(pk_b200_set_pdl) X(pk_b200_launch_count)      \
+  X(pk_b200_wait_errors_seen)                                                                                                               \
   X(pk_res32_skinny_proj) X(pk_convert) X(pk_gemm_strided) X(pk_proj_rows_f32out) X(pk_scale_to_f32) X(pk_top1_rows_f32)
 #define PV_MOE(X) X(pk_moe_down_combine) X(pk_moe_grouped_workspace_bytes) X(pk_moe_up_act_p) X(pk_moe_grouped_act_p)
 #define PV_DENSE(X) X(pk_act) X(pk_act_ex) X(pk_b200_gemv_fused) X(pk_b200_gemm_gated_ex)
@@ -270,6 +271,8 @@ struct Model {
     err = std::string(what) + ": " + cudaGetErrorString(e);
     return false;
   }
+  unsigned wait_base = 0;  // the library's count of run-out waits when the model was made
+  bool waits_ok() { return k.pk_b200_wait_errors_seen() == wait_base ? true : fail("a kernel gave up a wait: its results, and the state they went into, are not valid"); }
   bool rc(int r, const char* what) {
     if (r == 0) return true;
     err = std::string(what) + " failed (" + (r > 0 ? cudaGetErrorString((cudaError_t)r) : r == -1 ? "invalid argument" : "shape out of range") + ")";
@@ -1886,6 +1889,7 @@ bool Model::forward(int T, int n, int n_rows, int max_kv, int want_sample) {
 // greedy token of each row in sampled_h when want_sample).
 bool Model::step(int n, const int* tokens, const int* lens, const int* rids, int n_rows, const int* rows, int want_sample) {
   if (!finalized) return fail("model not finalized");
+  if (!waits_ok()) return false;
   if (n <= 0) return fail("empty step");
   int T = 0, pages_needed = 0;
   for (int i = 0; i < n; ++i) {
@@ -1999,7 +2003,7 @@ bool Model::step(int n, const int* tokens, const int* lens, const int* rids, int
     ok = forward(T, n, n_rows, max_kv, want_sample);
   }
   if (!ok) return false;
-  if (!cu(cudaStreamSynchronize(st), "step")) return false;
+  if (!cu(cudaStreamSynchronize(st), "step") || !waits_ok()) return false;
   txn.committed = true;
   return true;
 }
@@ -2028,6 +2032,7 @@ PV_API void* pv_create(const pv::ModelCfg* mc, const pv::LayerCfg* lc, const cha
   if (cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking) != cudaSuccess)
     return bail(std::string("stream creation failed: ") + cudaGetErrorString(cudaGetLastError()));
   m->k.cublas_init();
+  m->wait_base = m->k.pk_b200_wait_errors_seen();
   m->k.pk_b200_set_pdl(mc->enable_pdl);
   g_pv_err.clear();
   return m;

@@ -45,7 +45,7 @@ struct Lib {
   Q35_FN(prefill_attention_hd256_prep_cuda) Q35_FN(attention_gate_batch_hd256_cuda) Q35_FN(qk_norm_partial_rope_batched_decode_hd256_cuda)
   Q35_FN(paged_kv_scatter_cuda) Q35_FN(paged_attention_decode_cuda_hd256) Q35_FN(batch_prefill_paged_cuda_hd256)
   Q35_FN(silu_mul_triton_aot_cuda) Q35_FN(flashinfer_top1_cuda) Q35_FN(pk_b200_gemv_fused) Q35_FN(pk_b200_gemm_segments)
-  Q35_FN(pk_b200_set_pdl) Q35_FN(pk_b200_launch_count)
+  Q35_FN(pk_b200_set_pdl) Q35_FN(pk_b200_launch_count) Q35_FN(pk_b200_wait_errors_seen)
 #undef Q35_FN
   std::string load(const std::string& p) {
     handle = dlopen(p.c_str(), RTLD_NOW | RTLD_LOCAL);
@@ -61,7 +61,7 @@ struct Lib {
     Q35_REQ(attention_gate_batch_hd256_cuda) Q35_REQ(qk_norm_partial_rope_batched_decode_hd256_cuda) Q35_REQ(paged_kv_scatter_cuda)
     Q35_REQ(paged_attention_decode_cuda_hd256) Q35_REQ(batch_prefill_paged_cuda_hd256) Q35_REQ(silu_mul_triton_aot_cuda)
     Q35_REQ(flashinfer_top1_cuda) Q35_REQ(pk_b200_gemv_fused) Q35_REQ(pk_b200_gemm_segments) Q35_REQ(pk_b200_set_pdl)
-    Q35_REQ(pk_b200_launch_count)
+    Q35_REQ(pk_b200_launch_count) Q35_REQ(pk_b200_wait_errors_seen)
 #undef Q35_REQ
     return missing.empty() ? "" : "kernel library " + p + " lacks:" + missing;
   }
@@ -137,6 +137,8 @@ struct Model {
     err = std::string(what) + ": " + cudaGetErrorString(e);
     return false;
   }
+  unsigned wait_base = 0;  // the library's count of run-out waits when the model was made
+  bool waits_ok() { return k.pk_b200_wait_errors_seen() == wait_base ? true : fail("a kernel gave up a wait: its results, and the state they went into, are not valid"); }
   ~Model() {
     if (st) cudaStreamSynchronize(st);
     for (auto& g : graphs)
@@ -358,6 +360,7 @@ bool Model::layer_tail(Layer& L, int T, pk_bf16* hcur, pk_bf16* attn, pk_bf16* h
 
 bool Model::prefill(int rid, const uint32_t* tokens, int n, void** logits_out) {
   if (!finalized) return fail("model not finalized");
+  if (!waits_ok()) return false;
   if (rid < 0 || rid >= (int)reqs.size() || !reqs[rid].live) return fail("bad request id");
   if (n <= 0) return fail("empty prompt");
   Request& r = reqs[rid];
@@ -458,9 +461,7 @@ bool Model::prefill(int rid, const uint32_t* tokens, int n, void** logits_out) {
   }
   k.rms_norm_offset_cuda(h.bf() + (size_t)(T - 1) * H, norm.bf(), x.bf(), H, eps, st);
   k.gemm_graphsafe_cuda(embed.p(), x.bf(), logits.bf(), c.vocab_size, 1, H, st);
-  if (!cu(cudaStreamSynchronize(st), "prefill sync")) {
-    return false;
-  }
+  if (!cu(cudaStreamSynchronize(st), "prefill sync") || !waits_ok()) return false;
   r.seq_len += T;
   if (logits_out) *logits_out = logits.ptr;
   return true;
@@ -577,6 +578,7 @@ bool Model::decode_body_fused(Request& r) {
 
 bool Model::decode(int rid, uint32_t token, void** logits_out, int* sampled) {
   if (!finalized) return fail("model not finalized");
+  if (!waits_ok()) return false;
   if (rid < 0 || rid >= (int)reqs.size() || !reqs[rid].live) return fail("bad request id");
   Request& r = reqs[rid];
   if (r.seq_len + 1 > kMaxSeq) return fail("position beyond the 4096-entry RoPE table");
@@ -620,7 +622,7 @@ bool Model::decode(int rid, uint32_t token, void** logits_out, int* sampled) {
   if (logits_out) *logits_out = logits.ptr;
   if (sampled) {
     if (!cu(cudaMemcpyAsync(sample_h, sample_out.ptr, 4, cudaMemcpyDeviceToHost, st), "sample D2H")) return false;
-    if (!cu(cudaStreamSynchronize(st), "decode sync")) return false;
+    if (!cu(cudaStreamSynchronize(st), "decode sync") || !waits_ok()) return false;
     *sampled = sample_h[0];
   }
   return true;
@@ -663,6 +665,7 @@ V35 void* pq35_create(const pq35_config* c, const int* layer_is_full, const char
   m->device = c->device_ordinal;
   if (cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking) != cudaSuccess) return bail("stream creation failed");
   m->k.cublas_init();
+  m->wait_base = m->k.pk_b200_wait_errors_seen();
   m->k.pk_b200_set_pdl(c->enable_pdl);
   g35_err.clear();
   return m;
@@ -717,7 +720,7 @@ V35 int pq35_prefill(void* mp, int id, const uint32_t* tokens, int n, void** log
 V35 int pq35_decode(void* mp, int id, uint32_t token, void** logits_out, int* sampled) { return M35->decode(id, token, logits_out, sampled) ? 0 : -1; }
 V35 int pq35_copy_out(void* mp, void* dst, const void* src, int64_t bytes) {
   if (cudaMemcpyAsync(dst, src, (size_t)bytes, cudaMemcpyDefault, M35->st) != cudaSuccess) return -1;
-  return cudaStreamSynchronize(M35->st) == cudaSuccess ? 0 : -1;
+  return M35->cu(cudaStreamSynchronize(M35->st), "copy out") && M35->waits_ok() ? 0 : -1;
 }
 V35 int64_t pq35_launches_per_step(void* mp) { return M35->launches_per_step; }
 // Greedy generation timed like bench_serving.rs (TTFT = submit -> first token, then the gaps between tokens).
@@ -734,7 +737,7 @@ V35 int pq35_generate(void* mp, const uint32_t* prompt, int n_prompt, int max_to
     m->k.flashinfer_top1_cuda(static_cast<const pk_bf16*>(lg), static_cast<pk_bf16*>(m->top1_val.ptr), static_cast<uint8_t*>(m->top1_states.ptr),
                               m->sample_out.i32(), m->c.vocab_size, m->st);
     ok = cudaMemcpyAsync(m->sample_h, m->sample_out.ptr, 4, cudaMemcpyDeviceToHost, m->st) == cudaSuccess &&
-         cudaStreamSynchronize(m->st) == cudaSuccess;
+         cudaStreamSynchronize(m->st) == cudaSuccess && m->waits_ok();
     tok = m->sample_h[0];
   }
   auto tprev = clk::now();

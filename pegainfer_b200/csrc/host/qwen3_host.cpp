@@ -31,7 +31,7 @@ std::string KernelLib::load(const std::string& p) {
   PQ_REQ(batch_prefill_cta_tile_q_with_override) PQ_REQ(batch_prefill_paged_cuda_with_cta_tile_q)
   PQ_REQ(paged_attention_decode_cuda) PQ_REQ(paged_attention_decode_split_kv_cuda)
   PQ_REQ(flashinfer_top1_cuda)
-  PQ_OPT(pk_b200_launch_count) PQ_OPT(pk_b200_set_pdl) PQ_OPT(pk_b200_gemv_fused) PQ_OPT(pk_b200_gemm_segments)
+  PQ_OPT(pk_b200_launch_count) PQ_OPT(pk_b200_wait_errors_seen) PQ_OPT(pk_b200_set_pdl) PQ_OPT(pk_b200_gemv_fused) PQ_OPT(pk_b200_gemm_segments)
   PQ_OPT(pk_b200_decode_attention_fused) PQ_OPT(pk_tp_all_reduce_rows)
   PQ_OPT(pk_tp_all_reduce_add_rms_norm) PQ_OPT(pk_tp_max_rows)
   PQ_OPT(pk_b200_decode_attention_fused_prefetch) PQ_OPT(pk_b200_gemv_grid) PQ_OPT(pk_tp_top1_exchange) PQ_OPT(pk_b200_gemm_swiglu)
@@ -220,6 +220,9 @@ struct Qwen3Model {
     err = std::string(what) + ": " + cudaGetErrorString(e);
     return false;
   }
+  unsigned wait_base = 0;  // the library's count of run-out waits when the model was made (a library without the extensions has no such waits)
+  unsigned waits_seen() const { return k.pk_b200_wait_errors_seen ? k.pk_b200_wait_errors_seen() : 0; }
+  bool waits_ok() { return waits_seen() == wait_base ? true : fail("a kernel gave up a wait: its results, and the state they went into, are not valid"); }
 
   // ---- ops (pegainfer-kernels/src/ops/linear.rs) ----
   void gemm_rows_into(const DeviceMatrix& w, size_t row_off, size_t nrows, const pk_bf16* x, int T,
@@ -519,6 +522,7 @@ bool Qwen3Model::unified_step(int n_req, const uint32_t* tokens, const int* lens
   // data-dependent reason, and a CUDA failure later rolls them back (PrefillTxn). ----
   int T = 0;
   std::vector<int> starts(n_req);
+  if (!waits_ok()) return false;
   if (n_req <= 0) return fail("empty prefill batch");
   if (n_req + n_dec > max_bs) return fail("more prompts + decode requests than max_batch");
   int pages_needed = 0;
@@ -750,7 +754,7 @@ bool Qwen3Model::unified_step(int n_req, const uint32_t* tokens, const int* lens
       dec_logits_out[i - n_req] = lg;
     }
   }
-  if (!cu(cudaStreamSynchronize(st), "prefill sync")) return false;
+  if (!cu(cudaStreamSynchronize(st), "prefill sync") || !waits_ok()) return false;
   txn.committed = true;
   return true;
 }
@@ -1134,6 +1138,7 @@ bool Qwen3Model::run_step_kernels(int padded, bool split) {
 
 bool Qwen3Model::decode(int bs, const uint32_t* tokens, const int* kv_ids, void** logits_out, int* sampled) {
   if (!finalized) return fail("model not finalized");
+  if (!waits_ok()) return false;
   if (bs <= 0 || bs > max_bs) return fail("batch size out of range");
   const bool fused = rt.mode >= 1;
   // fused path: 1..4 requests run the GEMV graph of their exact size; larger batches pad to the reference's buckets
@@ -1149,7 +1154,7 @@ bool Qwen3Model::decode(int bs, const uint32_t* tokens, const int* kv_ids, void*
     if (fused) {
       if (!cu(cudaMemcpyAsync(sample_h, sample_out.ptr, (size_t)bs * 4, cudaMemcpyDeviceToHost, st), "sample D2H"))
         return false;
-      if (!cu(cudaStreamSynchronize(st), "decode sync")) return false;
+      if (!cu(cudaStreamSynchronize(st), "decode sync") || !waits_ok()) return false;
       for (int b = 0; b < bs; ++b) sampled[b] = sample_h[b];
     } else {
       for (int b = 0; b < bs; ++b)  // per request: top-1 kernel, sync, 4-byte D2H (sampling.rs:161-172)
@@ -1164,6 +1169,7 @@ bool Qwen3Model::decode(int bs, const uint32_t* tokens, const int* kv_ids, void*
 // and there is no host synchronisation inside the timed region (CUDA events on the launch stream).
 bool Qwen3Model::decode_burst(int kv_id, uint32_t first_token, int K, uint32_t* tokens_out, float* ms_total) {
   if (!finalized || rt.mode < 1) return fail("decode_burst needs the fused path");
+  if (!waits_ok()) return false;
   if (K <= 0) return fail("K must be positive");
   {  // all K steps must fit before the first one advances the request
     if (kv_id < 0 || kv_id >= (int)kv_states.size() || !kv_states[kv_id].live) return fail("bad kv id");
@@ -1200,7 +1206,7 @@ bool Qwen3Model::decode_burst(int kv_id, uint32_t first_token, int K, uint32_t* 
     ok = ok && cu(cudaMemcpyAsync(toks.i32() + i, sample_out.ptr, 4, cudaMemcpyDeviceToDevice, st), "tok save");
   }
   cudaEventRecord(e1, st);
-  ok = ok && cu(cudaStreamSynchronize(st), "burst sync");
+  ok = ok && cu(cudaStreamSynchronize(st), "burst sync") && waits_ok();
   float ms = 0.f;
   cudaEventElapsedTime(&ms, e0, e1);
   cudaEventDestroy(e0);
@@ -1271,7 +1277,7 @@ bool Qwen3Model::sample_greedy(const pk_bf16* lg, int* out) {
                             0x80000000u | (++host_sample_seq & 0x7fffffffu), ctx.stream) != 0)
     return fail("pk_tp_top1_exchange failed");
   if (!cu(cudaMemcpyAsync(sample_h, sample_out.ptr, 4, cudaMemcpyDeviceToHost, ctx.stream), "sample D2H")) return false;
-  if (!cu(cudaStreamSynchronize(ctx.stream), "sample sync")) return false;
+  if (!cu(cudaStreamSynchronize(ctx.stream), "sample sync") || !waits_ok()) return false;
   *out = sample_h[0];
   return true;
 }
@@ -1332,6 +1338,7 @@ __attribute__((visibility("default"))) void* pq_model_create(const pq_config* c,
   if (cudaStreamCreateWithFlags(&m->ctx.stream, cudaStreamNonBlocking) != cudaSuccess)
     return bail(std::string("stream creation failed: ") + cudaGetErrorString(cudaGetLastError()));
   m->k.cublas_init();
+  m->wait_base = m->waits_seen();
   if (m->k.pk_b200_set_pdl) m->k.pk_b200_set_pdl(r->enable_pdl);
   g_create_err.clear();
   return m;
@@ -1391,12 +1398,12 @@ __attribute__((visibility("default"))) int pq_sample_greedy(void* mp, const void
   return PQ_M->sample_greedy(static_cast<const pk_bf16*>(logits), out) ? 0 : -1;
 }
 __attribute__((visibility("default"))) int pq_sync(void* mp) {
-  return cudaStreamSynchronize(PQ_M->ctx.stream) == cudaSuccess ? 0 : -1;
+  return PQ_M->cu(cudaStreamSynchronize(PQ_M->ctx.stream), "sync") && PQ_M->waits_ok() ? 0 : -1;
 }
 // copy a device buffer produced on the model's stream into caller-owned memory (device or host)
 __attribute__((visibility("default"))) int pq_copy_out(void* mp, void* dst, const void* src, int64_t bytes) {
   if (cudaMemcpyAsync(dst, src, (size_t)bytes, cudaMemcpyDefault, PQ_M->ctx.stream) != cudaSuccess) return -1;
-  return cudaStreamSynchronize(PQ_M->ctx.stream) == cudaSuccess ? 0 : -1;
+  return PQ_M->cu(cudaStreamSynchronize(PQ_M->ctx.stream), "sync") && PQ_M->waits_ok() ? 0 : -1;
 }
 __attribute__((visibility("default"))) int64_t pq_launch_count(void* mp, int reset) {
   return PQ_M->k.pk_b200_launch_count ? PQ_M->k.pk_b200_launch_count(reset) : -1;

@@ -356,7 +356,7 @@ int launch_latent_attention_tc(const bf16* qa, const bf16* cache, const bf16* si
     }
     configured = true;
   }
-  const LtArgs a{sink, pos, req, page_off, pages, out, page_size, tokens, heads, rank, nc, halves, window, scale * 1.4426950408889634f, tls().wait_err};
+  const LtArgs a{sink, pos, req, page_off, pages, out, page_size, tokens, heads, rank, nc, halves, window, scale * 1.4426950408889634f, wait_err_word()};
   return (int)launch(latent_attention_tc_kernel, dim3((unsigned)(tiles * halves)), dim3(LT_THREADS), smem, st, true, mq, mk, a);
 }
 

@@ -431,7 +431,7 @@ extern "C" int pk_moe_grouped_act_p(const void* xa, const void* w_up, const void
   launch(moe_bucket_kernel, dim3(1), dim3(kBucketThreads), (size_t)(2 * experts + 66) * sizeof(int), st, true, ids, (int)pairs, experts, max_tiles, meta,
          slot_pair, pair_slot);
   launch(moe_gather_kernel, dim3((unsigned)pairs), dim3(width >= 2048 ? 256 : 128), 0, st, true, (const bf16*)xa, (const int*)slot_pair, xs, width, top);
-  MgArgs a{hid, meta, slot_pair, weights, experts, max_tiles, act ? 2 * ff : ff, width, p0, p1, tls().wait_err};
+  MgArgs a{hid, meta, slot_pair, weights, experts, max_tiles, act ? 2 * ff : ff, width, p0, p1, wait_err_word()};
   cudaError_t e = act == 2 ? mg_launch<3>(xs, pairs, w_up, a, st) : act == 1 ? mg_launch<2>(xs, pairs, w_up, a, st) : mg_launch<0>(xs, pairs, w_up, a, st);
   if (e != cudaSuccess) return (int)e;
   a.out = part;

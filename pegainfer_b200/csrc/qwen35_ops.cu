@@ -412,7 +412,7 @@ int pk_b200_gated_delta_rule_prefill_recurrent(const pk_bf16* qkv_seq, const pk_
   }
   return (int)launch(gated_delta_rule_seq_kernel, dim3(num_value_heads, GV / GC), dim3(kDcThreads), smem, stream, true, (const bf16*)qkv_seq,
                      (const bf16*)b_seq, (const bf16*)a_seq, (const bf16*)dt_bias, A_log, state, (bf16*)out_seq, num_key_heads, num_value_heads,
-                     seq_len, tls().wait_err);
+                     seq_len, wait_err_word());
 }
 void prefill_attention_hd256_prep_cuda(const pk_bf16* q_full_batch, const pk_bf16* k_batch, const pk_bf16* v_batch,
                                        const pk_bf16* q_norm_weight, const pk_bf16* k_norm_weight, const pk_bf16* cos_cache,

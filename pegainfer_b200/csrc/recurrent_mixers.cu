@@ -570,7 +570,7 @@ static void launch_delta_chunk(const SeqArgs& a, int entries, cudaStream_t st) {
     attr_set = true;
   }
   const bool vec = ((a.ld | a.q_off | a.k_off) & 7) == 0 && (reinterpret_cast<uintptr_t>(a.qkv) & 15) == 0;
-  launch(delta_chunk_kernel<DK>, dim3(entries, a.H, (a.vdim + COLS - 1) / COLS), dim3(kDcThreads), smem, st, true, a, vec, tls().wait_err);
+  launch(delta_chunk_kernel<DK>, dim3(entries, a.H, (a.vdim + COLS - 1) / COLS), dim3(kDcThreads), smem, st, true, a, vec, wait_err_word());
 }
 template <typename E, bool CH>
 static int launch_delta(const SeqArgs& a, int entries, cudaStream_t st) {

@@ -1,6 +1,9 @@
 // Per-thread runtime state: device binding, scratch, launch counter.
 // Replaces csrc/linear.cu:7-42 of the reference (thread-local cuBLAS handles + workspace):
 // same entry points, same "once per rank thread" contract, no cuBLAS.
+#include <atomic>
+#include <mutex>
+
 #include "common.cuh"
 
 namespace pk {
@@ -18,6 +21,31 @@ int sm_count() {
     if (ts.sm_count <= 0) ts.sm_count = 148;
   }
   return ts.sm_count;
+}
+static std::atomic<unsigned int*> g_wait_err{nullptr};
+unsigned int* wait_err_word() { return g_wait_err.load(std::memory_order_acquire); }
+static void make_wait_err_word() {
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  if (wait_err_word()) return;
+  void* p = nullptr;
+  if (cudaHostAlloc(&p, 64, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  memset(p, 0, 64);
+  g_wait_err.store(static_cast<unsigned int*>(p), std::memory_order_release);
+}
+// waits for a barrier that nothing completes, `spins` tries long
+__global__ void wait_probe_kernel(uint32_t spins, unsigned int* err) {
+  __shared__ uint64_t bar;
+  __shared__ int dead;
+  if (threadIdx.x != 0) return;
+  dead = 0;
+  mbar_init(&bar, 1);
+  mbar_fence_init();
+  const WaitFlag wf{&dead, err};
+  mbar_wait_bounded(&bar, 0, wf, spins);
 }
 }  // namespace pk
 
@@ -43,14 +71,7 @@ void cublas_init() {
       ts.scratch_bytes = 0;
     }
   }
-  if (ts.wait_err == nullptr) {
-    if (cudaMalloc(&ts.wait_err, 256) == cudaSuccess) {
-      cudaMemset(ts.wait_err, 0, 256);
-    } else {
-      ts.wait_err = nullptr;
-      cudaGetLastError();
-    }
-  }
+  pk::make_wait_err_word();
   (void)pk::sm_count();
 }
 
@@ -60,10 +81,6 @@ void cublas_destroy() {
     cudaFree(ts.scratch);
     ts.scratch = nullptr;
     ts.scratch_bytes = 0;
-  }
-  if (ts.wait_err != nullptr) {
-    cudaFree(ts.wait_err);
-    ts.wait_err = nullptr;
   }
 }
 
@@ -79,11 +96,18 @@ int64_t pk_b200_launch_count(int reset) {
 }
 
 int pk_b200_wait_errors(void) {
-  pk::ThreadState& ts = pk::tls();
-  unsigned int n = 0;
-  if (ts.wait_err == nullptr) return 0;
-  if (cudaMemcpy(&n, ts.wait_err, sizeof n, cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
-  return (int)n;
+  if (pk::wait_err_word() == nullptr || cudaDeviceSynchronize() != cudaSuccess) return -1;
+  return (int)pk_b200_wait_errors_seen();
+}
+
+unsigned int pk_b200_wait_errors_seen(void) {
+  const volatile unsigned int* w = pk::wait_err_word();
+  return w ? *w : 0u;
+}
+
+int pk_b200_wait_probe(int spins, pk_stream stream) {
+  if (spins <= 0 || spins > 1024 || pk::wait_err_word() == nullptr) return -1;
+  return (int)pk::launch(pk::wait_probe_kernel, dim3(1), dim3(32), 0, stream, false, (uint32_t)spins, pk::wait_err_word());
 }
 
 void pk_b200_set_pdl(int enable) { pk::tls().pdl = enable != 0; }

@@ -53,4 +53,62 @@ def test_the_word_that_counts_reaches_every_limited_wait(path):
         while depth:
             depth += {"(": 1, ")": -1}.get(text[j], 0)
             j += 1
-        assert re.search(r", wf\b[^,]*$", text[m.end():j - 1]), text[m.start():j]
+        assert re.search(r", wf\b", text[m.end():j - 1]), text[m.start():j]
+
+
+REFUSAL = """
+import torch
+from pegainfer_b200 import ffi
+from pegainfer_b200.config import QWEN3_TINY
+from pegainfer_b200.model import ModelRuntimeConfig, Qwen3Model
+from pegainfer_b200.qwen35 import QWEN35_TINY, Qwen35Model, iter_random_weights
+from pegainfer_b200.synthetic import random_weights
+from tests.test_vegodra_gpu import build, cfg_edges, make_weights
+
+lib = ffi.lib()
+assert lib.pk_b200_wait_errors() == -1 and lib.pk_b200_wait_errors_seen() == 0  # nothing is counted before the first cublas_init
+w3 = {k: v.cuda() for k, v in random_weights(QWEN3_TINY, seed=0).items()}
+w35 = {k: v.cuda() for k, v in iter_random_weights(QWEN35_TINY, seed=0)}
+cfg = cfg_edges()
+wv = make_weights(cfg, 1)
+
+
+def make():
+    a, b, c = Qwen3Model(QWEN3_TINY, w3, ModelRuntimeConfig(num_pages=16)), Qwen35Model(QWEN35_TINY, w35, num_pages=16), build(cfg, wv, torch.bfloat16)
+    kv, r35, rv = a.alloc_kv(), b.alloc_request(), c.alloc_request()
+    return (a, b, c), [("qwen3 prefill", lambda: a.prefill([[1, 2, 3]], [kv])), ("qwen3 decode", lambda: a.decode([4], [kv])),
+                       ("qwen3.5 prefill", lambda: b.prefill(r35, [1, 2, 3])), ("qwen3.5 decode", lambda: b.decode(r35, 4)),
+                       ("layer list", lambda: c.step([(rv, [1, 2, 3])]))]
+
+
+old, steps = make()
+for _, s in steps:
+    s()
+assert lib.pk_b200_wait_errors() == 0
+assert lib.pk_b200_wait_probe(0, None) == -1 and lib.pk_b200_wait_probe(4, None) == 0
+assert lib.pk_b200_wait_errors() == 1 and lib.pk_b200_wait_errors_seen() == 1
+for what, s in steps:
+    try:
+        s()
+    except RuntimeError as e:
+        assert "gave up a wait" in str(e), (what, str(e))
+    else:
+        raise AssertionError(what + " was not refused")
+new, steps = make()  # models made afterwards work
+for _, s in steps:
+    s()
+torch.cuda.synchronize()  # and the device does
+for m in old + new:
+    m.close()
+print("refused and served")
+"""
+
+
+@pytest.mark.gpu
+def test_steps_behind_a_run_out_wait_are_refused():
+    """in a process of its own: the count stays"""
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(CSRC))
+    run = subprocess.run([sys.executable, "-c", REFUSAL], cwd=root, env=dict(os.environ, PYTHONPATH=root), capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0 and "refused and served" in run.stdout, run.stdout[-2000:] + run.stderr[-4000:]
