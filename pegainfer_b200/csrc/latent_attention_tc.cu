@@ -325,7 +325,8 @@ int launch_latent_attention_tc(const bf16* qa, const bf16* cache, const bf16* si
                                bf16* out, long page_stride, int page_size, int tokens, int heads, int rank, int rot, float scale, int window,
                                cudaStream_t st) {
   const int D = rank + rot, nc = (D + 63) / 64, halves = (rank / 64 + LT_VC - 1) / LT_VC;
-  if (rank % 64 || D % 8 || nc > LT_MAXC || page_size < 8 || (page_size & (page_size - 1)) || page_stride % 8 || !(scale > 0.f) ||
+  // (rot % 16, rank <= 512: what the mma.sync kernel takes too.  The shapes beyond go to the generic kernel, whose weights stay fp32.)
+  if (rank % 64 || rot % 16 || rank > 512 || nc > LT_MAXC || page_size < 8 || (page_size & (page_size - 1)) || page_stride % 8 || !(scale > 0.f) ||
       ((reinterpret_cast<uintptr_t>(qa) | reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(out)) & 15))
     return -2;
   const long rows = (long)tokens * heads, tiles = (rows + LT_ROWS - 1) / LT_ROWS;

@@ -96,3 +96,27 @@ def test_as_near_to_64_bits_as_the_other_kernel(lib, spread):
         for i in range(2):
             err[i] += (out[i, :, h].double() - want).square().sum().item()
     assert (err[0] / err[1]) ** 0.5 < 1.03, err
+
+
+@pytest.mark.parametrize("rank,rot,H", [(64, 8, 8), (128, 24, 8), (576, 0, 8)])
+def test_shapes_of_the_generic_kernel_keep_its_weights(lib, rank, rot, H):
+    """what the mma.sync kernel does not take (rot off 16, rank above 512) runs with fp32 weights however many the tokens: only the result is rounded"""
+    T, ps, D = 1300, 16, rank + rot
+    g = torch.Generator(device="cuda").manual_seed(D)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    need = (T + ps - 1) // ps
+    cache, qa = torch.zeros(need * ps, D, device="cuda").bfloat16(), (2 * rn(T, H, D)).bfloat16()
+    cache[:T] = rn(T, D).bfloat16()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    pos, req, off, pages = torch.arange(T, device="cuda", dtype=torch.int32), i32([0] * T), i32([0]), i32(list(range(need)))
+    out = torch.zeros(T, H, rank, device="cuda").bfloat16()
+    assert lib.pk_latent_attention_ex(qa.data_ptr(), cache.data_ptr(), None, pos.data_ptr(), req.data_ptr(), off.data_ptr(), pages.data_ptr(), out.data_ptr(),
+                                      ps * D, ps, T, H, rank, rot, D ** -0.5, 0, T, 0, None) == 0
+    torch.cuda.synchronize()
+    hidden = torch.arange(T, device="cuda")[None] > torch.arange(T, device="cuda")[:, None]
+    kd = cache[:T].double()
+    for h in range(H):
+        p = torch.softmax((qa[:, h].double() @ kd.T * D ** -0.5).masked_fill(hidden, -float("inf")), -1)
+        want, size = p @ kd[:, :rank], p @ kd[:, :rank].abs()
+        # scores of a few units from fp32 sums of D products: a weight is off by 2^-18 at most, and so is the sum
+        assert ((out[:, h].double() - want).abs() <= want.abs() * 2 ** -8 + size * 2 ** -16).all()
