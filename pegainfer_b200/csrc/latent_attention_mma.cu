@@ -7,8 +7,9 @@
 //   S   = Q K^T   warp w owns keys [16w, 16w+16) of the tile over the whole feature axis (mma.sync m16n8k16, fp32 acc)
 //   row maxima / sums are exchanged through shared memory, P (bf16) goes to shared memory
 //   O  += P V     V = the first `rank` columns of the same key tile; warp w owns output columns [w*rank/4, (w+1)*rank/4)
-// A tile whose rows belong to several requests walks each request's keys in turn with the other rows masked (their
-// accumulators see p = 0 and a correction of 1).  The sink enters once, at the end (or in the merge of the splits).
+// A tile whose rows belong to several requests walks each request's keys in turn with the other rows masked, from empty accumulators, and writes that
+// request's rows behind it: p = 0 times a NaN of one request's cache never reaches another's rows.  The sink enters once, at the end (or in the merge of
+// the splits).
 // Tensor-bound for prompt portions (2 * rows * keys * (2 rank + rot) flop), HBM/L2-bound for decode (keys * (rank + rot) * 2 B).
 #include "common.cuh"
 #include "mma.cuh"
@@ -61,18 +62,6 @@ latent_attention_mma_kernel(const bf16* __restrict__ qa, const bf16* __restrict_
     row_tok[i] = R < total_rows ? R / heads : -1;
     row_pos[i] = row_tok[i] >= 0 ? pos[row_tok[i]] : -1;
   }
-  float m_run[NR], l_run[NR];
-#pragma unroll
-  for (int i = 0; i < NR; ++i) {
-    m_run[i] = kNegBig;
-    l_run[i] = 0.f;
-  }
-  float o[MT][NV][4];
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-    for (int i = 0; i < NV; ++i) o[mt][i][0] = o[mt][i][1] = o[mt][i][2] = o[mt][i][3] = 0.f;
-
   const int t_first = R0 / heads, t_last = (min(total_rows, R0 + ROWS) - 1) / heads;
   int t = t_first;
   while (t <= t_last) {
@@ -86,6 +75,18 @@ latent_attention_mma_kernel(const bf16* __restrict__ qa, const bf16* __restrict_
     bool act[NR];
 #pragma unroll
     for (int i = 0; i < NR; ++i) act[i] = row_tok[i] >= t && row_tok[i] <= t_end;
+
+    float m_run[NR], l_run[NR];
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      m_run[i] = kNegBig;
+      l_run[i] = 0.f;
+    }
+    float o[MT][NV][4];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int i = 0; i < NV; ++i) o[mt][i][0] = o[mt][i][1] = o[mt][i][2] = o[mt][i][3] = 0.f;
 
     auto load_keys = [&](int j0, int buf) {
       bf16* base = Ks + (size_t)buf * kMmaKeys * ldk;
@@ -224,37 +225,36 @@ latent_attention_mma_kernel(const bf16* __restrict__ qa, const bf16* __restrict_
         }
       }
     }
+    // ---- write: final rows (one split) or partial state (several)
+    const int wcol0 = warp * (rank / 4);
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      const int r = rb + g + 8 * i, R = R0 + r, mt = i >> 1, hf = i & 1;
+      if (!act[i]) continue;
+      if (nsplit == 1) {
+        const float sk = sink ? bf2f(sink[R % heads]) : kNegBig;
+        const float M = fmaxf(m_run[i], sk);
+        const float w = __expf(m_run[i] - M);
+        const float inv = w / (l_run[i] * w + (sink ? __expf(sk - M) : 0.f));
+#pragma unroll
+        for (int n = 0; n < NV; ++n)
+          if (n < nv)
+            *reinterpret_cast<uint32_t*>(out + (size_t)R * rank + wcol0 + n * 8 + 2 * tq) = pack_bf16(o[mt][n][2 * hf] * inv, o[mt][n][2 * hf + 1] * inv);
+      } else {
+        const size_t slot = ((size_t)blockIdx.x * nsplit + split) * ROWS + r;
+        if (warp == 0 && tq == 0) {
+          part_ml[slot * 2] = m_run[i];
+          part_ml[slot * 2 + 1] = l_run[i];
+        }
+#pragma unroll
+        for (int n = 0; n < NV; ++n)
+          if (n < nv) *reinterpret_cast<float2*>(part_o + slot * rank + wcol0 + n * 8 + 2 * tq) = make_float2(o[mt][n][2 * hf], o[mt][n][2 * hf + 1]);
+      }
+    }
     __syncthreads();  // the next request's first load reuses buffer 0
     t = t_end + 1;
   }
   cp_async_wait_all();  // a tile with no keys in this split still waits for its Q copy
-
-  // ---- write: final rows (one split) or partial state (several)
-  const int vcol0 = warp * (rank / 4);
-#pragma unroll
-  for (int i = 0; i < NR; ++i) {
-    const int r = rb + g + 8 * i, R = R0 + r, mt = i >> 1, hf = i & 1;
-    if (R >= total_rows) continue;
-    if (nsplit == 1) {
-      const float sk = sink ? bf2f(sink[R % heads]) : kNegBig;
-      const float M = fmaxf(m_run[i], sk);
-      const float w = __expf(m_run[i] - M);
-      const float inv = w / (l_run[i] * w + (sink ? __expf(sk - M) : 0.f));
-#pragma unroll
-      for (int n = 0; n < NV; ++n)
-        if (n < nv)
-          *reinterpret_cast<uint32_t*>(out + (size_t)R * rank + vcol0 + n * 8 + 2 * tq) = pack_bf16(o[mt][n][2 * hf] * inv, o[mt][n][2 * hf + 1] * inv);
-    } else {
-      const size_t slot = ((size_t)blockIdx.x * nsplit + split) * ROWS + r;
-      if (warp == 0 && tq == 0) {
-        part_ml[slot * 2] = m_run[i];
-        part_ml[slot * 2 + 1] = l_run[i];
-      }
-#pragma unroll
-      for (int n = 0; n < NV; ++n)
-        if (n < nv) *reinterpret_cast<float2*>(part_o + slot * rank + vcol0 + n * 8 + 2 * tq) = make_float2(o[mt][n][2 * hf], o[mt][n][2 * hf + 1]);
-    }
-  }
 }
 
 // one block per query row: combine the splits' (m, l, O) and the sink

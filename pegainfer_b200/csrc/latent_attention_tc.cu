@@ -10,8 +10,9 @@
 //             made the result's error 1.2 times as large for peaked scores)
 //   warp 4    MMA issuer     S = Q K^T (SS),  O += P V (A from TMEM, V = the key chunks read N-major)
 //   warp 5    TMA: Q once, then the pages of every key block
-// A tile whose rows belong to several requests walks each request's keys in turn with the other rows masked.  Keys outside the run (slots behind the
-// context's end, keys before the window) are masked in S, and their value rows are cleared in shared memory before P V: they may hold anything.
+// A tile whose rows belong to several requests walks each request's keys in turn with the other rows masked, starts O anew for each and writes that
+// request's rows behind it: what another request's cache holds (a NaN times a weight of zero) never reaches them.  Keys outside the run (slots behind
+// the context's end, keys before the window) are masked in S, and their value rows are cleared in shared memory before P V: they may hold anything.
 // Tensor-bound (operand reads of the narrow MMAs): 2 * rows * keys * (2 rank + rot) flop of result, 1.5 times that executed at rank 512.
 #include <cuda.h>
 
@@ -184,15 +185,19 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         if (x1 == a.nc) umma_commit(m.s_full + (n & 1));
       };
       mbar_wait_bounded(&m.q_full, 0, wf);
-      issue_s(0, 0, a.nc);
+      if (total_blocks > 0) issue_s(0, 0, a.nc);
+      uint32_t run_end = 0;  // block at which the next run starts
+      int run = 0;
       const uint64_t vd = make_sw128_mn_desc(smem_u32(Ks + (size_t)vc0 * LT_KC), LT_KC, 1024);
       for (uint32_t n = 0; n < total_blocks; ++n) {
         if (n + 1 < total_blocks) issue_s(n + 1, 0, n_other);
         mbar_wait_bounded(m.p_ready + (n & 1), (n >> 1) & 1, wf);
         tc_fence_after();
+        const bool anew = n == run_end;
+        while (n == run_end) run_end += blocks_of(m.runs[run++]);
 #pragma unroll
         for (int k = 0; k < LT_KEYS / 16; ++k)
-          umma_bf16_tmem_a(tmem + 256, tmem + (n & 1) * LT_KEYS + (uint32_t)(k * 8), vd + (uint64_t)(k * (2048 >> 4)), idesc_pv, (n > 0 || k > 0) ? 1u : 0u);
+          umma_bf16_tmem_a(tmem + 256, tmem + (n & 1) * LT_KEYS + (uint32_t)(k * 8), vd + (uint64_t)(k * (2048 >> 4)), idesc_pv, (!anew || k > 0) ? 1u : 0u);
         for (int c = vc0; c < vc0 + nvc; ++c) umma_commit(m.k_empty + c);
         umma_commit(&m.pv_done);
         if (n + 1 < total_blocks) issue_s(n + 1, n_other, a.nc);
@@ -208,12 +213,12 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
     const int tok = R < total ? R / a.heads - t_first : -1, my_pos = tok >= 0 ? m.tok_pos[tok] : -1;
     const int my_lo = a.window > 0 ? my_pos - a.window + 1 : 0;
     const uint32_t t_lane = tmem + ((uint32_t)(warp * 32) << 16), t_o = t_lane + 256;
-    float mx = -INFINITY, l = 0.f;  // running maximum (scaled, log2 units) and sum
     uint32_t n = 0;
     for (int i = 0; i < n_runs; ++i) {
       const LtRun r = m.runs[i];
       const bool act = tok >= r.t0 && tok <= r.t1;
       const int nb = blocks_of(r);
+      float mx = -INFINITY, l = 0.f;  // running maximum (scaled, log2 units) and sum
       for (int b = 0; b < nb; ++b, ++n) {
         const int j0 = r.k0 + b * LT_KEYS;
         mbar_wait_bounded(m.s_full + (n & 1), (n >> 1) & 1, wf);
@@ -243,7 +248,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
           const float to = grow ? blk : mx, corr = grow ? lt_exp2(mx - to) : 1.f;
           mx = to;
           l *= corr;
-          if (n > 0) {  // O holds the blocks before this one
+          if (b > 0) {  // O holds the blocks before this one
             mbar_wait_bounded(&m.pv_done, (n - 1) & 1, wf);
             __syncwarp();
             tc_fence_after();
@@ -286,28 +291,31 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         tc_fence_before();
         mbar_arrive(m.p_ready + (n & 1));
       }
-    }
-    // ---- O / l -> bf16
-    mbar_wait_bounded(&m.pv_done, (n - 1) & 1, wf);
-    __syncwarp();
-    tc_fence_after();
-    const float sk = a.sink && tok >= 0 ? bf2f(a.sink[R % a.heads]) * 1.4426950408889634f : -INFINITY;
-    const float M = fmaxf(mx, sk), w = lt_exp2(mx - M);
-    const float inv = tok >= 0 ? w / (l * w + (a.sink ? lt_exp2(sk - M) : 0.f)) : 0.f;
-    uint4* dst = reinterpret_cast<uint4*>(a.out + (size_t)(tok >= 0 ? R : 0) * a.rank + vc0 * 64);
-    for (int c = 0; c < nvc * 64; c += 64) {
-      uint32_t t[64];
-      tmem_ld32_nowait(t_o + c, t);
-      tmem_ld32_nowait(t_o + c + 32, t + 32);
-      tmem_ld_wait64(t);
-      if (tok >= 0) {
+      // ---- O / l -> bf16, the rows of this run (the next one's first P V waits for all 128 threads' next p_ready)
+      if (nb > 0) mbar_wait_bounded(&m.pv_done, (n - 1) & 1, wf);
+      __syncwarp();
+      tc_fence_after();
+      const float sk = a.sink && act ? bf2f(a.sink[R % a.heads]) * 1.4426950408889634f : -INFINITY;
+      const float M = fmaxf(mx, sk), w = lt_exp2(mx - M);
+      const float inv = w / (l * w + (a.sink ? lt_exp2(sk - M) : 0.f));
+      uint4* dst = reinterpret_cast<uint4*>(a.out + (size_t)(act ? R : 0) * a.rank + vc0 * 64);
+      for (int c = 0; c < nvc * 64; c += 64) {
+        uint32_t t[64] = {};
+        if (nb > 0) {  // no visible key at all (a position before the first): O is zero, as the sum is
+          tmem_ld32_nowait(t_o + c, t);
+          tmem_ld32_nowait(t_o + c + 32, t + 32);
+          tmem_ld_wait64(t);
+        }
+        if (act) {
 #pragma unroll
-        for (int x = 0; x < 64; x += 8)
-          dst[(c + x) >> 3] = make_uint4(pack_bf16(__uint_as_float(t[x]) * inv, __uint_as_float(t[x + 1]) * inv),
-                                         pack_bf16(__uint_as_float(t[x + 2]) * inv, __uint_as_float(t[x + 3]) * inv),
-                                         pack_bf16(__uint_as_float(t[x + 4]) * inv, __uint_as_float(t[x + 5]) * inv),
-                                         pack_bf16(__uint_as_float(t[x + 6]) * inv, __uint_as_float(t[x + 7]) * inv));
+          for (int x = 0; x < 64; x += 8)
+            dst[(c + x) >> 3] = make_uint4(pack_bf16(__uint_as_float(t[x]) * inv, __uint_as_float(t[x + 1]) * inv),
+                                           pack_bf16(__uint_as_float(t[x + 2]) * inv, __uint_as_float(t[x + 3]) * inv),
+                                           pack_bf16(__uint_as_float(t[x + 4]) * inv, __uint_as_float(t[x + 5]) * inv),
+                                           pack_bf16(__uint_as_float(t[x + 6]) * inv, __uint_as_float(t[x + 7]) * inv));
+        }
       }
+      tc_fence_before();
     }
   }
   tc_fence_before();

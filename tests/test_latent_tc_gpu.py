@@ -120,3 +120,55 @@ def test_shapes_of_the_generic_kernel_keep_its_weights(lib, rank, rot, H):
         want, size = p @ kd[:, :rank], p @ kd[:, :rank].abs()
         # scores of a few units from fp32 sums of D products: a weight is off by 2^-18 at most, and so is the sum
         assert ((out[:, h].double() - want).abs() <= want.abs() * 2 ** -8 + size * 2 ** -16).all()
+
+
+@pytest.mark.parametrize("H,ps", [(16, 16), (10, 64)])
+@pytest.mark.parametrize("sink", [False, True])
+def test_what_another_requests_cache_holds_stays_there(lib, H, ps, sink):
+    """a request whose visible keys are NaN beside others in the same 128-row tiles: their rows are those of a call where it is sound"""
+    rank, rot, lens = 512, 64, [290, 3, 309]
+    D, T = rank + rot, sum(lens)
+    g = torch.Generator(device="cuda").manual_seed(H)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    need = [(n + ps - 1) // ps for n in lens]
+    cache, qa, sk = rn(sum(need) * ps, D).bfloat16(), rn(T, H, D).bfloat16(), rn(H).bfloat16()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    off = [sum(need[:i]) for i in range(3)]
+    pos, req = i32([j for n in lens for j in range(n)]), i32([r for r, n in enumerate(lens) for _ in range(n)])
+    off_d, pages = i32(off), i32(list(range(sum(need))))
+
+    def run(c):
+        out = torch.zeros(T, H, rank, device="cuda").bfloat16()
+        assert lib.pk_latent_attention_ex(qa.data_ptr(), c.data_ptr(), sk.data_ptr() if sink else None, pos.data_ptr(), req.data_ptr(), off_d.data_ptr(),
+                                          pages.data_ptr(), out.data_ptr(), ps * D, ps, T, H, rank, rot, D ** -0.5, 0, max(lens), 0, None) == 0
+        torch.cuda.synchronize()
+        return out
+
+    sound = run(cache)
+    assert torch.isfinite(sound).all()
+    for bad in range(3):
+        c = cache.clone()
+        c[off[bad] * ps:(off[bad] + need[bad]) * ps, :64] = float("nan")
+        got, row = run(c), 0
+        for r, n in enumerate(lens):
+            if r != bad:
+                assert torch.equal(got[row:row + n], sound[row:row + n]), (bad, r)
+            else:
+                assert torch.isnan(got[row:row + n, :, :64]).all()
+            row += n
+
+
+def test_rows_without_a_visible_key(lib):
+    """positions before the first key, whole tiles of them and some beside others: a row of zeros with a sink (the other kernels' result)"""
+    T, H, rank, rot, ps = 600, 16, 512, 64, 16
+    D = rank + rot
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    cache, qa, sk = rn(304 * ps, D).bfloat16(), rn(T, H, D).bfloat16(), rn(H).bfloat16()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    pos, req = i32([-1] * 300 + list(range(300))), i32([0] * 300 + [1] * 300)
+    off, pages, out = i32([0, 2]), i32(list(range(304))), torch.full((T, H, rank), 3.0, device="cuda").bfloat16()
+    assert lib.pk_latent_attention_ex(qa.data_ptr(), cache.data_ptr(), sk.data_ptr(), pos.data_ptr(), req.data_ptr(), off.data_ptr(), pages.data_ptr(),
+                                      out.data_ptr(), ps * D, ps, T, H, rank, rot, D ** -0.5, 0, 300, 0, None) == 0
+    torch.cuda.synchronize()
+    assert (out[:300] == 0).all() and torch.isfinite(out[300:]).all() and (out[300:] != 0).any(-1).all() and lib.pk_b200_wait_errors() == 0
