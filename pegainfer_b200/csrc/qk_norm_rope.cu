@@ -38,11 +38,11 @@ __global__ void __launch_bounds__(128) qk_norm_rope_kernel(bf16* __restrict__ q,
     raw[i] = 2 * i + half < HEADS && head < heads ? piece(row_of(head), lane) : make_uint4(0, 0, 0, 0);
   }
   // table layout [pos*128 + i] duplicated for i and i+64 (weight_loader.rs:210-244)
-  float c[8], s[8], wq[8], wk[8];
+  float c[8], s[8], wq[8] = {}, wk[8] = {};
   unpack(piece(cosc + (size_t)pos * HD, lane & 7), c);
   unpack(piece(sinc + (size_t)pos * HD, lane & 7), s);
-  unpack(piece(qw, lane), wq);
-  unpack(piece(kw, lane), wk);
+  if (nq > 0) unpack(piece(qw, lane), wq);  // a call without query (key) heads may come without their weights
+  if (nkv > 0) unpack(piece(kw, lane), wk);
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     const int head = head0 + 2 * i + half;

@@ -81,6 +81,20 @@ def test_qk_norm_rope(lib, tokens, nq, nkv, shift):
         assert ((x.double() - y).abs() <= y.abs() * ULP + 1e-30).double().mean() > 0.98
 
 
+@pytest.mark.parametrize("tokens", [1, 9, 800])
+def test_qk_norm_rope_without_one_kind_of_heads(lib, tokens):
+    """no key heads (or no query heads) and null pointers in their place: the other kind's rows are those of the full call"""
+    n, eps = 5, 1e-6
+    q, k, qw, kw = rnd(20, tokens, n, 128), rnd(21, tokens, n, 128), rnd(22, 128), rnd(23, 128)
+    cos, sin = rnd(24, tokens, 128), rnd(25, tokens, 128)
+    a, b, c, d = q.clone(), k.clone(), q.clone(), k.clone()
+    lib.prefill_qk_norm_rope_only_cuda(a.data_ptr(), b.data_ptr(), qw.data_ptr(), kw.data_ptr(), cos.data_ptr(), sin.data_ptr(), n, n, 128, tokens, 0, eps, None)
+    lib.prefill_qk_norm_rope_only_cuda(c.data_ptr(), None, qw.data_ptr(), None, cos.data_ptr(), sin.data_ptr(), n, 0, 128, tokens, 0, eps, None)
+    lib.prefill_qk_norm_rope_only_cuda(None, d.data_ptr(), None, kw.data_ptr(), cos.data_ptr(), sin.data_ptr(), 0, n, 128, tokens, 0, eps, None)
+    torch.cuda.synchronize()
+    assert torch.equal(a, c) and torch.equal(b, d)
+
+
 @pytest.mark.parametrize("shift", [0, 4])
 @pytest.mark.parametrize("C", [8, 1032, 20])
 @pytest.mark.parametrize("T", [1, 2, 3, 15, 16, 17, 50])
