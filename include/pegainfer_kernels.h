@@ -192,7 +192,8 @@ void pk_b200_set_pdl(int enable);
 
 /* Tensor-core GEMM with up to three output segments (the fused q|k|v projection of prefill):
  * rows [0, seg_rows[0]) of W -> Y[0] (a HiddenStates [seg_rows[0], N]), the next seg_rows[1] -> Y[1], the
- * rest -> Y[2].  seg_rows must sum to M.  Same arithmetic as gemm_cuda. */
+ * rest -> Y[2].  seg_rows must sum to M.  Same arithmetic as gemm_cuda; from 129 tokens on, with K < 8192 and 64 or more features per segment, also
+ * bit for bit what a gemm_cuda call per segment gives (elsewhere the order of the sums over K may follow from M). */
 int pk_b200_gemm_segments(const pk_bf16* W, const pk_bf16* X, pk_bf16* const* Y, const int* seg_rows, int M, int N,
                           int K, pk_stream stream);
 

@@ -262,14 +262,16 @@ struct SkPlan {
 
 // The most K parts for which all tiles run at once, and the lowest tiles for which they still do, so that every SM has the same share of W.
 // Beyond 128 tokens gemm2.cu is the faster one as soon as its CTA pairs (256 tokens x 128 features each) are half in use; here -> gemm2.cu, us:
-// 2560 x 4096 18.9 -> 21.0 at 160 tokens, but 24.5 -> 21.1 at 400;  2560 x 9728 25.2 -> 35.1 and 37.4 -> 35.3;  4096 x 12288 43.2 -> 49.8 and 58.5 -> 51.3;
-// 6144 x 2560 19.2 -> 15.1 at 160.  Parts follow from K there (4 from 4096 on, where they fit, else 2), and a short K comes here for one feature tile only
-// (32 x 2560: 10.4 us at 160 tokens, 14.5 without parts), so that the projections that one call stacks and that three calls make one by one take the same
-// kernel and add up in the same order.
+// 2560 x 9728 25.2 -> 35.1 at 160 tokens and 37.4 -> 35.3 at 400;  4096 x 12288 43.2 -> 49.8 and 58.5 -> 51.3;  6144 x 2560 19.2 -> 15.1 at 160.
+// But gemm2.cu adds up over K in one go and this kernel in parts, and what a stack of projections gets in one call and each of them in a call of its own
+// is the same, bit for bit, only if both take the same kernel (pk_b200_gemm_segments promises it from 129 tokens on).  The number of features must not
+// decide, then, wherever it could differ between the two: only reductions of 8192 or more (they come from a feed-forward's inner width; projections are
+// stacked over the hidden width) and fewer than 64 features (gates of a head each, no head's row is so short) come here.  What that gives up at 160
+// tokens: 2560 x 4096 18.9 -> 21.0.  Parts follow from K (4 from 4096 on, where they fit, else 2; 32 x 2560: 10.4 us, 14.5 in gemm2.cu).
 // Measured on B200, us a launch in a train over cold weights (before: the split-K form of gemm.cu; from 129 tokens on gemm2.cu), M x K:
 //   tokens            8            48           128          160
 //   6144 x 2560   20.1 -> 9.5  19.9 -> 10.4  24.9 -> 12.6     (gemm2)
-//   2560 x 4096   15.9 -> 8.2  15.9 -> 9.2   18.7 -> 11.4  29.8 -> 12.6
+//   2560 x 4096   15.9 -> 8.2  15.9 -> 9.2   18.7 -> 11.4     (gemm2)
 //   2560 x 9728   20.0 -> 13.1 20.6 -> 13.5  23.5 -> 16.3  61.2 -> 20.5
 //   19456 x 2560  31.3 -> 20.2 23.5 -> 21.2     (gemm.cu)     (gemm2)
 //   24576 x 4096  49.1 -> 37.1 43.2 -> 38.6     (gemm.cu)     (gemm2)
@@ -294,11 +296,13 @@ SkPlan sk_plan(int M, int N, int K, int nt, int sms) {
   return SkPlan{0, 1, 0};
 }
 
+bool sk_many_tokens(int M, int N, int K, int sms) { return M < 64 || (K >= 8192 && (long)((N + 255) / 256) * ((M + 127) / 128) * 4 <= sms); }
+
 template <int NT>
 int sk_run(const bf16* W, const bf16* X, bf16* Y, bf16* Y1, bf16* Y2, int e0, int e1, int M, int N, int K, cudaStream_t stream) {
   const SkPlan p = sk_plan(M, N, K, NT, sm_count());
   if (p.rows == 0 || (p.splits == 1 && (N > 128 || (N > 64 && M > SK_BM * sm_count())))) return -2;
-  if (N > 128 && (K < 4096 ? M > SK_BM : (long)((N + 255) / 256) * ((M + 127) / 128) * 4 > sm_count())) return -2;
+  if (N > 128 && !sk_many_tokens(M, N, K, sm_count())) return -2;
   const int n_tiles = (N + NT - 1) / NT, tiles = ((M + p.rows - 1) / p.rows) * n_tiles;
   CUtensorMap mx, mw;
   if (!sk_make_map(&mx, X, N, K, NT) || !sk_make_map(&mw, W, M, K, p.rows)) return -2;

@@ -674,7 +674,7 @@ bool Qwen3Model::unified_step(int n_req, const uint32_t* tokens, const int* lens
     TransformerBlock& L = layers[li];
     k.rms_norm_batched_cuda(hcur, L.input_layernorm.data.bf(), nrm.data.bf(), H, T, eps, st);
     if (rt.mode >= 1 && k.pk_b200_gemm_segments && T > 1) {
-      // one tensor-core launch over the stacked [q;k;v] weight, three outputs (same arithmetic)
+      // one tensor-core launch over the stacked [q;k;v] weight, three outputs (bit for bit the three launches' from 129 tokens on)
       pk_bf16* outs[3] = {qb.data.bf(), kb.data.bf(), vb.data.bf()};
       const int segs[3] = {qd, kd, kd};
       if (k.pk_b200_gemm_segments(L.attention.qkv_proj.data.bf(), nrm.data.bf(), outs, segs, qd + 2 * kd, T, H, st) != 0)
@@ -979,7 +979,7 @@ bool Qwen3Model::decode_kernels_fused(int bs) {
 }
 
 // B200 path for the reference's decode buckets above 4 requests (batch_decode_buffers.rs:12: 8, 16, 32, 64): the
-// projections run on the tensor cores (skinny split-K GEMM: every SM streams a K slice of the weights), norms stay
+// projections run on the tensor cores (gemm_skinny.cu: every SM streams a share of the weights), norms stay
 // separate launches over [H, bs], QK-norm + RoPE + KV append + attention + merge is the one fused attention launch over
 // all requests (cluster size shrinks with the batch), and every row's greedy token is taken inside the graph.
 // Same rounding points as decode_kernels_compat (it IS that op sequence with three fusions).

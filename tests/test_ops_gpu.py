@@ -513,6 +513,26 @@ def test_gemm_segments_matches_three_gemms():
     assert_bf16_close(bits(outs[0]), want, 1, floor=float(np.abs(f32(want)).max()) / 64, frac_exact=0.9)
 
 
+@pytest.mark.parametrize("T", [129, 160, 256, 257, 700])
+@pytest.mark.parametrize("segs,H", [((4096, 1024, 1024), 4096), ((512, 128, 128), 2560), ((512, 64, 64), 4096), ((4096, 1024, 1024), 5120), ((1000, 64, 300), 8184)])
+def test_gemm_segments_are_the_single_calls_bit_for_bit(segs, H, T):
+    """what the header promises from 129 tokens on: hidden widths around and above 4096, one key / value head of a shard, odd sizes"""
+    lib = get_lib("b200")
+    import ctypes as C
+    g = torch.Generator(device="cuda").manual_seed(H + T)
+    W = torch.randn(sum(segs), H, generator=g, device="cuda").mul_(0.02).bfloat16()
+    X = torch.randn(T, H, generator=g, device="cuda").bfloat16()
+    outs = [torch.zeros((T, n), dtype=torch.bfloat16, device="cuda") for n in segs]
+    assert lib.pk_b200_gemm_segments(p(W), p(X), (C.c_void_p * 3)(*[o.data_ptr() for o in outs]), (C.c_int * 3)(*segs), sum(segs), T, H, stream()) == 0
+    row = 0
+    for o, n in zip(outs, segs):
+        ref = torch.zeros((T, n), dtype=torch.bfloat16, device="cuda")
+        lib.gemm_cuda(W.data_ptr() + row * H * 2, p(X), p(ref), n, T, H, stream())
+        torch.cuda.synchronize()
+        assert torch.equal(o, ref)
+        row += n
+
+
 @pytest.mark.parametrize("N", [1, 3])
 def test_gemv_fused_prologue_epilogue(N):
     """x_mode 1 (residual add + RMSNorm prologue) with three output segments, then epi 1 (SwiGLU)."""
