@@ -138,7 +138,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    // by elect.sync, not by `lane == 0`: the descriptors are uniform registers, which a thread picked by its lane fills through a vote per instruction
+    // the issuing thread by elect.sync; picked by `lane == 0` a K block took longer (measured in gemm2.cu)
     if (tc_elect_one()) {
       // instruction descriptor: D=f32 [4,6)=1, A=bf16 [7,10)=1, B=bf16 [10,13)=1, K-major both, N>>3 at [17,23), M>>4 at [24,29)
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);

@@ -19,8 +19,8 @@
 // of the up block (peer CTA) of the stacked [gate; up] weight, so columns [0,128) / [128,256) of every accumulator row
 // are gate / up of one feature: the epilogue writes bf16(silu(bf16(g)) * bf16(u)) (csrc/fused_proj.cu:44-63 rounding)
 // and the separate SiLU-mul pass over 2*I*T elements disappears.
-// The MMA issuer and the producer are threads chosen by elect.sync: picked by `lane == 0` they filled the descriptors' uniform registers through a vote
-// per instruction, and a K block took 0.42 us whatever the tile's width.  B200, us a launch over cold weights, before -> after (2048 tokens):
+// The MMA issuer and the producer are threads chosen by elect.sync: with threads picked by `lane == 0` a K block took 0.42 us whatever the tile's width.
+// B200, us a launch over cold weights, before -> after (2048 tokens):
 // 6144 x 2560 59.5 -> 48.4, 2560 x 4096 45.6 -> 37.5, 2560 x 9728 88.8 -> 74.3, 4096 x 12288 160.6 -> 144.1.
 // The gated epilogue evaluates its 32 columns side by side, on two warps per lane quarter; one after the other (a branch on the activation per
 // element) a tile's epilogue took 26 us and set the pace: 9728 x 2560 gated 253 -> 154, 12288 x 4096 gated (3001 tokens) 557 -> 433.
@@ -174,7 +174,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    // by elect.sync, not by `lane == 0`: the descriptors are uniform registers, which a thread picked by its lane fills through a vote per instruction
+    // by elect.sync, not by `lane == 0` (see the head of this file)
     if (leader && tc_elect_one()) {
       // instruction descriptor: D=f32 [4,6)=1, A=bf16 [7,10)=1, B=bf16 [10,13)=1, K-major both, N>>3 at [17,23), M>>4 at [24,29)
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);

@@ -104,8 +104,7 @@ __device__ __forceinline__ uint64_t make_sw128_mn_desc(uint32_t smem_addr, uint3
   d |= (uint64_t)2 << 61;
   return d;
 }
-// one lane of the (converged) warp; the compiler knows a single thread is active under this predicate, so the uniform-register operands of
-// tcgen05.mma / commit need no per-thread loop (unlike `lane == 0`)
+// one lane of the (converged) warp: the form to choose the thread that issues tcgen05.mma, commits and TMA copies (gemm2.cu has what `lane == 0` cost)
 __device__ __forceinline__ bool tc_elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));

@@ -30,7 +30,7 @@ from tests.helpers import bits, logits_agree, oracle_cfg
 pytestmark = [pytest.mark.gpu,
               pytest.mark.skipif(os.environ.get("PK_SKIP_FULLSIZE") == "1", reason="PK_SKIP_FULLSIZE=1")]
 
-# bf16 ulps at the row's max |logit| after 36 layers.  Measured on B200 (gpurun_out/c1_pytest.log, profiles/README.md):
+# bf16 ulps at the row's max |logit| after 36 layers.  Measured on B200 (profiles/README.md):
 # fused 7.4 worst over 65 steps of config 1, 5.4 on config 2; compat 5.9 / 5.0 -- rounding-point flips accumulate as
 # ~sqrt(layers) (the 2-4 layer configs of test_model_gpu.py sit at <= 2 with a bound of 6).  12 = 1.6 x the worst seen.
 TOL_ULP = 12

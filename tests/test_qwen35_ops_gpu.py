@@ -1,8 +1,6 @@
 """GPU parity of the Qwen3.5 hybrid-layer ops (pegainfer_b200/csrc/qwen35_ops.cu) against oracle/qwen35_oracle.py.
 
-First hardware run: round 2, session 1 (gpurun_out/c1_q35_tests.log: 12 passed on B200; the token-by-token hybrid
-forward of tests/tools/qwen35_bringup.py matches the oracle within 2.25 ulp at the row max over 24 steps) -- the
-round-1 opt-in gate is gone."""
+On a B200 the token-by-token hybrid forward of tests/tools/qwen35_bringup.py matches the oracle within 2.25 ulp at the row max over 24 steps."""
 import math
 import os
 

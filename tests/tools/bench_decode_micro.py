@@ -13,7 +13,7 @@ sweep), captured into ONE CUDA graph so no host launch gap sits between them, on
 per-launch time = total / N.  For our library it is reported with programmatic dependent launch off and on (on = what
 the decode graph runs: the next launch's weight / KV requests overlap this one's tail).
 
-Prints one JSON object; `python tests/tools/bench_decode_micro.py > gpurun_out/micro.json`.
+Prints one JSON object.
 """
 import json
 import math
