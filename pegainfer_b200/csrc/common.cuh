@@ -4,6 +4,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -31,6 +32,19 @@ int sm_count();
 // The word that counts waits that ran out (mbar_wait_bounded), in mapped host memory: one per process, made by the first cublas_init and kept, so that a
 // captured graph may hold it and any thread may read it after a synchronisation of its own.  Null before that.
 unsigned int* wait_err_word();
+
+// More dynamic shared memory than 48 KB for `kernel`: an attribute of the kernel on the current device, set by the first thread that launches it there.
+// `done` is the kernel's own (one bit per device); a failure is the caller's to return, and the next launch tries again.
+inline cudaError_t allow_smem(std::atomic<uint64_t>& done, const void* kernel, size_t bytes) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = 1ull << (dev & 63);
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
+}
 
 // Launch with optional programmatic dependent launch (PDL).  Kernels that opt in call
 // pdl_wait() before touching data produced by the previous kernel in the stream.

@@ -228,11 +228,8 @@ bool sk_make_map(CUtensorMap* map, const void* base, int rows, int K, int box_ro
 template <int NT>
 cudaError_t sk_launch(const CUtensorMap& mx, const CUtensorMap& mw, const SkArgs& a, int tiles, int splits, cudaStream_t stream) {
   auto kern = gemm_skinny_kernel<NT>;
-  static thread_local bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX) != cudaSuccess) return cudaErrorInvalidValue;
-    configured = true;
-  }
+  static std::atomic<uint64_t> smem_set{0};
+  if (const cudaError_t e = allow_smem(smem_set, (const void*)kern, SK_SMEM_MAX); e != cudaSuccess) return e;
   ThreadState& ts = tls();
   ts.launches++;
   cudaLaunchConfig_t cfg{};

@@ -357,14 +357,10 @@ int launch_latent_attention_tc(const bf16* qa, const bf16* cache, const bf16* si
       return -2;
   }
   const size_t smem = (size_t)nc * (LT_QC + LT_KC) + sizeof(LtSmem) + 1024;
-  static thread_local bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(latent_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_MAXC * (LT_QC + LT_KC) + (int)sizeof(LtSmem) + 1024) !=
-        cudaSuccess) {
-      cudaGetLastError();
-      return -2;
-    }
-    configured = true;
+  static std::atomic<uint64_t> smem_set{0};
+  if (allow_smem(smem_set, (const void*)latent_attention_tc_kernel, LT_MAXC * (LT_QC + LT_KC) + sizeof(LtSmem) + 1024) != cudaSuccess) {
+    cudaGetLastError();
+    return -2;
   }
   const LtArgs a{sink, pos, req, page_off, pages, out, page_size, tokens, heads, rank, nc, halves, window, scale * 1.4426950408889634f, wait_err_word()};
   return (int)launch(latent_attention_tc_kernel, dim3((unsigned)(tiles * halves)), dim3(LT_THREADS), smem, st, true, mq, mk, a);

@@ -375,12 +375,8 @@ static cudaError_t mg_launch(const void* rows, long n_rows, const void* w, const
   CUtensorMap mx, mw;
   if (!mg_map(&mx, rows, n_rows, a.K, 64) || !mg_map(&mw, w, (long)a.experts * a.N, a.K, 128)) return cudaErrorInvalidValue;
   auto kern = moe_grouped_gemm_kernel<EPI>;
-  static thread_local bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMgSmem);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static std::atomic<uint64_t> smem_set{0};
+  if (const cudaError_t e = allow_smem(smem_set, (const void*)kern, kMgSmem); e != cudaSuccess) return e;
   // as many CTAs as there can be tiles, one per SM at most
   const long tiles = (n_rows / kMoeTile + (n_rows < a.experts ? n_rows : a.experts)) * ((a.N + 127) / 128);
   return launch(kern, dim3((unsigned)(tiles < sm_count() ? tiles : sm_count())), dim3(kMgThreads), kMgSmem, st, true, mx, mw, a);

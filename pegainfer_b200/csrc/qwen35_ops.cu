@@ -404,12 +404,8 @@ int pk_b200_gated_delta_rule_prefill_recurrent(const pk_bf16* qkv_seq, const pk_
   if (key_dim != GK || val_dim != GV || num_value_heads <= 0 || num_key_heads <= 0) return -1;
   if (seq_len <= 0) return 0;
   constexpr size_t smem = DcSmem<GK, GC>::BYTES;
-  static thread_local bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(gated_delta_rule_seq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static std::atomic<uint64_t> smem_set{0};
+  if (const cudaError_t e = allow_smem(smem_set, (const void*)gated_delta_rule_seq_kernel, smem); e != cudaSuccess) return (int)e;
   return (int)launch(gated_delta_rule_seq_kernel, dim3(num_value_heads, GV / GC), dim3(kDcThreads), smem, stream, true, (const bf16*)qkv_seq,
                      (const bf16*)b_seq, (const bf16*)a_seq, (const bf16*)dt_bias, A_log, state, (bf16*)out_seq, num_key_heads, num_value_heads,
                      seq_len, wait_err_word());

@@ -544,42 +544,37 @@ __global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_kernel(SeqArgs a, b
 }
 
 template <typename E, int DK, bool CH>
-static void launch_delta_t(const SeqArgs& a, int entries, cudaStream_t st) {
+static cudaError_t launch_delta_t(const SeqArgs& a, int entries, cudaStream_t st) {
   constexpr int COLS = 128 / (DK / 16);
   constexpr size_t need = 2 * delta_stage_floats<DK, CH>() * sizeof(float), apart = 116 * 1024;
   const dim3 g(entries, a.H, (a.vdim + COLS - 1) / COLS);
   // the chain of tokens sets the time, so two CTAs never share an SM while there is one for each: a programmatic launch would otherwise place
   // them wherever the previous kernel's CTAs have just left
   const size_t smem = (long)g.x * g.y * g.z <= sm_count() ? (need > apart ? need : apart) : need;
-  static bool attr_set = false;  // per template instance
-  if (!attr_set) {
-    cudaFuncSetAttribute(delta_seq_kernel<E, DK, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(need > apart ? need : apart));
-    attr_set = true;
-  }
-  launch(delta_seq_kernel<E, DK, CH>, g, dim3(256), smem, st, true, a);
+  static std::atomic<uint64_t> smem_set{0};  // per template instance
+  if (const cudaError_t e = allow_smem(smem_set, (const void*)delta_seq_kernel<E, DK, CH>, need > apart ? need : apart); e != cudaSuccess) return e;
+  return launch(delta_seq_kernel<E, DK, CH>, g, dim3(256), smem, st, true, a);
 }
 // 2048 tokens, 16 heads of 128 x 128: 452 us token by token, 173 us in chunks (whole call, B200); error against 64 bits 1.7e-7 both.
 template <int DK>
-static void launch_delta_chunk(const SeqArgs& a, int entries, cudaStream_t st) {
+static cudaError_t launch_delta_chunk(const SeqArgs& a, int entries, cudaStream_t st) {
   constexpr int COLS = 128 / (DK / 16);
   constexpr size_t tokens = 2 * delta_stage_floats<DK, false>() * sizeof(float), chunks = DcSmem<DK, COLS>::BYTES;
   constexpr size_t smem = tokens > chunks ? tokens : chunks;  // more than half of an SM's: one CTA on an SM
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(delta_chunk_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr_set = true;
-  }
+  static std::atomic<uint64_t> smem_set{0};
+  if (const cudaError_t e = allow_smem(smem_set, (const void*)delta_chunk_kernel<DK>, smem); e != cudaSuccess) return e;
   const bool vec = ((a.ld | a.q_off | a.k_off) & 7) == 0 && (reinterpret_cast<uintptr_t>(a.qkv) & 15) == 0;
-  launch(delta_chunk_kernel<DK>, dim3(entries, a.H, (a.vdim + COLS - 1) / COLS), dim3(kDcThreads), smem, st, true, a, vec, wait_err_word());
+  return launch(delta_chunk_kernel<DK>, dim3(entries, a.H, (a.vdim + COLS - 1) / COLS), dim3(kDcThreads), smem, st, true, a, vec, wait_err_word());
 }
 template <typename E, bool CH>
 static int launch_delta(const SeqArgs& a, int entries, cudaStream_t st) {
   if (a.dim > 256) return -2;
-  if (a.dim <= 32) launch_delta_t<E, 32, CH>(a, entries, st);
-  else if (a.dim <= 64) launch_delta_t<E, 64, CH>(a, entries, st);
-  else if (a.dim <= 128) launch_delta_t<E, 128, CH>(a, entries, st);
-  else launch_delta_t<E, 256, CH>(a, entries, st);
-  return (int)cudaGetLastError();
+  const cudaError_t e = a.dim <= 32    ? launch_delta_t<E, 32, CH>(a, entries, st)
+                        : a.dim <= 64  ? launch_delta_t<E, 64, CH>(a, entries, st)
+                        : a.dim <= 128 ? launch_delta_t<E, 128, CH>(a, entries, st)
+                                       : launch_delta_t<E, 256, CH>(a, entries, st);
+  cudaGetLastError();
+  return (int)e;
 }
 
 // ---- gated linear attention.  CTA = (entry, head, COLS value columns), warp-specialised: warps 0-3 run the recurrence over stages of TB tokens,
@@ -1155,9 +1150,9 @@ extern "C" int pk_gated_delta_seq(const void* qkv, int ld, int q_off, int k_off,
   SeqArgs a{qkv, ld, q_off, k_off, v_off, z, ldz, decay_off, beta_off, a_log, dt_bias, state, slot_stride, slot, row0, len, out, nullptr,
             heads, kv_heads, dim, vdim, 0.f};
   if (!f32 && (dim == 64 || dim == 128)) {  // key sizes that need no padding
-    if (dim == 64) launch_delta_chunk<64>(a, entries, st);
-    else launch_delta_chunk<128>(a, entries, st);
-    return (int)cudaGetLastError();
+    const cudaError_t e = dim == 64 ? launch_delta_chunk<64>(a, entries, st) : launch_delta_chunk<128>(a, entries, st);
+    cudaGetLastError();
+    return (int)e;
   }
   return f32 ? launch_delta<float, false>(a, entries, st) : launch_delta<bf16, false>(a, entries, st);
 }
