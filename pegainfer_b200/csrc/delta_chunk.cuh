@@ -116,13 +116,13 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
   const int n = a.n, n_chunks = (n + kDcT - 1) / kDcT;
   uint64_t* full = reinterpret_cast<uint64_t*>(sm + L::BARS);
   uint64_t* empty = full + kDcPrep;
-  const WaitFlag wf{reinterpret_cast<int*>(empty + kDcPrep), a.err};
+  volatile int* dead = reinterpret_cast<volatile int*>(empty + kDcPrep);
   if (tid == 0) {
     for (int i = 0; i < kDcPrep; ++i) {
       mbar_init(full + i, 32);
       mbar_init(empty + i, 8);
     }
-    *wf.dead = 0;
+    *dead = 0;
     mbar_fence_init();
   }
   __syncthreads();
@@ -136,7 +136,7 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
     uint32_t ph = 1;
     for (int b = pw; b < n_chunks; b += kDcPrep, ph ^= 1u) {
       const int t0 = b * kDcT, nb = min(kDcT, n - t0);  // tokens past the end: zero rows, decay 1, write strength 0
-      mbar_wait_bounded(empty + pw, ph, wf);
+      mbar_wait_bounded(empty + pw, ph, dead);
       __syncwarp();
 #pragma unroll
       for (int i = 0; i < PR; ++i) {
@@ -263,6 +263,7 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
       }
       mbar_arrive(full + pw);
     }
+    asm volatile("bar.arrive 2, %0;" ::"n"(kDcThreads) : "memory");
     return;
   }
   const int pc = (tid & 127) % COLS, pt0 = (tid & 127) / COLS * NTK;  // triangle and read-out: column pc, tokens pt0 .. pt0 + NTK - 1
@@ -289,14 +290,14 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
       acc[i] += a1;
     }
   };
-  // Named barriers: 1 the state warps, 4 / 5 u and S0^T q of an even / odd chunk are there, 6 / 7 they have been read
+  // Named barriers: 1 the state warps, 2 the end, 4 / 5 u and S0^T q of an even / odd chunk are there, 6 / 7 they have been read
   if (warp >= 4) {
     // ---- read-out
     int slot = 0;
     uint32_t ph = 0;
     for (int b = 0; b < n_chunks; ++b) {
       const float* st = sm + slot * L::STAGE;
-      mbar_wait_bounded(full + slot, ph, wf);
+      mbar_wait_bounded(full + slot, ph, dead);
       __syncwarp();
       if (b & 1) asm volatile("bar.sync 5, 256;" ::: "memory");
       else asm volatile("bar.sync 4, 256;" ::: "memory");
@@ -320,6 +321,7 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
         ph ^= 1u;
       }
     }
+    asm volatile("bar.arrive 2, %0;" ::"n"(kDcThreads) : "memory");
     return;
   }
   // ---- state and products
@@ -352,7 +354,7 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
       for (int nt = 0; nt < 2 * MT; ++nt)
 #pragma unroll
         for (int i = 0; i < 2; ++i) dc_split(S[nt >> 1][2 * ks + i][(nt & 1) * 2], S[nt >> 1][2 * ks + i][(nt & 1) * 2 + 1], sp[ks][nt][i]);
-    mbar_wait_bounded(full + slot, ph, wf);
+    mbar_wait_bounded(full + slot, ph, dead);
     __syncwarp();
     // S0^T x over this warp's rows, x = k (0) or q (1)
     auto products = [&](int x, float (&p)[2 * MT][3][4]) {
@@ -453,6 +455,8 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
   each_state([](float& x, float* p, bool on) {
     if (on) *p = x;
   });
+  asm volatile("bar.sync 2, %0;" ::"n"(kDcThreads) : "memory");  // every role is through with its waits
+  if (tid == 0) count_run_out(dead, a.err);
 }
 
 }  // namespace pk

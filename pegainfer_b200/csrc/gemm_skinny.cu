@@ -77,7 +77,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   uint64_t* empty = full + SK_MAX_STAGES;
   uint64_t* done = empty + SK_MAX_STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
-  const WaitFlag wf{reinterpret_cast<int*>(tmem_slot + 1), a.err};
+  volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = gridDim.x, sp = (int)sk_rank();  // the cluster spans the whole x axis
@@ -91,7 +91,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       mbar_init(empty + s, 1);
     }
     mbar_init(done, 1);
-    *wf.dead = 0;
+    *dead = 0;
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
@@ -107,7 +107,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       int s = 0, i = 0;
       uint32_t ph = 1;
       for (; i < nk; ++i) {
-        if (!mbar_wait_bounded(empty + s, ph, wf)) break;
+        if (!mbar_wait_bounded(empty + s, ph, dead)) break;
         mbar_expect_tx(full + s, STAGE_BYTES);
         uint8_t* st = smem + (size_t)s * STAGE_BYTES;
         sk_tma_2d(st, &map_w, (kb0 + i) * SK_BK, m0, full + s);
@@ -127,7 +127,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       int s = 0;
       uint32_t ph = 0;
       for (int i = 0; i < nk; ++i) {
-        if (!mbar_wait_bounded(full + s, ph, wf)) break;
+        if (!mbar_wait_bounded(full + s, ph, dead)) break;
         tc_fence_after();
         const uint32_t a_addr = smem_u32(smem + (size_t)s * STAGE_BYTES);
         const uint64_t adesc = make_sw128_desc(a_addr), bdesc = make_sw128_desc(a_addr + A_BYTES);
@@ -144,7 +144,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     __syncwarp();
   }
   // ---- every MMA has read its operands once `done` completes: the ring now takes the partial [NT tokens][rows features]
-  if (!mbar_wait_bounded(done, 0, wf)) mbar_drain(done, 0);
+  if (!mbar_wait_bounded(done, 0, dead)) mbar_drain(done, 0);
   __syncwarp();
   tc_fence_after();
   float* part = reinterpret_cast<float*>(smem);
@@ -207,6 +207,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       }
     }
   }
+  if (threadIdx.x == 0) count_run_out(dead, a.err);  // (every wait lies before the barrier above)
+  __syncwarp();
   if (S > 1) sk_cluster_sync();  // the others may still read this CTA's partial
   if (warp == 1) {
     tc_fence_after();

@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
   uint8_t* Qs = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(lt_smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* Ks = Qs + (size_t)a.nc * LT_QC;
   LtSmem& m = *reinterpret_cast<LtSmem*>(Ks + (size_t)a.nc * LT_KC);
-  const WaitFlag wf{&m.dead, a.err};
+  volatile int* dead = &m.dead;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int half = blockIdx.x % a.halves, tile = gridDim.x / a.halves - 1 - blockIdx.x / a.halves;  // late tokens (long contexts) first
   const int R0 = tile * LT_ROWS, total = a.tokens * a.heads;
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         if (lane < pieces && b + 1 < nb) next = page_of(b + 1);
         for (int x = 0; x < a.nc; ++x, ++fills) {
           const int c = (x + vc0 + nvc) % a.nc;  // the value chunks last
-          on = __all_sync(0xffffffffu, mbar_wait_bounded(m.k_empty + c, (n & 1) ^ 1, wf));
+          on = __all_sync(0xffffffffu, mbar_wait_bounded(m.k_empty + c, (n & 1) ^ 1, dead));
           if (!on) break;
           if (lane == 0) mbar_expect_tx(m.k_full + c, LT_KC);
           __syncwarp();
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
       auto issue_s = [&](uint32_t n, int x0, int x1) {
         for (int x = x0; x < x1; ++x) {
           const int c = (x + vc0 + nvc) % a.nc;
-          mbar_wait_bounded(m.k_full + c, n & 1, wf);
+          mbar_wait_bounded(m.k_full + c, n & 1, dead);
           tc_fence_after();
           const uint64_t qd = make_sw128_desc(smem_u32(Qs + (size_t)c * LT_QC)), kd = make_sw128_desc(smem_u32(Ks + (size_t)c * LT_KC));
 #pragma unroll
@@ -184,14 +184,14 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         }
         if (x1 == a.nc) umma_commit(m.s_full + (n & 1));
       };
-      mbar_wait_bounded(&m.q_full, 0, wf);
+      mbar_wait_bounded(&m.q_full, 0, dead);
       if (total_blocks > 0) issue_s(0, 0, a.nc);
       uint32_t run_end = 0;  // block at which the next run starts
       int run = 0;
       const uint64_t vd = make_sw128_mn_desc(smem_u32(Ks + (size_t)vc0 * LT_KC), LT_KC, 1024);
       for (uint32_t n = 0; n < total_blocks; ++n) {
         if (n + 1 < total_blocks) issue_s(n + 1, 0, n_other);
-        mbar_wait_bounded(m.p_ready + (n & 1), (n >> 1) & 1, wf);
+        mbar_wait_bounded(m.p_ready + (n & 1), (n >> 1) & 1, dead);
         tc_fence_after();
         const bool anew = n == run_end;
         while (n == run_end) run_end += blocks_of(m.runs[run++]);
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         umma_commit(&m.pv_done);
         if (n + 1 < total_blocks) issue_s(n + 1, n_other, a.nc);
       }
-      if (wait_failed(wf)) {
+      if (*dead) {
         umma_commit(&m.done);
         mbar_drain(&m.done, 0);
       }
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
       float mx = -INFINITY, l = 0.f;  // running maximum (scaled, log2 units) and sum
       for (int b = 0; b < nb; ++b, ++n) {
         const int j0 = r.k0 + b * LT_KEYS;
-        mbar_wait_bounded(m.s_full + (n & 1), (n >> 1) & 1, wf);
+        mbar_wait_bounded(m.s_full + (n & 1), (n >> 1) & 1, dead);
         __syncwarp();
         tc_fence_after();
         const uint32_t t_s = t_lane + (n & 1) * LT_KEYS;
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
           mx = to;
           l *= corr;
           if (b > 0) {  // O holds the blocks before this one
-            mbar_wait_bounded(&m.pv_done, (n - 1) & 1, wf);
+            mbar_wait_bounded(&m.pv_done, (n - 1) & 1, dead);
             __syncwarp();
             tc_fence_after();
             for (int c = 0; c < nvc * 64; c += 64) {
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         mbar_arrive(m.p_ready + (n & 1));
       }
       // ---- O / l -> bf16, the rows of this run (the next one's first P V waits for all 128 threads' next p_ready)
-      if (nb > 0) mbar_wait_bounded(&m.pv_done, (n - 1) & 1, wf);
+      if (nb > 0) mbar_wait_bounded(&m.pv_done, (n - 1) & 1, dead);
       __syncwarp();
       tc_fence_after();
       const float sk = a.sink && act ? bf2f(a.sink[R % a.heads]) * 1.4426950408889634f : -INFINITY;
@@ -320,6 +320,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
   }
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0) count_run_out(dead, a.err);
   if (warp == 4) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);

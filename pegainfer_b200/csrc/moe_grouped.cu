@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
   uint64_t* tempty = tfull + 2;
   uint64_t* done = tempty + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
-  const WaitFlag wf{reinterpret_cast<int*>(tmem_slot + 1), a.err};
+  volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMgStages; ++s) {
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
       mbar_init(tempty + s, 4);
     }
     mbar_init(done, 1);
-    *wf.dead = 0;
+    *dead = 0;
     mbar_fence_init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
@@ -198,10 +198,10 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
     if (tc_elect_one()) {
       int s = 0, fills = 0;
       uint32_t ph = 1;
-      for (int t = blockIdx.x; t < tiles && !wait_failed(wf); t += gridDim.x) {
+      for (int t = blockIdx.x; t < tiles && !*dead; t += gridDim.x) {
         const int rt = t / n_ft, m0 = tr[rt], rows = tr[rt + 1] - m0, w0 = te[rt] * a.N + (t - rt * n_ft) * 128, boxes = (rows + 63) / 64;
         for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait_bounded(empty + s, ph, wf)) break;
+          if (!mbar_wait_bounded(empty + s, ph, dead)) break;
           ++fills;
           mbar_expect_tx(full + s, kMgA + boxes * kMgBox);
           uint8_t* st = smem + (size_t)s * kMgStage;
@@ -213,20 +213,20 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
           }
         }
       }
-      if (wait_failed(wf)) ring_drain(full, kMgStages, fills);
+      if (*dead) ring_drain(full, kMgStages, fills);
     }
   } else if (warp == 1) {
     if (tc_elect_one()) {
       int s = 0, lt = 0;
       uint32_t ph = 0;
-      for (int t = blockIdx.x; t < tiles && !wait_failed(wf); t += gridDim.x, ++lt) {
+      for (int t = blockIdx.x; t < tiles && !*dead; t += gridDim.x, ++lt) {
         const int rt = t / n_ft, n16 = (tr[rt + 1] - tr[rt] + 15) / 16, as = lt & 1;
         // instruction descriptor: D = f32 [4,6) = 1, A = bf16 [7,10) = 1, B = bf16 [10,13) = 1, both K-major, N >> 3 at [17,23), M >> 4 at [24,29)
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n16 * 2) << 17) | ((uint32_t)(128 >> 4) << 24);
-        if (!mbar_wait_bounded(tempty + as, (uint32_t)(((lt >> 1) & 1) ^ 1), wf)) break;
+        if (!mbar_wait_bounded(tempty + as, (uint32_t)(((lt >> 1) & 1) ^ 1), dead)) break;
         tc_fence_after();
         for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait_bounded(full + s, ph, wf)) break;
+          if (!mbar_wait_bounded(full + s, ph, dead)) break;
           tc_fence_after();
           const uint32_t a_addr = smem_u32(smem + (size_t)s * kMgStage);
           const uint64_t ad = make_sw128_desc(a_addr), bd = make_sw128_desc(a_addr + kMgA);
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
         }
         umma_commit(tfull + as);
       }
-      if (wait_failed(wf)) {
+      if (*dead) {
         umma_commit(done);
         mbar_drain(done, 0);
       }
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
     // (to the last tile even when a wait ran out: a warp that left on its own reading of the flag would leave the others at barrier 1)
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++lt) {
       const int rt = t / n_ft, m0 = tr[rt], rows = tr[rt + 1] - m0, f0 = (t - rt * n_ft) * 128, as = lt & 1;
-      mbar_wait_bounded(tfull + as, (uint32_t)((lt >> 1) & 1), wf);
+      mbar_wait_bounded(tfull + as, (uint32_t)((lt >> 1) & 1), dead);
       __syncwarp();
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * kMoeTile);
@@ -317,6 +317,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
   __syncwarp();
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0) count_run_out(dead, a.err);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);

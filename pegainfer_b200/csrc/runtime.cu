@@ -39,13 +39,13 @@ static void make_wait_err_word() {
 // waits for a barrier that nothing completes, `spins` tries long
 __global__ void wait_probe_kernel(uint32_t spins, unsigned int* err) {
   __shared__ uint64_t bar;
-  __shared__ int dead;
+  __shared__ int flag;
   if (threadIdx.x != 0) return;
-  dead = 0;
+  flag = 0;
   mbar_init(&bar, 1);
   mbar_fence_init();
-  const WaitFlag wf{&dead, err};
-  mbar_wait_bounded(&bar, 0, wf, spins);
+  mbar_wait_bounded(&bar, 0, &flag, spins);
+  count_run_out(&flag, err);
 }
 }  // namespace pk
 

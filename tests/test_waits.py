@@ -25,35 +25,26 @@ def block_after(text, at):
 def test_no_loop_with_a_barrier_ends_on_a_threads_own_view_of_the_flag(path):
     """A loop over a barrier of several warps must end for all of them alike: a warp that sees the flag before another leaves that one waiting for good."""
     text = open(path).read()
-    for m in re.finditer(r"\b(?:for|while) \([^{}]*(?:\*dead|wait_failed)[^{}]*\) \{", text):
+    for m in re.finditer(r"\b(?:for|while) \([^{}]*\*dead[^{}]*\) \{", text):
         body = block_after(text, m.end() - 1)
         assert not re.search(r"bar\.sync|__syncthreads|barrier\.cluster", body), f"{os.path.basename(path)}: {m.group(0)}"
 
 
-@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
-def test_a_run_out_wait_is_counted_where_it_runs_out(path):
-    """Counting at a kernel's end, by one thread, misses the waits of roles that run out after that thread has looked: only the wait itself counts."""
+@pytest.mark.parametrize("path", [p for p in SOURCES if os.path.basename(p) not in ("common.cuh", "qwen35_ops.cu", "recurrent_mixers.cu")], ids=os.path.basename)
+def test_run_outs_are_counted_behind_every_role(path):
+    """A thread that counts at the end of its own role misses what runs out in the others after that: behind the count's place no wait may follow, and a
+    barrier of all roles lies before it (a role that returns early arrives there)."""
     text = open(path).read()
-    counts = [m.start() for m in re.finditer(r"atomicAdd\([^;]*\berr\b", text)]
-    if os.path.basename(path) != "common.cuh":
-        assert not counts
-    else:
-        at = text.index("bool mbar_wait_bounded(")
-        assert len(counts) == 1 and block_after(text, at).find(text[counts[0]:counts[0] + 20]) >= 0
-
-
-@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
-def test_the_word_that_counts_reaches_every_limited_wait(path):
-    """every wait with a limit names the flag and the word (WaitFlag), not a flag alone"""
-    text = open(path).read()
-    for m in re.finditer(r"mbar_wait_bounded\(", text):
-        if os.path.basename(path) == "common.cuh":
-            continue
-        depth, j = 1, m.end()
-        while depth:
-            depth += {"(": 1, ")": -1}.get(text[j], 0)
-            j += 1
-        assert re.search(r", wf\b", text[m.end():j - 1]), text[m.start():j]
+    waits = [m.start() for m in re.finditer(r"mbar_wait_bounded\(", text)]
+    counts = [m.start() for m in re.finditer(r"count_run_out\(", text)]
+    assert len(counts) == (1 if waits else 0)
+    if waits and os.path.basename(path) != "runtime.cu":  # (one thread there)
+        assert max(waits) < counts[0]
+        gap = text[max(waits):counts[0]]
+        assert "__syncthreads();" in gap or 'bar.sync 2, %0;" ::"n"(kDcThreads)' in gap
+        for m in re.finditer(r"\n    return;\n", text[min(waits):counts[0]]):
+            before = text[min(waits):counts[0]][:m.start()]
+            assert before.endswith('asm volatile("bar.arrive 2, %0;" ::"n"(kDcThreads) : "memory");')
 
 
 REFUSAL = """
