@@ -7,12 +7,18 @@
 // has; S takes the others first, so the next block's chunks arrive under the softmax and its S is under way before P V.
 //   warps 0-3 softmax (thread = row; P goes back to TMEM over S and is the A operand of P V; O is scaled when a row's maximum has grown.  The reference
 //             is the maximum itself: the largest weight is then 1, which bf16 holds exactly -- behind a maximum that lags by up to 2^8 its rounding alone
-//             made the result's error 1.2 times as large for peaked scores)
+//             made the result's error 1.2 times as large for peaked scores; it saved 8 of 272 us)
 //   warp 4    MMA issuer     S = Q K^T (SS),  O += P V (A from TMEM, V = the key chunks read N-major)
 //   warp 5    TMA: Q once, then the pages of every key block
-// A tile whose rows belong to several requests walks each request's keys in turn with the other rows masked, starts O anew for each and writes that
-// request's rows behind it: what another request's cache holds (a NaN times a weight of zero) never reaches them.  Keys outside the run (slots behind
-// the context's end, keys before the window) are masked in S, and their value rows are cleared in shared memory before P V: they may hold anything.
+// Work item = (tile, run): the rows of a tile that belong to one request, with the tile's other rows masked, from an empty O.  What another request's
+// cache holds (a NaN times a weight of zero) never reaches a row, and requests that share a tile -- decoded tokens beside a prompt portion, each with a
+// context of its own -- do not wait for one another.  A tile's CTAs take its first run; the others, which start at a token whose first row is inside a
+// tile, go to the helper CTAs, every helpers-th token to the same ones, so that the decoded tokens of a step spread over the GPU.  A helper that finds
+// none ends at once.  Us, 16 heads, latent
+// 512 + 64 (walking a tile's runs one after the other; latent_attention_mma.cu for all): 2048-token portion + 8 tokens at contexts of 4096: 307 (2345;
+// 1169), 1000 + 24 tokens at 2000: 154 (1146; 444), 320 tokens at 1000: 376 (592; 334), a 2048-token prompt alone: 272 (270; 662).
+// Keys outside the run (slots behind the context's end, keys before the window) are masked in S, and their value rows are cleared in shared memory
+// before P V: they may hold anything.
 // Tensor-bound (operand reads of the narrow MMAs): 2 * rows * keys * (2 rank + rot) flop of result, 1.5 times that executed at rank 512.
 #include <cuda.h>
 
@@ -25,12 +31,12 @@ namespace {
 
 constexpr int LT_ROWS = 128, LT_KEYS = 64, LT_MAXC = 9, LT_VC = 4;  // rows, keys per block, feature chunks, value chunks per CTA
 constexpr int LT_QC = LT_ROWS * 128, LT_KC = LT_KEYS * 128;         // bytes of a chunk of Q / of keys
-constexpr int LT_THREADS = 192;
+constexpr int LT_THREADS = 192, LT_ITEMS = 128;  // items of a CTA at most
 
-struct LtRun {  // consecutive tokens of one request inside a tile
-  int t0, t1;    // first and last token
+struct LtItem {  // consecutive tokens of one request inside a tile
+  int R0, t0, t1;   // the tile's first row, first and last token
   int k0, lo, end;  // first key of the first block (on a page border), first visible key of any row, one past the last
-  int pages;     // offset of the request's page list
+  int pages;        // offset of the request's page list
 };
 
 struct LtArgs {
@@ -38,6 +44,7 @@ struct LtArgs {
   const int *pos, *req, *page_off, *pages;
   bf16* out;
   int page_size, tokens, heads, rank, nc, halves, window;
+  int helpers, helpers_first;  // helper CTAs per half; whether they come before the tiles' in the grid
   float scale_log2;
   unsigned int* err;
 };
@@ -61,11 +68,10 @@ __device__ __forceinline__ float lt_exp2(float x) {
 }
 
 struct LtSmem {  // behind Q and the key chunks
-  uint64_t q_full, k_full[LT_MAXC], k_empty[LT_MAXC], s_full[2], p_ready[2], pv_done, done;
+  uint64_t q_full, q_empty, k_full[LT_MAXC], k_empty[LT_MAXC], s_full[2], p_ready[2], pv_done, done;
   uint32_t tmem_slot;
-  int dead, n_runs;
-  int tok_req[LT_ROWS], tok_pos[LT_ROWS];
-  LtRun runs[LT_ROWS];
+  int dead, n_items, first_end;
+  LtItem items[LT_ITEMS];
 };
 
 __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -76,12 +82,25 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
   LtSmem& m = *reinterpret_cast<LtSmem*>(Ks + (size_t)a.nc * LT_KC);
   volatile int* dead = &m.dead;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int half = blockIdx.x % a.halves, tile = gridDim.x / a.halves - 1 - blockIdx.x / a.halves;  // late tokens (long contexts) first
-  const int R0 = tile * LT_ROWS, total = a.tokens * a.heads;
-  const int t_first = R0 / a.heads, n_tok = (min(total, R0 + LT_ROWS) - 1) / a.heads - t_first + 1;
+  const int half = blockIdx.x % a.halves, total = a.tokens * a.heads, tiles = (total + LT_ROWS - 1) / LT_ROWS;
+  const int group = blockIdx.x / a.halves, helper = a.helpers_first ? group : group - tiles;  // 0 .. helpers - 1: a helper
+  const bool help = helper >= 0 && helper < a.helpers;
+  auto item_of = [&](int R0, int t0, int t1) {
+    const int rq = a.req[t0], lo = a.window > 0 ? max(a.pos[t0] - a.window + 1, 0) : 0;
+    return LtItem{R0, t0, t1, lo / a.page_size * a.page_size, lo, a.pos[t1] + 1, a.page_off[rq]};
+  };
+  auto last_token = [&](int R0) { return (min(total, R0 + LT_ROWS) - 1) / a.heads; };
+  bool starts = false;  // this thread's token starts a run inside a tile
+  const int my_token = helper + (int)threadIdx.x * a.helpers;
+  if (help) {
+    pdl_wait();
+    if (threadIdx.x < LT_ITEMS && my_token > 0 && my_token < a.tokens && (long)my_token * a.heads % LT_ROWS != 0) starts = a.req[my_token] != a.req[my_token - 1];
+    if (__syncthreads_count(starts) == 0) return;
+  }
   const int vc0 = half * LT_VC, nvc = min(LT_VC, a.rank / 64 - vc0);
   if (threadIdx.x == 0) {
     mbar_init(&m.q_full, 1);
+    mbar_init(&m.q_empty, 1);
     for (int c = 0; c < LT_MAXC; ++c) {
       mbar_init(m.k_full + c, 1);
       mbar_init(m.k_empty + c, 1);
@@ -93,73 +112,71 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
     mbar_init(&m.pv_done, 1);
     mbar_init(&m.done, 1);
     m.dead = 0;
+    m.n_items = 0;
+    m.first_end = 0x7fffffff;
     mbar_fence_init();
   }
   if (warp == 4) tmem_alloc(&m.tmem_slot, 512);
-  pdl_wait();
-  for (int i = threadIdx.x; i < n_tok; i += LT_THREADS) {
-    m.tok_req[i] = a.req[t_first + i];
-    m.tok_pos[i] = a.pos[t_first + i];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int n = 0;
-    for (int t = 0; t < n_tok;) {
-      int e = t;
-      while (e + 1 < n_tok && m.tok_req[e + 1] == m.tok_req[t]) ++e;
-      LtRun r;
-      r.t0 = t;
-      r.t1 = e;
-      r.lo = a.window > 0 ? max(m.tok_pos[t] - a.window + 1, 0) : 0;
-      r.k0 = r.lo / a.page_size * a.page_size;
-      r.end = m.tok_pos[e] + 1;
-      r.pages = a.page_off[m.tok_req[t]];
-      m.runs[n++] = r;
-      t = e + 1;
-    }
-    m.n_runs = n;
-  }
+  if (!help) pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (help) {
+    if (starts) {
+      const int R0 = my_token * a.heads / LT_ROWS * LT_ROWS, last = last_token(R0), rq = a.req[my_token];
+      int e = my_token;
+      while (e < last && a.req[e + 1] == rq) ++e;
+      m.items[atomicAdd(&m.n_items, 1)] = item_of(R0, my_token, e);
+    }
+  } else {
+    const int tile = tiles - 1 - (a.helpers_first ? group - a.helpers : group);  // late tokens (long contexts) first
+    const int R0 = tile * LT_ROWS, t0 = R0 / a.heads, last = last_token(R0), t = t0 + 1 + (int)threadIdx.x;  // at most 128 tokens
+    if (t <= last && a.req[t] != a.req[t - 1]) atomicMin(&m.first_end, t - 1);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      m.items[0] = item_of(R0, t0, min(last, m.first_end));
+      m.n_items = 1;
+    }
+  }
+  __syncthreads();
   pdl_launch_dependents();  // after the allocation: a dependent that came first would hold the TMEM while it waits for this grid
   const uint32_t tmem = m.tmem_slot;
-  const int n_runs = m.n_runs;
-  auto blocks_of = [&](const LtRun& r) { return (r.end - r.k0 + LT_KEYS - 1) / LT_KEYS; };
+  const int n_items = m.n_items;
+  auto blocks_of = [&](const LtItem& r) { return (r.end - r.k0 + LT_KEYS - 1) / LT_KEYS; };  // 0: no visible key
 
   if (warp == 5) {
-    if (lane == 0) {
-      mbar_expect_tx(&m.q_full, (uint32_t)(a.nc * LT_QC));
-      for (int c = 0; c < a.nc; ++c) lt_tma_2d(Qs + (size_t)c * LT_QC, &map_q, c * 64, R0, &m.q_full);
-    }
     // lane j copies the j-th piece (a page, or 64 slots of one) of every chunk; its page number is looked up once per block, a block ahead
     const int box = min(a.page_size, LT_KEYS), pieces = LT_KEYS / box;
-    uint32_t n = 0;
-    int fills = 0;  // of the key chunks, in the order in which they are loaded
-    bool on = true;
-    for (int i = 0; i < n_runs && on; ++i) {
-      const LtRun r = m.runs[i];
+    uint32_t n = 0, q = 0;  // blocks and queries so far
+    for (int i = 0; i < n_items; ++i) {
+      const LtItem r = m.items[i];
       const int* pg = a.pages + r.pages;
       const int nb = blocks_of(r), last = (r.end - 1) / a.page_size;
+      if (nb <= 0) continue;
+      if (q > 0) mbar_wait_bounded(&m.q_empty, (q - 1) & 1, dead);
+      if (lane == 0) {
+        mbar_expect_tx(&m.q_full, (uint32_t)(a.nc * LT_QC));
+        for (int c = 0; c < a.nc; ++c) lt_tma_2d(Qs + (size_t)c * LT_QC, &map_q, c * 64, r.R0, &m.q_full);
+      }
+      ++q;
       auto page_of = [&](int b) { return pg[min((r.k0 + b * LT_KEYS + lane * box) / a.page_size, last)]; };  // behind the end: the last page again (masked)
       int next = lane < pieces ? page_of(0) : 0;
-      for (int b = 0; b < nb && on; ++b, ++n) {
+      for (int b = 0; b < nb; ++b, ++n) {
         const int page = next, slot = (r.k0 + b * LT_KEYS + lane * box) % a.page_size;
         if (lane < pieces && b + 1 < nb) next = page_of(b + 1);
-        for (int x = 0; x < a.nc; ++x, ++fills) {
+        for (int x = 0; x < a.nc; ++x) {
           const int c = (x + vc0 + nvc) % a.nc;  // the value chunks last
-          on = __all_sync(0xffffffffu, mbar_wait_bounded(m.k_empty + c, (n & 1) ^ 1, dead));
-          if (!on) break;
+          mbar_wait_bounded(m.k_empty + c, (n & 1) ^ 1, dead);
           if (lane == 0) mbar_expect_tx(m.k_full + c, LT_KC);
           __syncwarp();
           if (lane < pieces) lt_tma_3d(Ks + (size_t)c * LT_KC + lane * box * 128, &map_k, c * 64, slot, page, m.k_full + c);
         }
       }
     }
-    if (!on) {
-      mbar_drain(&m.q_full, 0);
-      for (int j = max(0, fills - a.nc); j < fills; ++j) mbar_drain(m.k_full + (j % a.nc + vc0 + nvc) % a.nc, (uint32_t)((j / a.nc) & 1));
-    }
+    // Behind a run-out the copies go on, in bounds but without waiting for their places, and no barrier says when the last has landed: two milliseconds,
+    // where a copy takes a thousandth of that
+    if (*dead)
+      for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     __syncwarp();
   } else if (warp == 4) {
     if (tc_elect_one()) {
@@ -167,8 +184,6 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
       constexpr uint32_t base = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(LT_ROWS >> 4) << 24);
       constexpr uint32_t idesc_s = base | ((uint32_t)(LT_KEYS >> 3) << 17);
       const uint32_t idesc_pv = base | (1u << 16) | ((uint32_t)(nvc * 8) << 17);
-      uint32_t total_blocks = 0;
-      for (int i = 0; i < n_runs; ++i) total_blocks += blocks_of(m.runs[i]);
       const int n_other = a.nc - nvc;
       // chunks [x0, x1) of block n in the order of the loads
       auto issue_s = [&](uint32_t n, int x0, int x1) {
@@ -184,23 +199,26 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         }
         if (x1 == a.nc) umma_commit(m.s_full + (n & 1));
       };
-      mbar_wait_bounded(&m.q_full, 0, dead);
-      if (total_blocks > 0) issue_s(0, 0, a.nc);
-      uint32_t run_end = 0;  // block at which the next run starts
-      int run = 0;
       const uint64_t vd = make_sw128_mn_desc(smem_u32(Ks + (size_t)vc0 * LT_KC), LT_KC, 1024);
-      for (uint32_t n = 0; n < total_blocks; ++n) {
-        if (n + 1 < total_blocks) issue_s(n + 1, 0, n_other);
-        mbar_wait_bounded(m.p_ready + (n & 1), (n >> 1) & 1, dead);
-        tc_fence_after();
-        const bool anew = n == run_end;
-        while (n == run_end) run_end += blocks_of(m.runs[run++]);
+      uint32_t n = 0, q = 0;  // blocks and queries so far
+      for (int i = 0; i < n_items; ++i) {
+        const uint32_t end = n + (uint32_t)max(blocks_of(m.items[i]), 0), first = n;
+        if (n == end) continue;
+        mbar_wait_bounded(&m.q_full, q++ & 1, dead);
+        issue_s(n, 0, a.nc);
+        if (n + 1 == end) umma_commit(&m.q_empty);
+        for (; n < end; ++n) {
+          if (n + 1 < end) issue_s(n + 1, 0, n_other);
+          mbar_wait_bounded(m.p_ready + (n & 1), (n >> 1) & 1, dead);
+          tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < LT_KEYS / 16; ++k)
-          umma_bf16_tmem_a(tmem + 256, tmem + (n & 1) * LT_KEYS + (uint32_t)(k * 8), vd + (uint64_t)(k * (2048 >> 4)), idesc_pv, (!anew || k > 0) ? 1u : 0u);
-        for (int c = vc0; c < vc0 + nvc; ++c) umma_commit(m.k_empty + c);
-        umma_commit(&m.pv_done);
-        if (n + 1 < total_blocks) issue_s(n + 1, n_other, a.nc);
+          for (int k = 0; k < LT_KEYS / 16; ++k)
+            umma_bf16_tmem_a(tmem + 256, tmem + (n & 1) * LT_KEYS + (uint32_t)(k * 8), vd + (uint64_t)(k * (2048 >> 4)), idesc_pv, (n > first || k > 0) ? 1u : 0u);
+          for (int c = vc0; c < vc0 + nvc; ++c) umma_commit(m.k_empty + c);
+          umma_commit(&m.pv_done);
+          if (n + 1 < end) issue_s(n + 1, n_other, a.nc);
+          if (n + 2 == end) umma_commit(&m.q_empty);  // the item's last scores: then the next one's queries may come
+        }
       }
       if (*dead) {
         umma_commit(&m.done);
@@ -209,15 +227,14 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
     }
     __syncwarp();
   } else {
-    const int row = threadIdx.x, R = R0 + row;  // 0 .. 127
-    const int tok = R < total ? R / a.heads - t_first : -1, my_pos = tok >= 0 ? m.tok_pos[tok] : -1;
-    const int my_lo = a.window > 0 ? my_pos - a.window + 1 : 0;
+    const int row = threadIdx.x;  // 0 .. 127
     const uint32_t t_lane = tmem + ((uint32_t)(warp * 32) << 16), t_o = t_lane + 256;
     uint32_t n = 0;
-    for (int i = 0; i < n_runs; ++i) {
-      const LtRun r = m.runs[i];
+    for (int i = 0; i < n_items; ++i) {
+      const LtItem r = m.items[i];
+      const int R = r.R0 + row, tok = R < total ? R / a.heads : -1, nb = blocks_of(r);
       const bool act = tok >= r.t0 && tok <= r.t1;
-      const int nb = blocks_of(r);
+      const int my_pos = act ? a.pos[tok] : -1, my_lo = a.window > 0 ? my_pos - a.window + 1 : 0;
       float mx = -INFINITY, l = 0.f;  // running maximum (scaled, log2 units) and sum
       for (int b = 0; b < nb; ++b, ++n) {
         const int j0 = r.k0 + b * LT_KEYS;
@@ -248,10 +265,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
           const float to = grow ? blk : mx, corr = grow ? lt_exp2(mx - to) : 1.f;
           mx = to;
           l *= corr;
-          if (b > 0) {  // O holds the blocks before this one
-            mbar_wait_bounded(&m.pv_done, (n - 1) & 1, dead);
-            __syncwarp();
-            tc_fence_after();
+          if (b > 0) {  // O holds the blocks before this one (their P V were issued before this block's last scores, so they are complete)
             for (int c = 0; c < nvc * 64; c += 64) {
               uint32_t t[64];
               tmem_ld32_nowait(t_o + c, t);
@@ -291,7 +305,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         tc_fence_before();
         mbar_arrive(m.p_ready + (n & 1));
       }
-      // ---- O / l -> bf16, the rows of this run (the next one's first P V waits for all 128 threads' next p_ready)
+      // ---- O / l -> bf16, the rows of this item (the next one's first P V waits for all 128 threads' next p_ready)
       if (nb > 0) mbar_wait_bounded(&m.pv_done, (n - 1) & 1, dead);
       __syncwarp();
       tc_fence_after();
@@ -339,7 +353,7 @@ int launch_latent_attention_tc(const bf16* qa, const bf16* cache, const bf16* si
       ((reinterpret_cast<uintptr_t>(qa) | reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(out)) & 15))
     return -2;
   const long rows = (long)tokens * heads, tiles = (rows + LT_ROWS - 1) / LT_ROWS;
-  if (tiles * halves < sm_count() / 2 || tiles * halves > 0x7fffffff || rows > 0x7fffffff) return -2;  // few rows: the key axis has to be split
+  if (tiles * halves < sm_count() / 2 || tiles * halves > 0x3fffffff || rows > 0x7fffffff) return -2;  // few rows: the key axis has to be split
   EncodeTiledFn fn = encode_fn();
   if (!fn) return -2;
   CUtensorMap mq, mk;
@@ -357,14 +371,18 @@ int launch_latent_attention_tc(const bf16* qa, const bf16* cache, const bf16* si
            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return -2;
   }
+  // Runs that start inside a tile are for the helpers, one CTA per half and SM (more where a helper would have over LT_ITEMS tokens to look at); none
+  // where each token fills whole tiles.  They come first, since their contexts may be the longest, unless all CTAs fit at once.
+  int helpers = heads % LT_ROWS == 0 ? 0 : (sm_count() + halves - 1) / halves;
+  if (helpers > 0 && helpers < (tokens + LT_ITEMS - 1) / LT_ITEMS) helpers = (tokens + LT_ITEMS - 1) / LT_ITEMS;
   const size_t smem = (size_t)nc * (LT_QC + LT_KC) + sizeof(LtSmem) + 1024;
   static std::atomic<uint64_t> smem_set{0};
   if (allow_smem(smem_set, (const void*)latent_attention_tc_kernel, LT_MAXC * (LT_QC + LT_KC) + sizeof(LtSmem) + 1024) != cudaSuccess) {
     cudaGetLastError();
     return -2;
   }
-  const LtArgs a{sink, pos, req, page_off, pages, out, page_size, tokens, heads, rank, nc, halves, window, scale * 1.4426950408889634f, wait_err_word()};
-  return (int)launch(latent_attention_tc_kernel, dim3((unsigned)(tiles * halves)), dim3(LT_THREADS), smem, st, true, mq, mk, a);
+  const LtArgs a{sink, pos, req, page_off, pages, out, page_size, tokens, heads, rank, nc, halves, window, helpers, tiles * halves > sm_count(), scale * 1.4426950408889634f, wait_err_word()};
+  return (int)launch(latent_attention_tc_kernel, dim3((unsigned)((tiles + helpers) * halves)), dim3(LT_THREADS), smem, st, true, mq, mk, a);
 }
 
 }  // namespace pk

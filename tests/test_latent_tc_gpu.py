@@ -172,3 +172,14 @@ def test_rows_without_a_visible_key(lib):
                                       out.data_ptr(), ps * D, ps, T, H, rank, rot, D ** -0.5, 0, 300, 0, None) == 0
     torch.cuda.synchronize()
     assert (out[:300] == 0).all() and torch.isfinite(out[300:]).all() and (out[300:] != 0).any(-1).all() and lib.pk_b200_wait_errors() == 0
+
+
+@pytest.mark.parametrize("starts,lens,H,window,ps,sink", [
+    ([0] + [60 * i + 5 for i in range(20)], [500] + [1] * 20, 16, 0, 16, True),            # a portion and decoded tokens behind it
+    ([40 * i for i in range(13)] + [100, 0], [1] * 13 + [290, 4], 16, 70, 8, False),      # in front of it, windows; odd rests
+    ([(7 * i) % 400 for i in range(300)], [1] * 300, 16, 0, 64, True),                    # decoded tokens alone
+    ([3, 500, 0, 77, 9, 1], [20, 1, 1, 30, 2, 1], 100, 0, 16, False),                     # tokens across the borders of tiles
+    ([3, 0, 77, 9], [17, 1, 20, 2], 128, 0, 16, True), ([3, 0, 77], [8, 1, 11], 256, 0, 16, False),  # tokens that fill whole tiles
+    ([i % 5 for i in range(9600)], [1] * 9600, 1, 0, 8, False)])                          # more runs than the helpers of one GPU's SMs list
+def test_many_requests_in_a_tile(lib, starts, lens, H, window, ps, sink):
+    test_against_64_bits(lib, starts, lens, H, window, ps, sink, 512, 64)
