@@ -292,9 +292,11 @@ constexpr int delta_stage_floats() {
 }
 
 template <typename E, int DK, bool CH>
-__device__ __forceinline__ void delta_tokens(const SeqArgs& a) {
+__global__ void __launch_bounds__(256) delta_seq_kernel(SeqArgs a) {
   constexpr int KS = DK / 16, COLS = 128 / KS, TB = kDeltaTB, NV = DK / 32, TW = TB / 4;  // TW: tokens a preparing warp handles per stage
   extern __shared__ __align__(16) float ds_sm[];
+  pdl_wait();
+  pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
   const int e = blockIdx.x, h = blockIdx.y, kvh = h / (a.H / a.G), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = a.len[e], r0 = a.row0[e], dim = a.dim, vdim = a.vdim, col0 = blockIdx.z * COLS;
   const int n_stages = (n + TB - 1) / TB;
@@ -431,7 +433,7 @@ __device__ __forceinline__ void delta_tokens(const SeqArgs& a) {
     finish(0);
     if (n_stages > 1) fetch(1);
     for (int b = 0; b < n_stages; ++b) {
-      asm volatile("bar.sync 3, 256;" ::: "memory");  // stage b is complete, and nobody reads the other one any more
+      __syncthreads();  // stage b is complete, and nobody reads the other one any more
       if (b + 1 < n_stages) {
         finish(b + 1);
         if (b + 2 < n_stages) fetch(b + 2);
@@ -452,7 +454,7 @@ __device__ __forceinline__ void delta_tokens(const SeqArgs& a) {
   const size_t out_ld = (size_t)a.H * vdim;
   float* out = a.out + (size_t)r0 * out_ld + h * vdim + col;
   for (int b = 0; b < n_stages; ++b) {
-    asm volatile("bar.sync 3, 256;" ::: "memory");
+    __syncthreads();
     const float* sm = ks_of(b);
     const int nb = min(TB, n - b * TB);
 #pragma unroll 4
@@ -506,27 +508,239 @@ __device__ __forceinline__ void delta_tokens(const SeqArgs& a) {
   }
 }
 
-template <typename E, int DK, bool CH>
-__global__ void __launch_bounds__(256) delta_seq_kernel(SeqArgs a) {
-  pdl_wait();
-  pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
-  delta_tokens<E, DK, CH>(a);
+// A portion of a few tokens (decoded tokens; up to kDeltaFew), inside the CTAs of delta_chunk_kernel.  Only one of these fits an SM (registers), where
+// delta_seq_kernel has three, so a CTA keeps more of the state in flight: 32, 64 or 128 value columns of a head in the registers of 8 warps; the CTAs
+// of the grid's z axis that this leaves over end at once.  Warp ks of KS (two groups of warps for DK = 64, each with half of the columns) has the state
+// rows that delta_seq_kernel's lane ks has, a lane has VC neighbouring columns, so that state rows move in whole lines; the warps' sums meet in shared
+// memory and are added in the order of that kernel's shuffles: an entry's result is the same, bit for bit, whatever the columns to a CTA.  Warps 8-11
+// prepare the tokens.  Bound by latency: state in, one exchange per token, state out.
+// B200, us, 1 / 2 / 4 / 6 / 24 decoding requests, 16 heads of 128 x 128: 3.0 3.9 5.7 7.4 26.7 (delta_seq_kernel's 256 threads inside each CTA of the
+// chunk kernel: 4.1 7.3 13.1 18.8 64.6; delta_seq_kernel itself 4.2 5.5 8.8 9.8 30.2); heads of 64 x 64: 2.7 2.8 2.9 2.9 7.7 (3.8 3.9 3.9 6.7 17.9; 3.8 3.8
+// 3.9 4.3 8.3).
+constexpr int kDeltaFew = 32;
+template <int DK>
+constexpr int delta_few_floats(int fc) { return kDeltaFew * (2 * DK + fc + 4) + 2 * 2 * (DK / 16) * fc; }
+template <int DK, int VC, int NB>
+__device__ __forceinline__ void delta_few(const SeqArgs& a, float* sm, int n) {
+  constexpr int KS = DK / 16, GR = 8 / KS, W = 32 * VC * GR, FC = W * NB, NV = DK / 32, VL = FC / 32, TW = kDeltaFew / 4;  // W: columns of a pass of 8 warps
+  constexpr int COLS = 128 / KS, Z = FC / COLS;
+  float *ks = sm, *qs = ks + kDeltaFew * DK, *vs = qs + kDeltaFew * DK, *sc = vs + kDeltaFew * FC;  // sc: decays, write strengths, k . q
+  float* part = sc + 4 * kDeltaFew;                                                                // two of [k S, q S][KS][FC]
+  const int e = blockIdx.x, h = blockIdx.y, kvh = h / (a.H / a.G), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int r0 = a.row0[e], vdim = a.vdim, col0 = blockIdx.z / Z * FC;
+  if (warp >= 8) {
+    // tokens warp - 8, + 4, ..: all loads on their way before the first is used
+    const int d0 = lane * NV;
+    bf16 qr[TW][NV], kr[TW][NV], vr[TW][VL];
+    float za[TW], zb[TW];
+#pragma unroll
+    for (int i = 0; i < TW; ++i) {
+      const int t = warp - 8 + 4 * i;
+      if (t >= n) break;
+      const bf16* X = static_cast<const bf16*>(a.qkv) + (size_t)(r0 + t) * a.ld;
+      const float* z = a.z + (size_t)(r0 + t) * a.ldz;
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        qr[i][j] = X[a.q_off + kvh * DK + d0 + j];
+        kr[i][j] = X[a.k_off + kvh * DK + d0 + j];
+      }
+#pragma unroll
+      for (int j = 0; j < VL; ++j) vr[i][j] = col0 + lane + 32 * j < vdim ? X[a.v_off + h * vdim + col0 + lane + 32 * j] : f2bf(0.f);
+      za[i] = z[a.za_off + h];
+      zb[i] = z[a.zb_off + h];
+    }
+    const float rate = expf(a.p0[h]), bias = a.p1[h], qscale = 1.f / sqrtf((float)DK);
+#pragma unroll
+    for (int i = 0; i < TW; ++i) {
+      const int t = warp - 8 + 4 * i;
+      if (t >= n) break;
+      float qq = 0.f, kk = 0.f, kq = 0.f;
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        const float q = bf2f(qr[i][j]), k = bf2f(kr[i][j]);
+        qq = fmaf(q, q, qq);
+        kk = fmaf(k, k, kk);
+        kq = fmaf(k, q, kq);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        qq += __shfl_xor_sync(0xffffffffu, qq, o);
+        kk += __shfl_xor_sync(0xffffffffu, kk, o);
+        kq += __shfl_xor_sync(0xffffffffu, kq, o);
+      }
+      const float qf = qscale / sqrtf(qq + 1e-6f), kf = 1.f / sqrtf(kk + 1e-6f);
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        ks[t * DK + d0 + j] = bf2f(kr[i][j]) * kf;
+        qs[t * DK + d0 + j] = bf2f(qr[i][j]) * qf;
+      }
+#pragma unroll
+      for (int j = 0; j < VL; ++j) vs[t * FC + lane + 32 * j] = bf2f(vr[i][j]);
+      if (lane == 0) {
+        sc[t] = expf(-rate * softplusf_(za[i] + bias));
+        sc[kDeltaFew + t] = sigmoidf_(zb[i]);
+        sc[2 * kDeltaFew + t] = kq * qf * kf;
+      }
+    }
+    __syncthreads();
+    return;
+  }
+  const int ksi = warp % KS, c0 = (warp / KS) * 32 * VC + lane * VC;  // this lane's first column of each W
+  float* S_g = a.state + (size_t)a.slot[e] * a.slot_stride + (size_t)h * DK * vdim;  // [DK][vdim]
+  auto row_of = [&](int j) { return ((j >> 1) * KS + ksi) * 4 + (j & 1) * 2; };      // of the packed pair j: this row and the next
+  // columns c0 .. of block x: moved as pairs where they lie on 8-byte borders
+  const bool pairs = VC == 2 && (vdim & 1) == 0 && (reinterpret_cast<uintptr_t>(S_g) & 7) == 0;
+  F2 S[NB][VC][8];
+#pragma unroll
+  for (int x = 0; x < NB; ++x)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float v[2][VC];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int col = col0 + W * x + c0;
+        const float* p = S_g + (size_t)(row_of(j) + i) * vdim + col;
+        if (pairs) {
+          const float2 w = col < vdim ? *reinterpret_cast<const float2*>(p) : make_float2(0.f, 0.f);
+          v[i][0] = w.x;
+          v[i][VC - 1] = w.y;
+        } else {
+#pragma unroll
+          for (int c = 0; c < VC; ++c) v[i][c] = col + c < vdim ? p[c] : 0.f;
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < VC; ++c) S[x][c][j] = f2_pack(v[0][c], v[1][c]);
+    }
+  __syncthreads();
+  const size_t out_ld = (size_t)a.H * vdim;
+  float* out = a.out + (size_t)r0 * out_ld + h * vdim + col0 + c0;
+  for (int t = 0; t < n; ++t) {
+    const ulonglong2* kp = reinterpret_cast<const ulonglong2*>(ks + t * DK) + ksi;
+    const ulonglong2* qp = reinterpret_cast<const ulonglong2*>(qs + t * DK) + ksi;
+    const float g = sc[t], beta = sc[kDeltaFew + t], kq = sc[2 * kDeltaFew + t];
+    const F2 g1 = f2_pack(g, g);
+    float* pt = part + (t & 1) * 2 * KS * FC;
+    F2 kk[8], qk[8];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const ulonglong2 k2 = kp[m * KS], q2 = qp[m * KS];
+      kk[2 * m].v = k2.x;
+      kk[2 * m + 1].v = k2.y;
+      qk[2 * m].v = q2.x;
+      qk[2 * m + 1].v = q2.y;
+    }
+#pragma unroll
+    for (int x = 0; x < NB; ++x) {
+      float kv[VC], o[VC];
+#pragma unroll
+      for (int c = 0; c < VC; ++c) {
+        F2 k0{0}, k1{0}, o0{0}, o1{0};
+        F2(&s)[8] = S[x][c];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          s[2 * m] = f2_mul(s[2 * m], g1);
+          s[2 * m + 1] = f2_mul(s[2 * m + 1], g1);
+          k0 = f2_fma(s[2 * m], kk[2 * m], k0);
+          k1 = f2_fma(s[2 * m + 1], kk[2 * m + 1], k1);
+          o0 = f2_fma(s[2 * m], qk[2 * m], o0);
+          o1 = f2_fma(s[2 * m + 1], qk[2 * m + 1], o1);
+        }
+        const float2 c2 = f2_unpack(f2_add(k0, k1)), o2 = f2_unpack(f2_add(o0, o1));
+        kv[c] = c2.x + c2.y;
+        o[c] = o2.x + o2.y;
+      }
+      float* p = pt + ksi * FC + W * x + c0;
+      if constexpr (VC == 2) {
+        *reinterpret_cast<float2*>(p) = make_float2(kv[0], kv[1]);
+        *reinterpret_cast<float2*>(p + KS * FC) = make_float2(o[0], o[1]);
+      } else {
+        p[0] = kv[0];
+        p[KS * FC] = o[0];
+      }
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");  // (the buffer of two tokens ago has been read by all: they were at the last token's barrier)
+    auto sums = [&](const float* p, float (&r)[VC]) {  // over the KS warps, in the order of a butterfly
+      float v[KS][VC];
+#pragma unroll
+      for (int i = 0; i < KS; ++i) {
+        if constexpr (VC == 2) {
+          const float2 w = *reinterpret_cast<const float2*>(p + i * FC);
+          v[i][0] = w.x;
+          v[i][1] = w.y;
+        } else {
+          v[i][0] = p[i * FC];
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < VC; ++c) {
+#pragma unroll
+        for (int s = 1; s < KS; s <<= 1)
+#pragma unroll
+          for (int i = 0; i < KS; i += 2 * s) v[i][c] += v[i + s][c];
+        r[c] = v[0][c];
+      }
+    };
+#pragma unroll
+    for (int x = 0; x < NB; ++x) {
+      const int col = W * x + c0;
+      float kv[VC], u[VC];
+      sums(pt + col, kv);
+#pragma unroll
+      for (int c = 0; c < VC; ++c) {
+        u[c] = beta * (vs[t * FC + col + c] - kv[c]);
+        const F2 u2 = f2_pack(u[c], u[c]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) S[x][c][j] = f2_fma(kk[j], u2, S[x][c][j]);
+      }
+      if (ksi == (t & (KS - 1))) {  // the warps take turns at the read-outs
+        float o[VC];
+        sums(pt + KS * FC + col, o);
+#pragma unroll
+        for (int c = 0; c < VC; ++c)
+          if (col0 + col + c < vdim) out[(size_t)t * out_ld + W * x + c] = fmaf(kq, u[c], o[c]);
+      }
+    }
+  }
+#pragma unroll
+  for (int x = 0; x < NB; ++x)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float2 v[VC];
+#pragma unroll
+      for (int c = 0; c < VC; ++c) v[c] = f2_unpack(S[x][c][j]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int col = col0 + W * x + c0;
+        float* p = S_g + (size_t)(row_of(j) + i) * vdim + col;
+        if (pairs) {
+          if (col < vdim) *reinterpret_cast<float2*>(p) = i ? make_float2(v[0].y, v[VC - 1].y) : make_float2(v[0].x, v[VC - 1].x);
+        } else {
+#pragma unroll
+          for (int c = 0; c < VC; ++c)
+            if (col + c < vdim) p[c] = i ? v[c].y : v[c].x;
+        }
+      }
+    }
 }
 
-// The same CTAs with the tokens in chunks of 16 (delta_chunk.cuh).  A portion of up to kDeltaFew tokens costs less token by token: a chunk's time
-// does not shrink with its tokens.  Which of the two an entry takes follows from its own length.
-constexpr int kDeltaFew = 4;
+// The same CTAs with the tokens in chunks of 16 (delta_chunk.cuh).  A portion of up to `few` tokens costs less token by token: a chunk's time does not
+// shrink with its tokens.  `few` follows from the CTAs of the call (launch_delta_chunk); the two forms differ in the order of their fp32 sums.
 template <int DK>
-__global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_kernel(SeqArgs a, bool vec, unsigned int* err) {
+__global__ void __launch_bounds__(kDcThreads, 1) delta_chunk_kernel(SeqArgs a, bool vec, int few, int few_cols, unsigned int* err) {
   constexpr int COLS = 128 / (DK / 16);
   extern __shared__ __align__(16) float ds_sm[];
   pdl_wait();
   pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
-  const int e = blockIdx.x, h = blockIdx.y, kvh = h / (a.H / a.G), n = a.len[e], r0 = a.row0[e], col0 = blockIdx.z * COLS;
-  if (n <= kDeltaFew) {
-    if (threadIdx.x < 256) delta_tokens<bf16, DK, false>(a);
+  const int e = blockIdx.x, h = blockIdx.y, kvh = h / (a.H / a.G), n = a.len[e];
+  if (n <= few) {
+    if (blockIdx.z % (few_cols / COLS) != 0) return;
+    if (few_cols == 128) delta_few<DK, DK == 128 ? 2 : 1, 2>(a, ds_sm, n);
+    else if (few_cols == 64) delta_few<DK, DK == 128 ? 2 : 1, 1>(a, ds_sm, n);
+    else if constexpr (DK == 128) delta_few<DK, 1, 1>(a, ds_sm, n);
     return;
   }
+  const int r0 = a.row0[e], col0 = blockIdx.z * COLS;
   const bf16* x = static_cast<const bf16*>(a.qkv) + (size_t)r0 * a.ld;
   const DeltaRows rows{x + a.q_off + kvh * DK, x + a.k_off + kvh * DK, x + a.v_off + h * a.vdim + col0, a.ld, n, vec,
                        a.state + (size_t)a.slot[e] * a.slot_stride + (size_t)h * DK * a.vdim, a.vdim, col0, 1e-6f, 1.f / sqrtf((float)DK), err};
@@ -559,12 +773,21 @@ static cudaError_t launch_delta_t(const SeqArgs& a, int entries, cudaStream_t st
 template <int DK>
 static cudaError_t launch_delta_chunk(const SeqArgs& a, int entries, cudaStream_t st) {
   constexpr int COLS = 128 / (DK / 16);
-  constexpr size_t tokens = 2 * delta_stage_floats<DK, false>() * sizeof(float), chunks = DcSmem<DK, COLS>::BYTES;
-  constexpr size_t smem = tokens > chunks ? tokens : chunks;  // more than half of an SM's: one CTA on an SM
+  constexpr size_t smem = DcSmem<DK, COLS>::BYTES;  // (one CTA on an SM, by its registers)
+  static_assert(delta_few_floats<DK>(128) * sizeof(float) <= smem, "room for a portion of a few tokens");
   static std::atomic<uint64_t> smem_set{0};
   if (const cudaError_t e = allow_smem(smem_set, (const void*)delta_chunk_kernel<DK>, smem); e != cudaSuccess) return e;
   const bool vec = ((a.ld | a.q_off | a.k_off) & 7) == 0 && (reinterpret_cast<uintptr_t>(a.qkv) & 15) == 0;
-  return launch(delta_chunk_kernel<DK>, dim3(entries, a.H, (a.vdim + COLS - 1) / COLS), dim3(kDcThreads), smem, st, true, a, vec, wait_err_word());
+  // as many columns to a CTA of the few-token form as it takes for all to fit the GPU at once
+  const long heads = (long)entries * a.H;
+  int cols = DK == 128 ? 32 : 64;
+  while (cols < 128 && cols < a.vdim && heads * ((a.vdim + cols - 1) / cols) > sm_count()) cols *= 2;
+  // A wave of CTAs in chunks takes about as long as ten tokens in the few-token form, which needs fewer CTAs.  B200, us, few -> chunks, 16 heads of 128:
+  // one request (one wave) of 8 tokens 6.1 -> 7.2, of 12 7.6 -> 7.3;  two (two) of 12 8.5 -> 12.3, of 28 14.4 -> 13.9;  three (three) of 24 15.9 -> 19.3;
+  // six (six) of 8 13.5 -> 30.0, of 32 28.6 -> 36.4.  (delta_seq_kernel 6.5, 7.3, 9.4, 15.6, 15.1, 15.2, 32.3.)
+  const long ctas = heads * ((a.vdim + COLS - 1) / COLS), waves = (ctas + sm_count() - 1) / sm_count();
+  const int few = waves >= 4 ? kDeltaFew : 10 * (int)waves;
+  return launch(delta_chunk_kernel<DK>, dim3(entries, a.H, (a.vdim + COLS - 1) / COLS), dim3(kDcThreads), smem, st, true, a, vec, few, cols, wait_err_word());
 }
 template <typename E, bool CH>
 static int launch_delta(const SeqArgs& a, int entries, cudaStream_t st) {

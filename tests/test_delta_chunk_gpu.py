@@ -80,6 +80,29 @@ def test_lengths(lib, lens, D, V):
     assert off(got, want) < 6e-7 and off(gs, ws) < 6e-7
 
 
+@pytest.mark.parametrize("D,V", [(64, 64), (64, 129), (64, 300), (128, 128), (128, 65), (128, 200), (128, 3)])
+@pytest.mark.parametrize("lens", [[1, 1, 1, 1, 1, 1], [2, 1, 3, 4], [1, 40, 2], [10, 11, 9], [20, 21, 33], [31, 32, 33, 7, 1, 12]])
+@pytest.mark.parametrize("H,G", [(4, 2), (24, 12)])
+def test_few_tokens(lib, lens, H, G, D, V):
+    """Portions of a few tokens: value columns on both sides of what a CTA takes (one, two and all CTAs of a head), both forms in one call, lengths on both
+    sides of the choice for one to many waves of CTAs, unaligned pairs of columns."""
+    a = inputs(lens, H, G, D, V, 0.0, -1.0)
+    (got, gs), (want, ws) = launch(lib, *a, lens, H, G, D, V), wanted(*a, lens, H, G, D, V)
+    assert off(got, want) < 6e-7 and off(gs, ws) < 6e-7
+
+
+@pytest.mark.parametrize("D,V", [(64, 64), (64, 129), (128, 128), (128, 65)])
+def test_a_decoded_tokens_result_does_not_depend_on_the_call(lib, D, V):
+    """the same bits alone and beside other requests, whatever the columns to a CTA"""
+    lens, H, G = [1, 4, 2, 10, 1, 1, 3, 1, 1, 1, 1, 9], 16, 8
+    x, z, a_log, dt, S0 = inputs(lens, H, G, D, V, 0.0, -1.0)
+    got, gs = launch(lib, x, z, a_log, dt, S0, lens, H, G, D, V)
+    for i, n in enumerate(lens):
+        r = sum(lens[:i])
+        alone, alone_s = launch(lib, x[r:r + n], z[r:r + n], a_log, dt, S0[i:i + 1], [n], H, G, D, V)
+        assert torch.equal(alone, got[r:r + n]) and torch.equal(alone_s[0], gs[i])
+
+
 @pytest.mark.parametrize("alike", [0.5, 0.9, 1.0])
 @pytest.mark.parametrize("rate", [-8.0, -1.0, 2.5])
 def test_alike_keys_and_strong_decays(lib, alike, rate):
