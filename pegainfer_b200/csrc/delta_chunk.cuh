@@ -16,41 +16,13 @@
 // The other warps each prepare every kDcPrep-th chunk by themselves, start to end (rows by cp.async, Gram matrices, decay products, the triangle's
 // inverse by forward substitution with a lane per column), so that their latency is spread over kDcPrep chunks; they hand it over in a ring of stages.
 // Bound by the chain products -> sum over the warps -> triangle -> update (three barriers of the four warps a chunk); the figures stand where it is launched.
-// Sums over s <= t leave the later tokens out by selection, not by a factor of zero: a NaN or an infinity reaches the same tokens as token by token.
+// Sums over s <= t leave the later tokens out by selection, not by a factor of zero: a NaN reaches the same tokens as token by token, and so does an
+// infinity, as a NaN (its parts are differences of infinities).
 #pragma once
 #include "common.cuh"
 #include "mma.cuh"
 
 namespace pk {
-
-struct F2 {  // a packed pair of floats
-  unsigned long long v;
-};
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
-  F2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
-  F2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-  F2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_pack(float lo, float hi) {
-  F2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 f2_unpack(F2 a) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
-  return r;
-}
 
 constexpr int kDcT = 16;    // tokens per chunk
 constexpr int kDcPrep = 4;  // preparing warps = stages; with 12 warps a thread may hold 168 registers (four of them were enough to keep the state warps busy)

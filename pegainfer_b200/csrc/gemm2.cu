@@ -308,17 +308,6 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
   }
 }
 
-bool g2_make_map(CUtensorMap* map, const void* base, int rows, int K, int box_rows) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-  cuuint32_t box[2] = {(cuuint32_t)G2_BK, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 template <int BN, int NSUB, int STAGES>
 cudaError_t g2_launch(const CUtensorMap& mx, const CUtensorMap& mw, const G2Args& a, cudaStream_t stream) {
   constexpr size_t smem = (size_t)STAGES * (G2_BM * G2_BK * 2 + NSUB * (BN / 2) * G2_BK * 2) + 1024 + 256;
@@ -403,9 +392,9 @@ int launch_gemm_pair(const bf16* W, const bf16* X, bf16* Y, bf16* Y1, bf16* Y2, 
   if (best < 0) return -2;
   G2Args a{Y, Y1, Y2, e0, e1, M, N, K, swiglu, ldy};
   CUtensorMap mx, mw;
-  if (!g2_make_map(&mx, X, N, K, G2_BM)) return -2;
+  if (!make_rows_map(&mx, X, N, K, G2_BM)) return -2;
   const int rows_w = swiglu ? 2 * M : M;
-  if (!g2_make_map(&mw, W, rows_w, K, g2_widths[best].bn / 2)) return -2;
+  if (!make_rows_map(&mw, W, rows_w, K, g2_widths[best].bn / 2)) return -2;
   cudaError_t e;
   switch (best) {
     case 0: e = g2_launch<256, 1, 6>(mx, mw, a, stream); break;

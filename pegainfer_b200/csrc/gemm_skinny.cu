@@ -41,13 +41,6 @@ __device__ __forceinline__ float4 sk_ld_dsmem(uint32_t addr, uint32_t rank) {
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
   return v;
 }
-__device__ __forceinline__ void sk_tma_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-      "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-      : "memory");
-}
-
 // two CTAs on an SM: at most half of its shared memory each
 constexpr int SK_SMEM_MAX = 112 * 1024;
 constexpr size_t sk_smem(int rows, int nt, int stages) {
@@ -110,8 +103,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         if (!mbar_wait_bounded(empty + s, ph, dead)) break;
         mbar_expect_tx(full + s, STAGE_BYTES);
         uint8_t* st = smem + (size_t)s * STAGE_BYTES;
-        sk_tma_2d(st, &map_w, (kb0 + i) * SK_BK, m0, full + s);
-        sk_tma_2d(st + A_BYTES, &map_x, (kb0 + i) * SK_BK, t0, full + s);
+        tma_load_2d(st, &map_w, (kb0 + i) * SK_BK, m0, full + s);
+        tma_load_2d(st + A_BYTES, &map_x, (kb0 + i) * SK_BK, t0, full + s);
         if (++s == stages) {
           s = 0;
           ph ^= 1u;
@@ -216,17 +209,6 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   }
 }
 
-bool sk_make_map(CUtensorMap* map, const void* base, int rows, int K, int box_rows) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-  cuuint32_t box[2] = {(cuuint32_t)SK_BK, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 template <int NT>
 cudaError_t sk_launch(const CUtensorMap& mx, const CUtensorMap& mw, const SkArgs& a, int tiles, int splits, cudaStream_t stream) {
   auto kern = gemm_skinny_kernel<NT>;
@@ -266,7 +248,7 @@ struct SkPlan {
 // is the same, bit for bit, only if both take the same kernel (pk_b200_gemm_segments promises it from 129 tokens on).  The number of features must not
 // decide, then, wherever it could differ between the two: only reductions of 8192 or more (they come from a feed-forward's inner width; projections are
 // stacked over the hidden width) and fewer than 64 features (gates of a head each, no head's row is so short) come here.  What that gives up at 160
-// tokens: 2560 x 4096 18.9 -> 21.0.  Parts follow from K (4 from 4096 on, where they fit, else 2; 32 x 2560: 10.4 us, 14.5 in gemm2.cu).
+// tokens: 2560 x 4096 13.7 -> 16.4, 1024 x 4096 11.7 -> 15.4.  Parts follow from K (4 from 4096 on, where they fit, else 2; 32 x 2560: 10.4 us, 14.5 in gemm2.cu).
 // Measured on B200, us a launch in a train over cold weights (before: the split-K form of gemm.cu; from 129 tokens on gemm2.cu), M x K:
 //   tokens            8            48           128          160
 //   6144 x 2560   20.1 -> 9.5  19.9 -> 10.4  24.9 -> 12.6     (gemm2)
@@ -304,7 +286,7 @@ int sk_run(const bf16* W, const bf16* X, bf16* Y, bf16* Y1, bf16* Y2, int e0, in
   if (N > 128 && !sk_many_tokens(M, N, K, sm_count())) return -2;
   const int n_tiles = (N + NT - 1) / NT, tiles = ((M + p.rows - 1) / p.rows) * n_tiles;
   CUtensorMap mx, mw;
-  if (!sk_make_map(&mx, X, N, K, NT) || !sk_make_map(&mw, W, M, K, p.rows)) return -2;
+  if (!make_rows_map(&mx, X, N, K, NT) || !make_rows_map(&mw, W, M, K, p.rows)) return -2;
   const SkArgs a{Y, Y1, Y2, e0, e1, M, N, K, n_tiles, p.rows, p.stages, wait_err_word()};
   return (int)sk_launch<NT>(mx, mw, a, tiles, p.splits, stream);
 }

@@ -9,14 +9,13 @@
 //             is the maximum itself: the largest weight is then 1, which bf16 holds exactly -- behind a maximum that lags by up to 2^8 its rounding alone
 //             made the result's error 1.2 times as large for peaked scores; it saved 8 of 272 us)
 //   warp 4    MMA issuer     S = Q K^T (SS),  O += P V (A from TMEM, V = the key chunks read N-major)
-//   warp 5    TMA: Q once, then the pages of every key block
+//   warp 5    TMA: the item's Q, then the pages of every key block
 // Work item = (tile, run): the rows of a tile that belong to one request, with the tile's other rows masked, from an empty O.  What another request's
 // cache holds (a NaN times a weight of zero) never reaches a row, and requests that share a tile -- decoded tokens beside a prompt portion, each with a
 // context of its own -- do not wait for one another.  A tile's CTAs take its first run; the others, which start at a token whose first row is inside a
 // tile, go to the helper CTAs, every helpers-th token to the same ones, so that the decoded tokens of a step spread over the GPU.  A helper that finds
-// none ends at once.  Us, 16 heads, latent
-// 512 + 64 (walking a tile's runs one after the other; latent_attention_mma.cu for all): 2048-token portion + 8 tokens at contexts of 4096: 307 (2345;
-// 1169), 1000 + 24 tokens at 2000: 154 (1146; 444), 320 tokens at 1000: 376 (592; 334), a 2048-token prompt alone: 272 (270; 662).
+// none ends at once.  B200, us, 16 heads, latent 512 + 64 (a tile's runs one after the other; latent_attention_mma.cu for all): 2048-token portion beside
+// 8 tokens at contexts of 4096 307 (2345; 1169), 1000 beside 24 at 2000 154 (1146; 444), 320 tokens at 1000 376 (592; 334), 2048 alone 272 (271; 662).
 // Keys outside the run (slots behind the context's end, keys before the window) are masked in S, and their value rows are cleared in shared memory
 // before P V: they may hold anything.
 // Tensor-bound (operand reads of the narrow MMAs): 2 * rows * keys * (2 rank + rot) flop of result, 1.5 times that executed at rank 512.
@@ -49,12 +48,6 @@ struct LtArgs {
   unsigned int* err;
 };
 
-__device__ __forceinline__ void lt_tma_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-      "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-      : "memory");
-}
 __device__ __forceinline__ void lt_tma_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
@@ -156,7 +149,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
       if (q > 0) mbar_wait_bounded(&m.q_empty, (q - 1) & 1, dead);
       if (lane == 0) {
         mbar_expect_tx(&m.q_full, (uint32_t)(a.nc * LT_QC));
-        for (int c = 0; c < a.nc; ++c) lt_tma_2d(Qs + (size_t)c * LT_QC, &map_q, c * 64, r.R0, &m.q_full);
+        for (int c = 0; c < a.nc; ++c) tma_load_2d(Qs + (size_t)c * LT_QC, &map_q, c * 64, r.R0, &m.q_full);
       }
       ++q;
       auto page_of = [&](int b) { return pg[min((r.k0 + b * LT_KEYS + lane * box) / a.page_size, last)]; };  // behind the end: the last page again (masked)
@@ -357,13 +350,7 @@ int launch_latent_attention_tc(const bf16* qa, const bf16* cache, const bf16* si
   EncodeTiledFn fn = encode_fn();
   if (!fn) return -2;
   CUtensorMap mq, mk;
-  {
-    cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)D * 2};
-    cuuint32_t box[2] = {64, LT_ROWS}, estr[2] = {1, 1};
-    if (fn(&mq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16*>(qa), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return -2;
-  }
+  if (!make_rows_map(&mq, qa, rows, D, LT_ROWS)) return -2;
   {
     cuuint64_t dims[3] = {(cuuint64_t)D, (cuuint64_t)page_size, (cuuint64_t)1 << 30}, strides[2] = {(cuuint64_t)D * 2, (cuuint64_t)page_stride * 2};
     cuuint32_t box[3] = {64, (cuuint32_t)(page_size < LT_KEYS ? page_size : LT_KEYS), 1}, estr[3] = {1, 1, 1};

@@ -18,7 +18,6 @@
 #include <cuda.h>
 
 #include "common.cuh"
-#include "mma.cuh"
 #include "tcgen05.cuh"
 
 namespace pk {
@@ -136,13 +135,6 @@ constexpr int kMgStages = 4, kMgThreads = 192, kMgChunk = 32;  // chunk: rows of
 constexpr int kMgA = 128 * 64 * 2, kMgBox = 64 * 64 * 2, kMgStage = kMgA + kMoeTile * 64 * 2;
 constexpr size_t kMgSmem = (size_t)kMgStages * kMgStage + 1024 + kMgChunk * 128 * 2 + (2 * kMgStages + 5) * 8 + 16;
 
-__device__ __forceinline__ void mg_tma_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-      "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-      : "memory");
-}
-
 struct MgArgs {
   void* out;
   const int* meta;
@@ -205,8 +197,8 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
           ++fills;
           mbar_expect_tx(full + s, kMgA + boxes * kMgBox);
           uint8_t* st = smem + (size_t)s * kMgStage;
-          mg_tma_2d(st, &map_w, kb * 64, w0, full + s);
-          for (int b = 0; b < boxes; ++b) mg_tma_2d(st + kMgA + b * kMgBox, &map_x, kb * 64, m0 + b * 64, full + s);
+          tma_load_2d(st, &map_w, kb * 64, w0, full + s);
+          for (int b = 0; b < boxes; ++b) tma_load_2d(st + kMgA + b * kMgBox, &map_x, kb * 64, m0 + b * 64, full + s);
           if (++s == kMgStages) {
             s = 0;
             ph ^= 1u;
@@ -360,21 +352,10 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
   }
 }
 
-static bool mg_map(CUtensorMap* map, const void* base, long rows, int K, int box_rows) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-  cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 template <int EPI>
 static cudaError_t mg_launch(const void* rows, long n_rows, const void* w, const MgArgs& a, cudaStream_t st) {
   CUtensorMap mx, mw;
-  if (!mg_map(&mx, rows, n_rows, a.K, 64) || !mg_map(&mw, w, (long)a.experts * a.N, a.K, 128)) return cudaErrorInvalidValue;
+  if (!make_rows_map(&mx, rows, n_rows, a.K, 64) || !make_rows_map(&mw, w, (long)a.experts * a.N, a.K, 128)) return cudaErrorInvalidValue;
   auto kern = moe_grouped_gemm_kernel<EPI>;
   static std::atomic<uint64_t> smem_set{0};
   if (const cudaError_t e = allow_smem(smem_set, (const void*)kern, kMgSmem); e != cudaSuccess) return e;
