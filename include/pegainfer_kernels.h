@@ -179,7 +179,7 @@ const char* pk_b200_version(void);
 /* Number of kernels launched by this library on the calling thread since the last
  * reset (bench.py's gpu_launches; counts launches recorded into a capture too). */
 int64_t pk_b200_launch_count(int reset);
-/* Kernels of this process with a wait that ran into its iteration limit since the first cublas_init (0 in a sound run; the results of such a
+/* CTAs of this process's kernels with a wait that ran into its iteration limit, since the first cublas_init (0 in a sound run; the results of such a
  * launch are not valid).  Synchronises the device; -1: no cublas_init yet, or the device reports an error.  _seen does not synchronise (0 before
  * the first cublas_init): for a caller that has just waited for its stream.  The hosts read it behind every synchronisation and refuse all steps
  * of a model from the first run-out on. */
