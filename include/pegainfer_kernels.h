@@ -205,7 +205,7 @@ int pk_b200_gemm_swiglu(const pk_bf16* W, const pk_bf16* X, pk_bf16* Y, int M, i
  * pk_b200_gemm_segments / pk_b200_gemm_swiglu make internally): 128 / 160 / 192 / 224 / 256 / 320 = tile width of the CTA-pair kernel
  * (gemm2.cu), -2 = another one (gemm_skinny.cu, gemm.cu).  Shapes of few output tiles beyond 128 tokens go to gemm_skinny.cu
  * whatever this says.  Pure host arithmetic, no CUDA call: the wave-count
- * cost model calibrated on B200 measurements (profiles/README.md round 2) is pinned by a CPU test. */
+ * cost model calibrated on B200 measurements is pinned by a CPU test. */
 int pk_b200_gemm_plan(int M, int N, int K, int swiglu, int sms);
 
 /* GEMV with fused prologue/epilogue for decode (N == 1..4 tokens), one launch:

@@ -472,7 +472,7 @@ static int pick_max_chunks(int bs, int nkv, int nq, size_t scratch_floats) {
 }
 
 
-// PK_ATTN = tma (default: decode_attention_tma.cu) | cluster (round-1 LDG cluster kernel) | ticket (global-memory merge)
+// PK_ATTN = tma (default: decode_attention_tma.cu) | cluster (LDG cluster kernel) | ticket (global-memory merge)
 static int attention_impl() {
   static int v = -1;
   if (v < 0) {
@@ -483,7 +483,7 @@ static int attention_impl() {
 }
 static bool use_cluster_attention() { return attention_impl() >= 1; }
 static int launch_cluster_or_tma(const ClusterAttnArgs& c, int nkv, int bs, cudaStream_t stream) {
-  if (attention_impl() == 2) {  // (the L2-prefetch spans are an experiment of the round-1 cluster kernel only)
+  if (attention_impl() == 2) {  // (the L2-prefetch spans are an experiment of the LDG cluster kernel only)
     const int rc = launch_decode_attention_tma(c, nkv, bs, stream);
     if (rc != -2) return rc;
   }

@@ -6,7 +6,7 @@
 // merges inside the CTA through shared memory, then writes its (max, denominator, 4 x 128 numerators) straight
 // into the LEADER CTA's shared memory over DSMEM (st.shared::cluster), one cluster barrier, and the leader
 // produces the bf16 output.  Compared with the ticket version in decode_attention.cu (profiles/README.md,
-// round 1 v3: 22 us per layer, of which the partial-store -> __threadfence -> atomic ticket -> L2 re-read chain
+// the kernel before it: 22 us per layer, of which the partial-store -> __threadfence -> atomic ticket -> L2 re-read chain
 // is 3-4 dependent global round trips) there is no global-memory synchronisation at all.
 // The CTA that owns the step's position also appends the normed/roped K and the V row to the paged cache and
 // injects the new token from shared memory.  Arithmetic and rounding points: see decode_attention.cu.

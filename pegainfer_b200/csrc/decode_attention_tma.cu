@@ -1,6 +1,6 @@
-// Fused decode attention, round-2 design: TMA page tiles + tensor-core (mma.sync) score / PV products.
+// Fused decode attention: TMA page tiles + tensor-core (mma.sync) score / PV products.
 //
-// Why: the round-1 cluster kernel (decode_attention_cluster.cu) reads K/V with per-lane LDGs and reduces every
+// Why: the LDG cluster kernel (decode_attention_cluster.cu) reads K/V with per-lane LDGs and reduces every
 // q.k product with a 4-level shuffle tree -- ncu (profiles/r1_v4_attn_cluster_full_details.txt) shows ~215 issued
 // instructions per token row and 2 warps per scheduler: latency-bound on its own instruction stream (6.8 cycles per
 // issue), 6 % of DRAM bandwidth, 64 CTAs on 148 SMs.  Here:
@@ -484,7 +484,7 @@ TmaAttnConfig& tma_attn_config() {
 
 }  // namespace
 
-// Returns cudaError as int; -2 when this kernel cannot take the call (caller falls back to the round-1 kernels).
+// Returns cudaError as int; -2 when this kernel cannot take the call (caller falls back to the other kernels).
 int launch_decode_attention_tma(const ClusterAttnArgs& c, int nkv, int bs, cudaStream_t stream) {
   TmaAttnConfig& cfg = tma_attn_config();
   if (!cfg.ok) return -2;

@@ -242,7 +242,7 @@ int launch_gemm_pair(const bf16* W, const bf16* X, bf16* Y, bf16* Y1, bf16* Y2, 
                      cudaStream_t stream);
 // gemm_skinny.cu: few output tiles, K cut over the CTAs of a cluster; -2 = not for this kernel
 int launch_gemm_skinny(const bf16* W, const bf16* X, bf16* Y, bf16* Y1, bf16* Y2, int e0, int e1, int M, int N, int K, cudaStream_t stream);
-static bool gemm_pair_enabled() {  // PK_GEMM_PAIR=0 keeps the round-1 single-CTA kernel for A/B runs
+static bool gemm_pair_enabled() {  // PK_GEMM_PAIR=0 keeps the single-CTA kernel for A/B runs
   static int v = -1;
   if (v < 0) {
     const char* e = getenv("PK_GEMM_PAIR");
@@ -267,7 +267,7 @@ void launch_gemm_seg(const bf16* W, const bf16* X, bf16* Y, bf16* Y1, bf16* Y2, 
   if (tma_ok && gemm_impl_mode() == 0) {
     // Tile width by wave count: tiles = ceil(N/128) * ceil(M/BN) on `sms` persistent CTAs; cost ~ waves * (BN + c).
     // M = 2560 outputs (o_proj / down_proj of Qwen3-4B) at 2048 tokens: BN 256 -> 160 tiles = 2 waves of 256-wide
-    // tiles, BN 160 -> 256 tiles = 2 waves of 160-wide tiles (profiles/README.md, r1 v3: tile quantisation).
+    // tiles, BN 160 -> 256 tiles = 2 waves of 160-wide tiles (tile quantisation).
     const int m_tiles = (N + BM - 1) / BM;
     const int sms = sm_count();
     int best_bn = 256;

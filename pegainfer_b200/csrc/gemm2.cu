@@ -1,6 +1,6 @@
-// Prefill GEMM on CTA PAIRS: Y[M, N] = W[M, K] x X[K, N] with tcgen05.mma.cta_group::2 (round 2).
+// Prefill GEMM on CTA PAIRS: Y[M, N] = W[M, K] x X[K, N] with tcgen05.mma.cta_group::2.
 //
-// Why: the round-1 kernel (gemm.cu, cta_group::1, M128 x N256 x K16 per instruction) reads 12 KB of operands from
+// Why: the single-CTA kernel (gemm.cu, cta_group::1, M128 x N256 x K16 per instruction) reads 12 KB of operands from
 // shared memory per 128-cycle instruction and TMA writes another 12 KB: ~190 B/clk against a 128 B/clk shared-memory
 // port.  ncu (profiles/r1_v3_gemm_full_details.txt) shows the tensor pipe 61-64 % active and cuBLAS' sm_100 kernels
 // 1.27-1.53 PFLOP/s against our 0.77-1.20 on the same shapes.  A CTA pair (two SMs of one TPC) computes a
@@ -372,7 +372,7 @@ static int g2_plan(int M, int N, int K, int swiglu, int sms) {
   if (!swiglu) {  // is the single-CTA kernel (gemm.cu: 128-token tiles of width 256 / 160 / 128 on every SM) strictly better?
     // One cost unit of the single-CTA kernel takes 1.75-2.3 x as long as one of the pair kernel (it is bound by its own
     // shared-memory port, see the header): at 2048 tokens o_proj 80.8 us (2 waves of 160-wide tiles, 384 units) vs 46.5 us
-    // for the pair's one wave of 320-wide tiles (458 units), down_proj 173 vs 88 us (profiles/README.md round 2).  Without
+    // for the pair's one wave of 320-wide tiles (458 units), down_proj 173 vs 88 us.  Without
     // the factor the model sent both back to the single-CTA kernel (r2_v3_prefill_decode_launches.csv: 2 x 89 us per layer).
     const long m1 = (N + G2_BM - 1) / G2_BM;
     const int w1[3] = {256, 160, 128};

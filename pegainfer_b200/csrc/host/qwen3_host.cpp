@@ -903,7 +903,7 @@ bool Qwen3Model::decode_kernels_fused(int bs) {
     const char* e = getenv("PK_TP_MODE");
     if (e && strcmp(e, "kernel") == 0) return 0;
     if (e && strcmp(e, "fused") == 0) return 1;
-    const char* f = getenv("PK_TP_FUSED");  // round-1 switch
+    const char* f = getenv("PK_TP_FUSED");  // A/B switch
     if (f && !e) return atoi(f) > 0 ? 1 : 0;
     return 2;
   }();

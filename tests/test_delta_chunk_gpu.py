@@ -63,7 +63,7 @@ def launch(lib, x, z, a_log, dt, S0, lens, H, G, D, V):
     assert lib.pk_gated_delta_seq(x.data_ptr(), x.stride(0), 0, G * D, 2 * G * D, z.data_ptr(), 2 * H, 0, H, a_log.data_ptr(), dt.data_ptr(), state.data_ptr(),
                                   H * D * V, slot.data_ptr(), row0.data_ptr(), ln.data_ptr(), out.data_ptr(), H, G, D, V, len(lens), 0, None) == 0
     torch.cuda.synchronize()
-    assert (out[-1] == 5.0).all()
+    assert (out[-1] == 5.0).all() and lib.pk_b200_wait_errors() == 0
     return out[:-1].view(-1, H, V), state
 
 

@@ -7,7 +7,7 @@ Attention: the reference's own case (1 layer, nq 32, nkv 8, hd 128, page 16, bs 
 4096*seq + 16 KiB, seq in {1, 128, 1024, 4096}.  When oracle/_ref/libkernels_ref.so is present the reference's own
 kernels (cuBLAS GEMV, FlashInfer decode) are timed beside ours under the same protocol.
 
-Round 2 adds the `train` protocol next to the single-launch one (single CUDA-event launches quantise to ~2 us and
+The `train` protocol stands next to the single-launch one (single CUDA-event launches quantise to ~2 us and
 cannot resolve the small shapes): N >= 32 launches over N DISTINCT cold buffers (together >= 2 x L2, after an L2
 sweep), captured into ONE CUDA graph so no host launch gap sits between them, one event pair around the replay;
 per-launch time = total / N.  For our library it is reported with programmatic dependent launch off and on (on = what
