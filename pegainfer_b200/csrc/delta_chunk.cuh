@@ -16,6 +16,9 @@
 // The other warps each prepare every kDcPrep-th chunk by themselves, start to end (rows by cp.async, Gram matrices, decay products, the triangle's
 // inverse by forward substitution with a lane per column), so that their latency is spread over kDcPrep chunks; they hand it over in a ring of stages.
 // Bound by the chain products -> sum over the warps -> triangle -> update (three barriers of the four warps a chunk); the figures stand where it is launched.
+// The roles' loops run side by side and have to share the SM's instruction cache: with the preparation unrolled to the end every role waited for its
+// instructions (hit rate 0.69 in one form), so its loops are rolled as far as their latency allows; keys of 64 gain nothing by it.  2048 tokens, 16 heads of 128: 173 -> 149 us,
+// 1024 tokens, 32 heads, 32 columns to a CTA: 180 -> 107 us, 24 tokens 7.4 -> 6.8 us (B200, the kernel alone; same sums in the same order).
 // Sums over s <= t leave the later tokens out by selection, not by a factor of zero: a NaN reaches the same tokens as token by token, and so does an
 // infinity, as a NaN (its parts are differences of infinities).
 #pragma once
@@ -51,8 +54,9 @@ struct DcSmem {
   static constexpr int CQ = CK + kDcT;                 // c_t qf_t
   static constexpr int CS = CQ + kDcT;                 // r(16, s) kf_s
   static constexpr int GC = CS + kDcT;                 // c_16 (4 floats)
-  static constexpr int GM = GC + 4;                    // scratch: [2][16][17] k . k and q . k, then A [16][16]
-  static constexpr int FT = GM + 2 * kDcT * 17;        // scratch: beta_t kf_t, qf_t, decays
+  static constexpr int GM = GC + 4;                    // scratch: [2][16][17] k . k and q . k
+  static constexpr int AM = GM + 2 * kDcT * 17;        // scratch: A [16][16]
+  static constexpr int FT = AM + 256;                  // scratch: beta_t kf_t, qf_t, decays
   static constexpr int STAGE = FT + 3 * kDcT;
   // the four state warps
   static constexpr int WLD = kDcT + 4;                 // a column's 16 tokens, 16-byte reads without conflicts
@@ -64,7 +68,7 @@ struct DcSmem {
   static constexpr int BARS = UB + 3 * COLS * UBLD / 2;
   static constexpr int FLOATS = BARS + 4 * kDcPrep + 4;
   static constexpr size_t BYTES = (size_t)FLOATS * 4;
-  static_assert(STAGE % 4 == 0 && PK % 4 == 0 && W % 4 == 0 && UB % 4 == 0 && BARS % 2 == 0, "alignment");
+  static_assert(STAGE % 4 == 0 && AM % 4 == 0 && PK % 4 == 0 && W % 4 == 0 && UB % 4 == 0 && BARS % 2 == 0, "alignment");
 };
 
 // x = hi + mid + lo, bf16 each: cut off after 8 and 16 of the 24 bits, so the sum is exact (for finite x that does not underflow)
@@ -102,6 +106,7 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
   if (warp >= 8) {
     // ---- preparation
     constexpr int PR = DK / 8, NVL = kDcT * COLS / 32;  // 16-byte pieces per row; values per lane
+    constexpr int ROLL_P = DK > 64 ? 4 : 8, ROLL_T = DK > 64 ? 8 : 16, ROLL_I = DK > 64 ? 1 : 4;  // rows of 64 leave room for more
     const int pw = warp - 8, half = lane >> 4, s = lane & 15;
     float* st = sm + pw * L::STAGE;
     bf16* raw = reinterpret_cast<bf16*>(st + L::RAW);
@@ -110,18 +115,22 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
       const int t0 = b * kDcT, nb = min(kDcT, n - t0);  // tokens past the end: zero rows, decay 1, write strength 0
       mbar_wait_bounded(empty + pw, ph, dead);
       __syncwarp();
-#pragma unroll
-      for (int i = 0; i < PR; ++i) {
-        const int p = lane + 32 * i, row = p / PR, c = (p % PR) * 8, t = row & (kDcT - 1);
-        const bf16* src = (row < kDcT ? a.k : a.q) + (size_t)(t0 + t) * a.ld + c;
-        bf16* dst = raw + row * LDR + c;
-        if (t >= nb) {
-          *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
-        } else if (a.vec) {
-          cp_async16(dst, src);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) dst[j] = src[j];
+      if (a.vec) {
+        const bf16* src = a.k + (size_t)t0 * a.ld + lane % PR * 8;
+        const ptrdiff_t to_q = a.q - a.k;
+        bf16* dst = raw + lane / PR * LDR + lane % PR * 8;
+#pragma unroll ROLL_P
+        for (int t = lane / PR; t < kDcT; t += 32 / PR, dst += 32 / PR * LDR) {
+          const bf16* row = src + (ptrdiff_t)min(t, nb - 1) * a.ld;
+          const uint32_t bytes = t < nb ? 16 : 0;  // zeros behind the end
+          cp_async16(dst, row, bytes);
+          cp_async16(dst + kDcT * LDR, row + to_q, bytes);
+        }
+      } else {
+#pragma unroll 8
+        for (int i = lane; i < 2 * kDcT * DK; i += 32) {
+          const int row = i / DK, t = row & (kDcT - 1);
+          raw[row * LDR + i % DK] = t < nb ? (row < kDcT ? a.k : a.q)[(size_t)(t0 + t) * a.ld + i % DK] : f2bf(0.f);
         }
       }
       cp_async_commit();
@@ -146,7 +155,7 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
       __syncwarp();
       // unit factors: lane = row
       float d[4] = {};
-#pragma unroll
+#pragma unroll ROLL_P
       for (int i = 0; i < PR; ++i) {
         const uint4 u = *reinterpret_cast<const uint4*>(raw + lane * LDR + i * 8);
         d[0] = fmaf(bf16_lo(u.x), bf16_lo(u.x), d[0]);
@@ -185,27 +194,19 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
         }
       __syncwarp();
       // lanes 0-15: column s of A;  16-31: column s of B
-      float gt[kDcT], f[kDcT], gm[kDcT];
-#pragma unroll
-      for (int t = 0; t < kDcT; t += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(st + L::FT + 2 * kDcT + t), y = *reinterpret_cast<const float4*>(st + L::FT + half * kDcT + t);
-        gt[t] = x.x; gt[t + 1] = x.y; gt[t + 2] = x.z; gt[t + 3] = x.w;
-        f[t] = y.x; f[t + 1] = y.y; f[t + 2] = y.z; f[t + 3] = y.w;
-      }
-#pragma unroll
-      for (int t = 0; t < kDcT; ++t) gm[t] = st[L::GM + half * kDcT * 17 + t * 17 + s];
       float r = 1.f, c = 1.f, cs = 1.f;
-#pragma unroll
-      for (int t = 0; t < kDcT; ++t) {
-        r = t > s ? r * gt[t] : r;
-        c *= gt[t];
-        cs = t == s ? c : cs;
-        gm[t] = t > s || (half && t == s) ? (f[t] * kf) * r * gm[t] : 0.f;
+      {
+        const float* gm = st + L::GM + half * kDcT * 17 + s;
+        float* to = st + (half ? L::BM : L::AM) + s;
+#pragma unroll ROLL_T
+        for (int t = 0; t < kDcT; ++t) {
+          const float gt = st[L::FT + 2 * kDcT + t], f = st[L::FT + half * kDcT + t], m = gm[t * 17];
+          r = t > s ? r * gt : r;
+          c *= gt;
+          cs = t == s ? c : cs;
+          to[t * kDcT] = t > s || (half && t == s) ? (f * kf) * r * m : 0.f;
+        }
       }
-      __syncwarp();  // the Gram matrices have been read
-      float* to = half ? st + L::BM : st + L::GM;
-#pragma unroll
-      for (int t = 0; t < kDcT; ++t) to[t * kDcT + s] = gm[t];
       st[(half ? L::CQ : L::CK) + s] = ft * cs;
       if (half == 0) st[L::CS + s] = r * kf;
       if (lane == 0) st[L::GC] = c;
@@ -215,23 +216,30 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
         st[L::VB + at] = __shfl_sync(0xffffffffu, beta, at / COLS) * bf2f(vr[i]);
       }
       __syncwarp();
-      float T[kDcT];  // column s of (I + A)^-1
+      // column s of (I + A)^-1, four rows at a time (both halves of the warp alike)
+#pragma unroll ROLL_I
+      for (int t = 0; t < kDcT; t += 4) {
+        const float4* A = reinterpret_cast<const float4*>(st + L::AM + t * kDcT);
+        float x[4];
 #pragma unroll
-      for (int t = 0; t < kDcT; ++t) {
-        float acc = t == s ? 1.f : 0.f;
+        for (int i = 0; i < 4; ++i) x[i] = t + i == s ? 1.f : 0.f;
+#pragma unroll ROLL_I
+        for (int j = 0; j < t; j += 4) {
+          float y[4];
 #pragma unroll
-        for (int s4 = 0; s4 < t; s4 += 4) {
-          const float4 x = *reinterpret_cast<const float4*>(st + L::GM + t * kDcT + s4);
-          acc = fmaf(-x.x, T[s4], acc);
-          if (s4 + 1 < t) acc = fmaf(-x.y, T[s4 + 1], acc);
-          if (s4 + 2 < t) acc = fmaf(-x.z, T[s4 + 2], acc);
-          if (s4 + 3 < t) acc = fmaf(-x.w, T[s4 + 3], acc);
+          for (int i = 0; i < 4; ++i) y[i] = st[L::TM + (j + i) * kDcT + s];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float4 w = A[i * 4 + (j >> 2)];
+            x[i] = fmaf(-w.w, y[3], fmaf(-w.z, y[2], fmaf(-w.y, y[1], fmaf(-w.x, y[0], x[i]))));
+          }
         }
-        T[t] = acc;
-      }
-      if (half == 0) {
+        const float4 w1 = A[4 + (t >> 2)], w2 = A[8 + (t >> 2)], w3 = A[12 + (t >> 2)];
+        x[1] = fmaf(-w1.x, x[0], x[1]);
+        x[2] = fmaf(-w2.y, x[1], fmaf(-w2.x, x[0], x[2]));
+        x[3] = fmaf(-w3.z, x[2], fmaf(-w3.y, x[1], fmaf(-w3.x, x[0], x[3])));
 #pragma unroll
-        for (int t = 0; t < kDcT; ++t) st[L::TM + t * kDcT + s] = T[t];
+        for (int i = 0; i < 4; ++i) st[L::TM + (t + i) * kDcT + s] = x[i];
       }
       mbar_arrive(full + pw);
     }

@@ -158,3 +158,18 @@ def test_hybrid_entry(lib, T, shift):
     o, S = rule(q, k, x[:, 2 * nk * 128:].view(T, nv, 128), dec, torch.sigmoid(b.double()), S0.double())
     assert off(state, S) < 6e-7
     assert ((out.view(T, nv, 128).double() - o).abs() <= o.abs() * 2 ** -8 + o.abs().max() * 1e-5).all()  # one bf16 rounding
+
+
+@pytest.mark.parametrize("n", [1, 3, 15, 17, 31])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_rows_behind_the_end_are_never_read(lib, n, D, aligned):
+    """the last chunk's missing tokens: zeros, whatever lies behind the portion (here NaN), by asynchronous copies and one by one; after a whole chunk, so
+    that the chunk form takes it"""
+    H, G, V, lens = 4, 2, D, [32 + n]
+    x, z, a_log, dt, S0 = inputs([lens[0] + 16], H, G, D, V, 0.0, -1.0, ld_extra=0 if aligned else 3)
+    want, ws = wanted(x[:lens[0]], z[:lens[0]], a_log, dt, S0, lens, H, G, D, V)
+    x[lens[0]:] = float("nan")
+    z[lens[0]:] = float("nan")
+    got, gs = launch(lib, x, z, a_log, dt, S0, lens, H, G, D, V)
+    assert off(got, want) < 6e-7 and off(gs, ws) < 6e-7
