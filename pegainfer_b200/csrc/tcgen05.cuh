@@ -130,6 +130,12 @@ __device__ __forceinline__ void tmem_put32(uint32_t taddr, const uint32_t* v) {
       "r"(v[31])
       : "memory");
 }
+__device__ __forceinline__ void tmem_put16(uint32_t taddr, const uint32_t* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
+               "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]),
+               "r"(v[14]), "r"(v[15])
+               : "memory");
+}
 __device__ __forceinline__ void tmem_put_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // generic-proxy shared-memory writes (st.shared, cp.async) -> visible to the async proxy (tcgen05.mma operand reads)
 __device__ __forceinline__ void fence_proxy_async_smem() {

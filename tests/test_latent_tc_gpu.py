@@ -21,6 +21,17 @@ def lib():
     ([0], [700], 16, 0, 16, False), ([0, 130, 5], [300, 333, 67], 16, 0, 16, True), ([500, 0], [400, 301], 16, 150, 8, True),
     ([40], [1300], 8, 64, 32, False), ([0] * 40, [17 + i for i in range(40)], 10, 0, 128, True), ([3, 900], [640, 1], 16, 1000, 64, False)])
 def test_against_64_bits(lib, starts, lens, H, window, ps, sink, rank, rot):
+    check_against_64_bits(lib, starts, lens, H, window, ps, sink, rank, rot)
+
+
+# other chunks of a CTA from none to eight (rings of 2, 8, 9, 7, 5 and 3 places), value chunks from one to four, and both in one launch
+@pytest.mark.parametrize("rank,rot", [(256, 0), (64, 64), (448, 64), (384, 48), (512, 16), (192, 384), (128, 448), (64, 512)])
+@pytest.mark.parametrize("starts,lens,H,window,ps,sink", [([0, 77], [900, 301], 16, 0, 16, True), ([300, 0, 9], [1, 700, 340], 16, 130, 128, False)])
+def test_places_for_chunks(lib, starts, lens, H, window, ps, sink, rank, rot):
+    check_against_64_bits(lib, starts, lens, H, window, ps, sink, rank, rot)
+
+
+def check_against_64_bits(lib, starts, lens, H, window, ps, sink, rank, rot):
     D, T = rank + rot, sum(lens)
     g = torch.Generator(device="cuda").manual_seed(T + rank)
     rn = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
