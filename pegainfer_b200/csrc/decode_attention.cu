@@ -608,6 +608,10 @@ static int decode_attention_fused_impl(
       c.pf[c.npf++] = PfSpan{static_cast<const uint8_t*>(sp.base), sp.rows, sp.row_bytes, sp.slices, sp.prefetch_rows};
     }
     c.pf_y = prefetch_cluster_rows();
+    if (attention_impl() == 2) {
+      const int rc = launch_decode_attention_flat(c, num_kv_heads, batch_size, partial_scratch, (long)batch_size * (max_chunks > 0 ? max_chunks : 1), counters, stream);
+      if (rc != -2) return rc;
+    }
     return launch_cluster_or_tma(c, num_kv_heads, batch_size, stream);
   }
   DecodeAttnArgs a{};

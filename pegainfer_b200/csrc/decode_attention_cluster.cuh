@@ -31,5 +31,7 @@ cudaError_t launch_decode_attention_cluster(const ClusterAttnArgs& a, int nkv, i
 // the default kernel (decode_attention_tma.cu): TMA page tiles + mma.sync, up to 16-CTA clusters.  Same argument block
 // (prefetch spans ignored).  Returns a cudaError, or -2 when it cannot take the call.
 int launch_decode_attention_tma(const ClusterAttnArgs& a, int nkv, int bs, cudaStream_t stream);
+// decode_attention_flat.cu: many requests, equal runs of pages for every SM.  -2: not a call for it
+int launch_decode_attention_flat(const ClusterAttnArgs& a, int nkv, int bs, float* partial, long places, int* counters, cudaStream_t stream);
 
 }  // namespace pk
