@@ -569,6 +569,295 @@ __global__ void gqa_attention_merge_kernel(const float* __restrict__ part_o, con
   }
 }
 
+// ---- fewer than 64 rows (decode steps, small portions), bf16: a cluster of CTAs per (tokens of one request, kv head).  The 16 rows of a tile are the group's
+// query heads, for as many tokens of the request as fit (a cluster is launched for every token, and the first of each tile's stays), so that a key is fetched
+// once for all of them and requests do not wait for one another.  A warp takes every (4 cs)-th tile of 16 visible keys through a cp.async ring of its own;
+// the warps' states meet in shared memory, the CTAs' in the cluster's.
+// Bound by latency: lookups, keys, exchange.  Figures at launch_gqa_mma.
+constexpr int kGdWarps = 4, kGdRing = 3;
+__device__ __forceinline__ uint32_t gd_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void gd_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float2 gd_remote(const float2* p, uint32_t rank) {  // the same place in another CTA of the cluster
+  uint32_t at;
+  float2 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(at) : "memory");
+  return v;
+}
+
+template <int D>
+__global__ void __launch_bounds__(kGdWarps * 32, 2) gqa_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache, const bf16* __restrict__ sink,
+                                                                    const int* __restrict__ pos, const int* __restrict__ req, const int* __restrict__ page_off,
+                                                                    const int* __restrict__ pages, bf16* __restrict__ out, long page_stride, int page_size, int T,
+                                                                    int H, int G, float scale, int chunk, AttnExtra x) {
+  constexpr int LD = D + 8, TILE = 16 * LD;
+  extern __shared__ __align__(16) unsigned char gd_smem[];  // [warps][ring][K, V][16][LD]; later the states, [warps][16][D] floats at the warps' rings
+  __shared__ long long s_off[kGdWarps][kGdRing][16];
+  __shared__ float2 s_ml[kGdWarps][16];  // (maximum, sum) of the warps' rows; later of the CTA's
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gq = lane >> 2, tq = lane & 3;
+  const int rank = (int)gd_rank(), cs = gridDim.x, g = blockIdx.y, t = blockIdx.z, R = H / G, per = 16 / R;
+  pdl_wait();
+  pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
+  // the tokens of this one's request around it
+  const int rq = req[t], r0 = lane < T ? req[lane] : -1, r1 = lane + 32 < T ? req[lane + 32] : -1;
+  const unsigned long long other = (unsigned long long)__ballot_sync(0xffffffffu, lane >= T || r0 != rq) |
+                                   (unsigned long long)__ballot_sync(0xffffffffu, lane + 32 >= T || r1 != rq) << 32;
+  const unsigned long long below = other & ((1ull << t) - 1), above = other >> t;  // (T < 64: there is one above)
+  const int start = below ? 64 - __clzll((long long)below) : 0, left = __ffsll((long long)above) - 1;
+  if ((t - start) % per != 0) return;  // (the whole cluster)
+  const int n_tok = min(per, left);
+  const int p_max = pos[t + n_tok - 1], lo = first_visible(pos[t], chunk, x.window), nf = min(x.keep_first, lo), n_vis = nf + p_max - lo + 1;
+  const int* pg = pages + page_off[rq];
+  const int tok = 2 * G * D, n_tiles = (n_vis + 15) / 16, step = cs * kGdWarps;
+  bf16* ring = reinterpret_cast<bf16*>(gd_smem) + warp * kGdRing * 2 * TILE;
+  auto key_of = [&](int i) { return i < nf ? i : lo + i - nf; };  // position of visible key i
+  auto load = [&](int tile, int st) {
+    if (tile < n_tiles) {
+      if (lane < 16) {
+        const int i = tile * 16 + lane, j = key_of(i);
+        s_off[warp][st][lane] = i < n_vis ? (long long)pg[j / page_size] * page_stride + (long long)(j % page_size) * tok + g * D : -1;
+      }
+      __syncwarp();
+      bf16* dst = ring + st * 2 * TILE;
+#pragma unroll
+      for (int c = lane; c < 16 * (D / 8); c += 32) {
+        const int r = c / (D / 8), cc = (c % (D / 8)) * 8;
+        const long long at = s_off[warp][st][r];
+        const bf16* src = cache + (at < 0 ? 0 : at) + cc;
+        const uint32_t bytes = at < 0 ? 0 : 16;  // zeros behind the last key
+        cp_async16(dst + r * LD + cc, src, bytes);
+        cp_async16(dst + TILE + r * LD + cc, at < 0 ? src : src + G * D, bytes);
+      }
+    }
+    cp_async_commit();
+  };
+  int tile = rank * kGdWarps + warp;
+#pragma unroll
+  for (int s = 0; s < kGdRing; ++s) load(tile + s * step, s);
+  // rows gq and gq + 8: (token, head) of the group
+  const int ta = gq / R, tb = (gq + 8) / R, ha = g * R + gq % R, hb = g * R + (gq + 8) % R;
+  const bool on_a = ta < n_tok, on_b = tb < n_tok;  // (n_tok <= per: rows behind R * per are off)
+  const int pos_a = on_a ? pos[t + ta] : -1, pos_b = on_b ? pos[t + tb] : -1;
+  uint32_t qa[D / 16][4];
+#pragma unroll
+  for (int kk = 0; kk < D / 16; ++kk) {
+    const bf16* qra = q + ((size_t)(t + (on_a ? ta : 0)) * H + ha) * D + kk * 16 + 2 * tq;
+    const bf16* qrb = q + ((size_t)(t + (on_b ? tb : 0)) * H + hb) * D + kk * 16 + 2 * tq;
+    qa[kk][0] = on_a ? *reinterpret_cast<const uint32_t*>(qra) : 0u;
+    qa[kk][1] = on_b ? *reinterpret_cast<const uint32_t*>(qrb) : 0u;
+    qa[kk][2] = on_a ? *reinterpret_cast<const uint32_t*>(qra + 8) : 0u;
+    qa[kk][3] = on_b ? *reinterpret_cast<const uint32_t*>(qrb + 8) : 0u;
+  }
+  // scores in units of log2, shaped as in the kernel above
+  const bool capped = x.softcap > 0.f;
+  const float cap2 = x.softcap * kLog2e, c1 = capped ? 2.f * scale / x.softcap * kLog2e : scale * kLog2e;
+  const float slope_a = head_slope(x.slope_log2, ha, H) * kLog2e, slope_b = head_slope(x.slope_log2, hb, H) * kLog2e;
+  const int lo_a = on_a ? first_visible(pos_a, chunk, x.window) : 0, lo_b = on_b ? first_visible(pos_b, chunk, x.window) : 0;
+  float oa[D / 8][4] = {};
+  float m_a = -INFINITY, m_b = -INFINITY, l_a = 0.f, l_b = 0.f;
+  for (int st = 0; tile < n_tiles; tile += step) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kGdRing - 1) : "memory");
+    __syncwarp();
+    const bf16 *Ks = ring + st * 2 * TILE, *Vs = Ks + TILE;
+    float s[2][4] = {}, s1[2][4] = {};  // even and odd k steps apart
+#pragma unroll
+    for (int kk = 0; kk < D / 16; ++kk) {
+      uint32_t b[4];
+      ldsm_x4(b, &Ks[((lane & 7) + ((lane >> 4) & 1) * 8) * LD + kk * 16 + ((lane >> 3) & 1) * 8]);
+      mma_bf16_16816(kk & 1 ? s1[0] : s[0], qa[kk], b[0], b[1]);
+      mma_bf16_16816(kk & 1 ? s1[1] : s[1], qa[kk], b[2], b[3]);
+    }
+    float mx_a = -INFINITY, mx_b = -INFINITY;
+#pragma unroll
+    for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = tile * 16 + ni * 8 + 2 * tq + (e & 1), j = key_of(i);
+        const bool top = e < 2;
+        const int dist = (top ? pos_a : pos_b) - j;
+        const bool ok = i < n_vis && dist >= 0 && (j >= (top ? lo_a : lo_b) || j < x.keep_first);
+        float v = (s[ni][e] + s1[ni][e]) * c1;
+        if (capped) v = fmaf(-2.f * cap2, __fdividef(1.f, fast_ex2(fminf(v, 80.f)) + 1.f), cap2);
+        v = fmaf(-(top ? slope_a : slope_b), (float)dist, v);
+        v = ok ? v : -INFINITY;
+        s[ni][e] = v;
+        if (top) mx_a = fmaxf(mx_a, v);
+        else mx_b = fmaxf(mx_b, v);
+      }
+    mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 1));
+    mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 2));
+    mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 1));
+    mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 2));
+    const float mn_a = fmaxf(m_a, mx_a), mn_b = fmaxf(m_b, mx_b);
+    const float sub_a = mn_a == -INFINITY ? 0.f : mn_a, sub_b = mn_b == -INFINITY ? 0.f : mn_b;
+    const float f_a = fast_ex2(m_a - sub_a), f_b = fast_ex2(m_b - sub_b);
+    uint32_t pa[4];  // P rounded to bf16 once, for the second product; the sums add the rounded values
+#pragma unroll
+    for (int ni = 0; ni < 2; ++ni) {
+      pa[ni * 2] = pack_bf16(fast_ex2(s[ni][0] - sub_a), fast_ex2(s[ni][1] - sub_a));
+      pa[ni * 2 + 1] = pack_bf16(fast_ex2(s[ni][2] - sub_b), fast_ex2(s[ni][3] - sub_b));
+    }
+    l_a = l_a * f_a + ((bf16_lo(pa[0]) + bf16_hi(pa[0])) + (bf16_lo(pa[2]) + bf16_hi(pa[2])));
+    l_b = l_b * f_b + ((bf16_lo(pa[1]) + bf16_hi(pa[1])) + (bf16_lo(pa[3]) + bf16_hi(pa[3])));
+    m_a = mn_a;
+    m_b = mn_b;
+#pragma unroll
+    for (int ni = 0; ni < D / 8; ++ni) {
+      oa[ni][0] *= f_a;
+      oa[ni][1] *= f_a;
+      oa[ni][2] *= f_b;
+      oa[ni][3] *= f_b;
+    }
+#pragma unroll
+    for (int np = 0; np < D / 16; ++np) {
+      uint32_t b[4];
+      ldsm_x4_trans(b, &Vs[((lane & 7) + ((lane >> 3) & 1) * 8) * LD + np * 16 + ((lane >> 4) & 1) * 8]);
+      mma_bf16_16816(oa[np * 2], pa, b[0], b[1]);
+      mma_bf16_16816(oa[np * 2 + 1], pa, b[2], b[3]);
+    }
+    __syncwarp();
+    load(tile + kGdRing * step, st);
+    if (++st == kGdRing) st = 0;
+  }
+  cp_async_wait_all();
+  __syncwarp();
+  l_a += __shfl_xor_sync(0xffffffffu, l_a, 1);
+  l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
+  l_b += __shfl_xor_sync(0xffffffffu, l_b, 1);
+  l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
+  // ---- the warps' states -> this CTA's
+  float* st_o = reinterpret_cast<float*>(gd_smem);
+  constexpr int WARP_F = kGdRing * TILE;  // floats of a warp's ring
+#pragma unroll
+  for (int ni = 0; ni < D / 8; ++ni) {
+    float* p = st_o + warp * WARP_F + gq * D + ni * 8 + 2 * tq;
+    *reinterpret_cast<float2*>(p) = make_float2(oa[ni][0], oa[ni][1]);
+    *reinterpret_cast<float2*>(p + 8 * D) = make_float2(oa[ni][2], oa[ni][3]);
+  }
+  if (tq == 0) {
+    s_ml[warp][gq] = make_float2(m_a, l_a);
+    s_ml[warp][gq + 8] = make_float2(m_b, l_b);
+  }
+  __syncthreads();
+  // rows by turns to the warps, two columns to a lane.  Row r: token t + r / R, head g R + r % R (a lane each: divisions once)
+  constexpr int PAIRS = D / 2, NP = (PAIRS + 31) / 32;
+  const int rows = R * n_tok, l_tok = lane / R, l_head = g * R + lane % R;
+  auto finish = [&](int r, float M, float den, float2 (&o)[NP]) {  // M: of the states; the sink and the gate join here
+    const int tt = t + __shfl_sync(0xffffffffu, l_tok, r), h = __shfl_sync(0xffffffffu, l_head, r);
+    float f = 1.f;
+    if (sink) {
+      const float sk = bf2f(sink[h]) * kLog2e, top = fmaxf(M, sk);
+      f = fast_ex2(M - top);
+      den = den * f + fast_ex2(sk - top);
+    }
+    f /= den;
+    if (x.gate && x.gate_per_head) f *= out_gate<bf16>(x, tt, h, 0, D);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int d = 2 * (lane + 32 * i);
+      if (d >= D) break;
+      float g0 = f, g1 = f;
+      if (x.gate && !x.gate_per_head) {
+        g0 *= out_gate<bf16>(x, tt, h, d, D);
+        g1 *= out_gate<bf16>(x, tt, h, d + 1, D);
+      }
+      *reinterpret_cast<uint32_t*>(out + (size_t)tt * x.out_ld + h * D + d) = pack_bf16(o[i].x * g0, o[i].y * g1);
+    }
+  };
+  for (int r = warp; r < rows; r += kGdWarps) {  // the four warps' states of a row -> this CTA's, in the first warp's place
+    float2 ml[kGdWarps], o[NP] = {};
+    float M = -INFINITY, den = 0.f;
+#pragma unroll
+    for (int w = 0; w < kGdWarps; ++w) {
+      ml[w] = s_ml[w][r];
+      M = fmaxf(M, ml[w].x);
+    }
+#pragma unroll
+    for (int w = 0; w < kGdWarps; ++w) {
+      const float f = ml[w].x == -INFINITY ? 0.f : fast_ex2(ml[w].x - M);
+      den = fmaf(ml[w].y, f, den);
+#pragma unroll
+      for (int i = 0; i < NP; ++i)
+        if (lane + 32 * i < PAIRS) {
+          const float2 v = *reinterpret_cast<const float2*>(st_o + w * WARP_F + r * D + 2 * (lane + 32 * i));
+          o[i].x = fmaf(v.x, f, o[i].x);
+          o[i].y = fmaf(v.y, f, o[i].y);
+        }
+    }
+    if (cs == 1) {
+      finish(r, M, den, o);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NP; ++i)
+        if (lane + 32 * i < PAIRS) *reinterpret_cast<float2*>(st_o + r * D + 2 * (lane + 32 * i)) = o[i];
+      __syncwarp();
+      if (lane == 0) s_ml[0][r] = make_float2(M, den);
+    }
+  }
+  if (cs == 1) return;
+  gd_cluster_sync();
+  for (int r = rank * kGdWarps + warp; r < rows; r += cs * kGdWarps) {  // the CTAs' states: every warp of the cluster finishes rows
+    float2 ml = make_float2(-INFINITY, 0.f), o[NP] = {};
+    if (lane < cs) ml = gd_remote(&s_ml[0][r], lane);
+    const float M = warp_max(ml.x), f = ml.x == -INFINITY ? 0.f : fast_ex2(ml.x - M), den = warp_sum(ml.y * f);
+    float2 v[8][NP];
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+#pragma unroll
+      for (int i = 0; i < NP; ++i)
+        if (c < cs && lane + 32 * i < PAIRS) v[c][i] = gd_remote(reinterpret_cast<const float2*>(st_o + r * D) + lane + 32 * i, c);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const float fc = __shfl_sync(0xffffffffu, f, c);
+#pragma unroll
+      for (int i = 0; i < NP; ++i)
+        if (c < cs && lane + 32 * i < PAIRS) {
+          o[i].x = fmaf(v[c][i].x, fc, o[i].x);
+          o[i].y = fmaf(v[c][i].y, fc, o[i].y);
+        }
+    }
+    finish(r, M, den, o);
+  }
+  gd_cluster_sync();  // nobody leaves while its states are read
+}
+
+template <int D>
+static cudaError_t launch_gqa_decode(const bf16* q, const bf16* cache, const bf16* sink, const int* pos, const int* req, const int* page_off, const int* pages,
+                                   bf16* out, long page_stride, int page_size, int T, int H, int G, float scale, int chunk, AttnExtra x, int span,
+                                   cudaStream_t st) {
+  constexpr size_t smem = (size_t)kGdWarps * kGdRing * 2 * 16 * (D + 8) * sizeof(bf16);
+  static std::atomic<uint64_t> smem_set{0};
+  if (const cudaError_t e = allow_smem(smem_set, (const void*)gqa_decode_kernel<D>, smem); e != cudaSuccess) return e;
+  // As many CTAs as the keys occupy and the GPU holds twice: of a portion's clusters most leave at once.  (60 tokens behind 400 cached: 16.1 us with what it
+  // holds once, 13.5 so; 16 requests of 2000 17.6 / 20.7.)  Steps of over 40 rows are portions more often: twice that again.
+  int cs = 8;
+  while (cs > 1 && ((long)cs * G * T > (T > 40 ? 8L : 4L) * sm_count() || (cs / 2) * kGdWarps * 16 >= span)) cs /= 2;
+  ThreadState& ts = tls();
+  ts.launches++;
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3(cs, G, T);
+  lc.blockDim = dim3(kGdWarps * 32);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cs;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = ts.pdl ? 1 : 0;
+  lc.attrs = at;
+  lc.numAttrs = 2;
+  return cudaLaunchKernelEx(&lc, gqa_decode_kernel<D>, q, cache, sink, pos, req, page_off, pages, out, page_stride, page_size, T, H, G, scale, chunk, x);
+}
+
 template <int DQ, int DV>
 static void launch_gqa_mma(const bf16* q, const bf16* cache, const bf16* sink, const int* pos, const int* req, const int* page_off, const int* pages,
                            bf16* out, long page_stride, int page_size, int T, int H, int G, float scale, int chunk, AttnExtra x, cudaStream_t st) {
@@ -578,12 +867,20 @@ static void launch_gqa_mma(const bf16* q, const bf16* cache, const bf16* sink, c
     cudaFuncSetAttribute(gqa_attention_mma_kernel<DQ, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     attr_set = true;
   }
-  // Few rows (decode steps): the key axis is dealt out to several CTAs per (tile, head) so that the step fills the GPU.  The span a
-  // row can see is bounded by the window / chunk, else by the longest context of the step (when the caller knows it).
+  // The span a row can see is bounded by the window / chunk, else by the longest context of the step (when the caller knows it).
+  // Fewer than 64 rows run request by request; more (and groups of over 16 heads) in tiles of 64, the few-row ones with the key axis dealt out to several
+  // CTAs per (tile, head) so that the step fills the GPU.  B200, us, 16 heads of 128 in 4 groups, tiles of 64 -> request by request: 1 / 4 / 16 / 32 decoding
+  // requests at 2048, 2048 (window 1024), 2000, 2000 12.0 18.9 85 187 -> 10.6 8.0 20.7 33.3; portions of one request, 8 / 32 / 60 tokens 5.6 6.8 8.9 ->
+  // 5.0 5.3 6.5, 16 / 60 behind 400 8.8 11.7 -> 8.8 12.1, two of 31 behind 2000 28.3 -> 21.6.
   const int tiles = (T + kAmRows - 1) / kAmRows;
   int span = x.max_kv_len;
   if (x.window > 0) span = span > 0 ? min(span, x.window + x.keep_first + T) : x.window + x.keep_first + T;
   if (chunk > 0) span = span > 0 ? min(span, chunk) : chunk;
+  if constexpr (DQ == DV)
+    if (T < kAmRows && H / G <= 16) {
+      launch_gqa_decode<DQ>(q, cache, sink, pos, req, page_off, pages, out, page_stride, page_size, T, H, G, scale, chunk, x, span > 0 ? span : 1 << 30, st);
+      return;
+    }
   int splits = 1;
   ThreadState& ts = tls();
   if (T < kAmRows && span > 2 * kAmKeys && ts.scratch) {
