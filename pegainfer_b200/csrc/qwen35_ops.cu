@@ -97,10 +97,11 @@ __global__ void conv1d_silu_kernel(const bf16* __restrict__ x, const bf16* __res
   out[(size_t)t * C + c] = f2bf(s / (1.0f + expf(-s)));
 }
 // Four taps, channels in 16-byte pieces: a thread slides over kConvTokens tokens of 8 channels, so an input is read once (and the three before its
-// first again) instead of once per tap, and no index is divided per element.  With it the linear-attention layer of the
-// hybrid model over 1024 tokens went from 372 to 334 us (B200).
-constexpr int kConvTokens = 16;
-__global__ void __launch_bounds__(128) conv1d_silu4_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* __restrict__ state,
+// first again) instead of once per tap, and no index is divided per element.  The threads of the first tokens, the only ones that read the old state, leave
+// the new one.  Bound by its arithmetic (exponential and division per element) once there are warps enough to hide it: four tokens a thread instead of 16,
+// and no second launch for the state: 8192 channels, 16 / 300 / 1024 / 2048 tokens 13.1 14.2 26.5 39.7 -> 6.3 7.8 15.4 27.7 us (B200).
+constexpr int kConvTokens = 4;
+__global__ void __launch_bounds__(128) conv1d_silu4_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* state,
                                                            bf16* __restrict__ out, int C, int T) {
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8, t0 = blockIdx.y * kConvTokens;
   pdl_wait();
@@ -151,6 +152,19 @@ __global__ void __launch_bounds__(128) conv1d_silu4_kernel(const bf16* __restric
     }
     reinterpret_cast<uint4*>(out + c)[(size_t)(t0 + i) * ld] =
         make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
+  }
+  if (t0 == 0) {  // the newest three inputs, oldest first
+    bf16 nw[3][8];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int src = T - 3 + i;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) nw[i][e] = src >= 0 ? x[(size_t)src * C + c + e] : state[(size_t)(c + e) * 3 + 3 + src];
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) state[(size_t)(c + e) * 3 + i] = nw[i][e];
   }
 }
 __global__ void conv1d_state_kernel(const bf16* __restrict__ x, bf16* __restrict__ state, int C, int T, int K) {
@@ -380,11 +394,12 @@ void conv1d_prefill_cuda(const pk_bf16* x_seq, const pk_bf16* conv_weight, pk_bf
   if (num_channels <= 0 || seq_len <= 0) return;
   if (kernel_size < 1 || kernel_size > 9) unsupported("conv1d_prefill_cuda", "kernel_size must be 1..9");
   const int64_t total = (int64_t)num_channels * seq_len;
-  if (kernel_size == 4 && num_channels % 8 == 0 && seq_len > 1 && seq_len <= 65535 * kConvTokens && q35_al16(x_seq) && q35_al16(conv_weight) && q35_al16(out_seq))
+  if (kernel_size == 4 && num_channels % 8 == 0 && seq_len > 1 && seq_len <= 65535 * kConvTokens && q35_al16(x_seq) && q35_al16(conv_weight) && q35_al16(out_seq)) {
     launch(conv1d_silu4_kernel, dim3((num_channels / 8 + 127) / 128, (seq_len + kConvTokens - 1) / kConvTokens), dim3(128), 0, stream, true,
-           (const bf16*)x_seq, (const bf16*)conv_weight, (const bf16*)conv_state, (bf16*)out_seq, num_channels, seq_len);
-  else
-    launch(conv1d_silu_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, true, (const bf16*)x_seq,
+           (const bf16*)x_seq, (const bf16*)conv_weight, (bf16*)conv_state, (bf16*)out_seq, num_channels, seq_len);
+    return;
+  }
+  launch(conv1d_silu_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, true, (const bf16*)x_seq,
          (const bf16*)conv_weight, (const bf16*)conv_state, (bf16*)out_seq, num_channels, seq_len, kernel_size);
   launch(conv1d_state_kernel, dim3((num_channels + 255) / 256), dim3(256), 0, stream, false, (const bf16*)x_seq, (bf16*)conv_state,
          num_channels, seq_len, kernel_size);
