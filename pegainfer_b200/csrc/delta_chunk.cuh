@@ -247,15 +247,17 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
     return;
   }
   const int pc = (tid & 127) % COLS, pt0 = (tid & 127) / COLS * NTK;  // triangle and read-out: column pc, tokens pt0 .. pt0 + NTK - 1
-  // sum over s <= t of m[t][s] x[s] for this thread's tokens
-  auto lower = [&](const float* m, const float* x, float (&acc)[NTK]) {
-    float4 v[kDcT / 4], w[NTK][kDcT / 4];
-#pragma unroll
-    for (int j = 0; j < kDcT / 4; ++j) v[j] = *reinterpret_cast<const float4*>(x + pc * L::WLD + 4 * j);
+  // sum over s <= t of m[t][s] x[s] for this thread's tokens, w: their rows of m
+  auto rows_of = [&](const float* m, float4 (&w)[NTK][kDcT / 4]) {
 #pragma unroll
     for (int i = 0; i < NTK; ++i)
 #pragma unroll
       for (int j = 0; j < kDcT / 4; ++j) w[i][j] = *reinterpret_cast<const float4*>(m + (pt0 + i) * kDcT + 4 * j);
+  };
+  auto lower = [&](const float4 (&w)[NTK][kDcT / 4], const float* x, float (&acc)[NTK]) {
+    float4 v[kDcT / 4];
+#pragma unroll
+    for (int j = 0; j < kDcT / 4; ++j) v[j] = *reinterpret_cast<const float4*>(x + pc * L::WLD + 4 * j);
 #pragma unroll
     for (int i = 0; i < NTK; ++i) {
       const int t = pt0 + i;
@@ -288,7 +290,9 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
         const int t = pt0 + i;
         o[i] = st[L::CQ + t] * ((pq[t * L::PLD] + pq[(kDcT + t) * L::PLD]) + (pq[(2 * kDcT + t) * L::PLD] + pq[(3 * kDcT + t) * L::PLD]));
       }
-      lower(st + L::BM, sm + L::U + (b & 1) * COLS * L::WLD, o);
+      float4 w[NTK][kDcT / 4];
+      rows_of(st + L::BM, w);
+      lower(w, sm + L::U + (b & 1) * COLS * L::WLD, o);
       if (b & 1) asm volatile("bar.arrive 7, 256;" ::: "memory");
       else asm volatile("bar.arrive 6, 256;" ::: "memory");
       __syncwarp();
@@ -323,6 +327,7 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
   bf16* ub = reinterpret_cast<bf16*>(sm + L::UB);
   int slot = 0;
   uint32_t ph = 0;
+  bool ready = false;  // the stage has been seen full
   for (int b = 0; b < n_chunks; ++b) {
     const float* st = sm + slot * L::STAGE;
     const bf16* raw = reinterpret_cast<const bf16*>(st + L::RAW);
@@ -334,7 +339,7 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
       for (int nt = 0; nt < 2 * MT; ++nt)
 #pragma unroll
         for (int i = 0; i < 2; ++i) dc_split(S[nt >> 1][2 * ks + i][(nt & 1) * 2], S[nt >> 1][2 * ks + i][(nt & 1) * 2 + 1], sp[ks][nt][i]);
-    mbar_wait_bounded(full + slot, ph, dead);
+    if (!ready) mbar_wait_bounded(full + slot, ph, dead);
     __syncwarp();
     // S0^T x over this warp's rows, x = k (0) or q (1)
     auto products = [&](int x, float (&p)[2 * MT][3][4]) {
@@ -384,10 +389,12 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
     }
     products(1, p);  // under the barrier and the triangle
     bar();
+    float4 tw[NTK][kDcT / 4];
+    rows_of(st + L::TM, tw);  // (asked for before the barrier they cost registers and 4 %)
     float u[NTK];
 #pragma unroll
     for (int i = 0; i < NTK; ++i) u[i] = 0.f;
-    lower(st + L::TM, sm + L::W, u);
+    lower(tw, sm + L::W, u);
     if (b >= 2) {  // the read-out warps are done with this buffer's last contents
       if (b & 1) asm volatile("bar.sync 7, 256;" ::: "memory");
       else asm volatile("bar.sync 6, 256;" ::: "memory");
@@ -400,6 +407,7 @@ __device__ __forceinline__ void delta_chunks(const DeltaRows a, float* sm, Gates
 #pragma unroll
       for (int part = 0; part < 3; ++part) *reinterpret_cast<uint32_t*>(ub + (part * COLS + pc) * L::UBLD + pt0 + i) = q[part];
     }
+    ready = mbar_test_wait(full + (slot + 1 == kDcPrep ? 0 : slot + 1), slot + 1 == kDcPrep ? ph ^ 1u : ph);  // the next stage
     bar();
     put(sm + L::PQ + (b & 1) * 4 * kDcT * L::PLD, p);
     if (b & 1) asm volatile("bar.arrive 5, 256;" ::: "memory");
