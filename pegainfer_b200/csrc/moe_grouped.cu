@@ -5,16 +5,20 @@
 //                            expert's rows in as few tiles of at most 256 as they need, of equal size.  Which slot a pair gets inside its
 //                            expert's run may vary from run to run; every row's result is independent of its slot, so outputs do not.
 //   2. moe_gather_kernel     xs[slot] = x[token(slot)]  (TMA then reads an expert's rows as a block)
+//      moe_place_kernel      both, for up to 32768 pairs
 //   3. moe_grouped_gemm<0>   hid[slot] = relu(W_up[e] xs[slot])^2
 //      moe_grouped_gemm<2>   hid[slot] = silu(W_gate[e] x) * (W_up[e] x)            (gated experts, gate / up rows interleaved)
 //      moe_grouped_gemm<3>   hid[slot] = g logistic(p1 g) (u + 1), g = min(W_gate[e] x, p0), u = clamp(W_up[e] x, -p0, p0)
 //   4. moe_grouped_gemm<1>   part[slot] = weight(pair) * W_down[e] hid[slot]     (fp32)
 //   5. moe_combine_kernel    y[t] = sum_k part[slot(t, k)] (+ logistic(g_t) * shared[t]), summed in the order of k
-// GEMM: tcgen05, persistent CTAs.  The weights are the M axis (128 features, TMEM lane = feature) and the rows the N axis (TMEM column = row), so that
-// a tile costs MMAs for its own rows (to the next 16) and not for a full tile of 128; an expert of the usual 100-250 rows reads its weights once.
-//   warp 0 TMA (4 stages of 64 deep) | warp 1 MMA | warps 2-5 epilogue from the other of two accumulators.
-// Bound: HBM for few rows per expert (all weights are read once), the tensor pipe and the operand traffic out of L2 for many.  2048 tokens, 64 experts
-// of 2048 x 1408, top 6 (B200, whole call): 1025 us with 64 x 64 tiles of mma.sync, 363 us so.
+// GEMM: tcgen05, persistent CTA pairs (cta_group::2).  The weights are the M axis (256 features, 128 to a CTA, TMEM lane = feature) and the rows the N axis
+// (TMEM column = row, half of them staged by each CTA), so that a tile costs MMAs for its own rows (to the next 16) and not for a full tile of 128; an
+// expert of the usual 100-250 rows reads its weights once.
+//   warp 0 TMA (6 stages of 64 deep) | warp 1 of the leader MMA | warps 2-9 epilogue from the other of two accumulators.
+// Bound: HBM for few rows per expert (all weights are read once), the operand traffic out of L2 for many: single CTAs read an expert's rows once per 128
+// features, 12 TB/s in all.  2048 tokens, 64 experts of 2048 x 1408, top 6 (B200, whole call): 1025 us with 64 x 64 tiles of mma.sync, 320 with single CTAs and
+// four epilogue warps, 312 in pairs, 281 with eight (the gated epilogue's exponentials and divisions set the pace), 278 with one launch for places and rows;
+// 32 tokens 187 -> 175, where the weights alone take 163.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -131,9 +135,80 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict_
   for (int i = threadIdx.x; i < nv; i += blockDim.x) dst[i] = src[i];
 }
 
-constexpr int kMgStages = 4, kMgThreads = 192, kMgChunk = 32;  // chunk: rows of an epilogue step
-constexpr int kMgA = 128 * 64 * 2, kMgBox = 64 * 64 * 2, kMgStage = kMgA + kMoeTile * 64 * 2;
-constexpr size_t kMgSmem = (size_t)kMgStages * kMgStage + 1024 + kMgChunk * 128 * 2 + (2 * kMgStages + 5) * 8 + 16;
+// Both at once, for up to kPlacePairs pairs and kPlaceThreads experts: each CTA takes an equal share of the pairs, counts all ids by itself (its own
+// pairs' predecessors in the upper half of the same word), so that it knows where its pairs go, and copies their rows; the first also writes the lists.  One
+// launch instead of two, and no step on a single SM (281 -> 278 us of the call above, 26.9 -> 25.7 of 64 tokens on 16 experts of 1024 x 768).
+constexpr int kPlacePairs = 32768, kPlaceThreads = 512;
+__global__ void __launch_bounds__(kPlaceThreads) moe_place_kernel(const int* __restrict__ ids, int pairs, int experts, int max_tiles, int* __restrict__ meta,
+                                                                  int* __restrict__ slot_pair, int* __restrict__ pair_slot, const bf16* __restrict__ x,
+                                                                  bf16* __restrict__ xs, int width, int top) {
+  __shared__ unsigned cnt[kPlaceThreads];  // all pairs of the expert | those before this CTA's << 16
+  __shared__ int cur[kPlaceThreads], wsum[2][kPlaceThreads / 32];
+  pdl_wait();
+  pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int first = (int)((long)blockIdx.x * pairs / gridDim.x), end = (int)((long)(blockIdx.x + 1) * pairs / gridDim.x);
+  cnt[tid] = 0;
+  __syncthreads();
+#pragma unroll 8
+  for (int p = tid; p < pairs; p += kPlaceThreads) atomicAdd(&cnt[ids[p]], p < first ? 0x10001u : 1u);
+  __syncthreads();
+  // exclusive scans of the row and the tile counts over the experts
+  const int c = tid < experts ? (int)(cnt[tid] & 0xffffu) : 0, before = tid < experts ? (int)(cnt[tid] >> 16) : 0, nt = (c + kMoeTile - 1) / kMoeTile;
+  int rc = c, rt = nt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, rc, o), b = __shfl_up_sync(0xffffffffu, rt, o);
+    if (lane >= o) {
+      rc += a;
+      rt += b;
+    }
+  }
+  if (lane == 31) {
+    wsum[0][warp] = rc;
+    wsum[1][warp] = rt;
+  }
+  __syncthreads();
+  int row = rc - c, tile = rt - nt;
+  for (int w = 0; w < warp; ++w) {
+    row += wsum[0][w];
+    tile += wsum[1][w];
+  }
+  cur[tid] = row + before;
+  if (blockIdx.x == 0 && tid <= experts) {
+    int *off = meta + 1, *te = meta + 2 + experts, *tr = te + max_tiles;
+    off[tid] = row;
+    if (tid == experts) {
+      tr[tile] = row;
+      meta[0] = tile;
+    } else {
+      const int size = nt ? ((c + nt - 1) / nt + 15) / 16 * 16 : 0;
+      for (int i = 0; i < nt; ++i) {
+        te[tile + i] = tid;
+        tr[tile + i] = row + i * size;
+      }
+    }
+  }
+  __syncthreads();
+  const int nv = width >> 3;
+  for (int p = first + warp; p < end; p += kPlaceThreads / 32) {
+    int s = 0;
+    if (lane == 0) {
+      s = atomicAdd(&cur[ids[p]], 1);
+      slot_pair[s] = p;
+      pair_slot[p] = s;
+    }
+    s = __shfl_sync(0xffffffffu, s, 0);
+    const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(p / top) * width);
+    uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)s * width);
+#pragma unroll 8
+    for (int i = lane; i < nv; i += 32) dst[i] = src[i];
+  }
+}
+
+constexpr int kMgStages = 6, kMgEpi = 8, kMgThreads = 64 + 32 * kMgEpi, kMgChunk = 32;  // chunk: rows of an epilogue step
+constexpr int kMgA = 128 * 64 * 2, kMgBox = 64 * 64 * 2, kMgStage = kMgA + kMoeTile / 2 * 64 * 2;  // bytes: a CTA's features, 64 rows, a stage
+constexpr size_t kMgSmem = (size_t)kMgStages * kMgStage + 1024 + kMgEpi / 4 * kMgChunk * 128 * 2 + (2 * kMgStages + 5) * 8 + 16;
 
 struct MgArgs {
   void* out;
@@ -149,12 +224,12 @@ struct MgArgs {
 // EPI 2: W rows interleaved (2f = gate f, 2f + 1 = up f): out bf16 [slots][N / 2] = silu(acc[2f]) * acc[2f + 1].
 // EPI 3: the same rows with clamped pre-activations: g = min(acc[2f], p0), u = clamp(acc[2f + 1], -p0, p0), out = g logistic(p1 g) (u + 1).
 template <int EPI>
-__global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                                                                         const MgArgs a) {
   extern __shared__ uint8_t mg_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(mg_smem_raw) + 1023) & ~(uintptr_t)1023);
-  bf16* tile = reinterpret_cast<bf16*>(smem + (size_t)kMgStages * kMgStage);  // epilogue: [32 rows][64 or 128 outputs]
-  uint64_t* full = reinterpret_cast<uint64_t*>(tile + kMgChunk * 128);
+  bf16* tiles_out = reinterpret_cast<bf16*>(smem + (size_t)kMgStages * kMgStage);  // epilogue, per four warps: [32 rows][64 or 128 outputs]
+  uint64_t* full = reinterpret_cast<uint64_t*>(tiles_out + kMgEpi / 4 * kMgChunk * 128);  // the leader's: bytes of both CTAs
   uint64_t* empty = full + kMgStages;
   uint64_t* tfull = empty + kMgStages;
   uint64_t* tempty = tfull + 2;
@@ -169,52 +244,56 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(tfull + s, 1);
-      mbar_init(tempty + s, 4);
+      mbar_init(tempty + s, 2 * kMgEpi);  // the leader's: an arrival per epilogue warp of both CTAs
     }
     mbar_init(done, 1);
     *dead = 0;
     mbar_fence_init();
   }
-  if (warp == 1) tmem_alloc(tmem_slot, 512);
+  if (warp == 1) g2_tmem_alloc(tmem_slot, 512);
   tc_fence_before();
   __syncthreads();
+  g2_cluster_sync();  // both CTAs' barriers and accumulators are there
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = *tmem_slot, rank = g2_rank();
   pdl_wait();
   pdl_launch_dependents();  // after the allocation: a dependent that came first would hold the TMEM while it waits for this grid
   const int* te = a.meta + 2 + a.experts;
   const int* tr = te + a.max_tiles;
-  const int n_ft = (a.N + 127) / 128, tiles = a.meta[0] * n_ft, k_blocks = (a.K + 63) / 64;
-  // neighbouring CTAs share an expert's rows
+  const int n_ft = (a.N + 255) / 256, tiles = a.meta[0] * n_ft, k_blocks = (a.K + 63) / 64;
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;  // neighbouring pairs share an expert's rows
   if (warp == 0) {
     if (tc_elect_one()) {
-      int s = 0, fills = 0;
+      int s = 0;
       uint32_t ph = 1;
-      for (int t = blockIdx.x; t < tiles && !*dead; t += gridDim.x) {
-        const int rt = t / n_ft, m0 = tr[rt], rows = tr[rt + 1] - m0, w0 = te[rt] * a.N + (t - rt * n_ft) * 128, boxes = (rows + 63) / 64;
+      for (int t = pair; t < tiles && !*dead; t += pairs) {
+        const int rt = t / n_ft, n16 = (tr[rt + 1] - tr[rt] + 15) / 16, boxes = (n16 * 8 + 63) / 64;
+        const int r0 = tr[rt] + (int)rank * n16 * 8, w0 = te[rt] * a.N + (t - rt * n_ft) * 256 + (int)rank * 128;
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (!mbar_wait_bounded(empty + s, ph, dead)) break;
-          ++fills;
-          mbar_expect_tx(full + s, kMgA + boxes * kMgBox);
+          const uint32_t fb = g2_map(smem_u32(full + s), 0);
+          if (rank == 0) mbar_expect_tx(full + s, 2 * (kMgA + boxes * kMgBox));
           uint8_t* st = smem + (size_t)s * kMgStage;
-          tma_load_2d(st, &map_w, kb * 64, w0, full + s);
-          for (int b = 0; b < boxes; ++b) tma_load_2d(st + kMgA + b * kMgBox, &map_x, kb * 64, m0 + b * 64, full + s);
+          g2_tma_2d(st, &map_w, kb * 64, w0, fb);
+          for (int b = 0; b < boxes; ++b) g2_tma_2d(st + kMgA + b * kMgBox, &map_x, kb * 64, r0 + b * 64, fb);
           if (++s == kMgStages) {
             s = 0;
             ph ^= 1u;
           }
         }
       }
-      if (*dead) ring_drain(full, kMgStages, fills);
+      // Behind a run-out no barrier of this CTA says when its copies under way have landed: two milliseconds, where a copy takes a thousandth of that
+      if (*dead)
+        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     }
   } else if (warp == 1) {
-    if (tc_elect_one()) {
+    if (rank == 0 && tc_elect_one()) {
       int s = 0, lt = 0;
       uint32_t ph = 0;
-      for (int t = blockIdx.x; t < tiles && !*dead; t += gridDim.x, ++lt) {
+      for (int t = pair; t < tiles && !*dead; t += pairs, ++lt) {
         const int rt = t / n_ft, n16 = (tr[rt + 1] - tr[rt] + 15) / 16, as = lt & 1;
         // instruction descriptor: D = f32 [4,6) = 1, A = bf16 [7,10) = 1, B = bf16 [10,13) = 1, both K-major, N >> 3 at [17,23), M >> 4 at [24,29)
-        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n16 * 2) << 17) | ((uint32_t)(128 >> 4) << 24);
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n16 * 2) << 17) | ((uint32_t)(256 >> 4) << 24);
         if (!mbar_wait_bounded(tempty + as, (uint32_t)(((lt >> 1) & 1) ^ 1), dead)) break;
         tc_fence_after();
         for (int kb = 0; kb < k_blocks; ++kb) {
@@ -224,38 +303,45 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
           const uint64_t ad = make_sw128_desc(a_addr), bd = make_sw128_desc(a_addr + kMgA);
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            umma_bf16(tmem_base + (uint32_t)(as * kMoeTile), ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          umma_commit(empty + s);
+            g2_umma(tmem_base + (uint32_t)(as * kMoeTile), ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          g2_commit_both(empty + s);
           if (++s == kMgStages) {
             s = 0;
             ph ^= 1u;
           }
         }
-        umma_commit(tfull + as);
+        g2_commit_both(tfull + as);
       }
       if (*dead) {
-        umma_commit(done);
+        g2_commit_both(done);
         mbar_drain(done, 0);
       }
     }
   } else {
-    const int q = warp & 3, et = threadIdx.x & 127;  // TMEM lane quarter this warp may read; thread of the four epilogue warps (2, 3, 4, 5 -> 64 .. 191)
+    // two groups of four warps take turns at the chunks.  TMEM lane quarter this warp may read; group; thread of the group
+    const int q = warp & 3, grp = (warp - 2) >> 2, et = (threadIdx.x - 64) & 127;
+    bf16* tile = tiles_out + grp * kMgChunk * 128;
+    auto group_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory"); };
     const int out_n = EPI >= 2 ? a.N / 2 : a.N;
+    const uint32_t tempty0 = g2_map(smem_u32(tempty), 0);
     int lt = 0;
     // (to the last tile even when a wait ran out: a warp that left on its own reading of the flag would leave the others at barrier 1)
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++lt) {
-      const int rt = t / n_ft, m0 = tr[rt], rows = tr[rt + 1] - m0, f0 = (t - rt * n_ft) * 128, as = lt & 1;
+    for (int t = pair; t < tiles; t += pairs, ++lt) {
+      const int rt = t / n_ft, m0 = tr[rt], rows = tr[rt + 1] - m0, f0 = (t - rt * n_ft) * 256 + (int)rank * 128, as = lt & 1;
       mbar_wait_bounded(tfull + as, (uint32_t)((lt >> 1) & 1), dead);
       __syncwarp();
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * kMoeTile);
-      for (int c = 0; c < rows; c += kMgChunk) {
+      auto weight_of = [&](int r) { return EPI == 1 && r < rows ? a.weights[a.slot_pair[m0 + r]] : 0.f; };  // asked for a chunk ahead
+      float next = weight_of(grp * kMgChunk + lane);
+      for (int c = grp * kMgChunk; c < rows; c += kMgEpi / 4 * kMgChunk) {
         uint32_t v[32];
+        const float wl = next;
+        next = weight_of(c + kMgEpi / 4 * kMgChunk + lane);
         tmem_ld32(t_row + (uint32_t)c, v);
         const int n = min(kMgChunk, rows - c);
         if (EPI == 1) {  // fp32: a row's 32 features of a warp are 128 contiguous bytes
           const int f = f0 + q * 32 + lane;
-          const float wl = lane < n ? a.weights[a.slot_pair[m0 + c + lane]] : 0.f;
           float* o = static_cast<float*>(a.out) + (size_t)(m0 + c) * a.N + f;
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
@@ -266,7 +352,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
         }
         // bf16: through shared memory, [row][output], so that a row leaves in 16-byte pieces
         constexpr int OW = EPI >= 2 ? 64 : 128;
-        asm volatile("bar.sync 1, 128;" ::: "memory");  // the last chunk has left
+        group_sync();  // the last chunk has left
         if (EPI == 0) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
@@ -293,7 +379,7 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
 #pragma unroll
           for (int j = 0; j < 16; ++j) tile[(2 * j + (lane & 1)) * OW + q * 16 + (lane >> 1)] = f2bf(gt[j] / den[j] * up[j]);
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        group_sync();
         const int o0 = EPI >= 2 ? f0 / 2 : f0;
         for (int i = et; i < kMgChunk * OW / 8; i += 128) {
           const int r = i / (OW / 8), p = (i % (OW / 8)) * 8;
@@ -303,16 +389,17 @@ __global__ void __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const _
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(tempty + as);
+      if (lane == 0) g2_arrive_cluster(tempty0 + (uint32_t)(as * 8));
     }
   }
   __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x == 0) count_run_out(dead, a.err);
+  g2_cluster_sync();  // the peer's MMAs and copies may still have this CTA's memory as their target
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    g2_tmem_dealloc(tmem_base, 512);
   }
 }
 
@@ -359,9 +446,10 @@ static cudaError_t mg_launch(const void* rows, long n_rows, const void* w, const
   auto kern = moe_grouped_gemm_kernel<EPI>;
   static std::atomic<uint64_t> smem_set{0};
   if (const cudaError_t e = allow_smem(smem_set, (const void*)kern, kMgSmem); e != cudaSuccess) return e;
-  // as many CTAs as there can be tiles, one per SM at most
-  const long tiles = (n_rows / kMoeTile + (n_rows < a.experts ? n_rows : a.experts)) * ((a.N + 127) / 128);
-  return launch(kern, dim3((unsigned)(tiles < sm_count() ? tiles : sm_count())), dim3(kMgThreads), kMgSmem, st, true, mx, mw, a);
+  // as many pairs as there can be tiles, one CTA per SM at most
+  const long tiles = (n_rows / kMoeTile + (n_rows < a.experts ? n_rows : a.experts)) * ((a.N + 255) / 256);
+  const long pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
+  return launch(kern, dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs))), dim3(kMgThreads), kMgSmem, st, true, mx, mw, a);
 }
 
 }  // namespace pk
@@ -406,9 +494,14 @@ extern "C" int pk_moe_grouped_act_p(const void* xa, const void* w_up, const void
   o += (pairs * ff * 2 + 255) / 256 * 256;
   float* part = reinterpret_cast<float*>(ws + o);
   bf16* xs = reinterpret_cast<bf16*>(part);  // done with when `part` is written
-  launch(moe_bucket_kernel, dim3(1), dim3(kBucketThreads), (size_t)(2 * experts + 66) * sizeof(int), st, true, ids, (int)pairs, experts, max_tiles, meta,
-         slot_pair, pair_slot);
-  launch(moe_gather_kernel, dim3((unsigned)pairs), dim3(width >= 2048 ? 256 : 128), 0, st, true, (const bf16*)xa, (const int*)slot_pair, xs, width, top);
+  if (pairs <= kPlacePairs && experts < kPlaceThreads) {
+    launch(moe_place_kernel, dim3((unsigned)(pairs < 2L * sm_count() ? pairs : 2L * sm_count())), dim3(kPlaceThreads), 0, st, true, ids, (int)pairs, experts, max_tiles, meta,
+           slot_pair, pair_slot, (const bf16*)xa, xs, width, top);
+  } else {
+    launch(moe_bucket_kernel, dim3(1), dim3(kBucketThreads), (size_t)(2 * experts + 66) * sizeof(int), st, true, ids, (int)pairs, experts, max_tiles, meta,
+           slot_pair, pair_slot);
+    launch(moe_gather_kernel, dim3((unsigned)pairs), dim3(width >= 2048 ? 256 : 128), 0, st, true, (const bf16*)xa, (const int*)slot_pair, xs, width, top);
+  }
   MgArgs a{hid, meta, slot_pair, weights, experts, max_tiles, act ? 2 * ff : ff, width, p0, p1, wait_err_word()};
   cudaError_t e = act == 2 ? mg_launch<3>(xs, pairs, w_up, a, st) : act == 1 ? mg_launch<2>(xs, pairs, w_up, a, st) : mg_launch<0>(xs, pairs, w_up, a, st);
   if (e != cudaSuccess) return (int)e;

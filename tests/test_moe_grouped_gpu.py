@@ -72,3 +72,16 @@ def test_many_pairs_and_experts(lib, T, top, E):
     got, want = run(lib, x, up, down, ids, wts, 1, 0.0, 0.0), wanted(x, up, down, ids, wts, 1, 0.0, 0.0)
     assert (got.double() - want).norm() <= 2e-3 * want.norm()
     assert torch.equal(got, run(lib, x, up, down, ids, wts, 1, 0.0, 0.0))  # a row does not depend on its slot
+
+
+@pytest.mark.parametrize("T,top,E", [(32768, 1, 3), (5462, 6, 64), (5500, 6, 64), (40, 3, 511), (40, 3, 512), (7, 1, 2), (297, 1, 511)])
+def test_both_forms_of_placing(lib, T, top, E):
+    """pairs and experts on both sides of what moe_place_kernel takes, fewer pairs than CTAs"""
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    W, ff = 64, 32
+    ids = torch.topk(rn(T, E), top).indices.to(torch.int32).contiguous()
+    x, up, down, wts = rn(T, W).bfloat16(), (rn(E, 2 * ff, W) / 8).bfloat16(), (rn(E, W, ff) / 6).bfloat16(), torch.rand(T, top, generator=g, device="cuda")
+    got, want = run(lib, x, up, down, ids, wts, 1, 0.0, 0.0), wanted(x, up, down, ids, wts, 1, 0.0, 0.0)
+    # as above: a hidden value may round to the other bf16 neighbour
+    assert (got.double() - want).norm() <= 2e-3 * want.norm()
