@@ -17,8 +17,13 @@
 //     so skipping it changes nothing), off the softmax warps' critical path;
 //   * P (bf16 pairs) is written with tcgen05.st over the first 64 columns of the tile's own S region and consumed as
 //     the A operand from TMEM: no 32 KB shared-memory round trip, no generic->async proxy fence per block.
+//   * P V of a block begins when the first EARLY_STEPS of its eight k-steps of P are stored, under the exponentials of the
+//     rest; the second tile starts with that signal too.  A block of a tile was a chain of S, maximum, exponentials, all of
+//     P V (600 of 4190 clocks).  2048 / 3 x 1111 / 8192 tokens, 32 heads (B200, us): all of P first 58.5 / 81.1 / 594,
+//     after four steps 58.5 / 80.5 / 594, after six 54.1 / 74.7 / 576, and the second tile with it 53.7 / 74.0 / 536.  The
+//     order of every sum is the same, so are the bits.
 //
-// Warps: 0-3 softmax tile 0 | 4-7 softmax tile 1 | 8-11 correction + epilogue | 12 MMA issuer | 13 TMA loader.
+// Warps: 0-3 softmax tile 0 | 4-7 softmax tile 1 | 8-11 correction + epilogue | 12, 13 MMA issuers | 14 TMA loader.
 // TMEM (512 columns): S0 [0,128) | S1 [128,256) | O0 [256,384) | O1 [384,512); P_i aliases S_i[0,64).
 // Shared memory: Q0, Q1 (32 KB each), K ring 2 x 32 KB, V ring 2 x 32 KB = 192 KB -> one CTA per SM.
 // Per KV block j the in-order tensor queue is  P V(0,j) . S(0,j+1) . P V(1,j) . S(1,j+1): 4 x 512 cycles of MMA against
@@ -39,6 +44,7 @@ constexpr int TILE_B = 2 * HALF_BYTES;
 constexpr int W_CORR = 8, W_MMA = 12, W_LOAD = 14;  // warps 12 / 13 issue the MMAs of tile 0 / tile 1
 constexpr int NTHREADS = 15 * 32;
 constexpr uint32_t TMEM_COLS = 512;
+constexpr int EARLY_STEPS = 6;         // k-steps of 16 kv of P V that are issued before the rest of P is there
 
 struct Args {
   const bf16* q;
@@ -153,12 +159,13 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
   uint64_t* v_full = bars + 4;        // [2]
   uint64_t* v_empty = bars + 6;       // [2] tcgen05.commit after the last P V of the block
   uint64_t* s_full = bars + 8;        // [tile] S(j) complete                        MMA -> softmax
-  uint64_t* po_ready = bars + 10;     // [tile] P(j) stored AND O scaled by alpha(j) (4 + 4 warp arrivals)  softmax, correction -> MMA
+  uint64_t* po_ready = bars + 10;     // [tile] P(j) stored up to EARLY_STEPS AND O scaled by alpha(j) (4 + 4 warp arrivals)  softmax, correction -> MMA
   uint64_t* a_ready = bars + 12;      // [tile] alpha(j) published (128 arrivals)     softmax -> correction
   uint64_t* pv_done = bars + 16;      // [tile] P V(j) complete                       MMA -> correction
   uint64_t* d_ready = bars + 18;      // [tile] final denominators published (128)   softmax -> correction
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
-  float* alpha_s = reinterpret_cast<float*>(bars + 22);  // [tile][128]
+  uint64_t* p_rest = bars + 20;       // [tile] the k-steps of P(j) from EARLY_STEPS on stored (4 warp arrivals)  softmax -> MMA
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
+  float* alpha_s = reinterpret_cast<float*>(bars + 24);  // [tile][128]
   float* denom_s = alpha_s + 2 * TQ;                     // [tile][128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -205,6 +212,7 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
       mbar_init(a_ready + s, 4);
       mbar_init(pv_done + s, 1);
       mbar_init(d_ready + s, 4);
+      mbar_init(p_rest + s, 4);
     }
     mbar_fence_init();
   }
@@ -295,7 +303,7 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
         if (i == 0) FA2_TRACE(1, j, 5);
       };
       if (n_i > 0) {
-        // Stagger the tiles by half a block: tile 1 starts when tile 0 has finished its first softmax, so that one
+        // Stagger the tiles by half a block: tile 1 starts when tile 0 has the first part of its first P, so that one
         // tile's exponentials run under the other's MMAs instead of both contending for the MUFU and then for the
         // tensor pipe (nothing re-synchronises them afterwards; measured with tools/fa2_trace.py).
         if (i == 1 && !(a.dbg & 128)) wait_or_trap(po_ready + 0, 0);
@@ -309,15 +317,23 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
         wait_or_trap(v_full + s, (uint32_t)((j >> 1) & 1));
         if (j + 1 < n_i) wait_or_trap(k_full + (s ^ 1), (uint32_t)(((j + 1) >> 1) & 1));
         if (i == 0) FA2_TRACE(1, j, 0);
-        wait_or_trap(po_ready + i, (uint32_t)(j & 1));  // P(j) stored and O scaled by alpha(j)
+        wait_or_trap(po_ready + i, (uint32_t)(j & 1));  // the first part of P(j) stored and O scaled by alpha(j)
         tc_fence_after();
         if (i == 0) FA2_TRACE(1, j, 1);
         const uint64_t v_desc = make_sw128_mn_desc(smem_u32(KVs + (size_t)s * 2 * TILE_B) + TILE_B, HALF_BYTES, 1024);
         const int ksteps = (a.dbg & 1) ? 0 : min(TKV / 16, np - j * (TKV / PAGE));  // one k-step = one 16-token page
         if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < TKV / 16; ++k)
+          for (int k = 0; k < EARLY_STEPS; ++k)
             if (k < ksteps) umma_bf16_ts(t_o, t_sp + (uint32_t)(k * 8), v_desc + (uint64_t)(k * (2048 >> 4)), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
+        }
+        __syncwarp();
+        wait_or_trap(p_rest + i, (uint32_t)(j & 1));  // the rest of P(j)
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int k = EARLY_STEPS; k < TKV / 16; ++k)
+            if (k < ksteps) umma_bf16_ts(t_o, t_sp + (uint32_t)(k * 8), v_desc + (uint64_t)(k * (2048 >> 4)), idesc_pv, 1u);
           umma_commit(pv_done + i);
           umma_commit(v_empty + s);
           if (j >= n_o) umma_commit(v_empty + s);
@@ -450,7 +466,10 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
       if (a.dbg & 4) {
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(po_ready + i);
+        if (lane == 0) {
+          mbar_arrive(po_ready + i);
+          mbar_arrive(p_rest + i);
+        }
         continue;
       }
       // ---- P = bf16(exp2(s * scale - ref)); the denominator sums the ROUNDED values (straight off the pair) ----
@@ -480,15 +499,20 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
       }
 #pragma unroll
       for (int x = 0; x < 16; ++x) w[x] = p_pair(w[2 * x], w[2 * x + 1], x);
+      tmem_put16(t_s + 32, w);  // P columns 32..47 = kv 64..95
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(po_ready + i);  // the first EARLY_STEPS k-steps may run
 #pragma unroll
-      for (int x = 0; x < 16; ++x) w[16 + x] = p_pair(v[32 + 2 * x], v[32 + 2 * x + 1], x);
-      tmem_st32(t_s + 32, w);  // P columns 32..63 = kv 64..127
+      for (int x = 0; x < 16; ++x) w[x] = p_pair(v[32 + 2 * x], v[32 + 2 * x + 1], x);
+      tmem_put16(t_s + 48, w);  // P columns 48..63 = kv 96..127
       if (warp == 0) FA2_TRACE(0, j, 2);
       tmem_st_wait();
       d = fmaf(d, alpha, (ds4[0] + ds4[1]) + (ds4[2] + ds4[3]));
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(po_ready + i);
+      if (lane == 0) mbar_arrive(p_rest + i);
       if (warp == 0) FA2_TRACE(0, j, 3);
     }
     if (n_i > 0) {

@@ -679,6 +679,31 @@ def test_prefill_attention_tc(starts, lens, nq, nkv, impl, monkeypatch):
                                             T, bs, L.page_stride, sm, stream()) == -1  # page size 32: unsupported
 
 
+@pytest.mark.parametrize("start,n", [(0, 1), (0, 80), (0, 96), (0, 97), (0, 112), (0, 113), (128, 95), (128, 96), (128, 97), (30, 200), (0, 352)])
+def test_prefill_attention_parts_of_p(start, n):
+    """Key counts around the six of eight 16-key steps of a block after which P V begins; against float64.  P and the result are each
+    rounded to bf16 (2^-9 relative at most) and the sum's denominator is that of the rounded P: 2^-8 in the norm, with room for fp32."""
+    lib = get_lib("b200")
+    nq, nkv, hd, layer = 8, 2, 128, 1
+    pg = Paged([start + n], nkv, seed=n)
+    L = pg.layout
+    q = rnd((n, nq * hd), n + 1)
+    out = torch.zeros((n, nq * hd), dtype=torch.bfloat16, device="cuda")
+    assert lib.pk_b200_prefill_attention_tc(p(dev(q)), p(out), p(dev(pg.kv)), L.k_offset(layer), L.v_offset(layer), p(i32(pg.pi)), p(i32(pg.ip)),
+                                            p(i32(pg.lpl)), p(i32(np.array([0, n], np.int32))), nq, nkv, hd, 16, n, 1, L.page_stride, 1 / math.sqrt(hd), stream()) == 0
+    kv = pg.kv.double()
+    def rows(off):
+        pages = [kv[off + int(i) * L.page_stride:][:16 * nkv * hd].view(16, nkv, hd) for i in pg.pi]
+        return torch.cat(pages)[:start + n].transpose(0, 1).repeat_interleave(nq // nkv, 0)
+    K, V = rows(L.k_offset(layer)), rows(L.v_offset(layer))
+    Q = q.double().cpu().view(n, nq, hd).transpose(0, 1)
+    s = Q @ K.transpose(1, 2) / math.sqrt(hd)
+    s.masked_fill_(torch.ones(n, start + n, dtype=torch.bool).triu(start + 1), -math.inf)
+    want = (s.softmax(-1) @ V).transpose(0, 1).reshape(n, -1)
+    got = out.cpu().double()
+    assert (got - want).norm() <= 2.0 ** -8 * want.norm()
+
+
 # ------------------------------------------------------------------ tensor-parallel collectives, two "ranks" on ONE GPU
 def _two_rank_comms(lib, staging_bytes=1 << 20):
     """Two communicators of a world of 2 whose staging / flag buffers all live on this GPU: the peer-memory protocols
