@@ -240,7 +240,7 @@ gated_delta_rule_decode_kernel(const bf16* __restrict__ qkv, const bf16* __restr
 }
 
 // The same recurrence over a whole sequence, 16 tokens at a time (delta_chunk.cuh): CTA = (value head, 32 value columns), state in registers from
-// the first token to the last, the gates computed beside it.  1024 tokens, 32 heads: the layer around it 827 -> 235 us (B200; this kernel 107; before: a pass for
+// the first token to the last, the gates computed beside it.  1024 tokens, 32 heads: the layer around it 827 -> 218 us (B200; this kernel 105; before: a pass for
 // norms and gates, then token by token with two block barriers each).
 __global__ void __launch_bounds__(kDcThreads, 1)
 gated_delta_rule_seq_kernel(const bf16* __restrict__ qkv_seq, const bf16* __restrict__ b_seq, const bf16* __restrict__ a_seq,
