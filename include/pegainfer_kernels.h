@@ -396,6 +396,9 @@ int64_t pk_tp_flag_bytes(void);
 pk_tp_comm* pk_tp_comm_create(int rank, int world, void* const* staging_ptrs,
                               void* const* flag_ptrs, int64_t staging_bytes);
 void pk_tp_comm_destroy(pk_tp_comm* comm);
+/* Limit of a wait for a peer, in looks at its line or flag (default 2^27, about a minute; > 0, else -1).  A wait that runs out is counted
+ * (pk_b200_wait_errors), and the communicator's other waits give up at once from then on. */
+int pk_tp_set_wait_limit(pk_tp_comm* comm, uint32_t spins);
 /* Largest row count one call can reduce for rows of hidden_dim bf16 (callers chunk above it). */
 int64_t pk_tp_max_rows(pk_tp_comm* comm, int hidden_dim);
 /* Vocab-sharded lm_head: combine every rank's (max logit, index inside its shard) into the global greedy token on

@@ -240,6 +240,8 @@ struct TpDev {
   int64_t raw_bytes;             // leading part of a region used for plain rows; the tail holds the two LL areas
   int64_t ll_off, ll_bytes;      // LL lines of the standalone all-reduce kernel (PK_TP_PROTO=ll)
   int64_t gll_off, gll_bytes;    // 8-byte LL lines of the GEMV-fused all-reduce (gemv.cu epi 3)
+  uint32_t spins;                // limit of a wait for a peer
+  unsigned int* err;             // wait_err_word(), as of the launch
 };
 
 __device__ __forceinline__ void st_release_sys(uint32_t* p, uint32_t v) {
@@ -257,6 +259,21 @@ __device__ __forceinline__ uint32_t ld_acquire_sys(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
+}
+// A wait for a peer, with a limit.  The first one of a communicator that runs out is counted where the host looks (wait_err_word), and the communicator is
+// marked as lost: its other waits give up after a short look, so that the step's remaining kernels end soon.  The caller goes on with whatever is there; the
+// host refuses the results.
+template <typename Ready>
+__device__ __forceinline__ void tp_wait(const TpDev& d, Ready ready) {
+  for (uint32_t spins = 0; !ready(); ++spins) {
+    if (spins < d.spins && (spins & 1023u) != 1023u) continue;
+    uint32_t* lost = d.flags[d.rank] + 2 * kTpMaxCtas * kTpMaxWorld + 3;
+    if (spins >= d.spins) {
+      if (atomicExch(lost, 1u) == 0u && d.err) atomicAdd(d.err, 1u);
+      return;
+    }
+    if (*reinterpret_cast<volatile uint32_t*>(lost)) return;
+  }
 }
 
 }  // namespace pk

@@ -160,8 +160,7 @@ gemv_stream_kernel(const GemvArgs a) {
         const int slot = (int)(seq & 1u);
         if (tid < a.tp.world) {
           const uint32_t* f = my_flags + (size_t)(slot * kTpMaxCtas) * kTpMaxWorld + tid;
-          for (uint32_t spins = 0; ld_acquire_sys(f) != seq; ++spins)
-            if (spins > (1u << 27)) __trap();
+          tp_wait(a.tp, [&] { return ld_acquire_sys(f) == seq; });
         }
         consumer_bar();
         stage_base = a.tp.stage[a.tp.rank] + (size_t)slot * a.tp.world * a.tp.slot_bytes;
@@ -363,11 +362,7 @@ gemv_stream_kernel(const GemvArgs a) {
         } else {
           const uint8_t* line = local + (size_t)q * a.tp.slot_bytes + ((size_t)pr * M + r0 + r) * 8;
           uint2 l;
-          uint32_t spins = 0;
-          do {
-            l = ld_volatile_v2(line);
-            if (++spins > (1u << 26)) __trap();  // a missing peer (~1 min) becomes a launch failure, not a hang
-          } while (l.y != seq);
+          tp_wait(a.tp, [&] { l = ld_volatile_v2(line); return l.y == seq; });
           v = l.x;
         }
         s0 += bf16_lo(v);
@@ -595,6 +590,7 @@ int pk_b200_gemv_fused(const pk_b200_gemv_args* g, pk_stream stream) {
     a.tp_step = g->tp_step;
     a.tp_op = g->tp_op;
   }
+  a.tp.err = wait_err_word();
   return (int)launch_gemv(a, g->N, stream);
 }
 

@@ -81,8 +81,7 @@ __global__ void __launch_bounds__(kTpThreads) tp_allreduce_kernel(const TpArgs a
       const int p = threadIdx.x;
       st_release_sys(a.d.flags[p] + (size_t)(slot * kTpMaxCtas + c) * kTpMaxWorld + me, seq);
       const uint32_t* f = my_flags + (size_t)(slot * kTpMaxCtas + c) * kTpMaxWorld + p;
-      for (uint32_t spins = 0; ld_acquire_sys(f) != seq; ++spins)
-        if (spins > (1u << 27)) __trap();  // a lost peer becomes a launch failure instead of a wedged GPU
+      tp_wait(a.d, [&] { return ld_acquire_sys(f) == seq; });
     }
     __syncthreads();
   }
@@ -101,9 +100,8 @@ __global__ void __launch_bounds__(kTpThreads) tp_allreduce_kernel(const TpArgs a
         } else if (LL) {
           const uint8_t* line = local + (size_t)r * a.d.slot_bytes + a.d.ll_off + ((size_t)t * nv + i) * 32;
           uint4 l0, l1;
-          uint32_t spins = 0;
-          do { l0 = ld_volatile_v4(line); if (++spins > (1u << 27)) __trap(); } while (l0.y != seq || l0.w != seq);
-          do { l1 = ld_volatile_v4(line + 16); if (++spins > (1u << 27)) __trap(); } while (l1.y != seq || l1.w != seq);
+          tp_wait(a.d, [&] { l0 = ld_volatile_v4(line); return l0.y == seq && l0.w == seq; });
+          tp_wait(a.d, [&] { l1 = ld_volatile_v4(line + 16); return l1.y == seq && l1.w == seq; });
           v = make_uint4(l0.x, l0.z, l1.x, l1.z);
         } else {
           v = __ldcg(reinterpret_cast<const uint4*>(local + (size_t)r * a.d.slot_bytes +
@@ -201,11 +199,7 @@ __global__ void __launch_bounds__(64) tp_top1_exchange_kernel(const TpTop1Args a
     if (q == me) continue;
     const uint8_t* line = a.d.stage[me] + (size_t)q * a.d.slot_bytes + off;
     uint4 l;
-    uint32_t spins = 0;
-    do {
-      asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(l.x), "=r"(l.y), "=r"(l.z), "=r"(l.w) : "l"(line) : "memory");
-      if (++spins > (1u << 26)) __trap();
-    } while (l.y != seq || l.w != seq);
+    tp_wait(a.d, [&] { l = ld_volatile_v4(line); return l.y == seq && l.w == seq; });
     const float ov = __uint_as_float(l.x);
     const int oi = (int)l.z;
     if (ov > bv || (ov == bv && oi < bi)) {
@@ -252,7 +246,14 @@ pk_tp_comm* pk_tp_comm_create(int rank, int world, void* const* staging_ptrs,
   c->d.ll_bytes = eighth;
   c->d.gll_off = c->d.raw_bytes + eighth;
   c->d.gll_bytes = eighth;
+  c->d.spins = 1u << 27;  // about a minute
   return c;
+}
+
+int pk_tp_set_wait_limit(pk_tp_comm* comm, uint32_t spins) {
+  if (!comm || spins == 0) return -1;
+  comm->d.spins = spins;
+  return 0;
 }
 
 void pk_tp_comm_destroy(pk_tp_comm* comm) { delete comm; }
@@ -266,6 +267,7 @@ static int tp_launch(pk_tp_comm* comm, const pk_bf16* partial, pk_bf16* hidden,
   if ((int64_t)T * dim * 2 > comm->d.raw_bytes) return -2;  // caller chunks larger messages
   TpArgs a{};
   a.d = comm->d;
+  a.d.err = wait_err_word();
   a.partial = (const bf16*)partial;
   a.hidden = (bf16*)hidden;
   a.weight = (const bf16*)weight;
@@ -307,6 +309,7 @@ int pk_tp_top1_exchange(pk_tp_comm* comm, const pk_bf16* local_max, int* index_i
   if (!comm || batch_size <= 0 || batch_size > 64 || comm->d.gll_bytes < 8192) return -1;
   TpTop1Args a{};
   a.d = comm->d;
+  a.d.err = wait_err_word();
   a.vals = (const bf16*)local_max;
   a.idx = index_inout;
   a.bs = batch_size;

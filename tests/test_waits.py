@@ -103,3 +103,63 @@ def test_steps_behind_a_run_out_wait_are_refused():
     root = os.path.dirname(os.path.dirname(CSRC))
     run = subprocess.run([sys.executable, "-c", REFUSAL], cwd=root, env=dict(os.environ, PYTHONPATH=root), capture_output=True, text=True, timeout=300)
     assert run.returncode == 0 and "refused and served" in run.stdout, run.stdout[-2000:] + run.stderr[-4000:]
+
+
+LOST_PEER = """
+import ctypes as C
+import torch
+from pegainfer_b200 import ffi
+
+lib = ffi.lib()
+lib.cuda_set_device(0)
+lib.cublas_init()
+assert lib.pk_tp_set_wait_limit(None, 5) == -1
+
+
+def comm():  # a rank of two whose peer never comes
+    stage = [torch.zeros(1 << 20, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    flags = [torch.zeros(int(lib.pk_tp_flag_bytes()), dtype=torch.uint8, device="cuda") for _ in range(2)]
+    c = lib.pk_tp_comm_create(0, 2, (C.c_void_p * 2)(*[s.data_ptr() for s in stage]), (C.c_void_p * 2)(*[f.data_ptr() for f in flags]), 1 << 20)
+    assert lib.pk_tp_set_wait_limit(c, 0) == -1 and lib.pk_tp_set_wait_limit(c, 5000) == 0
+    return c, stage, flags
+
+
+bf = lambda *s: torch.ones(*s, device="cuda").bfloat16()
+x, w, y, h, hidden = bf(1, 1024), bf(512, 1024), bf(1, 512), bf(4, 512), bf(1, 1024)
+step, idx = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+
+
+def gemv(c, x_mode, epi):
+    g = ffi.GemvArgs()
+    g.W, g.X, g.residual, g.norm_w = w.data_ptr(), x.data_ptr(), x.data_ptr(), x.data_ptr()
+    g.Y = (C.c_void_p * 3)(y.data_ptr(), None, None)
+    g.seg_rows = (C.c_int * 3)(512, 0, 0)
+    g.M, g.N, g.K, g.x_mode, g.epi, g.eps = 512, 1, 1024, x_mode, epi, 1e-6
+    g.hidden_out = hidden.data_ptr() if x_mode else None
+    g.tp_comm, g.tp_step, g.tp_op = c, step.data_ptr(), 0
+    return lib.pk_b200_gemv_fused(C.byref(g), None)
+
+
+calls = [lambda c: lib.pk_tp_all_reduce_rows(c, h.data_ptr(), 512, 4, None), lambda c: lib.pk_tp_top1_exchange(c, y.data_ptr(), idx.data_ptr(), 1, 0, None, 9, None),
+         lambda c: gemv(c, 0, 3), lambda c: gemv(c, 2, 0)]
+keep = []
+for n, call in enumerate(calls):
+    keep.append(comm())
+    if n == 3:  # x_mode 2 waits for the number that its own flags name
+        keep[-1][2][0].view(torch.int32)[2 * 64 * 8] = 1
+    torch.cuda.synchronize()
+    for _ in range(2):  # the second call's waits give up at once, and are not counted again
+        assert call(keep[-1][0]) == 0 and lib.pk_b200_wait_errors() == n + 1, n
+assert torch.equal(x + x, 2 * x)  # the context works
+print("counted and returned")
+"""
+
+
+@pytest.mark.gpu
+def test_a_peer_that_never_comes_is_counted():
+    """in a process of its own: the count stays"""
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(CSRC))
+    run = subprocess.run([sys.executable, "-c", LOST_PEER], cwd=root, env=dict(os.environ, PYTHONPATH=root), capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0 and "counted and returned" in run.stdout, run.stdout[-2000:] + run.stderr[-4000:]
