@@ -704,76 +704,104 @@ def test_prefill_attention_parts_of_p(start, n):
     assert (got - want).norm() <= 2.0 ** -8 * want.norm()
 
 
-# ------------------------------------------------------------------ tensor-parallel collectives, two "ranks" on ONE GPU
-def _two_rank_comms(lib, staging_bytes=1 << 20):
-    """Two communicators of a world of 2 whose staging / flag buffers all live on this GPU: the peer-memory protocols
-    (posted stores + sequence-stamped lines) run unchanged, the 'NVLink' writes are local.  The two ranks' kernels must be
-    co-resident (they wait for each other), so callers keep the grids small and use two streams."""
+# ------------------------------------------------------------------ tensor-parallel collectives, the peer's lines laid down on ONE GPU
+# Kernels that wait for one another never run side by side on one GPU: the ranks run one after the other, and what the first one waits for lies in its
+# staging buffer before it is launched.  So no wait goes round more than once.
+STAGING = 1 << 20
+SLOT = (STAGING // 4) & ~15  # bytes of a (slot, source) region of a world of two; its last eighth holds the lines
+LINES = SLOT - (SLOT // 8 & ~15)
+
+
+def _two_ranks(lib):
+    """Communicators of a world of two whose staging and flag buffers all lie on this GPU (the 'NVLink' writes are local)"""
     import ctypes as C
-    stage = [torch.zeros(staging_bytes, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    stage = [torch.zeros(STAGING, dtype=torch.uint8, device="cuda") for _ in range(2)]
     flags = [torch.zeros(int(lib.pk_tp_flag_bytes()), dtype=torch.uint8, device="cuda") for _ in range(2)]
     sp = (C.c_void_p * 2)(stage[0].data_ptr(), stage[1].data_ptr())
     fp = (C.c_void_p * 2)(flags[0].data_ptr(), flags[1].data_ptr())
-    comms = [lib.pk_tp_comm_create(r, 2, sp, fp, staging_bytes) for r in range(2)]
-    assert all(comms)
+    comms = [lib.pk_tp_comm_create(r, 2, sp, fp, STAGING) for r in range(2)]
+    assert all(comms) and all(lib.pk_tp_set_wait_limit(c, 1000) == 0 for c in comms)  # (a line in the wrong place ends as a test that fails)
     _keep.extend(stage + flags)
-    return comms
+    return comms, [s.view(torch.int32) for s in stage]
 
 
 @pytest.mark.parametrize("N", [1, 3])
-def test_gemv_ll_allreduce_two_ranks_one_gpu(N):
+def test_gemv_ll_allreduce_with_the_peers_lines(N):
     """epi 3: GEMV + all-reduce of the CTA's own rows in one kernel.  Each 'rank' holds a column slice of W and the
     matching slice of x (row-parallel o_proj / down_proj); both must write the rank-ordered bf16 sum of the two bf16
-    partials, bit-identical to the oracle's all-reduce model, for two consecutive ops (slot / sequence reuse)."""
+    partials, bit-identical to the oracle's all-reduce model, for consecutive ops (slot / sequence reuse)."""
     lib = get_lib("b200")
     import ctypes as C
-    M, K = 512, 1024  # 64 CTAs per rank: both grids are resident at once
-    comms = _two_rank_comms(lib)
-    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    M, K = 512, 1024
+    comms, stage = _two_ranks(lib)
     step = torch.tensor([7], dtype=torch.int32, device="cuda")
     for op in range(3):
         W, x = rnd((M, 2 * K), 70 + op, 0.05), rnd((N, 2 * K), 80 + op, 1.0)
-        parts, outs = [], []
-        torch.cuda.synchronize()
+        parts, outs, own, args = [], [], [], []
         for r in range(2):
             Wr = dev(W[:, r * K:(r + 1) * K].contiguous())
             xr = dev(x[:, r * K:(r + 1) * K].contiguous())
-            y = torch.zeros((N, M), dtype=torch.bfloat16, device="cuda")
+            y, partial = (torch.zeros((N, M), dtype=torch.bfloat16, device="cuda") for _ in range(2))
             g = ffi.GemvArgs()
             g.W, g.X = p(Wr), p(xr)
-            g.Y = (C.c_void_p * 3)(y.data_ptr(), None, None)
+            g.Y = (C.c_void_p * 3)(partial.data_ptr(), None, None)
             g.seg_rows = (C.c_int * 3)(M, 0, 0)
-            g.M, g.N, g.K, g.x_mode, g.epi = M, N, K, 0, 3
-            g.tp_comm, g.tp_step, g.tp_op = comms[r], step.data_ptr(), op
-            with torch.cuda.stream(streams[r]):
-                assert lib.pk_b200_gemv_fused(C.byref(g), streams[r].cuda_stream) == 0
+            g.M, g.N, g.K, g.x_mode, g.epi = M, N, K, 0, 0
+            assert lib.pk_b200_gemv_fused(C.byref(g), stream()) == 0  # the rank's partial rows
+            g.Y = (C.c_void_p * 3)(y.data_ptr(), None, None)
+            g.epi, g.tp_comm, g.tp_step, g.tp_op = 3, comms[r], step.data_ptr(), op
+            args.append(g)
             outs.append(y)
+            own.append(partial)
             parts.append(O.gemm(bits(W[:, r * K:(r + 1) * K].contiguous()), bits(x[:, r * K:(r + 1) * K].contiguous())))
+        # a line per pair of tokens and row: two bf16 values, the sequence number
+        pairs = torch.zeros(((N + 1) // 2, M, 2), dtype=torch.bfloat16, device="cuda")
+        for n in range(N):
+            pairs[n // 2, :, n % 2] = own[1][n]
+        lines = torch.stack([pairs.view(torch.int32)[..., 0], torch.full((pairs.shape[0], M), 7 * 256 + op + 1, dtype=torch.int32, device="cuda")], -1).flatten()
+        at = (((op & 1) * 2 + 1) * SLOT + LINES) // 4  # rank 1's region in rank 0's buffer
+        here = stage[0][at:at + lines.numel()]
+        here.copy_(lines)
         torch.cuda.synchronize()
+        assert lib.pk_b200_gemv_fused(C.byref(args[0]), stream()) == 0
+        torch.cuda.synchronize()
+        here.zero_()
+        torch.cuda.synchronize()
+        assert lib.pk_b200_gemv_fused(C.byref(args[1]), stream()) == 0  # finds what rank 0's kernel left
+        torch.cuda.synchronize()
+        assert lib.pk_b200_wait_errors() == 0 and torch.equal(here, lines)  # and leaves the lines that were laid down before
         want = O.all_reduce_sum(parts)
         assert (bits(outs[0]) == bits(outs[1])).all(), "ranks disagree"
         assert_bf16_close(bits(outs[0]), want, 2, floor=float(np.abs(f32(want)).max()) / 64, frac_exact=0.85, what=f"ll all-reduce op {op}")
 
 
-def test_tp_top1_exchange_two_ranks_one_gpu():
+def test_tp_top1_exchange_with_the_peers_lines():
     """Vocab-sharded greedy token: every rank ends with the same global (max, lowest index) winner."""
     lib = get_lib("b200")
-    comms = _two_rank_comms(lib)
-    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    comms, stage = _two_ranks(lib)
     step = torch.tensor([3], dtype=torch.int32, device="cuda")
-    vals = [from_bits(O.f32_to_bf16(np.array(v, np.float32)), "cuda") for v in ([1.5, 9.0, 2.0], [4.0, 9.0, -1.0])]
-    idx = [torch.tensor(i, dtype=torch.int32, device="cuda") for i in ([10, 20, 30], [5, 6, 7])]
-    torch.cuda.synchronize()
-    for r in range(2):
-        with torch.cuda.stream(streams[r]):
-            assert lib.pk_tp_top1_exchange(comms[r], p(vals[r]), p(idx[r]), 3, r * 1000, step.data_ptr(), 250, streams[r].cuda_stream) == 0
-    torch.cuda.synchronize()
+
+    def exchange(vals, local, step, op, seq, entry):
+        idx = [torch.tensor(i, dtype=torch.int32, device="cuda") for i in local]
+        v = [from_bits(O.f32_to_bf16(np.array(x, np.float32)), "cuda") for x in vals]
+        n = len(vals[0])
+        seq -= 1 << 32 if seq >> 31 else 0
+        lines = torch.stack([v[1].float().view(torch.int32), torch.full_like(idx[1], seq), idx[1] + 1000, torch.full_like(idx[1], seq)], 1).flatten()
+        at = (2 * SLOT - 4096 + entry * 16) // 4  # rank 1's region in rank 0's buffer
+        here = stage[0][at:at + 4 * n]
+        here.copy_(lines)
+        for r in range(2):
+            torch.cuda.synchronize()
+            assert lib.pk_tp_top1_exchange(comms[r], p(v[r]), p(idx[r]), n, r * 1000, step.data_ptr() if step is not None else None, op, stream()) == 0
+            torch.cuda.synchronize()
+            if r == 0:
+                here.zero_()
+        assert lib.pk_b200_wait_errors() == 0 and torch.equal(here, lines)
+        assert idx[0].tolist() == idx[1].tolist()
+        return idx[0].tolist()
+
     # request 0: rank 1 wins (4.0 at 1000+5); request 1: tie at 9.0 -> lowest global index (rank 0: 20); request 2: rank 0 (30)
-    assert idx[0].tolist() == idx[1].tolist() == [1005, 20, 30]
+    vals = ([1.5, 9.0, 2.0], [4.0, 9.0, -1.0])
+    assert exchange(vals, ([10, 20, 30], [5, 6, 7]), step, 250, 3 * 256 + 251, 0) == [1005, 20, 30]
     # host-path sequence numbers (no step counter) use separate lines
-    idx2 = [torch.tensor([3], dtype=torch.int32, device="cuda"), torch.tensor([4], dtype=torch.int32, device="cuda")]
-    for r in range(2):
-        with torch.cuda.stream(streams[r]):
-            assert lib.pk_tp_top1_exchange(comms[r], p(vals[r]), p(idx2[r]), 1, r * 1000, None, 0x80000001, streams[r].cuda_stream) == 0
-    torch.cuda.synchronize()
-    assert idx2[0].tolist() == idx2[1].tolist() == [1004]
+    assert exchange(([1.5], [4.0]), ([3], [4]), None, 0x80000001, 0x80000001, 64) == [1004]
