@@ -335,7 +335,9 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         for (int x = 0; x < 32; ++x) m4[x & 3] = fmaxf(m4[x & 3], __uint_as_float(v[x]));
         const float own = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * a.scale_log2;
         m.top[n & 1][threadIdx.x] = own;
-        both_halves();  // (and both have read their scores: P may take their place)
+        tc_fence_before();  // both have read their scores: P may take their place
+        both_halves();
+        tc_fence_after();
         const float blk = fmaxf(own, m.top[n & 1][threadIdx.x ^ LT_ROWS]);
         const bool grow = blk > mx, any = __any_sync(0xffffffffu, grow);
         const float to = grow ? blk : mx, corr = grow ? lt_exp2(mx - to) : 1.f;
@@ -353,6 +355,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         l = l * corr + ((s4[0] + s4[1]) + (s4[2] + s4[3]));
         tmem_put16(t_s + side * 16, p);
         if (any && b > 0) {  // O holds the blocks before this one, once their last P V is through
+          // (blocks whose pv_done this thread did not wait for have left the barrier no phase behind: the P V of block n - 2 was complete when these scores were)
           mbar_wait_bounded(&m.pv_done, (n - 1) & 1, dead);
           __syncwarp();
           tc_fence_after();
