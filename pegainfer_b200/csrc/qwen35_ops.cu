@@ -102,8 +102,9 @@ __global__ void conv1d_silu_kernel(const bf16* __restrict__ x, const bf16* __res
 // and no second launch for the state: 8192 channels, 16 / 300 / 1024 / 2048 tokens 13.1 14.2 26.5 39.7 -> 6.3 7.8 15.4 27.7 us (B200).
 constexpr int kConvTokens = 4;
 __global__ void __launch_bounds__(128) conv1d_silu4_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* state,
-                                                           bf16* __restrict__ out, int C, int T) {
-  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8, t0 = blockIdx.y * kConvTokens;
+                                                           bf16* __restrict__ out, int C, int T, int groups) {
+  // (blocks of `groups` channel groups one after the other: the grid's first axis has room for any number of tokens)
+  const int c = (int)((blockIdx.x % groups * blockDim.x + threadIdx.x) * 8), t0 = (int)(blockIdx.x / groups) * kConvTokens;
   pdl_wait();
   if (c >= C) return;
   auto unpack = [](const uint4& u, float (&v)[8]) {
@@ -394,9 +395,10 @@ void conv1d_prefill_cuda(const pk_bf16* x_seq, const pk_bf16* conv_weight, pk_bf
   if (num_channels <= 0 || seq_len <= 0) return;
   if (kernel_size < 1 || kernel_size > 9) unsupported("conv1d_prefill_cuda", "kernel_size must be 1..9");
   const int64_t total = (int64_t)num_channels * seq_len;
-  if (kernel_size == 4 && num_channels % 8 == 0 && seq_len > 1 && seq_len <= 65535 * kConvTokens && q35_al16(x_seq) && q35_al16(conv_weight) && q35_al16(out_seq)) {
-    launch(conv1d_silu4_kernel, dim3((num_channels / 8 + 127) / 128, (seq_len + kConvTokens - 1) / kConvTokens), dim3(128), 0, stream, true,
-           (const bf16*)x_seq, (const bf16*)conv_weight, (bf16*)conv_state, (bf16*)out_seq, num_channels, seq_len);
+  const int64_t groups = (num_channels / 8 + 127) / 128, blocks = groups * ((seq_len - 1) / kConvTokens + 1);
+  if (kernel_size == 4 && num_channels % 8 == 0 && seq_len > 1 && blocks <= 0x7fffffff && q35_al16(x_seq) && q35_al16(conv_weight) && q35_al16(out_seq)) {
+    launch(conv1d_silu4_kernel, dim3((unsigned)blocks), dim3(128), 0, stream, true,
+           (const bf16*)x_seq, (const bf16*)conv_weight, (bf16*)conv_state, (bf16*)out_seq, num_channels, seq_len, (int)groups);
     return;
   }
   launch(conv1d_silu_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, true, (const bf16*)x_seq,

@@ -112,6 +112,12 @@ def test_conv(lib, T, C, shift):
     assert torch.equal(state, full[-3:].T.bfloat16()) and (out[T] == 0).all()
 
 
+@pytest.mark.parametrize("T", [262140, 262145, 1048581])
+def test_conv_of_many_tokens(lib, T):
+    """more blocks of four tokens than the second axis of a grid has places"""
+    test_conv(lib, T, 8, 0)
+
+
 @pytest.mark.parametrize("shift", [0, 4])
 @pytest.mark.parametrize("heads,dim", [(1, 128), (15, 128), (16, 128), (33, 128), (7, 96)])
 def test_gated_norm(lib, heads, dim, shift):
