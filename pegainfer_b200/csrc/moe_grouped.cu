@@ -17,8 +17,8 @@
 //   warp 0 TMA (6 stages of 64 deep) | warp 1 of the leader MMA | warps 2-9 epilogue from the other of two accumulators.
 // Bound: HBM for few rows per expert (all weights are read once), the operand traffic out of L2 for many: single CTAs read an expert's rows once per 128
 // features, 12 TB/s in all.  2048 tokens, 64 experts of 2048 x 1408, top 6 (B200, whole call): 1025 us with 64 x 64 tiles of mma.sync, 320 with single CTAs and
-// four epilogue warps, 312 in pairs, 281 with eight (the gated epilogue's exponentials and divisions set the pace), 278 with one launch for places and rows;
-// 32 tokens 187 -> 175, where the weights alone take 163.
+// four epilogue warps, 312 in pairs, 281 with eight (the gated epilogue's exponentials and divisions set the pace), 278 with one launch for places and rows
+// (one box under one clock; on three others 357 to 360 -> 310 to 315); 32 tokens 187 -> 175, where the weights alone take 163.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict_
 // Both at once, for up to kPlacePairs pairs and kPlaceThreads experts: each CTA takes an equal share of the pairs, counts all ids by itself (its own
 // pairs' predecessors in the upper half of the same word), so that it knows where its pairs go, and copies their rows; the first also writes the lists.  One
 // launch instead of two, and no step on a single SM (281 -> 278 us of the call above, 26.9 -> 25.7 of 64 tokens on 16 experts of 1024 x 768).
-constexpr int kPlacePairs = 32768, kPlaceThreads = 512;
+constexpr int kPlacePairs = 32768, kPlaceThreads = 512, kPlaceHead = 8;
 __global__ void __launch_bounds__(kPlaceThreads) moe_place_kernel(const int* __restrict__ ids, int pairs, int experts, int max_tiles, int* __restrict__ meta,
                                                                   int* __restrict__ slot_pair, int* __restrict__ pair_slot, const bf16* __restrict__ x,
                                                                   bf16* __restrict__ xs, int width, int top) {
@@ -148,6 +148,12 @@ __global__ void __launch_bounds__(kPlaceThreads) moe_place_kernel(const int* __r
   pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int first = (int)((long)blockIdx.x * pairs / gridDim.x), end = (int)((long)(blockIdx.x + 1) * pairs / gridDim.x);
+  // the warp's first pair's row, under way while its place is looked for
+  const int nv = width >> 3;
+  uint4 head[kPlaceHead];
+#pragma unroll
+  for (int i = 0; i < kPlaceHead; ++i)
+    if (first + warp < end && lane + 32 * i < nv) head[i] = reinterpret_cast<const uint4*>(x + (size_t)((first + warp) / top) * width)[lane + 32 * i];
   cnt[tid] = 0;
   __syncthreads();
 #pragma unroll 8
@@ -190,7 +196,6 @@ __global__ void __launch_bounds__(kPlaceThreads) moe_place_kernel(const int* __r
     }
   }
   __syncthreads();
-  const int nv = width >> 3;
   for (int p = first + warp; p < end; p += kPlaceThreads / 32) {
     int s = 0;
     if (lane == 0) {
@@ -201,8 +206,14 @@ __global__ void __launch_bounds__(kPlaceThreads) moe_place_kernel(const int* __r
     s = __shfl_sync(0xffffffffu, s, 0);
     const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(p / top) * width);
     uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)s * width);
+    int i = lane;
+    if (p == first + warp) {
+#pragma unroll
+      for (int k = 0; k < kPlaceHead; ++k, i += 32)
+        if (i < nv) dst[i] = head[k];
+    }
 #pragma unroll 8
-    for (int i = lane; i < nv; i += 32) dst[i] = src[i];
+    for (; i < nv; i += 32) dst[i] = src[i];
   }
 }
 
