@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) decode_attention_flat_kernel(con
     }
     const int first = b_first - base, last = __shfl_sync(0xffffffffu, w_ptr, b - w0) - base;  // the request's pages
     const int piece = start + i, end = min(last, start + count);
-    const int len = (last - first - 1) * F_PAGE + len16, own = first + (pos >> 4);  // own: the page of the step's row
+    const int len = (last - first - 1) * F_PAGE + len16, own = pos >> 4 < (len + F_PAGE - 1) / F_PAGE ? first + (pos >> 4) : -1;  // own: the page of the step's row
     {
       const uint2* q = reinterpret_cast<const uint2*>(a.q + ((size_t)b * NQ + head * F_GROUP) * F_HD);
       uint2 raw[F_GROUP];
@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(F_THREADS, 1) decode_attention_flat_kernel(con
         if (lane < 16) *reinterpret_cast<uint4*>(k_tile + f_at(r, lane)) = reinterpret_cast<const uint4*>(k_s)[lane];
         else *reinterpret_cast<uint4*>(v_tile + f_at(r, lane - 16)) = reinterpret_cast<const uint4*>(v_s)[lane - 16];
       }
-      if (at == last - 1 && (len & 15) != 0)  // rows past the context: V zero, so that 0 times what lies there stays 0
-        for (int x = lane; x < (16 - (len & 15)) * 16; x += 32) *reinterpret_cast<uint4*>(v_tile + f_at((len & 15) + (x >> 4), x & 15)) = make_uint4(0, 0, 0, 0);
+      if (at == last - 1 && len16 < F_PAGE)  // rows past the context (a page may be there before its first token): V zero, so that 0 times what lies there stays 0
+        for (int x = lane; x < (F_PAGE - len16) * 16; x += 32) *reinterpret_cast<uint4*>(v_tile + f_at(len16 + (x >> 4), x & 15)) = make_uint4(0, 0, 0, 0);
       __syncwarp();
       const uint32_t kt = smem_u32(k_tile), vt = smem_u32(v_tile);
       float s[2][4] = {}, s1[2][4] = {};  // even and odd k steps apart: half as long a chain

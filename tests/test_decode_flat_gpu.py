@@ -10,7 +10,7 @@ import torch
 from pegainfer_b200 import ffi
 
 pytestmark = pytest.mark.gpu
-NQ, NKV, HD, PS = 32, 8, 128, 16
+NQ, NKV, HD, PS, MIN_PAGES = 32, 8, 128, 16, 2
 
 
 @pytest.fixture(scope="module")
@@ -21,23 +21,14 @@ def lib():
     return l
 
 
-def rope(x, cos, sin):
-    a, b = x.chunk(2, -1)
-    return (x.float() * cos[:, None].float() + torch.cat([-b, a], -1).float() * sin[:, None].float()).bfloat16()
-
-
-def normed(x, w):  # the rounding points of qk_norm_rope.cu
-    inv = torch.rsqrt(x.float().square().mean(-1, keepdim=True) + 1e-6)
-    return ((x.float() * inv).bfloat16().float() * w.float()).bfloat16()
-
-
-def check(lib, lens, v_first=False, empty=(), rounds=1, places=37):
-    """empty: requests without a page (their length is taken for zero)"""
+def check(lib, lens, v_first=False, empty=(), rounds=1, places=37, spare=()):
+    """empty: requests without a page (their length is taken for zero); spare: requests whose last page holds no token yet (last_page_len 0)"""
     g = torch.Generator(device="cuda").manual_seed(sum(lens) + len(lens))
     rn = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
     lens = [0 if i in empty else n for i, n in enumerate(lens)]
-    bs, need = len(lens), [(n + PS - 1) // PS for n in lens]
+    lens = [(n + PS - 1) // PS * PS if i in spare else n for i, n in enumerate(lens)]
+    bs, need = len(lens), [(n + PS - 1) // PS + (i in spare) for i, n in enumerate(lens)]
     order = (torch.randperm(sum(need), generator=g, device="cuda") + 1).tolist()
     ptr = [0]
     for m in need:
@@ -58,8 +49,11 @@ def check(lib, lens, v_first=False, empty=(), rounds=1, places=37):
     ang = torch.arange(4096, device="cuda")[:, None] * inv
     cos, sin = torch.cat([ang.cos()] * 2, 1).bfloat16(), torch.cat([ang.sin()] * 2, 1).bfloat16()
     pos = i32([max(n - 1, 0) for n in lens])
-    last, order_d, ptr_d = i32([(n - 1) % PS + 1 if n else 0 for n in lens]), i32(order), i32(ptr)
+    last, order_d, ptr_d = i32([0 if i in spare else (n - 1) % PS + 1 if n else 0 for i, n in enumerate(lens)]), i32(order), i32(ptr)
     partial, counters = torch.full((bs * places * NQ * (HD + 2),), float("nan"), device="cuda"), torch.zeros(bs * NKV, dtype=torch.int32, device="cuda")
+    # the kernel leaves states in `partial` where a request lies in several runs, as one of more pages than a run must; the cluster form never touches it
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    flat, run = bs * NKV > sms and bs * places >= 2 * sms, max((sum(need) + sms - 1) // sms, MIN_PAGES + 1)
     half, before = PS * NKV * HD, pool.clone()
     got = []
     for _ in range(rounds):
@@ -70,26 +64,30 @@ def check(lib, lens, v_first=False, empty=(), rounds=1, places=37):
                                                   bs, 2 * half, HD ** -0.5, None) == 0
         torch.cuda.synchronize()
         assert (out[bs] == 7.0).all() and lib.pk_b200_wait_errors() == 0 and not counters.any()
+        if max(need) > run or not flat:
+            assert partial.isnan().all().item() != flat
         got.append(out[:bs].clone())
     assert all(torch.equal(x, got[0]) for x in got)
-    at = pos.long()
-    qr, kr = rope(normed(q, qw), cos[at], sin[at]), rope(normed(k, kw), cos[at], sin[at])
+    qr, kr = q.clone(), k.clone()  # normed and rotated by the kernel of the same arithmetic (tested by itself)
+    lib.qk_norm_rope_batched_decode_cuda(qr.data_ptr(), kr.data_ptr(), qw.data_ptr(), kw.data_ptr(), cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), NQ, NKV, HD,
+                                         bs, 1e-6, None)
+    torch.cuda.synchronize()
     for i, n in enumerate(lens):
         if not n:
             assert not got[0][i].any()
             continue
         page, row = order[ptr[i] + (n - 1) // PS], (n - 1) % PS
-        new_k = pool[page, kx, row].float()
-        # one bf16 rounding of the norm and one of the rotation may fall to the other side
-        assert ((new_k - kr[i].float()).abs() <= 2 ** -6 * kr[i].float().abs() + 2 ** -7).all() and torch.equal(pool[page, vx, row], v[i])
+        assert torch.equal(pool[page, kx, row], kr[i]) and torch.equal(pool[page, vx, row], v[i])
         before[page, :, row] = pool[page, :, row]
         keys, vals = ctx[i][0, :n].double(), ctx[i][1, :n].double()
-        keys[n - 1], vals[n - 1] = new_k.double(), v[i].double()
+        keys[n - 1], vals[n - 1] = kr[i].double(), v[i].double()
         for h in range(NQ):
             p = torch.softmax(keys[:, h // 4] @ qr[i, h].double() * HD ** -0.5, 0)
             want = p @ vals[:, h // 4]
-            # q as the kernel rounds it may be an ulp off in single entries (scores move by 2^-8 of their spread); the result is rounded once
-            assert (got[0][i, h].double() - want).norm() <= 2 ** -6 * want.norm() + 1e-3, (i, h)
+            # The result is rounded to bf16 once (2^-8 of an entry).  Weights are held to 16 bits; an entry of q whose norm or rotation rounds the other way
+            # than in the kernel that qr comes from (entries below 4: 2^-6, by a key's 2, by the scale 2^-3.5) moves them by 2^-8
+            size, off = p @ vals[:, h // 4].abs(), (got[0][i, h].double() - want).abs()
+            assert (off <= 2 ** -8 * (want.abs() + size)).all() and off.norm() <= 2 ** -8 * want.norm() + 2 ** -10 * size.norm(), (i, h)
     assert torch.equal(pool.nan_to_num(), before.nan_to_num())  # nothing else was written
 
 
@@ -98,6 +96,12 @@ def check(lib, lens, v_first=False, empty=(), rounds=1, places=37):
     [33] * 70, [2048] * 19, [5, 900, 16, 2047, 31, 32, 64] * 5])
 def test_against_64_bits(lib, lens):
     check(lib, lens, rounds=2)
+
+
+def test_last_pages_without_a_token(lib):
+    """a page that was taken ahead of its first token, first in a run, last in one and alone in one; what lies there (NaN) is not looked at"""
+    check(lib, [100 + 31 * i for i in range(20)], spare=range(0, 20, 3))
+    check(lib, [16] * 30, spare=range(30))
 
 
 def test_values_before_keys(lib):
