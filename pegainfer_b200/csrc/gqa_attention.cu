@@ -308,30 +308,26 @@ __global__ void __launch_bounds__(kGqaWarps * 32) gqa_attention_kernel(const E* 
 // next block's copy overlaps this block's products); S = Q K^T and O += P V with mma.sync m16n8k16, P rounded to bf16 for the
 // second product, statistics in fp32.
 constexpr int kAmRows = 64, kAmKeys = 64;
+constexpr int kGdTileFrom = 8;  // tokens of a request, at least, that run in tiles in a step of few rows
 
+// Rows t0 .. min(t0 + 64, t_end) - 1 of head h; of every request's 64-key blocks share `split` of `nsplit`, whose states go to part_o / part_ml
+// [head][part_ld][T] where there are several
 template <int DQ, int DV>
-__global__ void __launch_bounds__(128, 3) gqa_attention_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache, const bf16* __restrict__ sink,
-                                                               const int* __restrict__ pos, const int* __restrict__ req,
-                                                               const int* __restrict__ page_off, const int* __restrict__ pages,
-                                                               bf16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
-                                                               long page_stride, int page_size, int T, int H, int G, float scale, int chunk,
-                                                               AttnExtra x) {
-  constexpr int LDK = DQ + 8, LDV = DV + 8;
-  extern __shared__ __align__(16) unsigned char am_smem[];  // two stages of [keys][LDK] K and [keys][LDV] V
+__device__ __forceinline__ void gqa_tile(unsigned char* am_smem, const bf16* __restrict__ q, const bf16* __restrict__ cache, const bf16* __restrict__ sink,
+                                         const int* __restrict__ pos, const int* __restrict__ req, const int* __restrict__ page_off, const int* __restrict__ pages,
+                                         bf16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml, long page_stride, int page_size, int T,
+                                         int H, int G, float scale, int chunk, const AttnExtra& x, int t0, int t_end, int h, int split, int nsplit, int part_ld) {
+  constexpr int LDK = DQ + 8, LDV = DV + 8;  // am_smem: two stages of [keys][LDK] K and [keys][LDV] V
   bf16* const Ks0 = reinterpret_cast<bf16*>(am_smem);
   bf16* const Vs0 = Ks0 + 2 * kAmKeys * LDK;
   __shared__ int s_req[kAmRows], s_pos[kAmRows];
   __shared__ long long s_slot[2][kAmKeys];  // per stage: element offset of every key row's cache slot (-1: not to be read)
-  pdl_wait();
-  pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
-  // grid (head, tile, split): the heads of a tile start together (a group's heads read the same keys), and the tiles run from the
-  // end of the step backwards, so that the CTAs that start last are the ones with the fewest visible keys
-  const int t0 = (gridDim.y - 1 - blockIdx.y) * kAmRows, h = blockIdx.x, g = h / (H / G);
+  const int g = h / (H / G);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gq = lane >> 2, tq = lane & 3;
   if (tid < kAmRows) {
     const int t = t0 + tid;
-    s_req[tid] = t < T ? req[t] : -1;
-    s_pos[tid] = t < T ? pos[t] : -1;
+    s_req[tid] = t < t_end ? req[t] : -1;
+    s_pos[tid] = t < t_end ? pos[t] : -1;
   }
   __syncthreads();
   const int tok = G * (DQ + DV);
@@ -345,7 +341,6 @@ __global__ void __launch_bounds__(128, 3) gqa_attention_mma_kernel(const bf16* _
   const bool capped = x.softcap > 0.f;
   const float slope2 = head_slope(x.slope_log2, h, H) * kLog2e, cap2 = x.softcap * kLog2e;
   const float c1 = capped ? 2.f * scale / x.softcap * kLog2e : scale * kLog2e;  // raw score -> ex2 argument of e^(2z) / -> plain scaled score
-  const int split = blockIdx.z, nsplit = gridDim.z;  // few rows: every request's 64-key blocks are dealt out to gridDim.z CTAs
   // Q fragments (A operand, row-major 16 x DQ)
   uint32_t qa[DQ / 16][4];
 #pragma unroll
@@ -493,7 +488,7 @@ __global__ void __launch_bounds__(128, 3) gqa_attention_mma_kernel(const bf16* _
     r_first = r_last + 1;
   }
   if (nsplit > 1) {  // partial state (running maximum, sum, unnormalised output) of this split; gqa_attention_merge_kernel finishes the rows
-    const size_t sa = ((size_t)(h * nsplit + split) * T + (t0 + ra)), sb = ((size_t)(h * nsplit + split) * T + (t0 + rb));
+    const size_t sa = ((size_t)(h * part_ld + split) * T + (t0 + ra)), sb = ((size_t)(h * part_ld + split) * T + (t0 + rb));
     if (req_a >= 0 && tq == 0) part_ml[sa * 2] = m_a * kLn2, part_ml[sa * 2 + 1] = l_a;  // maxima leave in natural units
     if (req_b >= 0 && tq == 0) part_ml[sb * 2] = m_b * kLn2, part_ml[sb * 2 + 1] = l_b;
 #pragma unroll
@@ -526,6 +521,51 @@ __global__ void __launch_bounds__(128, 3) gqa_attention_mma_kernel(const bf16* _
     if (req_a >= 0) *reinterpret_cast<uint32_t*>(out + (size_t)(t0 + ra) * x.out_ld + h * DV + c) = pack_bf16(oa[ni][0] * i_a * g0, oa[ni][1] * i_a * g1);
     if (req_b >= 0) *reinterpret_cast<uint32_t*>(out + (size_t)(t0 + rb) * x.out_ld + h * DV + c) = pack_bf16(oa[ni][2] * i_b * g2, oa[ni][3] * i_b * g3);
   }
+}
+
+template <int DQ, int DV>
+__global__ void __launch_bounds__(128, 3) gqa_attention_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache, const bf16* __restrict__ sink,
+                                                               const int* __restrict__ pos, const int* __restrict__ req,
+                                                               const int* __restrict__ page_off, const int* __restrict__ pages,
+                                                               bf16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
+                                                               long page_stride, int page_size, int T, int H, int G, float scale, int chunk,
+                                                               AttnExtra x) {
+  extern __shared__ __align__(16) unsigned char am_smem[];
+  pdl_wait();
+  pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
+  // grid (head, tile, split): the heads of a tile start together (a group's heads read the same keys), and the tiles run from the
+  // end of the step backwards, so that the CTAs that start last are the ones with the fewest visible keys
+  // few rows: every request's 64-key blocks are dealt out to gridDim.z CTAs
+  gqa_tile<DQ, DV>(am_smem, q, cache, sink, pos, req, page_off, pages, out, part_o, part_ml, page_stride, page_size, T, H, G, scale, chunk, x,
+                   (gridDim.y - 1 - blockIdx.y) * kAmRows, T, blockIdx.x, blockIdx.z, gridDim.z, gridDim.z);
+}
+
+// Steps of fewer than 64 rows (below): how a request with several tokens in the step runs.  Launched are cs CTAs for each of its tokens and kv heads; request by
+// request most of them leave, and what stays walks long contexts in tiles of 16 keys, a chain of about 1.2 us each (0.9 for heads of 64).  In tiles of 64 rows all
+// of them take a share of the keys, which needs a merge.
+struct GdRun {
+  int start, len;  // its tokens of the step
+  int shares;      // 0: request by request (gqa_decode_kernel); else in tiles of 64 rows per query head, the keys dealt out to so many CTAs each
+};
+// All lanes of a warp call; T < 64.  `slots`: CTAs that the GPU holds at once (0: never in tiles); a request counts on its part of them.
+__device__ __forceinline__ GdRun gd_run(const int* req, const int* pos, int T, int t, int H, int G, int cs, int keep_first, int window, int chunk, int slots, int from) {
+  const int lane = threadIdx.x & 31, rq = req[t], r0 = lane < T ? req[lane] : -1, r1 = lane + 32 < T ? req[lane + 32] : -1;
+  const int p0 = slots > 0 && lane < T ? pos[lane] : 0, p1 = slots > 0 && lane + 32 < T ? pos[lane + 32] : 0;
+  const unsigned long long other = (unsigned long long)__ballot_sync(0xffffffffu, lane >= T || r0 != rq) |
+                                   (unsigned long long)__ballot_sync(0xffffffffu, lane + 32 >= T || r1 != rq) << 32;
+  const unsigned long long below = other & ((1ull << t) - 1), above = other >> t;  // (T < 64: there is one above)
+  GdRun r;
+  r.start = below ? 64 - __clzll((long long)below) : 0;
+  r.len = t + __ffsll((long long)above) - 1 - r.start;
+  r.shares = 0;
+  if (slots > 0 && r.len >= kGdTileFrom) {
+    auto pos_of = [&](int u) { return __shfl_sync(0xffffffffu, u < 32 ? p0 : p1, u & 31); };
+    const int lo = first_visible(pos_of(r.start), chunk, window), seen = min(keep_first, lo) + pos_of(r.start + r.len - 1) - lo + 1;
+    const int n = min(slots * r.len / (T * H), r.len * G * cs / H);
+    // a CTA of a tile walks 1 / n of the keys, a warp of a cluster 1 / (4 cs), which take it twice as long
+    if (seen > from && n >= 2 * cs) r.shares = min(min(n, 64), (seen + kAmKeys - 1) / kAmKeys + 1);
+  }
+  return r;
 }
 
 // one CTA per (row, head): combine the splits' (m, l, O), join the sink, apply the output gate
@@ -569,12 +609,68 @@ __global__ void gqa_attention_merge_kernel(const float* __restrict__ part_o, con
   }
 }
 
+// The same for a step whose requests may run in tiles (gd_run): a warp per (row, head), and rows of requests that do not stay as they are.  What the choice
+// follows from is older than the kernel before this one, so it is looked at ahead of the wait for it.
+template <int D>
+__global__ void __launch_bounds__(256) gqa_run_merge_kernel(const float* __restrict__ part, const bf16* __restrict__ sink, const int* __restrict__ pos,
+                                                           const int* __restrict__ req, bf16* __restrict__ out, int most, int T, int H, int G, int cs, int chunk,
+                                                           AttnExtra x, int slots, int from) {
+  const int t = blockIdx.x, lane = threadIdx.x & 31, h = blockIdx.y * 8 + (threadIdx.x >> 5);
+  const GdRun run = gd_run(req, pos, T, t, H, G, cs, x.keep_first, x.window, chunk, slots, from);
+  pdl_wait();
+  pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
+  if (run.shares < 2 || h >= H) return;
+  const float* ml = part + (size_t)H * most * T * D;
+  const size_t row0 = (size_t)h * most * T + t;  // row of share s: row0 + s T
+  float m[2], l[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int s = lane + 32 * i;
+    m[i] = s < run.shares ? ml[(row0 + (size_t)s * T) * 2] : -INFINITY;
+    l[i] = s < run.shares ? ml[(row0 + (size_t)s * T) * 2 + 1] : 0.f;
+  }
+  const float sk = sink ? bf2f(sink[h]) : -INFINITY, M = fmaxf(warp_max(fmaxf(m[0], m[1])), sk);  // finite: a query always sees its own position
+#pragma unroll
+  for (int i = 0; i < 2; ++i) m[i] = m[i] == -INFINITY ? 0.f : expf(m[i] - M);
+  const float inv = 1.f / (warp_sum(l[0] * m[0] + l[1] * m[1]) + (sink ? expf(sk - M) : 0.f));
+  constexpr int PAIRS = D / 2, NP = (PAIRS + 31) / 32;
+  float2 o[NP] = {};
+  constexpr int AT_ONCE = 12 / NP;  // loads under way
+  for (int s0 = 0; s0 < run.shares; s0 += AT_ONCE) {
+    float2 v[AT_ONCE][NP];
+#pragma unroll
+    for (int u = 0; u < AT_ONCE; ++u)
+#pragma unroll
+      for (int i = 0; i < NP; ++i)
+        v[u][i] = s0 + u < run.shares && lane + 32 * i < PAIRS ? *reinterpret_cast<const float2*>(part + (row0 + (size_t)(s0 + u) * T) * D + 2 * (lane + 32 * i))
+                                                              : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < AT_ONCE; ++u) {
+      const int s = s0 + u;
+      const float w = s < run.shares ? __shfl_sync(0xffffffffu, s < 32 ? m[0] : m[1], s & 31) * inv : 0.f;
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        o[i].x = fmaf(v[u][i].x, w, o[i].x);
+        o[i].y = fmaf(v[u][i].y, w, o[i].y);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NP; ++i)
+    if (lane + 32 * i < PAIRS) {
+      const int d = 2 * (lane + 32 * i);
+      const float g0 = x.gate ? out_gate<bf16>(x, t, h, d, D) : 1.f, g1 = x.gate ? out_gate<bf16>(x, t, h, d + 1, D) : 1.f;
+      *reinterpret_cast<uint32_t*>(out + (size_t)t * x.out_ld + h * D + d) = pack_bf16(o[i].x * g0, o[i].y * g1);
+    }
+}
+
 // ---- fewer than 64 rows (decode steps, small portions), bf16: a cluster of CTAs per (tokens of one request, kv head).  The 16 rows of a tile are the group's
 // query heads, for as many tokens of the request as fit (a cluster is launched for every token, and the first of each tile's stays), so that a key is fetched
 // once for all of them and requests do not wait for one another.  A warp takes every (4 cs)-th tile of 16 visible keys through a cp.async ring of its own;
 // the warps' states meet in shared memory, the CTAs' in the cluster's.
 // Bound by latency: lookups, keys, exchange.  Figures at launch_gqa_mma.
 constexpr int kGdWarps = 4, kGdRing = 3;
+constexpr size_t kGdScratch = 256 * 1024;  // of the thread's scratch memory: its first part holds counters of paged_attention_decode_cuda, which stay zero between calls
 __device__ __forceinline__ uint32_t gd_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -592,11 +688,12 @@ __device__ __forceinline__ float2 gd_remote(const float2* p, uint32_t rank) {  /
   return v;
 }
 
-template <int D>
-__global__ void __launch_bounds__(kGdWarps * 32, 2) gqa_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache, const bf16* __restrict__ sink,
+// TILES: requests with several tokens of the step may run in tiles (gd_run)
+template <int D, bool TILES>
+__global__ void __launch_bounds__(kGdWarps * 32, TILES && D <= 64 ? 3 : 2) gqa_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache, const bf16* __restrict__ sink,
                                                                     const int* __restrict__ pos, const int* __restrict__ req, const int* __restrict__ page_off,
                                                                     const int* __restrict__ pages, bf16* __restrict__ out, long page_stride, int page_size, int T,
-                                                                    int H, int G, float scale, int chunk, AttnExtra x) {
+                                                                    int H, int G, float scale, int chunk, AttnExtra x, float* __restrict__ part, int most, int slots, int from) {
   constexpr int LD = D + 8, TILE = 16 * LD;
   extern __shared__ __align__(16) unsigned char gd_smem[];  // [warps][ring][K, V][16][LD]; later the states, [warps][16][D] floats at the warps' rings
   __shared__ long long s_off[kGdWarps][kGdRing][16];
@@ -606,15 +703,19 @@ __global__ void __launch_bounds__(kGdWarps * 32, 2) gqa_decode_kernel(const bf16
   pdl_wait();
   pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
   // the tokens of this one's request around it
-  const int rq = req[t], r0 = lane < T ? req[lane] : -1, r1 = lane + 32 < T ? req[lane + 32] : -1;
-  const unsigned long long other = (unsigned long long)__ballot_sync(0xffffffffu, lane >= T || r0 != rq) |
-                                   (unsigned long long)__ballot_sync(0xffffffffu, lane + 32 >= T || r1 != rq) << 32;
-  const unsigned long long below = other & ((1ull << t) - 1), above = other >> t;  // (T < 64: there is one above)
-  const int start = below ? 64 - __clzll((long long)below) : 0, left = __ffsll((long long)above) - 1;
+  const GdRun run = gd_run(req, pos, T, t, H, G, cs, x.keep_first, x.window, chunk, TILES ? slots : 0, from);
+  if (TILES && run.shares > 0) {
+    const int nth = ((t - run.start) * G + g) * cs + rank;
+    if (nth < H * run.shares)
+      gqa_tile<D, D>(gd_smem, q, cache, sink, pos, req, page_off, pages, out, part, part + (size_t)H * most * T * D, page_stride, page_size, T, H, G, scale, chunk, x,
+                     run.start, run.start + run.len, nth % H, nth / H, run.shares, most);
+    return;  // (the whole cluster)
+  }
+  const int start = run.start, left = run.start + run.len - t;
   if ((t - start) % per != 0) return;  // (the whole cluster)
   const int n_tok = min(per, left);
   const int p_max = pos[t + n_tok - 1], lo = first_visible(pos[t], chunk, x.window), nf = min(x.keep_first, lo), n_vis = nf + p_max - lo + 1;
-  const int* pg = pages + page_off[rq];
+  const int* pg = pages + page_off[req[t]];
   const int tok = 2 * G * D, n_tiles = (n_vis + 15) / 16, step = cs * kGdWarps;
   bf16* ring = reinterpret_cast<bf16*>(gd_smem) + warp * kGdRing * 2 * TILE;
   auto key_of = [&](int i) { return i < nf ? i : lo + i - nf; };  // position of visible key i
@@ -833,13 +934,28 @@ static cudaError_t launch_gqa_decode(const bf16* q, const bf16* cache, const bf1
                                    bf16* out, long page_stride, int page_size, int T, int H, int G, float scale, int chunk, AttnExtra x, int span,
                                    cudaStream_t st) {
   constexpr size_t smem = (size_t)kGdWarps * kGdRing * 2 * 16 * (D + 8) * sizeof(bf16);
-  static std::atomic<uint64_t> smem_set{0};
-  if (const cudaError_t e = allow_smem(smem_set, (const void*)gqa_decode_kernel<D>, smem); e != cudaSuccess) return e;
-  // As many CTAs as the keys occupy and the GPU holds twice: of a portion's clusters most leave at once.  (60 tokens behind 400 cached: 16.1 us with what it
-  // holds once, 13.5 so; 16 requests of 2000 17.6 / 20.7.)  Steps of over 40 rows are portions more often: twice that again.
+  static_assert(smem >= (size_t)2 * kAmKeys * 2 * (D + 8) * sizeof(bf16), "gqa_tile's stages");
+  static std::atomic<uint64_t> smem_set[2];
+  // No more CTAs than the keys occupy, and as many as the GPU holds twice (four times from 41 tokens on: portions more often, of whose clusters most leave at
+  // once), but not where each token, or every second one, has a tile of its own.  B200, us, in a graph, by cluster size 1 / 2 / 4 / 8.  16 heads of 128 in 4 groups,
+  // 1 / 16 / 32 / 48 / 63 decoding requests at 2000: 40.0 24.6 15.0 10.1 | 40.6 25.3 18.8 24.3 | 43.3 35.0 39.3 51.1 | 53.0 62.3 57.4 75.4 | 55.1 65.5 74.4 98.6;
+  // portions of 8 / 16 / 32 / 60 tokens behind 400: 12.4 11.0 8.5 8.6 | 12.4 11.1 9.9 9.2 | 12.5 12.8 10.3 12.4 | 16.0 13.7 12.8 20.5 (a step's requests are not
+  // known here: the rule lies between the two).  In one group, 40 behind 400: 12.5 11.2 10.4 16.4.  64 heads of 64 in 8 groups, 60 behind 400: 14.4 19.9 23.2 36.4.
+  const int per = 16 / (H / G);
+  const long hold = (per == 1 ? 2L : per > 2 && T > 40 ? 8L : 4L) * sm_count();
   int cs = 8;
-  while (cs > 1 && ((long)cs * G * T > (T > 40 ? 8L : 4L) * sm_count() || (cs / 2) * kGdWarps * 16 >= span)) cs /= 2;
+  while (cs > 1 && ((long)cs * G * T > hold || (cs / 2) * kGdWarps * 16 >= span)) cs /= 2;
+  // A request with several tokens may run in tiles (gd_run) where its keys are many: below, the merge and the tiles' longer start cost more than they save.
+  // slots: at 128 entries a head two CTAs fit on an SM, but clusters of 8 not on every pair of them (304 of 296 or 288: a second round, 48 instead of 31 us).
+  // B200, us, in a graph, request by request -> in tiles (tiles of 64 rows for all requests, as before there was a choice): 16 heads of 128 in 4 groups, 24
+  // tokens behind 2000 18.7 -> 16.2 (15.7), 40 behind 2000 31.6 -> 16.1 (19.4), 60 behind 8000 59.3 -> 39.9 (42.4); in 8 groups, 24 behind 400 12.7 -> 9.9 (9.3);
+  // 16 heads of 64 in 16 groups, 24 behind 2000 / 8000 32.6 -> 14.5 (12.5), 118.7 -> 24.3 (23.4); 64 heads of 64 in 8 groups, 60 behind 8000 160 -> 84 (75).
   ThreadState& ts = tls();
+  const int from = max((D <= 64 ? 600 : cs == 8 ? 300 : 150) * cs, 400);
+  const int slots = (D <= 64 ? 20 : 14) * sm_count() / 8, most = min(max(slots / H, 1), 64);
+  const bool tiles = T >= kGdTileFrom && span > from && kGdScratch + (size_t)H * most * T * (D + 2) * sizeof(float) <= ts.scratch_bytes;
+  auto kern = tiles ? gqa_decode_kernel<D, true> : gqa_decode_kernel<D, false>;
+  if (const cudaError_t e = allow_smem(smem_set[tiles], (const void*)kern, smem); e != cudaSuccess) return e;
   ts.launches++;
   cudaLaunchConfig_t lc{};
   lc.gridDim = dim3(cs, G, T);
@@ -855,45 +971,48 @@ static cudaError_t launch_gqa_decode(const bf16* q, const bf16* cache, const bf1
   at[1].val.programmaticStreamSerializationAllowed = ts.pdl ? 1 : 0;
   lc.attrs = at;
   lc.numAttrs = 2;
-  return cudaLaunchKernelEx(&lc, gqa_decode_kernel<D>, q, cache, sink, pos, req, page_off, pages, out, page_stride, page_size, T, H, G, scale, chunk, x);
+  float* part = tiles ? reinterpret_cast<float*>(static_cast<char*>(ts.scratch) + kGdScratch) : nullptr;
+  const cudaError_t e = cudaLaunchKernelEx(&lc, kern, q, cache, sink, pos, req, page_off, pages, out, page_stride, page_size, T, H, G, scale, chunk, x, part, most, slots, from);
+  if (e != cudaSuccess || !tiles) return e;
+  return launch(gqa_run_merge_kernel<D>, dim3(T, (H + 7) / 8), dim3(256), 0, st, true, (const float*)part, sink, pos, req, out, most, T, H, G, cs, chunk, x, slots, from);
 }
 
-template <int DQ, int DV>
+template <int D>
 static void launch_gqa_mma(const bf16* q, const bf16* cache, const bf16* sink, const int* pos, const int* req, const int* page_off, const int* pages,
                            bf16* out, long page_stride, int page_size, int T, int H, int G, float scale, int chunk, AttnExtra x, cudaStream_t st) {
-  const size_t smem = (size_t)2 * kAmKeys * (DQ + 8 + DV + 8) * sizeof(bf16);
+  const size_t smem = (size_t)2 * kAmKeys * 2 * (D + 8) * sizeof(bf16);
   static bool attr_set = false;  // per template instance
   if (!attr_set) {
-    cudaFuncSetAttribute(gqa_attention_mma_kernel<DQ, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(gqa_attention_mma_kernel<D, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     attr_set = true;
   }
   // The span a row can see is bounded by the window / chunk, else by the longest context of the step (when the caller knows it).
-  // Fewer than 64 rows run request by request; more (and groups of over 16 heads) in tiles of 64, the few-row ones with the key axis dealt out to several
-  // CTAs per (tile, head) so that the step fills the GPU.  B200, us, 16 heads of 128 in 4 groups, tiles of 64 -> request by request: 1 / 4 / 16 / 32 decoding
-  // requests at 2048, 2048 (window 1024), 2000, 2000 12.0 18.9 85 187 -> 10.6 8.0 20.7 33.3; portions of one request, 8 / 32 / 60 tokens 5.6 6.8 8.9 ->
-  // 5.0 5.3 6.5, 16 / 60 behind 400 8.8 11.7 -> 8.8 12.1, two of 31 behind 2000 28.3 -> 21.6.
+  // Fewer than 64 rows run request by request (requests with many tokens and keys in tiles, in the same launch); more, and groups of over 16 heads, in tiles of
+  // 64, the few-row ones with the key axis dealt out to several CTAs per (tile, head) so that the step fills the GPU.  B200, us, in a graph, 16 heads of 128 in 4
+  // groups, tiles of 64 -> the other form: 4 / 16 / 32 / 63 decoding requests at 2000 (the first with a window of 1024) 18.8 107 221 429 -> 8.5 23.7 39.0 73.7.
+  // One token of up to 16 heads of up to 64 entries behind more than 5000 stays in tiles: 8000 keys, 8 heads in 4 groups 15.1 there, 18.8 in a cluster (16 heads in
+  // 16 groups 19.4, 21.6; behind 2000 9.8, 8.1).
   const int tiles = (T + kAmRows - 1) / kAmRows;
   int span = x.max_kv_len;
   if (x.window > 0) span = span > 0 ? min(span, x.window + x.keep_first + T) : x.window + x.keep_first + T;
   if (chunk > 0) span = span > 0 ? min(span, chunk) : chunk;
-  if constexpr (DQ == DV)
-    if (T < kAmRows && H / G <= 16) {
-      launch_gqa_decode<DQ>(q, cache, sink, pos, req, page_off, pages, out, page_stride, page_size, T, H, G, scale, chunk, x, span > 0 ? span : 1 << 30, st);
-      return;
-    }
+  if (T < kAmRows && H / G <= 16 && !(T == 1 && D <= 64 && H <= 16 && span > 5000)) {
+    launch_gqa_decode<D>(q, cache, sink, pos, req, page_off, pages, out, page_stride, page_size, T, H, G, scale, chunk, x, span > 0 ? span : 1 << 30, st);
+    return;
+  }
   int splits = 1;
   ThreadState& ts = tls();
   if (T < kAmRows && span > 2 * kAmKeys && ts.scratch) {
     const int blocks = (span + kAmKeys - 1) / kAmKeys + 1;
     splits = min(min(blocks, (2 * sm_count() + tiles * H - 1) / (tiles * H)), 64);
-    while (splits > 1 && (size_t)H * splits * T * (DV + 2) * sizeof(float) > ts.scratch_bytes) --splits;
+    while (splits > 1 && (size_t)H * splits * T * (D + 2) * sizeof(float) > ts.scratch_bytes) --splits;
   }
   float* po = static_cast<float*>(ts.scratch);
-  float* pml = po ? po + (size_t)H * splits * T * DV : nullptr;
-  launch(gqa_attention_mma_kernel<DQ, DV>, dim3(H, tiles, splits), dim3(128), smem, st, true, q, cache, sink, pos, req, page_off, pages, out, po, pml,
+  float* pml = po ? po + (size_t)H * splits * T * D : nullptr;
+  launch(gqa_attention_mma_kernel<D, D>, dim3(H, tiles, splits), dim3(128), smem, st, true, q, cache, sink, pos, req, page_off, pages, out, po, pml,
          page_stride, page_size, T, H, G, scale, chunk, x);
   if (splits > 1)
-    launch(gqa_attention_merge_kernel, dim3(T, H), dim3(DV >= 128 ? 128 : 64), 0, st, true, (const float*)po, (const float*)pml, sink, out, splits, T, H, DV, x);
+    launch(gqa_attention_merge_kernel, dim3(T, H), dim3(D >= 128 ? 128 : 64), 0, st, true, (const float*)po, (const float*)pml, sink, out, splits, T, H, D, x);
 }
 
 }  // namespace pk
@@ -979,7 +1098,7 @@ extern "C" int pk_gqa_attention_ex(const void* q, const void* cache, const void*
   // bf16 prompt portions always; single decoded tokens too when the caller asked through the _ex entry (the key axis is then split)
   if (!f32 && (tokens >= 32 || extra) && aligned && dim == vdim && (dim == 64 || dim == 128 || dim == 32 || dim == 96) && (dim * kv_heads) % 8 == 0) {
 #define PK_GQA_MMA(D) \
-  launch_gqa_mma<D, D>((const bf16*)q, (const bf16*)cache, (const bf16*)sink, positions, req, page_off, pages, (bf16*)out, page_stride, page_size, tokens, heads, kv_heads, scale, chunk, x, st)
+  launch_gqa_mma<D>((const bf16*)q, (const bf16*)cache, (const bf16*)sink, positions, req, page_off, pages, (bf16*)out, page_stride, page_size, tokens, heads, kv_heads, scale, chunk, x, st)
     if (dim == 32) PK_GQA_MMA(32);
     else if (dim == 64) PK_GQA_MMA(64);
     else if (dim == 96) PK_GQA_MMA(96);

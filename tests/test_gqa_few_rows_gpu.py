@@ -96,5 +96,14 @@ def test_options(lib, steps, opts):
     check(lib, steps, 16, 4, 128, **opts)
 
 
+@pytest.mark.parametrize("H,G,D", [(16, 4, 128), (8, 8, 64), (16, 8, 96), (6, 2, 32), (24, 3, 128), (16, 1, 128)])
+@pytest.mark.parametrize("steps", [[(24, 2500)], [(8, 4200)], [(1, 6000)], [(60, 900)], [(9, 2600), (1, 9), (3, 0)], [(20, 130), (1, 3000), (30, 97), (12, 800)]])
+def test_requests_that_run_in_tiles(lib, H, G, D, steps):
+    """several tokens behind many keys: a request's clusters become the CTAs of tiles of 64 rows, beside requests that run by themselves"""
+    check(lib, steps, H, G, D)
+    check(lib, steps, H, G, D, window=700, keep=9, softcap=25.0, gate="entry")
+    check(lib, steps, H, G, D, chunk=512, slope=6.0, sink=False, gate="head", known=False)
+
+
 def test_more_heads_to_a_group_than_a_tile_has_rows(lib):
     check(lib, [(1, 300), (7, 20)], 40, 2, 64)
