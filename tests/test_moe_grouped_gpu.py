@@ -62,6 +62,13 @@ def test_rows_per_expert(lib, counts, W, ff, act):
     assert (got.double() - want).norm() <= 2e-3 * want.norm()
 
 
+@pytest.mark.parametrize("W", [248, 2040, 2048, 2056, 4104])
+@pytest.mark.parametrize("counts", [[0, 1, 15, 5], [300, 12, 500]])
+def test_rows_around_what_is_fetched_ahead(lib, counts, W):
+    """moe_place_kernel holds the first 2048 entries of a warp's first row while it looks for the row's place"""
+    test_rows_per_expert(lib, counts, W, 24, 0)
+
+
 @pytest.mark.parametrize("T,top,E", [(33, 6, 64), (3000, 6, 64), (700, 2, 1500)])
 def test_many_pairs_and_experts(lib, T, top, E):
     g = torch.Generator(device="cuda").manual_seed(T)
