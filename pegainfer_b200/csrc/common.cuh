@@ -21,9 +21,12 @@ constexpr int kWarp = 32;
 struct ThreadState {
   int64_t launches = 0;
   bool pdl = false;
-  // scratch created by cublas_init()
+  // scratch created by cublas_init(): counters that are zero between calls (paged_attention_decode_cuda's), behind them work memory of any contents
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
+  static constexpr size_t kCounterBytes = 256 * 1024;
+  float* work() const { return scratch ? reinterpret_cast<float*>(static_cast<char*>(scratch) + kCounterBytes) : nullptr; }
+  size_t work_bytes() const { return scratch_bytes > kCounterBytes ? scratch_bytes - kCounterBytes : 0; }
   int sm_count = 0;
   int device = -1;
 };

@@ -533,8 +533,7 @@ int paged_attention_decode_cuda(const pk_bf16* q, pk_bf16* output, const pk_bf16
     return launch_cluster_or_tma(c, num_kv_heads, batch_size, stream);
   }
   ThreadState& ts = tls();
-  // scratch layout: [counters: bs*nkv ints, padded to 4 KB][fp32 partials]
-  const size_t counter_bytes = 4096 + (((size_t)batch_size * num_kv_heads * 4 + 4095) & ~(size_t)4095);
+  const size_t counter_bytes = (size_t)batch_size * num_kv_heads * 4;
   DecodeAttnArgs a{};
   a.q = (const bf16*)q; a.out = (bf16*)output; a.kv = (bf16*)kv_data;
   a.k_off = k_offset_elems; a.v_off = v_offset_elems;
@@ -543,11 +542,11 @@ int paged_attention_decode_cuda(const pk_bf16* q, pk_bf16* output, const pk_bf16
   a.nq = num_qo_heads; a.nkv = num_kv_heads; a.page_size = page_size; a.stride_page = stride_page;
   a.sm_scale_log2 = sm_scale * 1.44269504088896340736f;
   a.min_chunk = 64;
-  if (ts.scratch != nullptr && ts.scratch_bytes > counter_bytes) {
+  if (ts.work() && counter_bytes <= ThreadState::kCounterBytes) {
     a.counters = reinterpret_cast<int*>(ts.scratch);
-    a.partial = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ts.scratch) + counter_bytes);
+    a.partial = ts.work();
     a.max_chunks = pick_max_chunks(batch_size, num_kv_heads, num_qo_heads,
-                                   (ts.scratch_bytes - counter_bytes) / 4);
+                                   ts.work_bytes() / 4);
   } else {
     a.max_chunks = 1;  // cublas_init() not called on this thread: no split (reference behaviour)
   }

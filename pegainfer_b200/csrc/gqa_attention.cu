@@ -493,7 +493,6 @@ __global__ void __launch_bounds__(256) gqa_run_merge_kernel(const float* __restr
 // the warps' states meet in shared memory, the CTAs' in the cluster's.
 // Bound by latency: lookups, keys, exchange.  Figures at launch_gqa_mma.
 constexpr int kGdWarps = 4, kGdRing = 3;
-constexpr size_t kGdScratch = 256 * 1024;  // of the thread's scratch memory: its first part holds counters of paged_attention_decode_cuda, which stay zero between calls
 __device__ __forceinline__ uint32_t gd_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -776,7 +775,7 @@ static cudaError_t launch_gqa_decode(const bf16* q, const bf16* cache, const bf1
   ThreadState& ts = tls();
   const int from = max((D <= 64 ? 600 : cs == 8 ? 300 : 150) * cs, 400);
   const int slots = (D <= 64 ? 20 : 14) * sm_count() / 8, most = min(max(slots / H, 1), 64);
-  const bool tiles = T >= kGdTileFrom && span > from && kGdScratch + (size_t)H * most * T * (D + 2) * sizeof(float) <= ts.scratch_bytes;
+  const bool tiles = T >= kGdTileFrom && span > from && (size_t)H * most * T * (D + 2) * sizeof(float) <= ts.work_bytes();
   auto kern = tiles ? gqa_decode_kernel<D, true> : gqa_decode_kernel<D, false>;
   if (const cudaError_t e = allow_smem(smem_set[tiles], (const void*)kern, smem); e != cudaSuccess) return e;
   ts.launches++;
@@ -794,7 +793,7 @@ static cudaError_t launch_gqa_decode(const bf16* q, const bf16* cache, const bf1
   at[1].val.programmaticStreamSerializationAllowed = ts.pdl ? 1 : 0;
   lc.attrs = at;
   lc.numAttrs = 2;
-  float* part = tiles ? reinterpret_cast<float*>(static_cast<char*>(ts.scratch) + kGdScratch) : nullptr;
+  float* part = tiles ? ts.work() : nullptr;
   const cudaError_t e = cudaLaunchKernelEx(&lc, kern, q, cache, sink, pos, req, page_off, pages, out, page_stride, page_size, T, H, G, scale, chunk, x, part, most, slots, from);
   if (e != cudaSuccess || !tiles) return e;
   return launch(gqa_run_merge_kernel<D>, dim3(T, (H + 7) / 8), dim3(256), 0, st, true, (const float*)part, sink, pos, req, out, most, T, H, G, cs, chunk, x, slots, from);
@@ -825,12 +824,12 @@ static void launch_gqa_mma(const bf16* q, const bf16* cache, const bf16* sink, c
   }
   int splits = 1;
   ThreadState& ts = tls();
-  if (T < kAmRows && span > 2 * kAmKeys && ts.scratch) {
+  if (T < kAmRows && span > 2 * kAmKeys && ts.work()) {
     const int blocks = (span + kAmKeys - 1) / kAmKeys + 1;
     splits = min(min(blocks, (2 * sm_count() + tiles * H - 1) / (tiles * H)), 64);
-    while (splits > 1 && (size_t)H * splits * T * (D + 2) * sizeof(float) > ts.scratch_bytes) --splits;
+    while (splits > 1 && (size_t)H * splits * T * (D + 2) * sizeof(float) > ts.work_bytes()) --splits;
   }
-  float* po = static_cast<float*>(ts.scratch);
+  float* po = ts.work();
   float* pml = po ? po + (size_t)H * splits * T * D : nullptr;
   launch(gqa_attention_mma_kernel<D, D>, dim3(H, tiles, splits), dim3(128), smem, st, true, q, cache, sink, pos, req, page_off, pages, out, po, pml,
          page_stride, page_size, T, H, G, scale, chunk, x);

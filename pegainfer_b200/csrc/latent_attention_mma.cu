@@ -330,11 +330,11 @@ int launch_latent_attention_mma(const bf16* qa, const bf16* cache, const bf16* s
   const int tiles = (total + rows - 1) / rows;
   int splits = 1;
   ThreadState& ts = tls();
-  if (max_kv_len > 2 * kMmaKeys && tiles < 2 * sm_count() && ts.scratch) {
+  if (max_kv_len > 2 * kMmaKeys && tiles < 2 * sm_count() && ts.work()) {
     splits = min(min((2 * sm_count() + tiles - 1) / tiles, (max_kv_len + kMmaKeys - 1) / kMmaKeys), 64);
-    while (splits > 1 && (size_t)tiles * splits * rows * (rank + 2) * 4 > ts.scratch_bytes) --splits;
+    while (splits > 1 && (size_t)tiles * splits * rows * (rank + 2) * 4 > ts.work_bytes()) --splits;
   }
-  float* po = static_cast<float*>(ts.scratch);
+  float* po = ts.work();
   float* pml = po ? po + (size_t)tiles * splits * rows * rank : nullptr;
   const dim3 grid(tiles, splits);
   const int nv = rank / 32;

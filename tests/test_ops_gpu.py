@@ -329,6 +329,27 @@ def test_paged_attention_decode(lib, seq_lens, nq, nkv):
     assert_bf16_close(bits(out), want, 3, floor=float(np.abs(f32(want)).max()) / 32, what="decode attn")
 
 
+@pytest.mark.parametrize("dirty", ["latent", "grouped"])
+def test_paged_attention_decode_behind_other_splits(dirty):
+    """The counters of the split decode attention live in the thread's scratch memory and have to be zero: kernels that leave partial sums of their own there in
+    between must not touch them (they did, and outputs stayed unwritten)."""
+    lib = get_lib("b200")
+    bf = lambda *s: (1 + torch.rand(*s, device="cuda")).bfloat16()  # noqa: E731
+    n, H = 3000, 20
+    pages, zero, pos = i32(np.arange(n // 16 + 1, dtype=np.int32)), i32(np.zeros(1, np.int32)), i32(np.array([n - 1], np.int32))
+    if dirty == "latent":
+        q, cache, out = bf(H, 192), bf(n // 16 + 1, 16, 192), bf(H, 128)
+        assert lib.pk_latent_attention_ex(p(q), p(cache), None, p(pos), p(zero), p(zero), p(pages), p(out), 16 * 192, 16, 1, H, 128, 64, 0.07, 0, n, 0, stream()) == 0
+    else:  # over 16 heads to a group: tiles of 64 rows with the keys dealt out
+        q, cache, out = bf(H, 128), bf(n // 16 + 1, 16, 256), bf(H, 128)
+        ex = ffi.AttnExtra(window=0, softcap=0.0, slope_log2=0.0, keep_first=0, gate=None, gate_ld=0, gate_per_head=0, max_kv_len=n)
+        import ctypes as C
+        assert lib.pk_gqa_attention_ex(p(q), p(cache), None, p(pos), p(zero), p(zero), p(pages), p(out), 16 * 256, 16, 1, H, 1, 128, 128, 0.09, 0, C.byref(ex), 0,
+                                       stream()) == 0
+    torch.cuda.synchronize()
+    test_paged_attention_decode(lib, [3000, 17, 640], 16, 8)
+
+
 @pytest.mark.parametrize("seq_lens", [[1024], [2300, 1100]])
 def test_paged_attention_decode_split_kv(lib, seq_lens):
     nq, nkv, hd, layer, bs = 32, 8, 128, 0, len(seq_lens)
