@@ -18,8 +18,7 @@ namespace pk {
 namespace {
 
 constexpr int F_HD = 128, F_GROUP = 4, F_PAGE = 16, F_WARPS = 8, F_THREADS = F_WARPS * 32;
-constexpr int F_HALF = F_PAGE * 128;  // bytes of 64 columns of a page of one head
-constexpr int F_TILE = 4 * F_HALF;    // K lo | K hi | V lo | V hi (V first where it lies first in the pool)
+constexpr int F_TILE = 4 * kDaHalf;    // K lo | K hi | V lo | V hi (V first where it lies first in the pool)
 constexpr int F_SLOTS = 3;
 constexpr int F_MIN_PAGES = 2;        // pages of a CTA at least
 
@@ -36,49 +35,11 @@ struct FlatArgs {
   unsigned int* err;
 };
 
-__device__ __forceinline__ float f_ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 __device__ __forceinline__ void f_tma_page(uint32_t dst, const CUtensorMap* map, int head, int page, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %2, %3, %2, %4}], [%5];" ::"r"(dst),
       "l"(map), "r"(0), "r"(2 * head), "r"(page), "r"(smem_u32(bar))
       : "memory");
-}
-__device__ __forceinline__ void f_ldsm4(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void f_ldsm4_t(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-// A operand: rows 0-3 are the query heads, rows 8-15 are zero
-__device__ __forceinline__ void f_mma(float (&c)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%5}, {%7,%8}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1));
-}
-// byte offset of 16-byte piece c (0..15) of row r of a K (V) tile: two halves with the 128-byte swizzle
-__device__ __forceinline__ uint32_t f_at(int r, int c) { return (uint32_t)((c >> 3) * F_HALF + r * 128 + (((c & 7) ^ (r & 7)) << 4)); }
-
-// norm + rotation of one head, four entries to a lane (the arithmetic of qk_norm_rope.cu)
-__device__ __forceinline__ void f_norm_rope(uint2 raw, uint2 wr, uint2 cr, uint2 sr, float eps, bf16* dst, int lane) {
-  const float v[4] = {bf16_lo(raw.x), bf16_hi(raw.x), bf16_lo(raw.y), bf16_hi(raw.y)};
-  float ss = v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3];
-  ss = warp_sum(ss);
-  const float inv = rsqrtf(ss / (float)F_HD + eps);
-  const float wv[4] = {bf16_lo(wr.x), bf16_hi(wr.x), bf16_lo(wr.y), bf16_hi(wr.y)};
-  const float c[4] = {bf16_lo(cr.x), bf16_hi(cr.x), bf16_lo(cr.y), bf16_hi(cr.y)};
-  const float s[4] = {bf16_lo(sr.x), bf16_hi(sr.x), bf16_lo(sr.y), bf16_hi(sr.y)};
-  float o[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float t = round_bf16(round_bf16(v[j] * inv) * wv[j]);
-    const float other = __shfl_xor_sync(0xffffffffu, t, 16);
-    o[j] = lane < 16 ? t * c[j] - other * s[j] : other * s[j] + t * c[j];
-  }
-  reinterpret_cast<uint2*>(dst)[lane] = make_uint2(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]));
 }
 
 __global__ void __launch_bounds__(F_THREADS, 1) decode_attention_flat_kernel(const __grid_constant__ CUtensorMap map, const FlatArgs a) {
@@ -176,11 +137,11 @@ __global__ void __launch_bounds__(F_THREADS, 1) decode_attention_flat_kernel(con
 #pragma unroll
       for (int h = 0; h < F_GROUP; ++h) raw[h] = q[h * 32 + lane];
 #pragma unroll
-      for (int h = 0; h < F_GROUP; ++h) f_norm_rope(raw[h], qw, cr, sr, a.eps, q_s + h * F_HD, lane);
+      for (int h = 0; h < F_GROUP; ++h) da_norm_rope(raw[h], qw, cr, sr, a.eps, q_s + h * F_HD, lane);
       if (own >= piece && own < end) {
         const size_t row = ((size_t)b * F_WARPS + head) * F_HD;
         const uint2 kr = reinterpret_cast<const uint2*>(a.k_new + row)[lane], vr = reinterpret_cast<const uint2*>(a.v_new + row)[lane];
-        f_norm_rope(kr, kw, cr, sr, a.eps, k_s, lane);
+        da_norm_rope(kr, kw, cr, sr, a.eps, k_s, lane);
         reinterpret_cast<uint2*>(v_s)[lane] = vr;
         __syncwarp();
         const int64_t dst = (int64_t)pages[own - start] * a.stride_page + ((int64_t)(pos & 15) * F_WARPS + head) * F_HD;
@@ -205,23 +166,23 @@ __global__ void __launch_bounds__(F_THREADS, 1) decode_attention_flat_kernel(con
       mbar_wait_bounded(full + slot, par, dead);
       __syncwarp();
       uint8_t* k_tile = tiles + (size_t)slot * F_TILE + a.k_at;
-      uint8_t* v_tile = tiles + (size_t)slot * F_TILE + (2 * F_HALF - a.k_at);
+      uint8_t* v_tile = tiles + (size_t)slot * F_TILE + (2 * kDaHalf - a.k_at);
       if (at == own) {  // the step's own row: the copy may have come before it was written
         const int r = pos & 15;
-        if (lane < 16) *reinterpret_cast<uint4*>(k_tile + f_at(r, lane)) = reinterpret_cast<const uint4*>(k_s)[lane];
-        else *reinterpret_cast<uint4*>(v_tile + f_at(r, lane - 16)) = reinterpret_cast<const uint4*>(v_s)[lane - 16];
+        if (lane < 16) *reinterpret_cast<uint4*>(k_tile + da_at(r, lane)) = reinterpret_cast<const uint4*>(k_s)[lane];
+        else *reinterpret_cast<uint4*>(v_tile + da_at(r, lane - 16)) = reinterpret_cast<const uint4*>(v_s)[lane - 16];
       }
       if (at == last - 1 && len16 < F_PAGE)  // rows past the context (a page may be there before its first token): V zero, so that 0 times what lies there stays 0
-        for (int x = lane; x < (F_PAGE - len16) * 16; x += 32) *reinterpret_cast<uint4*>(v_tile + f_at(len16 + (x >> 4), x & 15)) = make_uint4(0, 0, 0, 0);
+        for (int x = lane; x < (F_PAGE - len16) * 16; x += 32) *reinterpret_cast<uint4*>(v_tile + da_at(len16 + (x >> 4), x & 15)) = make_uint4(0, 0, 0, 0);
       __syncwarp();
       const uint32_t kt = smem_u32(k_tile), vt = smem_u32(v_tile);
       float s[2][4] = {}, s1[2][4] = {};  // even and odd k steps apart: half as long a chain
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk) {
         uint32_t r[4];
-        f_ldsm4(kt + f_at(k_tok, kk * 2 + k_c), r);
-        f_mma(kk & 1 ? s1[0] : s[0], qa[kk][0], qa[kk][1], r[0], r[1]);
-        f_mma(kk & 1 ? s1[1] : s[1], qa[kk][0], qa[kk][1], r[2], r[3]);
+        da_ldsm4(kt + da_at(k_tok, kk * 2 + k_c), r);
+        da_mma(kk & 1 ? s1[0] : s[0], qa[kk][0], qa[kk][1], r[0], r[1]);
+        da_mma(kk & 1 ? s1[1] : s[1], qa[kk][0], qa[kk][1], r[2], r[3]);
       }
       const int tb = (at - first) * F_PAGE + 2 * tq;
       float mx = -INFINITY;
@@ -233,13 +194,13 @@ __global__ void __launch_bounds__(F_THREADS, 1) decode_attention_flat_kernel(con
       }
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-      const float m_new = fmaxf(m_run, mx), m_safe = m_new == -INFINITY ? 0.f : m_new, alpha = f_ex2(m_run - m_safe);
+      const float m_new = fmaxf(m_run, mx), m_safe = m_new == -INFINITY ? 0.f : m_new, alpha = da_ex2(m_run - m_safe);
       m_run = m_new;
       uint32_t ph[2], pl[2];  // P = hi + lo, bf16 each: 16 bits of p
       float sum = 0.f;
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const float p0 = f_ex2(s[j][0] - m_safe), p1 = f_ex2(s[j][1] - m_safe);
+        const float p0 = da_ex2(s[j][0] - m_safe), p1 = da_ex2(s[j][1] - m_safe);
         sum += p0 + p1;
         ph[j] = pack_bf16(p0, p1);
         pl[j] = pack_bf16(p0 - bf16_lo(ph[j]), p1 - bf16_hi(ph[j]));
@@ -253,11 +214,11 @@ __global__ void __launch_bounds__(F_THREADS, 1) decode_attention_flat_kernel(con
 #pragma unroll
       for (int dp = 0; dp < 8; ++dp) {
         uint32_t r[4];
-        f_ldsm4_t(vt + f_at(v_tok, dp * 2 + v_c), r);
-        f_mma(o[2 * dp], ph[0], ph[1], r[0], r[1]);
-        f_mma(o[2 * dp + 1], ph[0], ph[1], r[2], r[3]);
-        f_mma(o[2 * dp], pl[0], pl[1], r[0], r[1]);
-        f_mma(o[2 * dp + 1], pl[0], pl[1], r[2], r[3]);
+        da_ldsm4_t(vt + da_at(v_tok, dp * 2 + v_c), r);
+        da_mma(o[2 * dp], ph[0], ph[1], r[0], r[1]);
+        da_mma(o[2 * dp + 1], ph[0], ph[1], r[2], r[3]);
+        da_mma(o[2 * dp], pl[0], pl[1], r[0], r[1]);
+        da_mma(o[2 * dp + 1], pl[0], pl[1], r[2], r[3]);
       }
       __syncwarp();
       if (i + F_SLOTS < count && lane == 0 && !*dead) {
@@ -313,7 +274,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) decode_attention_flat_kernel(con
       for (int h = 0; h < F_GROUP; ++h) {
         const float2 ml = __ldcg(reinterpret_cast<const float2*>(pm + (at + h) * 2));
         const float4 x = __ldcg(reinterpret_cast<const float4*>(a.partial + (at + h) * F_HD) + lane);
-        const float w = ml.x == -INFINITY ? 0.f : f_ex2(ml.x - M[h]);
+        const float w = ml.x == -INFINITY ? 0.f : da_ex2(ml.x - M[h]);
         L[h] = fmaf(ml.y, w, L[h]);
         acc[h] = make_float4(fmaf(x.x, w, acc[h].x), fmaf(x.y, w, acc[h].y), fmaf(x.z, w, acc[h].z), fmaf(x.w, w, acc[h].w));
       }
@@ -369,7 +330,7 @@ int launch_decode_attention_flat(const ClusterAttnArgs& c, int nkv, int bs, floa
     return -2;
   }
   const FlatArgs a{c.q, c.k_new, c.v_new, c.out, c.kv, c.k_off, c.v_off, c.stride_page, c.page_indices, c.page_indptr, c.last_page_len, c.positions,
-                   c.qw, c.kw, c.cosc, c.sinc, c.eps, c.sm_scale_log2, bs, c.k_off < c.v_off ? 0 : 2 * F_HALF, partial, counters, wait_err_word()};
+                   c.qw, c.kw, c.cosc, c.sinc, c.eps, c.sm_scale_log2, bs, c.k_off < c.v_off ? 0 : 2 * kDaHalf, partial, counters, wait_err_word()};
   return (int)launch(decode_attention_flat_kernel, dim3(sms), dim3(F_THREADS), smem, stream, true, map, a);
 }
 

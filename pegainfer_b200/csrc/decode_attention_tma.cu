@@ -38,8 +38,7 @@ constexpr int T_WARPS = 8;
 constexpr int T_THREADS = T_WARPS * 32;
 constexpr int T_GROUP = 4;
 constexpr int T_PAGE = 16;
-constexpr int T_HALF = T_PAGE * 128;        // bytes of one 64-column half of a page tile (16 rows x 128 B)
-constexpr int T_SLOT = 4 * T_HALF;          // K lo | K hi | V lo | V hi = 8 KB
+constexpr int T_SLOT = 4 * kDaHalf;          // K lo | K hi | V lo | V hi = 8 KB
 constexpr int T_MAX_CLUSTER = 16;
 constexpr int T_MAX_SLOTS = 24;
 
@@ -54,11 +53,6 @@ struct TmaAttnArgs {
   int nq, nkv, nslot;
 };
 
-__device__ __forceinline__ float t_ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 __device__ __forceinline__ uint32_t t_cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -106,55 +100,12 @@ __device__ __forceinline__ void t_wait_or_trap(uint64_t* bar, uint32_t parity) {
   for (uint32_t spins = 0; !mbar_try_wait(bar, parity); ++spins)
     if (spins > (1u << 26)) __trap();
 }
-__device__ __forceinline__ void t_ldsm4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-               : "r"(addr));
-}
-__device__ __forceinline__ void t_ldsm4_t(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-               : "r"(addr));
-}
-__device__ __forceinline__ void t_mma(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// byte offset of 16-byte chunk c16 (0..15) of token row r (0..15) inside one K (or V) page tile: two 64-column halves,
-// each [16 rows x 128 B] with the TMA 128-byte swizzle (chunk ^= row & 7)
-__device__ __forceinline__ uint32_t t_sw(int r, int c16) {
-  return (uint32_t)((c16 >> 3) * T_HALF + r * 128 + (((c16 & 7) ^ (r & 7)) << 4));
-}
-
-// warp-level QK RMSNorm + RoPE of one 128-wide head (qk_norm_rope.cu arithmetic), result to shared memory
-__device__ __forceinline__ void t_norm_rope(const bf16* __restrict__ src, const bf16* __restrict__ w,
-                                            const bf16* __restrict__ cosc, const bf16* __restrict__ sinc, int pos,
-                                            float eps, bf16* dst, int lane) {
-  const uint2 raw = reinterpret_cast<const uint2*>(src)[lane];
-  const float v[4] = {bf16_lo(raw.x), bf16_hi(raw.x), bf16_lo(raw.y), bf16_hi(raw.y)};
-  float ss = v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3];
-  ss = warp_sum(ss);
-  const float inv = rsqrtf(ss / (float)T_HD + eps);
-  const uint2 wr = reinterpret_cast<const uint2*>(w)[lane];
-  const float wv[4] = {bf16_lo(wr.x), bf16_hi(wr.x), bf16_lo(wr.y), bf16_hi(wr.y)};
-  const int ci = (lane & 15) * 4;
-  const uint2 cr = reinterpret_cast<const uint2*>(cosc + (size_t)pos * T_HD + ci)[0];
-  const uint2 sr = reinterpret_cast<const uint2*>(sinc + (size_t)pos * T_HD + ci)[0];
-  const float c[4] = {bf16_lo(cr.x), bf16_hi(cr.x), bf16_lo(cr.y), bf16_hi(cr.y)};
-  const float s[4] = {bf16_lo(sr.x), bf16_hi(sr.x), bf16_lo(sr.y), bf16_hi(sr.y)};
-  float o[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float t = round_bf16(round_bf16(v[j] * inv) * wv[j]);
-    const float other = __shfl_xor_sync(0xffffffffu, t, 16);
-    o[j] = lane < 16 ? t * c[j] - other * s[j] : other * s[j] + t * c[j];
-  }
-  uint2 res;
-  res.x = pack_bf16(o[0], o[1]);
-  res.y = pack_bf16(o[2], o[3]);
-  reinterpret_cast<uint2*>(dst)[lane] = res;
+// norm + rotation of one head, result to shared memory
+__device__ __forceinline__ void t_norm_rope(const bf16* __restrict__ src, const bf16* __restrict__ w, const bf16* __restrict__ cosc, const bf16* __restrict__ sinc,
+                                            int pos, float eps, bf16* dst, int lane) {
+  const size_t at = (size_t)pos * T_HD + (lane & 15) * 4;
+  da_norm_rope(reinterpret_cast<const uint2*>(src)[lane], reinterpret_cast<const uint2*>(w)[lane], *reinterpret_cast<const uint2*>(cosc + at),
+               *reinterpret_cast<const uint2*>(sinc + at), eps, dst, lane);
 }
 
 __global__ void __launch_bounds__(T_THREADS, 1)
@@ -214,9 +165,9 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     const uint32_t dst = smem_u32(tiles + (size_t)slot * T_SLOT);
     mbar_expect_tx(full + slot, T_SLOT);
     t_tma_4d(dst, &map_k, 0, kvh, 0, page, full + slot);
-    t_tma_4d(dst + T_HALF, &map_k, 64, kvh, 0, page, full + slot);
-    t_tma_4d(dst + 2 * T_HALF, &map_v, 0, kvh, 0, page, full + slot);
-    t_tma_4d(dst + 3 * T_HALF, &map_v, 64, kvh, 0, page, full + slot);
+    t_tma_4d(dst + kDaHalf, &map_k, 64, kvh, 0, page, full + slot);
+    t_tma_4d(dst + 2 * kDaHalf, &map_v, 0, kvh, 0, page, full + slot);
+    t_tma_4d(dst + 3 * kDaHalf, &map_v, 64, kvh, 0, page, full + slot);
   };
   // first pass over the ring: each slot's owner warp (slot & 7) requests its page now
   if (lane == 0)
@@ -271,27 +222,27 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     const int gp = p_lo + lp;
     if (lp == pos_lp) {  // patch the step's own row into the tile (the TMA saw the slot before it was written)
       const int r = pos & 15;
-      if (lane < 16) *reinterpret_cast<uint4*>(tile + t_sw(r, lane)) = reinterpret_cast<const uint4*>(k_s)[lane];
-      else *reinterpret_cast<uint4*>(tile + 2 * T_HALF + t_sw(r, lane - 16)) = reinterpret_cast<const uint4*>(v_s)[lane - 16];
+      if (lane < 16) *reinterpret_cast<uint4*>(tile + da_at(r, lane)) = reinterpret_cast<const uint4*>(k_s)[lane];
+      else *reinterpret_cast<uint4*>(tile + 2 * kDaHalf + da_at(r, lane - 16)) = reinterpret_cast<const uint4*>(v_s)[lane - 16];
     }
     if (gp == tot_pages - 1 && (len & 15) != 0) {  // rows past the context: zero V so that 0 * garbage stays 0
       for (int i = lane; i < (16 - (len & 15)) * 16; i += 32) {
         const int r = (len & 15) + (i >> 4);
-        *reinterpret_cast<uint4*>(tile + 2 * T_HALF + t_sw(r, i & 15)) = make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4*>(tile + 2 * kDaHalf + da_at(r, i & 15)) = make_uint4(0, 0, 0, 0);
       }
     }
     __syncwarp();
-    const uint32_t kt = smem_u32(tile), vt = kt + 2 * T_HALF;
+    const uint32_t kt = smem_u32(tile), vt = kt + 2 * kDaHalf;
     // ---- S[16 x 16] = Q K^T ----
     float s[2][4];
 #pragma unroll
     for (int j = 0; j < 2; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) {
-      uint32_t b0, b1, b2, b3;
-      t_ldsm4(kt + t_sw(k_tok, kk * 2 + k_c), b0, b1, b2, b3);
-      t_mma(s[0], qa[kk][0], 0u, qa[kk][1], 0u, b0, b1);
-      t_mma(s[1], qa[kk][0], 0u, qa[kk][1], 0u, b2, b3);
+      uint32_t r[4];
+      da_ldsm4(kt + da_at(k_tok, kk * 2 + k_c), r);
+      da_mma(s[0], qa[kk][0], qa[kk][1], r[0], r[1]);
+      da_mma(s[1], qa[kk][0], qa[kk][1], r[2], r[3]);
     }
     // ---- online softmax on row g (lanes g >= 4 carry all-zero rows: harmless) ----
     const int tb = gp * T_PAGE + 2 * tq;
@@ -306,13 +257,13 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
     const float m_new = fmaxf(m_run, mx);
     const float m_safe = m_new == -INFINITY ? 0.f : m_new;
-    const float alpha = t_ex2(m_run - m_safe);
+    const float alpha = da_ex2(m_run - m_safe);
     m_run = m_new;
     float p[2][2];
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      p[j][0] = t_ex2(s[j][0] - m_safe);
-      p[j][1] = t_ex2(s[j][1] - m_safe);
+      p[j][0] = da_ex2(s[j][0] - m_safe);
+      p[j][1] = da_ex2(s[j][1] - m_safe);
     }
     l_run = l_run * alpha + ((p[0][0] + p[0][1]) + (p[1][0] + p[1][1]));
 #pragma unroll
@@ -330,12 +281,12 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     // ---- O[16 x 128] += P V ----
 #pragma unroll
     for (int dp = 0; dp < 8; ++dp) {
-      uint32_t v0, v1, v2, v3;
-      t_ldsm4_t(vt + t_sw(v_tok, dp * 2 + v_c), v0, v1, v2, v3);
-      t_mma(o[2 * dp], ph[0], 0u, ph[1], 0u, v0, v1);
-      t_mma(o[2 * dp], pl[0], 0u, pl[1], 0u, v0, v1);
-      t_mma(o[2 * dp + 1], ph[0], 0u, ph[1], 0u, v2, v3);
-      t_mma(o[2 * dp + 1], pl[0], 0u, pl[1], 0u, v2, v3);
+      uint32_t r[4];
+      da_ldsm4_t(vt + da_at(v_tok, dp * 2 + v_c), r);
+      da_mma(o[2 * dp], ph[0], ph[1], r[0], r[1]);
+      da_mma(o[2 * dp], pl[0], pl[1], r[0], r[1]);
+      da_mma(o[2 * dp + 1], ph[0], ph[1], r[2], r[3]);
+      da_mma(o[2 * dp + 1], pl[0], pl[1], r[2], r[3]);
     }
     // refill: this warp is the only reader of the slot -> request the page that reuses it
     if (lp + nslot < my_pages) {
@@ -378,7 +329,7 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
         for (int w = 0; w < T_WARPS; ++w) {
           const float mw = st_m[w * T_GROUP + h];
           if (mw != -INFINITY) {
-            const float wt = t_ex2(mw - mx);
+            const float wt = da_ex2(mw - mx);
             dd = fmaf(st_d[w * T_GROUP + h], wt, dd);
             oo = fmaf(st_o[((size_t)w * T_GROUP + h) * T_HD + dim], wt, oo);
           }
@@ -410,7 +361,7 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
       for (int r = 0; r < cs; ++r) {
         const float mr = c_m[e0 + r];
         if (mr != -INFINITY) {
-          const float wt = t_ex2(mr - mx);
+          const float wt = da_ex2(mr - mx);
           dd = fmaf(c_d[e0 + r], wt, dd);
           oo = fmaf(c_o[(e0 + r) * T_HD + threadIdx.x], wt, oo);
         }

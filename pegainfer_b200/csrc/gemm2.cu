@@ -76,7 +76,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = g2_rank();
+  const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int M = a.M, N = a.N, K = a.K;
   const int m_tiles = (N + 2 * G2_BM - 1) / (2 * G2_BM);  // pair tiles along tokens
@@ -99,7 +99,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
   if (warp == 1) g2_tmem_alloc(tmem_slot, TMEM_COLS);
   tc_fence_before();
   __syncthreads();
-  g2_cluster_sync();  // both CTAs' barriers are initialised and both TMEM allocations are done
+  cluster_barrier();  // both CTAs' barriers are initialised and both TMEM allocations are done
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();
@@ -254,7 +254,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
   }
   tc_fence_before();
   __syncthreads();
-  g2_cluster_sync();  // the peer's MMAs / loads may still target this CTA's shared memory and TMEM
+  cluster_barrier();  // the peer's MMAs / loads may still target this CTA's shared memory and TMEM
   if (warp == 1) {
     tc_fence_after();
     g2_tmem_dealloc(tmem_base, TMEM_COLS);

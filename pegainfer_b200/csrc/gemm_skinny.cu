@@ -25,15 +25,6 @@ namespace {
 constexpr int SK_BM = 128, SK_BK = 64, SK_THREADS = 192;
 constexpr int SK_MAX_SPLIT = 8, SK_MAX_STAGES = 12;  // 8: the portable cluster size
 
-__device__ __forceinline__ uint32_t sk_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void sk_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float4 sk_ld_dsmem(uint32_t addr, uint32_t rank) {
   uint32_t a;
   float4 v;
@@ -73,7 +64,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int S = gridDim.x, sp = (int)sk_rank();  // the cluster spans the whole x axis
+  const int S = gridDim.x, sp = (int)cluster_ctarank();  // the cluster spans the whole x axis
   const int m0 = (blockIdx.y / a.n_tiles) * rows, t0 = (blockIdx.y % a.n_tiles) * NT;
   const int k_blocks = (a.K + SK_BK - 1) / SK_BK;
   const int kb0 = (sp * k_blocks) / S, nk = ((sp + 1) * k_blocks) / S - kb0;
@@ -164,7 +155,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   }
   tc_fence_before();
   __syncthreads();
-  if (S > 1) sk_cluster_sync();
+  if (S > 1) cluster_barrier();
   // ---- this CTA's share of the tile: (token, 4 features) items, added up in rank order
   const int quads = rows / 4, items = min(NT, a.N - t0) * quads;
   const int i0 = (sp * items) / S, i1 = ((sp + 1) * items) / S;
@@ -202,7 +193,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   }
   if (threadIdx.x == 0) count_run_out(dead, a.err);  // (every wait lies before the barrier above)
   __syncwarp();
-  if (S > 1) sk_cluster_sync();  // the others may still read this CTA's partial
+  if (S > 1) cluster_barrier();  // the others may still read this CTA's partial
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);

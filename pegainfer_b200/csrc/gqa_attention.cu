@@ -18,6 +18,7 @@
 //   gqa_attention_kernel        one CTA per (query row, query head): warps stride over the visible keys with an online
 //                               softmax each (lanes split the features), merged with the sink at the end.  Any sizes.
 //   gqa_attention_mma_kernel    bf16 prompt portions on the tensor cores (64 query rows of one head per CTA).
+//   gqa_decode_kernel           bf16, fewer than 64 rows: request by request on the tensor cores, a group's query heads as the rows of a tile.
 #include "common.cuh"
 #include "mma.cuh"
 #include "typed.cuh"
@@ -493,15 +494,6 @@ __global__ void __launch_bounds__(256) gqa_run_merge_kernel(const float* __restr
 // the warps' states meet in shared memory, the CTAs' in the cluster's.
 // Bound by latency: lookups, keys, exchange.  Figures at launch_gqa_mma.
 constexpr int kGdWarps = 4, kGdRing = 3;
-__device__ __forceinline__ uint32_t gd_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void gd_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float2 gd_remote(const float2* p, uint32_t rank) {  // the same place in another CTA of the cluster
   uint32_t at;
   float2 v;
@@ -521,7 +513,7 @@ __global__ void __launch_bounds__(kGdWarps * 32, TILES && D <= 64 ? 3 : 2) gqa_d
   __shared__ long long s_off[kGdWarps][kGdRing][16];
   __shared__ float2 s_ml[kGdWarps][16];  // (maximum, sum) of the warps' rows; later of the CTA's
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gq = lane >> 2, tq = lane & 3;
-  const int rank = (int)gd_rank(), cs = gridDim.x, g = blockIdx.y, t = blockIdx.z, R = H / G, per = 16 / R;
+  const int rank = (int)cluster_ctarank(), cs = gridDim.x, g = blockIdx.y, t = blockIdx.z, R = H / G, per = 16 / R;
   pdl_wait();
   pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
   // the tokens of this one's request around it
@@ -725,7 +717,7 @@ __global__ void __launch_bounds__(kGdWarps * 32, TILES && D <= 64 ? 3 : 2) gqa_d
     }
   }
   if (cs == 1) return;
-  gd_cluster_sync();
+  cluster_barrier();
   for (int r = rank * kGdWarps + warp; r < rows; r += cs * kGdWarps) {  // the CTAs' states: every warp of the cluster finishes rows
     float2 ml = make_float2(-INFINITY, 0.f), o[NP] = {};
     if (lane < cs) ml = gd_remote(&s_ml[0][r], lane);
@@ -748,7 +740,7 @@ __global__ void __launch_bounds__(kGdWarps * 32, TILES && D <= 64 ? 3 : 2) gqa_d
     }
     finish(r, M, den, o);
   }
-  gd_cluster_sync();  // nobody leaves while its states are read
+  cluster_barrier();  // nobody leaves while its states are read
 }
 
 template <int D>

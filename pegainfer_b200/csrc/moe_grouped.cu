@@ -264,9 +264,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMgThreads, 1) moe_g
   if (warp == 1) g2_tmem_alloc(tmem_slot, 512);
   tc_fence_before();
   __syncthreads();
-  g2_cluster_sync();  // both CTAs' barriers and accumulators are there
+  cluster_barrier();  // both CTAs' barriers and accumulators are there
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot, rank = g2_rank();
+  const uint32_t tmem_base = *tmem_slot, rank = cluster_ctarank();
   pdl_wait();
   pdl_launch_dependents();  // after the allocation: a dependent that came first would hold the TMEM while it waits for this grid
   const int* te = a.meta + 2 + a.experts;
@@ -407,7 +407,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMgThreads, 1) moe_g
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x == 0) count_run_out(dead, a.err);
-  g2_cluster_sync();  // the peer's MMAs and copies may still have this CTA's memory as their target
+  cluster_barrier();  // the peer's MMAs and copies may still have this CTA's memory as their target
   if (warp == 1) {
     tc_fence_after();
     g2_tmem_dealloc(tmem_base, 512);

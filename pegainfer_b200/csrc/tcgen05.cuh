@@ -143,19 +143,10 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 }
 
 // ---- CTA pairs (cluster of two, cta_group::2): gemm2.cu, moe_grouped.cu
-__device__ __forceinline__ uint32_t g2_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
 __device__ __forceinline__ uint32_t g2_map(uint32_t smem_addr, uint32_t rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
-}
-__device__ __forceinline__ void g2_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // TMA tile load whose completion bytes land on a barrier given as a shared::cluster address (the leader's)
 __device__ __forceinline__ void g2_tma_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar_cluster_addr) {
