@@ -18,7 +18,8 @@
 // Bound by the chain products -> sum over the warps -> triangle -> update (three barriers of the four warps a chunk); the figures stand where it is launched.
 // The roles' loops run side by side and have to share the SM's instruction cache: with the preparation unrolled to the end every role waited for its
 // instructions (hit rate 0.69 in one form), so its loops are rolled as far as their latency allows; keys of 64 gain nothing by it.  2048 tokens, 16 heads of 128: 173 -> 149 us,
-// 1024 tokens, 32 heads, 32 columns to a CTA: 180 -> 107 us, 24 tokens 7.4 -> 6.8 us (B200, the kernel alone; same sums in the same order).
+// 1024 tokens, 32 heads, 32 columns to a CTA: 180 -> 107 us (105 with the stages looked at early), 24 tokens 7.4 -> 6.8 us (B200, the kernel alone; same
+// sums in the same order).
 // Sums over s <= t leave the later tokens out by selection, not by a factor of zero: a NaN reaches the same tokens as token by token, and so does an
 // infinity, as a NaN (its parts are differences of infinities).
 #pragma once

@@ -24,7 +24,8 @@ def test_against_64_bits(lib, starts, lens, H, window, ps, sink, rank, rot):
     check_against_64_bits(lib, starts, lens, H, window, ps, sink, rank, rot)
 
 
-# other chunks of a CTA from none to eight (rings of 2, 8, 9, 7, 5 and 3 places), value chunks from one to four, and both in one launch
+# other chunks of a CTA from none to eight, value chunks from one to four, and both in one launch.  Rings of 0, 2, 6 and 8 places (two blocks' other
+# chunks) and of 9, which is less than two blocks' from five other chunks on: 448 + 64, 384 + 48 (one of the halves), 512 + 16 and the last three
 @pytest.mark.parametrize("rank,rot", [(256, 0), (64, 64), (448, 64), (384, 48), (512, 16), (192, 384), (128, 448), (64, 512)])
 @pytest.mark.parametrize("starts,lens,H,window,ps,sink", [([0, 77], [900, 301], 16, 0, 16, True), ([300, 0, 9], [1, 700, 340], 16, 130, 128, False)])
 def test_places_for_chunks(lib, starts, lens, H, window, ps, sink, rank, rot):
