@@ -502,12 +502,16 @@ __device__ __forceinline__ float2 gd_remote(const float2* p, uint32_t rank) {  /
   return v;
 }
 
-// TILES: requests with several tokens of the step may run in tiles (gd_run)
+// TILES: requests with several tokens of the step may run in tiles (gd_run), `most` shares at most, whose states go to `part`
+struct GdExtra : AttnExtra {
+  float* part;
+  int most, slots, from;
+};
 template <int D, bool TILES>
 __global__ void __launch_bounds__(kGdWarps * 32, TILES && D <= 64 ? 3 : 2) gqa_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache, const bf16* __restrict__ sink,
                                                                     const int* __restrict__ pos, const int* __restrict__ req, const int* __restrict__ page_off,
                                                                     const int* __restrict__ pages, bf16* __restrict__ out, long page_stride, int page_size, int T,
-                                                                    int H, int G, float scale, int chunk, AttnExtra x, float* __restrict__ part, int most, int slots, int from) {
+                                                                    int H, int G, float scale, int chunk, std::conditional_t<TILES, GdExtra, AttnExtra> x) {
   constexpr int LD = D + 8, TILE = 16 * LD;
   extern __shared__ __align__(16) unsigned char gd_smem[];  // [warps][ring][K, V][16][LD]; later the states, [warps][16][D] floats at the warps' rings
   __shared__ long long s_off[kGdWarps][kGdRing][16];
@@ -517,13 +521,18 @@ __global__ void __launch_bounds__(kGdWarps * 32, TILES && D <= 64 ? 3 : 2) gqa_d
   pdl_wait();
   pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
   // the tokens of this one's request around it
-  const GdRun run = gd_run(req, pos, T, t, H, G, cs, x.keep_first, x.window, chunk, TILES ? slots : 0, from);
-  if (TILES && run.shares > 0) {
-    const int nth = ((t - run.start) * G + g) * cs + rank;
-    if (nth < H * run.shares)
-      gqa_tile_of_run<D, D>(gd_smem, q, cache, sink, pos, req, page_off, pages, out, part, part + (size_t)H * most * T * D, page_stride, page_size, T, H, G, scale, chunk,
-                            x, run, nth % H, nth / H, most);
-    return;  // (the whole cluster)
+  GdRun run;
+  if constexpr (TILES) {
+    run = gd_run(req, pos, T, t, H, G, cs, x.keep_first, x.window, chunk, x.slots, x.from);
+    if (run.shares > 0) {
+      const int nth = ((t - run.start) * G + g) * cs + rank;
+      if (nth < H * run.shares)
+        gqa_tile_of_run<D, D>(gd_smem, q, cache, sink, pos, req, page_off, pages, out, x.part, x.part + (size_t)H * x.most * T * D, page_stride, page_size, T, H, G,
+                              scale, chunk, x, run, nth % H, nth / H, x.most);
+      return;  // (the whole cluster)
+    }
+  } else {
+    run = gd_run(req, pos, T, t, H, G, cs, x.keep_first, x.window, chunk, 0, 0);
   }
   const int start = run.start, left = run.start + run.len - t;
   if ((t - start) % per != 0) return;  // (the whole cluster)
@@ -749,7 +758,6 @@ static cudaError_t launch_gqa_decode(const bf16* q, const bf16* cache, const bf1
                                    cudaStream_t st) {
   constexpr size_t smem = (size_t)kGdWarps * kGdRing * 2 * 16 * (D + 8) * sizeof(bf16);
   static_assert(smem >= (size_t)2 * kAmKeys * 2 * (D + 8) * sizeof(bf16), "gqa_tile's stages");
-  static std::atomic<uint64_t> smem_set[2];
   // No more CTAs than the keys occupy, and as many as the GPU holds twice (four times from 41 tokens on: portions more often, of whose clusters most leave at
   // once), but not where each token, or every second one, has a tile of its own.  B200, us, in a graph, by cluster size 1 / 2 / 4 / 8.  16 heads of 128 in 4 groups,
   // 1 / 16 / 32 / 48 / 63 decoding requests at 2000: 40.0 24.6 15.0 10.1 | 40.6 25.3 18.8 24.3 | 43.3 35.0 39.3 51.1 | 53.0 62.3 57.4 75.4 | 55.1 65.5 74.4 98.6;
@@ -759,18 +767,7 @@ static cudaError_t launch_gqa_decode(const bf16* q, const bf16* cache, const bf1
   const long hold = (per == 1 ? 2L : per > 2 && T > 40 ? 8L : 4L) * sm_count();
   int cs = 8;
   while (cs > 1 && ((long)cs * G * T > hold || (cs / 2) * kGdWarps * 16 >= span)) cs /= 2;
-  // A request with several tokens may run in tiles (gd_run) where its keys are many: below, the merge and the tiles' longer start cost more than they save.
-  // slots: at 128 entries a head two CTAs fit on an SM, but clusters of 8 not on every pair of them (304 of 296 or 288: a second round, 48 instead of 31 us).
-  // B200, us, in a graph, request by request -> in tiles (tiles of 64 rows for all requests, as before there was a choice): 16 heads of 128 in 4 groups, 24
-  // tokens behind 2000 18.7 -> 16.2 (15.7), 40 behind 2000 31.6 -> 16.1 (19.4), 60 behind 8000 59.3 -> 39.9 (42.4); in 8 groups, 24 behind 400 12.7 -> 9.9 (9.3);
-  // 16 heads of 64 in 16 groups, 24 behind 2000 / 8000 32.6 -> 14.5 (12.5), 118.7 -> 24.3 (23.4); 64 heads of 64 in 8 groups, 60 behind 8000 160 -> 84 (75).
   ThreadState& ts = tls();
-  const int from = max((D <= 64 ? 600 : cs == 8 ? 300 : 150) * cs, 400);
-  const int slots = (D <= 64 ? 20 : 14) * sm_count() / 8, most = min(max(slots / H, 1), 64);
-  const bool tiles = T >= kGdTileFrom && span > from && (size_t)H * most * T * (D + 2) * sizeof(float) <= ts.work_bytes();
-  auto kern = tiles ? gqa_decode_kernel<D, true> : gqa_decode_kernel<D, false>;
-  if (const cudaError_t e = allow_smem(smem_set[tiles], (const void*)kern, smem); e != cudaSuccess) return e;
-  ts.launches++;
   cudaLaunchConfig_t lc{};
   lc.gridDim = dim3(cs, G, T);
   lc.blockDim = dim3(kGdWarps * 32);
@@ -785,10 +782,31 @@ static cudaError_t launch_gqa_decode(const bf16* q, const bf16* cache, const bf1
   at[1].val.programmaticStreamSerializationAllowed = ts.pdl ? 1 : 0;
   lc.attrs = at;
   lc.numAttrs = 2;
-  float* part = tiles ? ts.work() : nullptr;
-  const cudaError_t e = cudaLaunchKernelEx(&lc, kern, q, cache, sink, pos, req, page_off, pages, out, page_stride, page_size, T, H, G, scale, chunk, x, part, most, slots, from);
-  if (e != cudaSuccess || !tiles) return e;
-  return launch(gqa_run_merge_kernel<D>, dim3(T, (H + 7) / 8), dim3(256), 0, st, true, (const float*)part, sink, pos, req, out, most, T, H, G, cs, chunk, x, slots, from);
+  // A request with several tokens may run in tiles (gd_run) where its keys are many: below, the merge and the tiles' longer start cost more than they save.
+  // slots: at 128 entries a head two CTAs fit on an SM, but clusters of 8 not on every pair of them (304 of 296 or 288: a second round, 48 instead of 31 us).
+  // B200, us, in a graph, request by request -> in tiles (tiles of 64 rows for all requests, as before there was a choice): 16 heads of 128 in 4 groups, 24
+  // tokens behind 2000 18.7 -> 16.2 (15.7), 40 behind 2000 31.6 -> 16.1 (19.4), 60 behind 8000 59.3 -> 39.9 (42.4); in 8 groups, 24 behind 400 12.7 -> 9.9 (9.3);
+  // 16 heads of 64 in 16 groups, 24 behind 2000 / 8000 32.6 -> 14.5 (12.5), 118.7 -> 24.3 (23.4); 64 heads of 64 in 8 groups, 60 behind 8000 160 -> 84 (75).
+  const int from = max((D <= 64 ? 600 : cs == 8 ? 300 : 150) * cs, 400);
+  if (T >= kGdTileFrom && span > from) {
+    const int slots = (D <= 64 ? 20 : 14) * sm_count() / 8, most = min(max(slots / H, 1), 64);
+    if ((size_t)H * most * T * (D + 2) * sizeof(float) <= ts.work_bytes()) {
+      static std::atomic<uint64_t> smem_set{0};
+      if (const cudaError_t e = allow_smem(smem_set, (const void*)gqa_decode_kernel<D, true>, smem); e != cudaSuccess) return e;
+      float* part = ts.work();
+      ts.launches++;
+      if (const cudaError_t e = cudaLaunchKernelEx(&lc, gqa_decode_kernel<D, true>, q, cache, sink, pos, req, page_off, pages, out, page_stride, page_size, T, H, G, scale,
+                                                   chunk, GdExtra{x, part, most, slots, from});
+          e != cudaSuccess)
+        return e;
+      return launch(gqa_run_merge_kernel<D>, dim3(T, (H + 7) / 8), dim3(256), 0, st, true, (const float*)part, sink, pos, req, out, most, T, H, G, cs, chunk, x, slots,
+                    from);
+    }
+  }
+  static std::atomic<uint64_t> smem_set{0};
+  if (const cudaError_t e = allow_smem(smem_set, (const void*)gqa_decode_kernel<D, false>, smem); e != cudaSuccess) return e;
+  ts.launches++;
+  return cudaLaunchKernelEx(&lc, gqa_decode_kernel<D, false>, q, cache, sink, pos, req, page_off, pages, out, page_stride, page_size, T, H, G, scale, chunk, x);
 }
 
 template <int D>
