@@ -45,6 +45,7 @@ struct GemvArgs {
   int tp_op;                // epi 3: collective index inside the step
   int stages;
   int kc;       // K elements per row segment per stage (multiple of 256); stage = 8 segments
+  int block_rows, part_ld;  // gemv_rows_kernel: row pairs whose sums are kept at once, floats of them per token
   int y_ld;     // gated epilogues (1, 4, 5, 6): elements from one token's output row to the next
 };
 
@@ -63,6 +64,90 @@ __device__ __forceinline__ float dot8(const uint4& w, const uint4& x, float acc)
 }
 
 __device__ __forceinline__ void consumer_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+
+// Rows [r0, r0 + nrows) of this CTA are in ybuf ([NTOK][ld], fp32, written before a barrier of the calling threads).
+template <int NTOK, int THREADS>
+__device__ __forceinline__ void tp_reduce_rows(const GemvArgs& a, const float* ybuf, int ld, int r0, int nrows) {
+  const int M = a.M;
+  // ---- GEMV + all-reduce in one kernel, row tile by row tile.  Every rank runs the same grid, so CTA c owns rows
+  // [r0, r1) on every rank: push my bf16 partials of these rows to the peers as 8-byte {2 x bf16, seq} lines (the
+  // sequence number travels with the data: one posted NVLink store per line, no fence / flag / ticket), then poll
+  // the peers' lines for the SAME rows in local memory and sum in rank order (fp32, one bf16 rounding: the
+  // collective's bf16 result, bit-identical on every rank). ----
+  const int me = a.tp.rank, W = a.tp.world;
+  const uint32_t seq = (*a.tp_step) * 256u + (uint32_t)a.tp_op + 1u;  // read after griddepcontrol.wait
+  const int slot = a.tp_op & 1;
+  constexpr int NP = (NTOK + 1) / 2;  // token pairs per row
+  const int items = nrows * NP;
+  auto payload = [&](int it) -> uint32_t {
+    const int r = it % nrows, pr = it / nrows;
+    const float v0 = ybuf[(2 * pr) * ld + r];
+    const float v1 = (2 * pr + 1 < NTOK) ? ybuf[(2 * pr + 1) * ld + r] : 0.f;
+    return pack_bf16(v0, v1);
+  };
+  for (int idx = threadIdx.x; idx < items * (W - 1); idx += THREADS) {
+    const int pi = idx / items, it = idx - pi * items;
+    const int p = pi >= me ? pi + 1 : pi;
+    const int r = it % nrows, pr = it / nrows;
+    uint8_t* line = a.tp.stage[p] + (size_t)(slot * W + me) * a.tp.slot_bytes + a.tp.gll_off +
+                    ((size_t)pr * M + r0 + r) * 8;
+    st_volatile_v2(line, payload(it), seq);
+  }
+  const uint8_t* local = a.tp.stage[me] + (size_t)slot * W * a.tp.slot_bytes + a.tp.gll_off;
+  for (int it = threadIdx.x; it < items; it += THREADS) {
+    const int r = it % nrows, pr = it / nrows;
+    float s0 = 0.f, s1 = 0.f;
+    for (int q = 0; q < W; ++q) {
+      uint32_t v;
+      if (q == me) {
+        v = payload(it);
+      } else {
+        const uint8_t* line = local + (size_t)q * a.tp.slot_bytes + ((size_t)pr * M + r0 + r) * 8;
+        uint2 l;
+        tp_wait(a.tp, [&] { l = ld_volatile_v2(line); return l.y == seq; });
+        v = l.x;
+      }
+      s0 += bf16_lo(v);
+      s1 += bf16_hi(v);
+    }
+    a.Y[0][(size_t)(2 * pr) * M + r0 + r] = f2bf(s0);
+    if (2 * pr + 1 < NTOK) a.Y[0][(size_t)(2 * pr + 1) * M + r0 + r] = f2bf(s1);
+  }
+}
+template <int NTOK, int THREADS, typename Bar>
+__device__ __forceinline__ void tp_push_rows(const GemvArgs& a, const float* ybuf, int ld, int r0, int nrows, Bar all_here) {
+  const int M = a.M, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // ---- fused GEMV -> all-reduce (push half): store this CTA's partial rows straight into every rank's
+  // staging slot [seq parity][my rank] over NVLink (consumer warp w serves peer w, 32 consecutive rows per
+  // coalesced transaction), then the LAST CTA of the grid publishes the sequence flag to every rank with
+  // release.sys.  The matching reduce + residual add + RMSNorm runs in the prologue (x_mode 2) of the next
+  // GEMV on every rank: no standalone collective kernel.
+  const int me = a.tp.rank, W = a.tp.world;
+  uint32_t* my_flags = a.tp.flags[me];
+  uint32_t* ctl = my_flags + 2 * kTpMaxCtas * kTpMaxWorld;  // [0] = seq, [2] = CTA ticket of this op
+  const uint32_t seq = *reinterpret_cast<volatile uint32_t*>(ctl) + 1u;  // read after griddepcontrol.wait
+  const int slot = (int)(seq & 1u);
+  for (int p = warp; p < W; p += THREADS / 32) {
+    bf16* dst = reinterpret_cast<bf16*>(a.tp.stage[p] + (size_t)(slot * W + me) * a.tp.slot_bytes);
+#pragma unroll
+    for (int n = 0; n < NTOK; ++n)
+      for (int r = lane; r < nrows; r += 32) dst[(size_t)n * M + r0 + r] = f2bf(ybuf[n * ld + r]);
+  }
+  __threadfence_system();
+  all_here();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    const uint32_t t = atomicAdd(ctl + 2, 1u);
+    if (t == gridDim.x - 1) {
+      __threadfence_system();
+      for (int p = 0; p < W; ++p)
+        st_release_sys(a.tp.flags[p] + (size_t)(slot * kTpMaxCtas) * kTpMaxWorld + me, seq);
+      ctl[2] = 0;
+      __threadfence();
+      *reinterpret_cast<volatile uint32_t*>(ctl) = seq;
+    }
+  }
+}
 
 #ifndef PK_GEMV_MIN_CTAS
 #define PK_GEMV_MIN_CTAS 1  // occupancy hint of the streaming kernel (register cap = 64K / (288 * this))
@@ -324,87 +409,242 @@ gemv_stream_kernel(const GemvArgs a) {
       }
     }
   }
-  if (a.epi == 3) {
-    // ---- GEMV + all-reduce in one kernel, row tile by row tile.  Every rank runs the same grid, so CTA c owns rows
-    // [r0, r1) on every rank: push my bf16 partials of these rows to the peers as 8-byte {2 x bf16, seq} lines (the
-    // sequence number travels with the data: one posted NVLink store per line, no fence / flag / ticket), then poll
-    // the peers' lines for the SAME rows in local memory and sum in rank order (fp32, one bf16 rounding: the
-    // collective's bf16 result, bit-identical on every rank). ----
+  if (a.epi == 3 || a.epi == 2) {
     consumer_bar();
-    const int me = a.tp.rank, W = a.tp.world;
-    const uint32_t seq = (*a.tp_step) * 256u + (uint32_t)a.tp_op + 1u;  // read after griddepcontrol.wait
-    const int slot = a.tp_op & 1;
-    const int nrows = r1 - r0;
-    constexpr int NP = (NTOK + 1) / 2;  // token pairs per row
-    const int items = nrows * NP;
-    auto payload = [&](int it) -> uint32_t {
-      const int r = it % nrows, pr = it / nrows;
-      const float v0 = ybuf[(2 * pr) * 64 + r];
-      const float v1 = (2 * pr + 1 < NTOK) ? ybuf[(2 * pr + 1) * 64 + r] : 0.f;
-      return pack_bf16(v0, v1);
-    };
-    for (int idx = threadIdx.x; idx < items * (W - 1); idx += kConsumerThreads) {
-      const int pi = idx / items, it = idx - pi * items;
-      const int p = pi >= me ? pi + 1 : pi;
-      const int r = it % nrows, pr = it / nrows;
-      uint8_t* line = a.tp.stage[p] + (size_t)(slot * W + me) * a.tp.slot_bytes + a.tp.gll_off +
-                      ((size_t)pr * M + r0 + r) * 8;
-      st_volatile_v2(line, payload(it), seq);
+    if (a.epi == 3) tp_reduce_rows<NTOK, kConsumerThreads>(a, ybuf, 64, r0, r1 - r0);
+    else tp_push_rows<NTOK, kConsumerThreads>(a, ybuf, 64, r0, r1 - r0, [] { consumer_bar(); });
+  }
+}
+
+// ---- the same product for 2 to 4 tokens.  There the kernel above is bound by its eight consumer warps (unpacking and FMAs grow with the tokens),
+// by the rings that two CTAs' copies of the activations leave room for, and by its one producer warp, whose lanes' copies are issued one after the other,
+// about 160 clocks each.  So: one CTA of 16 warps per SM; a warp takes two weight rows at once (gate and up of a feature, or neighbours), so that a
+// token's elements are read and unpacked once for both, multiplies packed pairs (fma.rn.f32x2), and refills a ring of its own.  Work is cut by (row pair,
+// chunk of the row) into equal runs for the warps; the chunks' sums meet in shared memory and are added in order, so a row's result does not depend on
+// where it lies.  x_mode 2 (tensor parallel) stays with the kernel above.
+constexpr int kRw = 16, kRwThreads = 32 * kRw, kRwStages = 6;
+constexpr int kRwOwn = 128;    // epi 2, 3: rows of a CTA at most
+constexpr int kRwSums = 1024;  // floats of a block of row pairs' sums per token at most
+
+__device__ __forceinline__ void fma2(float2& acc, const float2& w, const float2& x) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(reinterpret_cast<uint64_t&>(acc)) : "l"(reinterpret_cast<const uint64_t&>(w)), "l"(reinterpret_cast<const uint64_t&>(x)));
+}
+__device__ __forceinline__ float2 unpack2(uint32_t u) { return make_float2(bf16_lo(u), bf16_hi(u)); }
+
+// sums over the lanes of 2 N values v[row][token] (N <= 4), each left in lanes of its own: returns the sum of value (lane >> 2), in the order v[0][0..],
+// v[1][0..] padded to four tokens; the exchange halves the values with every step
+template <int N>
+__device__ __forceinline__ float sums_by_lane(const float (&v)[2][N], int lane) {
+  float a[4];
+#pragma unroll
+  for (int n = 0; n < 4; ++n) {
+    const float lo = n < N ? v[0][n < N ? n : 0] : 0.f, hi = n < N ? v[1][n < N ? n : 0] : 0.f;
+    a[n] = n < N ? (lane & 16 ? hi : lo) + __shfl_xor_sync(0xffffffffu, lane & 16 ? lo : hi, 16) : 0.f;
+  }
+  float b[2];
+#pragma unroll
+  for (int n = 0; n < 2; ++n) b[n] = (lane & 8 ? a[n + 2] : a[n]) + __shfl_xor_sync(0xffffffffu, lane & 8 ? a[n] : a[n + 2], 8);
+  float c = (lane & 4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, lane & 4 ? b[0] : b[1], 4);
+  c += __shfl_xor_sync(0xffffffffu, c, 2);
+  return c + __shfl_xor_sync(0xffffffffu, c, 1);
+}
+
+template <int NTOK>
+__global__ void __launch_bounds__(kRwThreads, 1) gemv_rows_kernel(const GemvArgs a) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  const int stages = a.stages, kc = a.kc, seg = kc * 2;  // bytes of a row's chunk
+  bf16* xs = reinterpret_cast<bf16*>(smem + (size_t)kRw * stages * 2 * seg);  // [NTOK][K]
+  uint64_t* full = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(xs) + (size_t)NTOK * a.K * 2);
+  float* red = reinterpret_cast<float*>(full + kRw * kRwStages);  // [2][8]
+  float* ybuf = red + 16;                                         // epi 2, 3: [NTOK][kRwOwn]
+  float* part = ybuf + NTOK * kRwOwn;                             // [NTOK][part_ld]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, M = a.M, K = a.K;
+  const bool glu = a.epi == 1 || a.epi >= 4;
+  // output rows of this CTA; plain: in pairs
+  const int units_all = glu ? M : (M + 1) / 2;
+  const int p0 = (int)((int64_t)blockIdx.x * units_all / gridDim.x), pairs_all = (int)((int64_t)(blockIdx.x + 1) * units_all / gridDim.x) - p0;
+  const int chunks = (K + kc - 1) / kc;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kRw * kRwStages; ++s) mbar_init(full + s, 1);
+    mbar_fence_init();
+  }
+  __syncthreads();
+  pdl_launch_dependents();
+  uint8_t* ring = smem + (size_t)warp * stages * 2 * seg;
+  full += warp * kRwStages;
+  const uint64_t pol = l2_evict_first_policy();
+  struct Cursor {  // the warp's place: first pair of the block, (pair, chunk) units left there, pair of the block, chunk
+    int blk, left, pair, chunk;
+  };
+  auto enter = [&](Cursor& c, int blk) {
+    const int n = min(a.block_rows, pairs_all - blk) * chunks, first = n * warp / kRw;
+    c.blk = blk;
+    c.left = n * (warp + 1) / kRw - first;
+    c.pair = first / chunks;
+    c.chunk = first % chunks;
+  };
+  auto step = [&](Cursor& c) {
+    --c.left;
+    if (++c.chunk == chunks) {
+      c.chunk = 0;
+      ++c.pair;
     }
-    const uint8_t* local = a.tp.stage[me] + (size_t)slot * W * a.tp.slot_bytes + a.tp.gll_off;
-    for (int it = threadIdx.x; it < items; it += kConsumerThreads) {
-      const int r = it % nrows, pr = it / nrows;
-      float s0 = 0.f, s1 = 0.f;
-      for (int q = 0; q < W; ++q) {
-        uint32_t v;
-        if (q == me) {
-          v = payload(it);
-        } else {
-          const uint8_t* line = local + (size_t)q * a.tp.slot_bytes + ((size_t)pr * M + r0 + r) * 8;
-          uint2 l;
-          tp_wait(a.tp, [&] { l = ld_volatile_v2(line); return l.y == seq; });
-          v = l.x;
+  };
+  Cursor ahead;
+  enter(ahead, 0);
+  auto refill = [&](int slot) {
+    while (ahead.left == 0) {
+      if (ahead.blk + a.block_rows >= pairs_all) return;
+      enter(ahead, ahead.blk + a.block_rows);
+    }
+    const int p = p0 + ahead.blk + ahead.pair, row0 = glu ? p : 2 * p, row1 = glu ? M + p : 2 * p + 1, k0 = ahead.chunk * kc;
+    const bool two = glu || row1 < M;  // (an odd last row)
+    const uint32_t bytes = (uint32_t)(min(kc, K - k0) * 2);
+    if (lane == 0) {
+      mbar_expect_tx(full + slot, two ? 2 * bytes : bytes);
+      bulk_g2s(ring + (size_t)slot * 2 * seg, a.W + (size_t)row0 * K + k0, bytes, full + slot, pol);
+      if (two) bulk_g2s(ring + (size_t)slot * 2 * seg + seg, a.W + (size_t)row1 * K + k0, bytes, full + slot, pol);
+    }
+    step(ahead);
+  };
+  for (int s = 0; s < stages; ++s) refill(s);
+
+  pdl_wait();  // activations come from the previous kernel
+  if (a.x_mode == 0) {
+    for (int i = threadIdx.x; i < NTOK * K / 8; i += kRwThreads) reinterpret_cast<uint4*>(xs)[i] = reinterpret_cast<const uint4*>(a.X)[i];
+  } else {
+    // x = bf16((h + r) * rsqrt(mean((h + r)^2) + eps) * w), as in the kernel above; two tokens at a time, 256 threads each
+    constexpr int kMaxVec = 5;  // K <= 10240
+    const int half = threadIdx.x >> 8, t = threadIdx.x & 255, nv = K >> 3;
+    for (int n0 = 0; n0 < NTOK; n0 += 2) {
+      const int n = n0 + half;
+      const bool on = n < NTOK;
+      float v[kMaxVec][8], ss = 0.f;
+#pragma unroll
+      for (int j = 0; j < kMaxVec; ++j) {
+        const int i = t + j * 256;
+        if (!on || i >= nv) continue;
+        const uint4 h = reinterpret_cast<const uint4*>(a.X + (size_t)n * K)[i], r = reinterpret_cast<const uint4*>(a.residual + (size_t)n * K)[i];
+        const uint32_t hw[4] = {h.x, h.y, h.z, h.w}, rw[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          v[j][2 * e] = bf16_lo(hw[e]) + bf16_lo(rw[e]);
+          v[j][2 * e + 1] = bf16_hi(hw[e]) + bf16_hi(rw[e]);
         }
-        s0 += bf16_lo(v);
-        s1 += bf16_hi(v);
+        if (a.x_mode == 3) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[j][e] = round_bf16(v[j][e]);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss = fmaf(v[j][e], v[j][e], ss);
       }
-      a.Y[0][(size_t)(2 * pr) * M + r0 + r] = f2bf(s0);
-      if (2 * pr + 1 < NTOK) a.Y[0][(size_t)(2 * pr + 1) * M + r0 + r] = f2bf(s1);
+      ss = warp_sum(ss);
+      __syncthreads();  // (the last pair of tokens' sums have been read)
+      if (lane == 0) red[warp] = ss;
+      __syncthreads();
+      float tot = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) tot += red[half * 8 + w];
+      const float rinv = rsqrtf(tot / (float)K + a.eps), wo = a.x_mode == 3 ? 1.0f : 0.0f;
+#pragma unroll
+      for (int j = 0; j < kMaxVec; ++j) {
+        const int i = t + j * 256;
+        if (!on || i >= nv) continue;
+        const uint4 g = reinterpret_cast<const uint4*>(a.norm_w)[i];
+        const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
+        uint32_t o[4], hs[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          o[e] = pack_bf16(v[j][2 * e] * rinv * (wo + bf16_lo(gw[e])), v[j][2 * e + 1] * rinv * (wo + bf16_hi(gw[e])));
+          hs[e] = pack_bf16(v[j][2 * e], v[j][2 * e + 1]);
+        }
+        reinterpret_cast<uint4*>(xs + (size_t)n * K)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+        if (blockIdx.x == 0) {
+          reinterpret_cast<uint4*>(a.hidden_out + (size_t)n * K)[i] = make_uint4(hs[0], hs[1], hs[2], hs[3]);
+          if (a.normed_out) reinterpret_cast<uint4*>(a.normed_out + (size_t)n * K)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+      }
     }
   }
-  if (a.epi == 2) {
-    // ---- fused GEMV -> all-reduce (push half): store this CTA's partial rows straight into every rank's
-    // staging slot [seq parity][my rank] over NVLink (consumer warp w serves peer w, 32 consecutive rows per
-    // coalesced transaction), then the LAST CTA of the grid publishes the sequence flag to every rank with
-    // release.sys.  The matching reduce + residual add + RMSNorm runs in the prologue (x_mode 2) of the next
-    // GEMV on every rank: no standalone collective kernel.
-    consumer_bar();
-    const int me = a.tp.rank, W = a.tp.world;
-    uint32_t* my_flags = a.tp.flags[me];
-    uint32_t* ctl = my_flags + 2 * kTpMaxCtas * kTpMaxWorld;  // [0] = seq, [2] = CTA ticket of this op
-    const uint32_t seq = *reinterpret_cast<volatile uint32_t*>(ctl) + 1u;  // read after griddepcontrol.wait
-    const int slot = (int)(seq & 1u);
-    const int nrows = r1 - r0;
-    for (int p = warp; p < W; p += kCW) {
-      bf16* dst = reinterpret_cast<bf16*>(a.tp.stage[p] + (size_t)(slot * W + me) * a.tp.slot_bytes);
+  __syncthreads();
+
+  int s = 0;
+  uint32_t ph = 0;
+  for (int blk = 0; blk < pairs_all; blk += a.block_rows) {
+    Cursor c;
+    for (enter(c, blk); c.left > 0; step(c)) {
+      const int k0 = c.chunk * kc, nvec = min(kc, K - k0) >> 3;
+      const uint4* w0 = reinterpret_cast<const uint4*>(ring + (size_t)s * 2 * seg);
+      const uint4* w1 = reinterpret_cast<const uint4*>(ring + (size_t)s * 2 * seg + seg);
+      const uint4* xp = reinterpret_cast<const uint4*>(xs + k0);
+      float2 acc[2][NTOK][2];
 #pragma unroll
-      for (int n = 0; n < NTOK; ++n)
-        for (int r = lane; r < nrows; r += 32) dst[(size_t)n * M + r0 + r] = f2bf(ybuf[n * 64 + r]);
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int n = 0; n < NTOK; ++n) acc[r][n][0] = acc[r][n][1] = make_float2(0.f, 0.f);
+      mbar_wait(full + s, ph);
+#pragma unroll 2
+      for (int i = lane; i < nvec; i += 32) {
+        const uint4 u0 = w0[i], u1 = w1[i];
+        const float2 a0[4] = {unpack2(u0.x), unpack2(u0.y), unpack2(u0.z), unpack2(u0.w)};
+        const float2 a1[4] = {unpack2(u1.x), unpack2(u1.y), unpack2(u1.z), unpack2(u1.w)};
+#pragma unroll
+        for (int n = 0; n < NTOK; ++n) {
+          const uint4 xv = xp[(size_t)n * (K >> 3) + i];
+          const float2 x[4] = {unpack2(xv.x), unpack2(xv.y), unpack2(xv.z), unpack2(xv.w)};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            fma2(acc[0][n][e & 1], a0[e], x[e]);
+            fma2(acc[1][n][e & 1], a1[e], x[e]);
+          }
+        }
+      }
+      __syncwarp();
+      refill(s);
+      if (++s == stages) {
+        s = 0;
+        ph ^= 1u;
+      }
+      float v[2][NTOK];
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int n = 0; n < NTOK; ++n) v[r][n] = (acc[r][n][0].x + acc[r][n][0].y) + (acc[r][n][1].x + acc[r][n][1].y);
+      const float sum = sums_by_lane<NTOK>(v, lane);
+      const int n = (lane >> 2) & 3;
+      if ((lane & 3) == 0 && n < NTOK) part[n * a.part_ld + (2 * c.pair + (lane >> 4)) * chunks + c.chunk] = sum;
     }
-    __threadfence_system();
-    consumer_bar();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      const uint32_t t = atomicAdd(ctl + 2, 1u);
-      if (t == gridDim.x - 1) {
-        __threadfence_system();
-        for (int p = 0; p < W; ++p)
-          st_release_sys(a.tp.flags[p] + (size_t)(slot * kTpMaxCtas) * kTpMaxWorld + me, seq);
-        ctl[2] = 0;
-        __threadfence();
-        *reinterpret_cast<volatile uint32_t*>(ctl) = seq;
+    __syncthreads();
+    auto total = [&](int n, int row) {  // a row's chunks in order
+      const float* p = part + n * a.part_ld + row * chunks;
+      float t = p[0];
+      for (int i = 1; i < chunks; ++i) t += p[i];
+      return t;
+    };
+    const int pairs = min(a.block_rows, pairs_all - blk), outs = glu ? pairs : 2 * pairs;
+    for (int i = threadIdx.x; i < outs * NTOK; i += kRwThreads) {
+      const int n = i / outs, o = i % outs, out_row = (glu ? p0 + blk : 2 * (p0 + blk)) + o;
+      if (out_row >= M) continue;
+      if (a.epi == 2 || a.epi == 3) {
+        ybuf[n * kRwOwn + 2 * blk + o] = total(n, o);
+      } else if (!glu) {
+        const int sg = out_row < a.seg_end[0] ? 0 : (out_row < a.seg_end[1] ? 1 : 2);
+        const int lo = sg == 0 ? 0 : a.seg_end[sg - 1];
+        a.Y[sg][(size_t)n * (a.seg_end[sg] - lo) + (out_row - lo)] = f2bf(total(n, o));
+      } else {
+        const float gt = round_bf16(total(n, 2 * o)), up = round_bf16(total(n, 2 * o + 1));  // gate_up_out is bf16 in the reference
+        float sl = a.epi == 5 ? fmaxf(gt, 0.f) : a.epi == 6 ? gelu_tanh_gate(gt) : gt / (1.0f + expf(-gt));
+        if (a.epi == 4) sl = round_bf16(sl);
+        a.Y[0][(size_t)n * a.y_ld + out_row] = f2bf(sl * up);
       }
     }
+    if (blk + a.block_rows < pairs_all) __syncthreads();  // the sums have been read
+  }
+  if (a.epi == 3 || a.epi == 2) {
+    __syncthreads();
+    const int r0 = 2 * p0, nrows = min(2 * pairs_all, M - r0);
+    if (a.epi == 3) tp_reduce_rows<NTOK, kRwThreads>(a, ybuf, kRwOwn, r0, nrows);
+    else tp_push_rows<NTOK, kRwThreads>(a, ybuf, kRwOwn, r0, nrows, [] { __syncthreads(); });
   }
 }
 
@@ -490,12 +730,41 @@ static cudaError_t launch_gemv_t(GemvArgs a, cudaStream_t stream) {
   return launch(kern, dim3(grid), dim3(kConsumerThreads + 32), smem, stream, true, a);
 }
 
+template <int NTOK>
+static cudaError_t launch_gemv_rows(GemvArgs a, cudaStream_t stream) {
+  constexpr size_t most = 224 * 1024;
+  const size_t x_bytes = (size_t)NTOK * a.K * 2, fixed = kRw * kRwStages * sizeof(uint64_t) + (16 + NTOK * kRwOwn) * sizeof(float);
+  const bool glu = a.epi == 1 || a.epi >= 4;
+  const int units = glu ? a.M : (a.M + 1) / 2, grid = units < sm_count() ? units : sm_count(), mine = (units + grid - 1) / grid;
+  size_t sums = 0;
+  auto plan = [&](int kc) {  // stages that fit
+    const int chunks = (a.K + kc - 1) / kc, fit = kRwSums / (2 * chunks);
+    a.kc = kc;
+    a.block_rows = mine < fit ? mine : fit > 0 ? fit : 1;
+    a.part_ld = a.block_rows * 2 * chunks;
+    sums = (size_t)NTOK * a.part_ld * sizeof(float);
+    const size_t used = x_bytes + fixed + sums;
+    const size_t n = used < most ? (most - used) / ((size_t)kRw * 4 * kc) : 0;
+    return (int)(n > kRwStages ? kRwStages : n);
+  };
+  // long chunks (fewer waits and sums) while three of them are under way
+  a.stages = plan(a.K >= 1024 ? 1024 : 512);
+  if (a.stages < 3) a.stages = plan(512);
+  if (a.stages < 2) a.stages = plan(256);
+  if (a.stages < 1 || ((a.epi == 2 || a.epi == 3) && 2 * mine > kRwOwn)) return cudaErrorInvalidValue;
+  const size_t smem = (size_t)kRw * a.stages * 4 * a.kc + x_bytes + fixed + sums;
+  static std::atomic<uint64_t> smem_set{0};
+  if (const cudaError_t e = allow_smem(smem_set, (const void*)gemv_rows_kernel<NTOK>, most); e != cudaSuccess) return e;
+  return launch(gemv_rows_kernel<NTOK>, dim3(grid), dim3(kRwThreads), smem, stream, true, a);
+}
+
 cudaError_t launch_gemv(const GemvArgs& a, int N, cudaStream_t stream) {
+  const bool rows = a.x_mode != 2;
   switch (N) {
     case 1: return launch_gemv_t<1>(a, stream);
-    case 2: return launch_gemv_t<2>(a, stream);
-    case 3: return launch_gemv_t<3>(a, stream);
-    case 4: return launch_gemv_t<4>(a, stream);
+    case 2: return rows ? launch_gemv_rows<2>(a, stream) : launch_gemv_t<2>(a, stream);
+    case 3: return rows ? launch_gemv_rows<3>(a, stream) : launch_gemv_t<3>(a, stream);
+    case 4: return rows ? launch_gemv_rows<4>(a, stream) : launch_gemv_t<4>(a, stream);
     default: return cudaErrorInvalidValue;
   }
 }
