@@ -43,9 +43,9 @@ def _run(cmd: list[str]) -> None:
 # What one design needs when nothing is built yet (a fresh checkout asked to serve that design compiles these files and no
 # others): kernel sources, host sources.  A later full build adds the rest and links both libraries again.
 PARTS_OF = {
-    "Vamadra": (("runtime.cu", "gemm.cu", "gemm2.cu", "gemm_skinny.cu", "gemv.cu", "sampling.cu", "residual32_ops.cu", "gemm_batched_mma.cu", "latent_attention.cu", "latent_attention_mma.cu", "latent_attention_tc.cu", "moe.cu", "moe_grouped.cu"),
+    "Vamadra": (("runtime.cu", "gemm.cu", "gemm2.cu", "gemm_skinny.cu", "gemv.cu", "sampling.cu", "residual32_ops.cu", "gemm_batched_mma.cu", "latent_attention.cu", "latent_attention_mma.cu", "latent_attention_tc.cu", "moe.cu", "moe_few.cu", "moe_grouped.cu"),
                 ("qwen3_host.cpp", "layered_host.cpp")),
-    "Risolorn": (("runtime.cu", "gemm.cu", "gemm2.cu", "gemm_skinny.cu", "gemv.cu", "sampling.cu", "residual32_ops.cu", "gemm_batched_mma.cu", "gqa_attention.cu", "recurrent_mixers.cu", "moe.cu", "moe_grouped.cu"),
+    "Risolorn": (("runtime.cu", "gemm.cu", "gemm2.cu", "gemm_skinny.cu", "gemv.cu", "sampling.cu", "residual32_ops.cu", "gemm_batched_mma.cu", "gqa_attention.cu", "recurrent_mixers.cu", "moe.cu", "moe_few.cu", "moe_grouped.cu"),
                  ("qwen3_host.cpp", "layered_host.cpp")),
     "Nagosun": (("runtime.cu", "gemm.cu", "gemm2.cu", "gemm_skinny.cu", "gemv.cu", "sampling.cu", "residual32_ops.cu", "gemm_batched_mma.cu", "gqa_attention.cu", "latent_attention.cu", "latent_attention_mma.cu", "latent_attention_tc.cu"),
                 ("qwen3_host.cpp", "layered_host.cpp")),

@@ -17,6 +17,12 @@
 
 namespace pk {
 
+// bf16, up to 192 pairs (moe_few.cu); -2: not for those kernels
+int launch_moe_up_few(const bf16* x, const bf16* w, const int* ids, bf16* hid, int tokens, int top, int width, int ff, int act, float p0, float p1,
+                      cudaStream_t st);
+int launch_moe_down_few(const bf16* hid, const bf16* w, const int* ids, const float* wts, const bf16* shared, const float* sg, float* y, int tokens, int top,
+                        int width, int ff, cudaStream_t st);
+
 // (value, index) arg-max over a warp, lowest index on ties
 __device__ __forceinline__ void warp_argmax(float& v, int& i) {
 #pragma unroll
@@ -217,6 +223,10 @@ extern "C" int pk_moe_up_act(const void* xa, const void* w_up, const int* ids, v
 extern "C" int pk_moe_up_act_p(const void* xa, const void* w_up, const int* ids, void* hid, int tokens, int top, int width, int ff, int act, float p0,
                                float p1, int f32, pk_stream st) {
   if (!xa || !w_up || !ids || !hid || tokens <= 0 || top <= 0 || width <= 0 || ff <= 0 || act < 0 || act > 2 || (act == 2 && !(p0 > 0.f))) return -1;
+  if (!f32) {
+    const int rc = launch_moe_up_few((const bf16*)xa, (const bf16*)w_up, ids, (bf16*)hid, tokens, top, width, ff, act, p0, p1, st);
+    if (rc != -2) return rc;
+  }
   const size_t smem = (size_t)width * sizeof(float);
   const dim3 grid(tokens, top, (ff + kMoeRowsPerBlock - 1) / kMoeRowsPerBlock);
 #define PK_UP(E, G) launch(moe_up_kernel<E, G>, grid, dim3(256), smem, st, true, (const E*)xa, (const E*)w_up, ids, (E*)hid, width, ff, p0, p1)
@@ -251,6 +261,10 @@ extern "C" int pk_moe_down_combine(const void* hid, const void* w_down, const in
   if (!hid || !w_down || !ids || !weights || !y || tokens <= 0 || top <= 0 || width <= 0 || ff <= 0) return -1;
   const size_t smem = (size_t)top * ((ff + 3) & ~3) * sizeof(float);
   if (smem > 200 * 1024) return -2;
+  if (!f32) {
+    const int rc = launch_moe_down_few((const bf16*)hid, (const bf16*)w_down, ids, weights, (const bf16*)shared, shared_gate, y, tokens, top, width, ff, st);
+    if (rc != -2) return rc;
+  }
   if (f32) {
     if (smem > 48 * 1024) cudaFuncSetAttribute(moe_down_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     launch(moe_down_kernel<float>, dim3(tokens, (width + kMoeDownRowsPerBlock - 1) / kMoeDownRowsPerBlock), dim3(256), smem, st, true, (const float*)hid, (const float*)w_down, ids, weights,
