@@ -239,7 +239,8 @@ struct SkPlan {
 // is the same, bit for bit, only if both take the same kernel (pk_b200_gemm_segments promises it from 129 tokens on).  The number of features must not
 // decide, then, wherever it could differ between the two: only reductions of 8192 or more (they come from a feed-forward's inner width; projections are
 // stacked over the hidden width) and fewer than 64 features (gates of a head each, no head's row is so short) come here.  What that gives up at 160
-// tokens: 2560 x 4096 13.7 -> 16.4, 1024 x 4096 11.7 -> 15.4.  Parts follow from K (4 from 4096 on, where they fit, else 2; 32 x 2560: 10.4 us, 14.5 in gemm2.cu).
+// tokens: 2560 x 4096 13.7 -> 16.4, 1024 x 4096 11.7 -> 15.4.  Parts follow from K (4 from 4096 on, where they fit, else 2), and
+// below 64 features, which no stacking has to agree with, they are as many as fit: 32 x 2560 of 300 / 1024 / 2048 tokens 9.0 9.1 9.2 us with two, 6.1 6.3 7.0.
 // Measured on B200, us a launch in a train over cold weights (before: the split-K form of gemm.cu; from 129 tokens on gemm2.cu), M x K:
 //   tokens            8            48           128          160
 //   6144 x 2560   20.1 -> 9.5  19.9 -> 10.4  24.9 -> 12.6     (gemm2)
@@ -253,7 +254,7 @@ struct SkPlan {
 // gemm.cu are as fast (24.3 us both at 19456 x 2560), and from 129 on gemm2.cu is faster.
 SkPlan sk_plan(int M, int N, int K, int nt, int sms) {
   const int n_tiles = (N + nt - 1) / nt, kb = (K + SK_BK - 1) / SK_BK;
-  for (int S = N <= 128 ? SK_MAX_SPLIT : K >= 4096 ? 4 : 2; S >= 1; S /= 2) {
+  for (int S = N <= 128 || M < 64 ? SK_MAX_SPLIT : K >= 4096 ? 4 : 2; S >= 1; S /= 2) {
     if (S > 1 && S > kb / 4) continue;  // at least 4 K blocks per part
     const int fit = sk_resident(S, sms) / n_tiles;  // feature tiles
     if ((long)fit * SK_BM < M) continue;
