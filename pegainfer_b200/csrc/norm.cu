@@ -3,8 +3,8 @@
 //   rms_norm        : out = bf16(x * rsqrt(mean(x^2)+eps) * w), fp32 throughout, ONE rounding
 //   fused_add_norm  : x = f32(hidden)+f32(residual); hidden = bf16(x);
 //                     out = bf16(x * rsqrt(mean(x^2)+eps) * w) on the UNROUNDED x
-// Unlike the reference there is no residual->out staging memcpy.  One CTA per token; the row is
-// read from HBM once (16-B vectors) and parked in shared memory as fp32 between the two passes.
+// Unlike the reference there is no residual->out staging memcpy.  Rows of up to 4096 elements on 16-byte boundaries go to norm_rows.cuh; here one CTA per
+// token, the row read from HBM once (16-B vectors) and parked in shared memory as fp32 between the two passes.
 #include "common.cuh"
 #include "norm_rows.cuh"
 
@@ -79,7 +79,7 @@ static void launch_norm(const pk_bf16* x, pk_bf16* hidden, const pk_bf16* residu
                         pk_stream stream) {
   if (dim <= 0 || rows <= 0) return;
   const bool vec = dim % 8 == 0 && al16(x) && al16(hidden) && al16(residual) && al16(w) && al16(out);
-  if (vec && rms_rows_fit(dim, rows)) {
+  if (vec && rms_rows_fit(dim)) {
     launch_rms_rows<kFusedAdd ? 1 : 0>((const bf16*)x, (bf16*)hidden, (const bf16*)residual, (const bf16*)w, (bf16*)out, dim, rows, eps, stream);
     return;
   }
