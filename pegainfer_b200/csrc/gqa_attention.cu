@@ -309,6 +309,12 @@ __global__ void __launch_bounds__(kGqaWarps * 32) gqa_attention_kernel(const E* 
 // next block's copy overlaps this block's products); S = Q K^T and O += P V with mma.sync m16n8k16, P rounded to bf16 for the
 // second product, statistics in fp32.
 constexpr int kAmRows = 64, kAmKeys = 64;
+// two floats at this address of CTA `rank` of the cluster
+__device__ __forceinline__ void gqa_ld_state(uint32_t addr, uint32_t rank, float& a, float& b) {
+  uint32_t at;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(at) : "memory");
+}
 constexpr int kGdTileFrom = 8;  // tokens of a request, at least, that run in tiles in a step of few rows
 
 template <int DQ, int DV>
@@ -330,11 +336,45 @@ __global__ void __launch_bounds__(128, 3) gqa_attention_mma_kernel(const bf16* _
   // end of the step backwards, so that the CTAs that start last are the ones with the fewest visible keys
   const int t0 = (gridDim.y - 1 - blockIdx.y) * kAmRows, h = blockIdx.x, g = h / (H / G);
 #define GQA_T_END T
+#define GQA_CLUSTER 0
 #define GQA_SPLIT blockIdx.z
 #define GQA_SPLITS gridDim.z
 #define GQA_PART_LD nsplit
 #include "gqa_tile.cuh"
 #undef GQA_T_END
+#undef GQA_CLUSTER
+#undef GQA_SPLIT
+#undef GQA_SPLITS
+#undef GQA_PART_LD
+}
+
+// The same for steps whose (tile, head) pairs leave SMs idle: the keys are dealt out to the CTAs of a cluster (the grid's z axis), which combine their states
+// over distributed shared memory.  B200, us, with the append (heads / groups x size): 229 tokens of 6 requests behind 480 (8 / 2 x 128) 91.6 -> 48.6,
+// 100 behind 500 (8 / 4 x 64) 26.9 -> 21.7, 1500 behind 400 (8 / 4 x 64) 80.6 -> 60.7.
+template <int DQ, int DV>
+__global__ void __launch_bounds__(128, 3) gqa_attention_cluster_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache, const bf16* __restrict__ sink,
+                                                               const int* __restrict__ pos, const int* __restrict__ req,
+                                                               const int* __restrict__ page_off, const int* __restrict__ pages,
+                                                               bf16* __restrict__ out,
+                                                               long page_stride, int page_size, int T, int H, int G, float scale, int chunk,
+                                                               AttnExtra x) {
+  constexpr int LDK = DQ + 8, LDV = DV + 8;
+  extern __shared__ __align__(16) unsigned char am_smem[];  // two stages of [keys][LDK] K and [keys][LDV] V
+  bf16* const Ks0 = reinterpret_cast<bf16*>(am_smem);
+  bf16* const Vs0 = Ks0 + 2 * kAmKeys * LDK;
+  __shared__ int s_req[kAmRows], s_pos[kAmRows];
+  __shared__ long long s_slot[2][kAmKeys];  // per stage: element offset of every key row's cache slot (-1: not to be read)
+  pdl_wait();
+  pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
+  const int t0 = (gridDim.y - 1 - blockIdx.y) * kAmRows, h = blockIdx.x, g = h / (H / G);
+#define GQA_T_END T
+#define GQA_CLUSTER 1
+#define GQA_SPLIT blockIdx.z
+#define GQA_SPLITS gridDim.z
+#define GQA_PART_LD nsplit
+#include "gqa_tile.cuh"
+#undef GQA_T_END
+#undef GQA_CLUSTER
 #undef GQA_SPLIT
 #undef GQA_SPLITS
 #undef GQA_PART_LD
@@ -382,11 +422,13 @@ __device__ __forceinline__ void gqa_tile_of_run(unsigned char* am_smem, const bf
   __shared__ long long s_slot[2][kAmKeys];  // per stage: element offset of every key row's cache slot (-1: not to be read)
   const int t0 = run.start, g = h / (H / G);
 #define GQA_T_END run.start + run.len
+#define GQA_CLUSTER 0
 #define GQA_SPLIT share
 #define GQA_SPLITS run.shares
 #define GQA_PART_LD most
 #include "gqa_tile.cuh"
 #undef GQA_T_END
+#undef GQA_CLUSTER
 #undef GQA_SPLIT
 #undef GQA_SPLITS
 #undef GQA_PART_LD
@@ -841,6 +883,33 @@ static void launch_gqa_mma(const bf16* q, const bf16* cache, const bf16* sink, c
   }
   float* po = ts.work();
   float* pml = po ? po + (size_t)H * splits * T * D : nullptr;
+  // From 64 rows on: as many CTAs of a cluster (8 at most) to a (tile, head) as the GPU holds at once, while each has a few blocks of keys to walk (a context
+  // no longer than the step is a prompt from its start, whose rows see half of it); the exchange takes about 5 us.
+  int cs = 1;
+  if (T >= kAmRows)
+    while (cs < 8 && (long)H * tiles * cs * 2 <= 3 * sm_count() && (span <= 0 || (span > T ? span : span / 2) >= 4 * cs * kAmKeys)) cs *= 2;
+  if (cs > 1) {
+    static std::atomic<uint64_t> smem_set{0};  // per template instance
+    if (allow_smem(smem_set, (const void*)gqa_attention_cluster_kernel<D, D>, smem) == cudaSuccess) {
+      cudaLaunchConfig_t lc{};
+      lc.gridDim = dim3(H, tiles, cs);
+      lc.blockDim = dim3(128);
+      lc.dynamicSmemBytes = smem;
+      lc.stream = st;
+      cudaLaunchAttribute attr[2];
+      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[0].val.programmaticStreamSerializationAllowed = ts.pdl ? 1 : 0;
+      attr[1].id = cudaLaunchAttributeClusterDimension;
+      attr[1].val.clusterDim.x = attr[1].val.clusterDim.y = 1;
+      attr[1].val.clusterDim.z = cs;
+      lc.attrs = attr;
+      lc.numAttrs = 2;
+      ts.launches++;
+      cudaLaunchKernelEx(&lc, gqa_attention_cluster_kernel<D, D>, q, cache, sink, pos, req, page_off, pages, out, page_stride, page_size, T, H, G, scale, chunk, x);
+      return;
+    }
+    cudaGetLastError();
+  }
   launch(gqa_attention_mma_kernel<D, D>, dim3(H, tiles, splits), dim3(128), smem, st, true, q, cache, sink, pos, req, page_off, pages, out, po, pml,
          page_stride, page_size, T, H, G, scale, chunk, x);
   if (splits > 1)

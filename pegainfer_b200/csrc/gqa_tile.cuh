@@ -166,6 +166,56 @@
     }
     r_first = r_last + 1;
   }
+#if GQA_CLUSTER
+  {
+    // this share's state of its 64 rows over the key blocks, then each CTA finishes every nsplit-th part of the rows, a warp per row
+    constexpr int LDO = DV + 2;  // [DV] unnormalised output, maximum, sum
+    float* st = reinterpret_cast<float*>(Ks0);
+    __syncthreads();  // the last block has been read
+#pragma unroll
+    for (int ni = 0; ni < DV / 8; ++ni) {
+      const int c = ni * 8 + 2 * tq;
+      *reinterpret_cast<float2*>(st + ra * LDO + c) = make_float2(oa[ni][0], oa[ni][1]);
+      *reinterpret_cast<float2*>(st + rb * LDO + c) = make_float2(oa[ni][2], oa[ni][3]);
+    }
+    if (tq == 0) {
+      *reinterpret_cast<float2*>(st + ra * LDO + DV) = make_float2(m_a, l_a);
+      *reinterpret_cast<float2*>(st + rb * LDO + DV) = make_float2(m_b, l_b);
+    }
+    cluster_barrier();
+    const float sk = sink ? bf2f(sink[h]) * kLog2e : -INFINITY;
+    const uint32_t base = smem_u32(st);
+    const int rows = kAmRows / nsplit;
+    for (int r = split * rows + warp; r < (split + 1) * rows; r += 4) {
+      if (s_req[r] < 0) continue;
+      const int t = t0 + r;
+      float m = -INFINITY, l = 0.f;
+      if (lane < nsplit) gqa_ld_state(base + (uint32_t)(r * LDO + DV) * 4, lane, m, l);
+      const float top = fmaxf(warp_max(m), sk), e = m == -INFINITY ? 0.f : exp2f(m - top);
+      const float wgt = e / (warp_sum(l * e) + (sink ? exp2f(sk - top) : 0.f));
+      float w[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) w[i] = __shfl_sync(0xffffffffu, wgt, i);  // (lanes of no share: zero)
+      for (int d = 2 * lane; d < DV; d += 64) {
+        float o0 = 0.f, o1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (i >= nsplit) break;
+          float x0, x1;
+          gqa_ld_state(base + (uint32_t)(r * LDO + d) * 4, i, x0, x1);
+          o0 = fmaf(x0, w[i], o0);
+          o1 = fmaf(x1, w[i], o1);
+        }
+        if (x.gate) {
+          o0 *= out_gate<bf16>(x, t, h, d, DV);
+          o1 *= out_gate<bf16>(x, t, h, d + 1, DV);
+        }
+        *reinterpret_cast<uint32_t*>(out + (size_t)t * x.out_ld + h * DV + d) = pack_bf16(o0, o1);
+      }
+    }
+    cluster_barrier();  // the other CTAs have read this one's shared memory
+  }
+#else
   if (nsplit > 1) {  // partial state (running maximum, sum, unnormalised output) of this split; gqa_attention_merge_kernel finishes the rows
     const size_t sa = ((size_t)(h * GQA_PART_LD + split) * T + (t0 + ra)), sb = ((size_t)(h * GQA_PART_LD + split) * T + (t0 + rb));
     if (req_a >= 0 && tq == 0) part_ml[sa * 2] = m_a * kLn2, part_ml[sa * 2 + 1] = l_a;  // maxima leave in natural units
@@ -200,3 +250,4 @@
     if (req_a >= 0) *reinterpret_cast<uint32_t*>(out + (size_t)(t0 + ra) * x.out_ld + h * DV + c) = pack_bf16(oa[ni][0] * i_a * g0, oa[ni][1] * i_a * g1);
     if (req_b >= 0) *reinterpret_cast<uint32_t*>(out + (size_t)(t0 + rb) * x.out_ld + h * DV + c) = pack_bf16(oa[ni][2] * i_b * g2, oa[ni][3] * i_b * g3);
   }
+#endif
