@@ -11,15 +11,20 @@
 //               rounding alone made the result's error 1.2 times as large for peaked scores
 //   warp 8      MMA issuer     S = Q K^T,  O += P V (A from TMEM, V = the key chunks read N-major)
 //   warps 9-14  TMA: Q and the pages of every key block
-// B200, 2048-token prompt, 16 heads: latent 512 + 64 271 -> 132 us, 256 + 32 100 -> 58 us (before: one block of keys in shared memory, four softmax
-// warps, one loading warp with a lane per page: a block's loads, scores, softmax and values followed one another).  Bound by the tensor cores and, for
+//   warp 15     items, in a queue to all roles: those of this CTA, then those of the grid's next CTA, taken away from the launch when the loads of the
+//               last item near their end (earlier, and a long tile could be held here that another SM would begin sooner).  A CTA's start and end are 12 us:
+//               the launch, page numbers, Q, the first scores, O; here the next item's Q and scores come under the last products and results of this one
+// Rows of Q and of the result are 1 KB and more apart: a thread that moves its own row touches a line per 16 bytes (the Q of an item took 3500 clocks, its
+// result 4000).  Four lanes move 64 bytes of a row at a time and exchange pieces by shuffles.
+// B200, us, 16 heads: 2048-token prompt, latent 512 + 64 132 -> 106 (a tile after the other by the launch 132, taken 117, and by 64 bytes 106); 3 prompts
+// of 2048 tokens in all 82 -> 58; latent 256 + 32 58 -> 52; 592 tokens, one tile per SM, 27 -> 24.  Bound by the tensor cores and, for
 // the operands outside TMEM, their shared-memory reads: a block of 64 keys takes 3000 clocks, 20 score MMAs of 78, 16 of 46 and 4 value MMAs of 142 2860.
 // Work item = (tile, run): the rows of a tile that belong to one request, with the tile's other rows masked, from an empty O.  What another request's
 // cache holds (a NaN times a weight of zero) never reaches a row, and requests that share a tile -- decoded tokens beside a prompt portion, each with a
 // context of its own -- do not wait for one another.  A tile's CTAs take its first run; the others, which start at a token whose first row is inside a
 // tile, go to the helper CTAs, every helpers-th token to the same ones, so that the decoded tokens of a step spread over the GPU.  A helper that finds
-// none ends at once.  B200, us, 16 heads, latent 512 + 64 (latent_attention_mma.cu in brackets): 2048-token portion beside 8
-// tokens at contexts of 4096 147 (1169), 1000 beside 24 at 2000 71 (444), 320 tokens at 1000 159 (334), 2048 alone 133 (662).
+// none goes on with a tile.  B200, us, 16 heads, latent 512 + 64 (latent_attention_mma.cu in brackets): 2048-token portion beside 8
+// tokens at contexts of 4096 123 (1169), 1000 beside 24 at 2000 64 (444), 320 tokens at 1000 150 (334).
 // Keys outside the run (slots behind the context's end, keys before the window) are masked in S, and their value rows are cleared in shared memory
 // before P V: they may hold anything.
 // 2 * rows * keys * (2 rank + rot) flop of result, 1.5 times that executed at rank 512.
@@ -34,7 +39,8 @@ namespace {
 
 constexpr int LT_ROWS = 128, LT_KEYS = 64, LT_MAXC = 9, LT_VC = 4;  // rows, keys per block, feature chunks, value chunks per CTA
 constexpr int LT_SOFT = 256, LT_LOAD_O = 2, LT_LOADS = LT_LOAD_O + LT_VC;  // softmax threads (two per row); loading warps
-constexpr int LT_THREADS = LT_SOFT + 32 + 32 * LT_LOADS, LT_ITEMS = 128;   // items of a CTA at most
+constexpr int LT_THREADS = LT_SOFT + 32 + 32 * LT_LOADS + 32, LT_SCAN = 128;  // tokens that a helper looks at, at most
+constexpr int LT_QUEUE = 4, LT_READERS = LT_SOFT / 32 + 1 + LT_LOADS;  // items on their way to the roles; softmax warps, MMA issuer, loaders
 constexpr int LT_QC = LT_ROWS * 128, LT_KC = LT_KEYS * 128;         // bytes of a chunk of Q / of keys
 // places for other chunks: two blocks' or what Q and two blocks' value chunks leave of 216 KB, and never less than one block's (S waits for all of them)
 constexpr int LT_RING = 9;
@@ -55,6 +61,7 @@ struct LtItem {  // consecutive tokens of one request inside a tile
   int R0, t0, t1;   // the tile's first row, first and last token
   int k0, lo, end;  // first key of the first block (on a page border), first visible key of any row, one past the last
   int pages;        // offset of the request's page list
+  int vc0;          // first value chunk of the half
 };
 
 struct LtArgs {
@@ -63,6 +70,7 @@ struct LtArgs {
   bf16* out;
   int page_size, tokens, heads, rank, D, nc, halves, window;
   int helpers, helpers_first;  // helper CTAs per half; whether they come before the tiles' in the grid
+  int take;                    // whether a CTA goes on with the grid's next one
   float scale_log2;
   unsigned int* err;
 };
@@ -79,19 +87,57 @@ __device__ __forceinline__ float lt_exp2(float x) {
   return y;
 }
 
+// v[4 p ..]: piece p (16 bytes) of this lane's row <-> piece `lane & 3` of row p of the four lanes
+__device__ __forceinline__ void lt_transpose4(uint32_t* v, int lane) {
+#pragma unroll
+  for (int d = 1; d <= 2; d *= 2) {
+    const bool up = lane & d;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      if (p & d) continue;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        uint32_t &lo = v[4 * p + x], &hi = v[4 * (p + d) + x];
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, up ? lo : hi, d);
+        (up ? lo : hi) = other;
+      }
+    }
+  }
+}
+// The grid's next CTA that has not begun, taken away from the launch: the answer (16 bytes) comes with the barrier's phase
+__device__ __forceinline__ void lt_take_next(void* answer, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(answer)), "r"(smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ int lt_taken(const void* answer) {  // its blockIdx.x; -1: there is none
+  int x;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
+      "ld.shared.b128 h, [%1];\n\t"
+      "mov.b32 %0, -1;\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, h;\n\t}"
+      : "=r"(x)
+      : "r"(smem_u32(answer))
+      : "memory");
+  return x;
+}
+
 struct LtSmem {  // behind Q and the key chunks
-  uint64_t q_full, q_empty, q_tmem, k_full[2], k_empty[LT_RING], v_full[2], v_empty[2], s_full[2], p_ready[2], pv_done, done;
+  alignas(16) uint4 answer;
+  uint64_t item_full[LT_QUEUE], item_empty[LT_QUEUE], taken, q_full, q_empty, q_tmem, k_full[2], k_empty[LT_RING], v_full[2], v_empty[2], s_full[2], p_ready[2], pv_done, done;
   uint32_t tmem_slot;
-  int dead, n_items, first_end;
+  int dead, near_end;  // near_end: items whose last blocks are being loaded, or that are done
   float top[2][LT_SOFT], sum[LT_SOFT];  // of the half rows: maxima (by the block's parity), sums
-  LtItem items[LT_ITEMS];
+  LtItem items[LT_QUEUE];
 };
 
 __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                                                           const LtArgs a) {
   extern __shared__ uint8_t lt_smem_raw[];
   uint8_t* Qs = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(lt_smem_raw) + 1023) & ~(uintptr_t)1023);
-  const int vc0 = (int)(blockIdx.x % a.halves) * LT_VC, nvc = min(LT_VC, a.rank / 64 - vc0), n_other = a.nc - nvc;
+  // (where CTAs go on with others, the halves are alike)
+  const int nvc = min(LT_VC, a.rank / 64 - (int)(blockIdx.x % a.halves) * LT_VC), n_other = a.nc - nvc;
   const int ring = lt_ring(n_other, nvc);
   uint8_t* Vs = Qs + (size_t)n_other * LT_QC;          // two of nvc chunks
   uint8_t* Ks = Vs + (size_t)2 * nvc * LT_KC;          // the ring of other chunks
@@ -99,19 +145,16 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
   volatile int* dead = &m.dead;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int total = a.tokens * a.heads, tiles = (total + LT_ROWS - 1) / LT_ROWS;
-  const int group = blockIdx.x / a.halves, helper = a.helpers_first ? group : group - tiles;  // 0 .. helpers - 1: a helper
-  const bool help = helper >= 0 && helper < a.helpers;
-  auto item_of = [&](int R0, int t0, int t1) {
-    const int rq = a.req[t0], lo = a.window > 0 ? max(a.pos[t0] - a.window + 1, 0) : 0;
-    return LtItem{R0, t0, t1, lo / a.page_size * a.page_size, lo, a.pos[t1] + 1, a.page_off[rq]};
+  // which helper the grid's CTA `id` is, or -1
+  auto helper_of = [&](int id) {
+    const int group = id / a.halves, h = a.helpers_first ? group : group - tiles;
+    return h >= 0 && h < a.helpers ? h : -1;
   };
-  auto last_token = [&](int R0) { return (min(total, R0 + LT_ROWS) - 1) / a.heads; };
-  bool starts = false;  // this thread's token starts a run inside a tile
-  const int my_token = helper + (int)threadIdx.x * a.helpers;
-  if (help) {
+  auto starts = [&](int t) { return t > 0 && t < a.tokens && (long)t * a.heads % LT_ROWS != 0 && a.req[t] != a.req[t - 1]; };  // a run begins inside a tile
+  const int help = helper_of(blockIdx.x);
+  if (help >= 0 && !a.take) {
     pdl_wait();
-    if (threadIdx.x < LT_ITEMS && my_token > 0 && my_token < a.tokens && (long)my_token * a.heads % LT_ROWS != 0) starts = a.req[my_token] != a.req[my_token - 1];
-    if (__syncthreads_count(starts) == 0) return;
+    if (__syncthreads_count(threadIdx.x < LT_SCAN && starts(help + (int)threadIdx.x * a.helpers)) == 0) return;
   }
   if (threadIdx.x == 0) {
     mbar_init(&m.q_full, 1);
@@ -127,40 +170,108 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
     }
     mbar_init(&m.pv_done, 1);
     mbar_init(&m.done, 1);
+    mbar_init(&m.taken, 1);
+    for (int i = 0; i < LT_QUEUE; ++i) {
+      mbar_init(m.item_full + i, 1);
+      mbar_init(m.item_empty + i, LT_READERS);
+    }
     m.dead = 0;
-    m.n_items = 0;
-    m.first_end = 0x7fffffff;
+    m.near_end = 0;
     mbar_fence_init();
   }
   if (warp == LT_SOFT / 32) tmem_alloc(&m.tmem_slot, 512);
-  if (!help) pdl_wait();
+  pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (help) {
-    if (starts) {
-      const int R0 = my_token * a.heads / LT_ROWS * LT_ROWS, last = last_token(R0), rq = a.req[my_token];
-      int e = my_token;
-      while (e < last && a.req[e + 1] == rq) ++e;
-      m.items[atomicAdd(&m.n_items, 1)] = item_of(R0, my_token, e);
-    }
-  } else {
-    const int tile = tiles - 1 - (a.helpers_first ? group - a.helpers : group);  // late tokens (long contexts) first
-    const int R0 = tile * LT_ROWS, t0 = R0 / a.heads, last = last_token(R0), t = t0 + 1 + (int)threadIdx.x;  // at most 128 tokens
-    if (t <= last && a.req[t] != a.req[t - 1]) atomicMin(&m.first_end, t - 1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      m.items[0] = item_of(R0, t0, min(last, m.first_end));
-      m.n_items = 1;
-    }
-  }
-  __syncthreads();
   pdl_launch_dependents();  // after the allocation: a dependent that came first would hold the TMEM while it waits for this grid
   const uint32_t tmem = m.tmem_slot;
-  const int n_items = m.n_items;
+  // the CTA's k-th item, in the order of all roles; false: no more
+  auto item = [&](uint32_t k, LtItem& r) {
+    if (!mbar_wait_bounded(m.item_full + k % LT_QUEUE, (k / LT_QUEUE) & 1, dead)) return false;
+    r = m.items[k % LT_QUEUE];
+    return r.R0 >= 0;
+  };
   auto blocks_of = [&](const LtItem& r) { return (r.end - r.k0 + LT_KEYS - 1) / LT_KEYS; };  // 0: no visible key
 
-  if (warp > LT_SOFT / 32) {
+  if (warp == LT_THREADS / 32 - 1) {
+    // Items: those of this CTA, then, while the last one's end is being computed, those of the grid's next CTA
+    uint32_t n = 0, asked = 0;
+    auto give = [&](const LtItem& r) {  // by one lane
+      if (mbar_wait_bounded(m.item_empty + n % LT_QUEUE, ((n / LT_QUEUE) & 1) ^ 1, dead)) {
+        m.items[n % LT_QUEUE] = r;
+        mbar_arrive(m.item_full + n % LT_QUEUE);
+      }
+    };
+    auto item_of = [&](int R0, int t0, int t1, int half) {
+      const int rq = a.req[t0], lo = a.window > 0 ? max(a.pos[t0] - a.window + 1, 0) : 0;
+      return LtItem{R0, t0, t1, lo / a.page_size * a.page_size, lo, a.pos[t1] + 1, a.page_off[rq], half * LT_VC};
+    };
+    auto last_token = [&](int R0) { return (min(total, R0 + LT_ROWS) - 1) / a.heads; };
+    int id = blockIdx.x;
+    while (id >= 0) {
+      const int half = id % a.halves, h = helper_of(id);
+      if (h >= 0) {
+        bool st[LT_SCAN / 32];
+#pragma unroll
+        for (int j = 0; j < LT_SCAN / 32; ++j) st[j] = starts(h + (lane + 32 * j) * a.helpers);
+#pragma unroll
+        for (int j = 0; j < LT_SCAN / 32; ++j) {
+          uint32_t which = __ballot_sync(0xffffffffu, st[j]);
+          if (which == 0) continue;
+          LtItem r{};
+          if (st[j]) {
+            const int t = h + (lane + 32 * j) * a.helpers, R0 = t * a.heads / LT_ROWS * LT_ROWS, last = last_token(R0), rq = a.req[t];
+            int e = t;
+            while (e < last && a.req[e + 1] == rq) ++e;
+            r = item_of(R0, t, e, half);
+          }
+          for (; which; which &= which - 1, ++n) {
+            if (lane == __ffs(which) - 1) give(r);
+            __syncwarp();
+          }
+        }
+      } else {
+        const int group = id / a.halves, tile = tiles - 1 - (a.helpers_first ? group - a.helpers : group);  // late tokens (long contexts) first
+        const int R0 = tile * LT_ROWS, t0 = R0 / a.heads, last = last_token(R0);
+        int end = last;
+        for (int t = t0 + 1; t <= last; t += 32) {  // (at most 128 tokens)
+          const uint32_t other = __ballot_sync(0xffffffffu, t + lane <= last && a.req[min(t + lane, last)] != a.req[t0]);
+          if (other) {
+            end = t + __ffs(other) - 2;
+            break;
+          }
+        }
+        if (lane == 0) give(item_of(R0, t0, end, half));
+        __syncwarp();
+        ++n;
+      }
+      id = -1;
+      if (!a.take) break;
+      if (lane == 0) {
+        // not before: what is taken early may be a long tile that another CTA could begin sooner
+        for (uint32_t spins = 0; *reinterpret_cast<volatile int*>(&m.near_end) < (int)n && !*dead; ++spins) {
+          __nanosleep(64);
+          if (spins > kWaitSpins) *dead = 1;
+        }
+        if (!*dead) {
+          fence_proxy_async_smem();  // the last answer has been read
+          mbar_expect_tx(&m.taken, 16);
+          lt_take_next(&m.answer, &m.taken);
+          if (mbar_wait_bounded(&m.taken, asked & 1, dead)) id = lt_taken(&m.answer);
+          else mbar_drain(&m.taken, asked & 1);
+        }
+      }
+      ++asked;
+      id = __shfl_sync(0xffffffffu, id, 0);
+    }
+    if (lane == 0) {
+      LtItem none{};
+      none.R0 = -1;
+      give(none);
+    }
+    __syncwarp();
+  } else if (warp > LT_SOFT / 32) {
     // Loads: two warps take the other chunks in turn (one of them their Q), one warp each the value chunks.  One thread of a warp issues (the operands of a
     // copy are uniform registers: with a lane per page the compiler walked through the lanes, about 200 clocks each), which takes 400 clocks for the four
     // pages of a chunk; page numbers are looked up a block ahead.
@@ -170,11 +281,16 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
       const int box = min(a.page_size, LT_KEYS), pieces = LT_KEYS / box;
       uint32_t n = 0, q = 0, place = 0, par = 1;  // blocks and queries so far; the ring's next place and its parity
       bool go = true;  // false behind a run-out: a barrier must not be armed twice in one phase
-      for (int i = 0; i < n_items && go; ++i) {
-        const LtItem r = m.items[i];
+      LtItem r;
+      for (uint32_t k = 0; go && item(k, r); ++k) {
+        mbar_arrive(m.item_empty + k % LT_QUEUE);
+        const int vc0 = r.vc0;
         const int* pg = a.pages + r.pages;
         const int nb = blocks_of(r), last = (r.end - 1) / a.page_size;
-        if (nb <= 0) continue;
+        if (nb <= 0) {
+          if (v == 0) *reinterpret_cast<volatile int*>(&m.near_end) = (int)k + 1;
+          continue;
+        }
         if (me == 0) {
           if (q > 0 && !mbar_wait_bounded(&m.q_empty, (q - 1) & 1, dead)) break;
           mbar_expect_tx(&m.q_full, (uint32_t)(n_other * LT_QC));
@@ -203,6 +319,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
             if (v >= nvc) continue;
             go = mbar_wait_bounded(m.v_empty + (n & 1), ((n >> 1) & 1) ^ 1, dead);
             if (!go) break;
+            if (v == 0 && b == max(nb - 2, 0)) *reinterpret_cast<volatile int*>(&m.near_end) = (int)k + 1;
             if (v == 0) mbar_expect_tx(m.v_full + (n & 1), (uint32_t)(nvc * LT_KC));  // (the other warps' bytes may be counted before)
             copy(Vs + (size_t)((n & 1) * nvc + v) * LT_KC, vc0 + v, m.v_full + (n & 1));
           } else {
@@ -255,8 +372,10 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         umma_commit(m.s_full + (n & 1));
       };
       uint32_t n = 0, q = 0;  // blocks and queries so far
-      for (int i = 0; i < n_items; ++i) {
-        const uint32_t end = n + (uint32_t)max(blocks_of(m.items[i]), 0), first = n;
+      LtItem r;
+      for (uint32_t k = 0; item(k, r); ++k) {
+        mbar_arrive(m.item_empty + k % LT_QUEUE);
+        const uint32_t end = n + (uint32_t)max(blocks_of(r), 0), first = n;
         if (n == end) continue;
         mbar_wait_bounded(&m.q_full, q & 1, dead);
         mbar_wait_bounded(&m.q_tmem, q++ & 1, dead);
@@ -288,33 +407,52 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
     const int row = threadIdx.x & (LT_ROWS - 1), side = threadIdx.x >> 7, ow = nvc * 32;
     const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16), t_o = t_lane + 256 + side * ow;
     auto both_halves = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 3)) : "memory"); };  // the two warps of 32 rows
-    uint32_t n = 0;
-    for (int i = 0; i < n_items; ++i) {
-      const LtItem r = m.items[i];
+    auto both_have = [&](bool x) {  // (behind a run-out the two could part, and wait for each other)
+      uint32_t y;
+      asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, %2, 64, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                   : "=r"(y)
+                   : "r"((uint32_t)x), "r"(1 + (warp & 3))
+                   : "memory");
+      return y != 0;
+    };
+    // the value chunks' Q of an item, once the last one's scores are complete
+    auto put_q = [&](const LtItem& r) {
+      const int R = r.R0 + (warp & 3) * 32 + (lane & ~3);  // four lanes read 64 bytes of a row at a time: a lane by itself would touch a line per 16 bytes
+      for (int c = side; c < nvc; c += 2) {
+        uint32_t t[32];
+        const bf16* src = a.qa + (size_t)R * a.D + (r.vc0 + c) * 64 + (lane & 3) * 8;
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+          const uint4 u = R + (x & 3) < total ? *reinterpret_cast<const uint4*>(src + (size_t)(x & 3) * a.D + (x >> 2) * 32) : make_uint4(0, 0, 0, 0);
+          t[4 * x] = u.x;
+          t[4 * x + 1] = u.y;
+          t[4 * x + 2] = u.z;
+          t[4 * x + 3] = u.w;
+        }
+        lt_transpose4(t, lane);
+        lt_transpose4(t + 16, lane);
+        tmem_put32(t_lane + 128 + c * 32, t);
+      }
+      tmem_put_wait();
+      tc_fence_before();
+      mbar_arrive(&m.q_tmem);
+    };
+    uint32_t n = 0, k = 0;
+    auto next_item = [&](LtItem& r) {
+      const bool more = item(k, r);
+      __syncwarp();
+      if (!both_have(more)) return false;
+      if (lane == 0) mbar_arrive(m.item_empty + k % LT_QUEUE);
+      ++k;
+      if (blocks_of(r) > 0) put_q(r);
+      return true;
+    };
+    LtItem r, ahead;
+    for (bool more = next_item(r); more; r = ahead) {
       const int R = r.R0 + row, tok = R < total ? R / a.heads : -1, nb = blocks_of(r);
       const bool act = tok >= r.t0 && tok <= r.t1;
       const int my_pos = act ? a.pos[tok] : -1, my_lo = a.window > 0 ? my_pos - a.window + 1 : 0;
       float mx = -INFINITY, l = 0.f;  // running maximum of the row (scaled, log2 units) and sum of the half
-      if (nb > 0) {  // the value chunks' Q (the last item's products are complete: its last P V was waited for)
-        for (int c = side; c < nvc; c += 2) {
-          uint32_t t[32] = {};
-          if (R < total) {
-            const uint4* src = reinterpret_cast<const uint4*>(a.qa + (size_t)R * a.D + (vc0 + c) * 64);
-#pragma unroll
-            for (int x = 0; x < 8; ++x) {
-              const uint4 u = src[x];
-              t[4 * x] = u.x;
-              t[4 * x + 1] = u.y;
-              t[4 * x + 2] = u.z;
-              t[4 * x + 3] = u.w;
-            }
-          }
-          tmem_put32(t_lane + 128 + c * 32, t);
-        }
-        tmem_put_wait();
-        tc_fence_before();
-        mbar_arrive(&m.q_tmem);
-      }
       for (int b = 0; b < nb; ++b, ++n) {
         const int j0 = r.k0 + b * LT_KEYS, h0 = j0 + side * 32;
         mbar_wait_bounded(m.s_full + (n & 1), (n >> 1) & 1, dead);
@@ -381,6 +519,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         tc_fence_before();
         mbar_arrive(m.p_ready + (n & 1));
       }
+      more = next_item(ahead);  // its first scores are computed under what follows
       // ---- O / l -> bf16, the rows of this item (the next one's first P V waits for all threads' next p_ready)
       if (nb > 0) mbar_wait_bounded(&m.pv_done, (n - 1) & 1, dead);
       __syncwarp();
@@ -392,18 +531,18 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
       const float sk = a.sink && act ? bf2f(a.sink[R % a.heads]) * 1.4426950408889634f : -INFINITY;
       const float M = fmaxf(mx, sk), w = lt_exp2(mx - M);
       const float inv = w / (l * w + (a.sink ? lt_exp2(sk - M) : 0.f));
-      uint4* dst = reinterpret_cast<uint4*>(a.out + (size_t)(act ? R : 0) * a.rank + vc0 * 64 + side * ow);
+      const uint32_t rows = __ballot_sync(0xffffffffu, act);
+      bf16* dst = a.out + (size_t)(r.R0 + (warp & 3) * 32 + (lane & ~3)) * a.rank + r.vc0 * 64 + side * ow + (lane & 3) * 8;
       for (int c = 0; c < ow; c += 32) {
-        uint32_t t[32] = {};
+        uint32_t t[32] = {}, u[16];
         if (nb > 0) tmem_ld32(t_o + c, t);  // no visible key at all (a position before the first): O is zero, as the sum is
-        if (act) {
 #pragma unroll
-          for (int x = 0; x < 32; x += 8)
-            dst[(c + x) >> 3] = make_uint4(pack_bf16(__uint_as_float(t[x]) * inv, __uint_as_float(t[x + 1]) * inv),
-                                           pack_bf16(__uint_as_float(t[x + 2]) * inv, __uint_as_float(t[x + 3]) * inv),
-                                           pack_bf16(__uint_as_float(t[x + 4]) * inv, __uint_as_float(t[x + 5]) * inv),
-                                           pack_bf16(__uint_as_float(t[x + 6]) * inv, __uint_as_float(t[x + 7]) * inv));
-        }
+        for (int x = 0; x < 16; ++x) u[x] = pack_bf16(__uint_as_float(t[2 * x]) * inv, __uint_as_float(t[2 * x + 1]) * inv);
+        lt_transpose4(u, lane);
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+          if (rows >> ((lane & ~3) + x) & 1)
+            *reinterpret_cast<uint4*>(dst + (size_t)x * a.rank + c) = make_uint4(u[4 * x], u[4 * x + 1], u[4 * x + 2], u[4 * x + 3]);
       }
       tc_fence_before();
     }
@@ -441,10 +580,10 @@ int launch_latent_attention_tc(const bf16* qa, const bf16* cache, const bf16* si
            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return -2;
   }
-  // Runs that start inside a tile are for the helpers, one CTA per half and SM (more where a helper would have over LT_ITEMS tokens to look at); none
+  // Runs that start inside a tile are for the helpers, one CTA per half and SM (more where a helper would have over LT_SCAN tokens to look at); none
   // where each token fills whole tiles.  They come first, since their contexts may be the longest, unless all CTAs fit at once.
   int helpers = heads % LT_ROWS == 0 ? 0 : (sm_count() + halves - 1) / halves;
-  if (helpers > 0 && helpers < (tokens + LT_ITEMS - 1) / LT_ITEMS) helpers = (tokens + LT_ITEMS - 1) / LT_ITEMS;
+  if (helpers > 0 && helpers < (tokens + LT_SCAN - 1) / LT_SCAN) helpers = (tokens + LT_SCAN - 1) / LT_SCAN;
   const int v0 = rank / 64 < LT_VC ? rank / 64 : LT_VC, v1 = halves == 1 ? v0 : rank / 64 - LT_VC;  // value chunks of the halves
   const size_t b0 = lt_bytes(nc - v0, v0), b1 = lt_bytes(nc - v1, v1), smem = (b0 > b1 ? b0 : b1) + sizeof(LtSmem) + 1024, most = 216 * 1024 + sizeof(LtSmem) + 1024;
   static_assert(most <= 227 * 1024, "shared memory");
@@ -453,7 +592,7 @@ int launch_latent_attention_tc(const bf16* qa, const bf16* cache, const bf16* si
     cudaGetLastError();
     return -2;
   }
-  const LtArgs a{qa, sink, pos, req, page_off, pages, out, page_size, tokens, heads, rank, D, nc, halves, window, helpers, tiles * halves > sm_count(), scale * 1.4426950408889634f, wait_err_word()};
+  const LtArgs a{qa, sink, pos, req, page_off, pages, out, page_size, tokens, heads, rank, D, nc, halves, window, helpers, tiles * halves > sm_count(), v0 == v1, scale * 1.4426950408889634f, wait_err_word()};
   return (int)launch(latent_attention_tc_kernel, dim3((unsigned)((tiles + helpers) * halves)), dim3(LT_THREADS), smem, st, true, mq, mk, a);
 }
 
