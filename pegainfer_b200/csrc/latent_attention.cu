@@ -224,9 +224,10 @@ __global__ void latent_attention_kernel(const E* __restrict__ qa, const E* __res
 int launch_latent_attention_mma(const bf16* qa, const bf16* cache, const bf16* sink, const int* pos, const int* req, const int* page_off,
                                 const int* pages, bf16* out, long page_stride, int page_size, int tokens, int heads, int rank, int rot, float scale,
                                 int window, int max_kv_len, cudaStream_t st);
-// latent_attention_tc.cu: tcgen05 kernel for prompt portions (enough rows to fill the GPU without cutting the key axis); -2 = not for this shape
+// latent_attention_tc.cu: tcgen05 kernel for prompt portions (rows enough, or contexts short enough, to leave the key axis in one piece); -2 = not for this shape
 int launch_latent_attention_tc(const bf16* qa, const bf16* cache, const bf16* sink, const int* pos, const int* req, const int* page_off, const int* pages,
-                               bf16* out, long page_stride, int page_size, int tokens, int heads, int rank, int rot, float scale, int window, cudaStream_t st);
+                               bf16* out, long page_stride, int page_size, int tokens, int heads, int rank, int rot, float scale, int window, int max_kv_len,
+                               cudaStream_t st);
 static bool latent_mma_enabled() {  // PK_LATENT_ATTN=generic keeps the generic kernel for A/B runs
   static int v = -1;
   if (v < 0) {
@@ -294,7 +295,7 @@ extern "C" int pk_latent_attention_ex(const void* qa, const void* cache, const v
   if (!qa || !cache || !positions || !req || !page_off || !pages || !out || tokens <= 0 || heads <= 0 || rank <= 0 || rot < 0 || window < 0) return -1;
   if (!f32 && latent_mma_enabled()) {
     int rc = launch_latent_attention_tc((const bf16*)qa, (const bf16*)cache, (const bf16*)sink, positions, req, page_off, pages, (bf16*)out, page_stride,
-                                        page_size, tokens, heads, rank, rot, scale, window, st);
+                                        page_size, tokens, heads, rank, rot, scale, window, max_kv_len, st);
     if (rc != -2) return rc;
     rc = launch_latent_attention_mma((const bf16*)qa, (const bf16*)cache, (const bf16*)sink, positions, req, page_off, pages, (bf16*)out,
                                                page_stride, page_size, tokens, heads, rank, rot, scale, window, max_kv_len, st);

@@ -561,14 +561,24 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
 // 0 = launched; -2 = shape / alignment outside this kernel (the caller runs the mma.sync kernel)
 int launch_latent_attention_tc(const bf16* qa, const bf16* cache, const bf16* sink, const int* pos, const int* req, const int* page_off, const int* pages,
                                bf16* out, long page_stride, int page_size, int tokens, int heads, int rank, int rot, float scale, int window,
-                               cudaStream_t st) {
+                               int max_kv_len, cudaStream_t st) {
   const int D = rank + rot, nc = (D + 63) / 64, halves = (rank / 64 + LT_VC - 1) / LT_VC;
   // (rot % 16, rank <= 512: what the mma.sync kernel takes too.  The shapes beyond go to the generic kernel, whose weights stay fp32.)
   if (rank % 64 || rot % 16 || rank > 512 || nc > LT_MAXC || page_size < 8 || (page_size & (page_size - 1)) || page_stride % 8 || !(scale > 0.f) ||
       ((reinterpret_cast<uintptr_t>(qa) | reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(out)) & 15))
     return -2;
   const long rows = (long)tokens * heads, tiles = (rows + LT_ROWS - 1) / LT_ROWS;
-  if (tiles * halves < sm_count() / 2 || tiles * halves > 0x3fffffff || rows > 0x7fffffff) return -2;  // few rows: the key axis has to be split
+  if (tiles * halves > 0x3fffffff || rows > 0x7fffffff) return -2;
+  const int v0 = rank / 64 < LT_VC ? rank / 64 : LT_VC, v1 = halves == 1 ? v0 : rank / 64 - LT_VC;  // value chunks of the halves
+  // Few CTAs: the key axis has to be cut, which the mma.sync kernel does, unless contexts are short.  This kernel takes 11 us and 1.3 to 1.5 for every 64
+  // keys of the longest context; that one 11 and, for every 16 rows of 64 keys, 0.05 (latent 512), 0.02 (256) or 0.007 (128), so that short contexts cancel
+  // out and the number of rows decides.  Up to 512 keys a request that is longer than all others costs little here (140 decoding, one of them
+  // at 510, latent 512 + 64, 8 heads, 33.3 31.2), and one CTA in twelve SMs is enough; latents below 128 and unequal halves, which gain less, take one
+  // in six.  One or two blocks of keys are one pass in that kernel.  Us, 16 heads, 512 + 64, that kernel and this one: 200 tokens 51.7 16.8, 150 37.4 14.9,
+  // 100 behind 400 keys 57.9 23.1, 80 decoding at 480 55.8 39.3; 8 heads, 500 tokens 92.7 23.0; latent 256 + 32, 16 heads, 200 tokens 27.0 14.8.
+  const int keys = window > 0 && window + (long)tokens < max_kv_len ? window + tokens : max_kv_len;
+  const bool few_keys = keys > (rank > 256 ? 1 : 2) * LT_KEYS && keys <= 8 * LT_KEYS;
+  if (tiles * halves < sm_count() / (!few_keys ? 2 : rank < 128 || v0 != v1 ? 6 : 12)) return -2;
   EncodeTiledFn fn = encode_fn();
   if (!fn) return -2;
   CUtensorMap mq, mk;
@@ -584,7 +594,6 @@ int launch_latent_attention_tc(const bf16* qa, const bf16* cache, const bf16* si
   // where each token fills whole tiles.  They come first, since their contexts may be the longest, unless all CTAs fit at once.
   int helpers = heads % LT_ROWS == 0 ? 0 : (sm_count() + halves - 1) / halves;
   if (helpers > 0 && helpers < (tokens + LT_SCAN - 1) / LT_SCAN) helpers = (tokens + LT_SCAN - 1) / LT_SCAN;
-  const int v0 = rank / 64 < LT_VC ? rank / 64 : LT_VC, v1 = halves == 1 ? v0 : rank / 64 - LT_VC;  // value chunks of the halves
   const size_t b0 = lt_bytes(nc - v0, v0), b1 = lt_bytes(nc - v1, v1), smem = (b0 > b1 ? b0 : b1) + sizeof(LtSmem) + 1024, most = 216 * 1024 + sizeof(LtSmem) + 1024;
   static_assert(most <= 227 * 1024, "shared memory");
   static std::atomic<uint64_t> smem_set{0};

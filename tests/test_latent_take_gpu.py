@@ -1,5 +1,5 @@
 """The latent attention of prompt portions where its CTAs go on with the grid's next ones: several tiles a CTA, more runs that start inside tiles than its
-queue has places, runs of one block and of many in turn, and halves of unequal width, whose CTAs do not."""
+queue has places, runs of one block and of many in turn, and halves of unequal width, whose CTAs do not.  And few rows with short contexts."""
 import pytest
 import torch
 
@@ -13,6 +13,15 @@ pytestmark = pytest.mark.gpu
     ([0], [3333], 16, 0, 16, False), ([50] * 600, [5] * 600, 10, 0, 16, True), ([0, 2000, 5], [1500, 700, 900], 16, 300, 32, True),
     ([3000, 0] * 12, [1, 130] * 12, 16, 0, 16, False), ([0] * 300, [9] * 300, 24, 0, 8, False)])
 def test_against_64_bits(lib, starts, lens, H, window, ps, sink, rank, rot):  # noqa: F811
+    check_against_64_bits(lib, starts, lens, H, window, ps, sink, rank, rot)
+
+
+# on both sides of the rule that takes few rows with short contexts here: 12 CTAs (one in twelve SMs) or not, contexts of 64, 128, 129, 512 and 513 keys
+@pytest.mark.parametrize("rank,rot", [(512, 64), (256, 32), (128, 32), (64, 16), (320, 0)])
+@pytest.mark.parametrize("starts,lens,H,window,ps,sink", [
+    ([0], [64], 16, 0, 16, False), ([0], [128], 16, 0, 16, True), ([0, 28], [60, 101], 16, 0, 16, False), ([412], [100], 16, 0, 16, True), ([413], [100], 16, 0, 16, False),
+    ([0], [512], 8, 0, 32, False), ([900], [100], 16, 300, 16, False), ([3, 511, 60, 0] * 25, [1] * 100, 20, 0, 16, True), ([0], [90], 16, 0, 16, False)])
+def test_few_rows(lib, starts, lens, H, window, ps, sink, rank, rot):  # noqa: F811
     check_against_64_bits(lib, starts, lens, H, window, ps, sink, rank, rot)
 
 
