@@ -234,7 +234,8 @@ struct MgArgs {
 // EPI 0: out bf16 [slots][N] = relu(acc)^2.   EPI 1: out fp32 [slots][N] = acc * weights[pair of the slot].
 // EPI 2: W rows interleaved (2f = gate f, 2f + 1 = up f): out bf16 [slots][N / 2] = silu(acc[2f]) * acc[2f + 1].
 // EPI 3: the same rows with clamped pre-activations: g = min(acc[2f], p0), u = clamp(acc[2f + 1], -p0, p0), out = g logistic(p1 g) (u + 1).
-template <int EPI>
+// W_FIRST: the weights are the first to leave L2.
+template <int EPI, bool W_FIRST>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMgThreads, 1) moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                                                                         const MgArgs a) {
   extern __shared__ uint8_t mg_smem_raw[];
@@ -277,6 +278,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMgThreads, 1) moe_g
     if (tc_elect_one()) {
       int s = 0;
       uint32_t ph = 1;
+      [[maybe_unused]] const uint64_t first = W_FIRST ? l2_evict_first_policy() : 0;
       for (int t = pair; t < tiles && !*dead; t += pairs) {
         const int rt = t / n_ft, n16 = (tr[rt + 1] - tr[rt] + 15) / 16, boxes = (n16 * 8 + 63) / 64;
         const int r0 = tr[rt] + (int)rank * n16 * 8, w0 = te[rt] * a.N + (t - rt * n_ft) * 256 + (int)rank * 128;
@@ -285,7 +287,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMgThreads, 1) moe_g
           const uint32_t fb = g2_map(smem_u32(full + s), 0);
           if (rank == 0) mbar_expect_tx(full + s, 2 * (kMgA + boxes * kMgBox));
           uint8_t* st = smem + (size_t)s * kMgStage;
-          g2_tma_2d(st, &map_w, kb * 64, w0, fb);
+          if constexpr (W_FIRST) g2_tma_2d(st, &map_w, kb * 64, w0, fb, first);
+          else g2_tma_2d(st, &map_w, kb * 64, w0, fb);
           for (int b = 0; b < boxes; ++b) g2_tma_2d(st + kMgA + b * kMgBox, &map_x, kb * 64, r0 + b * 64, fb);
           if (++s == kMgStages) {
             s = 0;
@@ -423,9 +426,9 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
   const float g = shared ? (sg ? 1.f / (1.f + expf(-sg[t])) : 1.f) : 0.f;
   for (int i = threadIdx.x; i < nv; i += blockDim.x) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
+#pragma unroll 2
     for (int k = 0; k < top; ++k) {
-      const float4 p = reinterpret_cast<const float4*>(part + (size_t)pair_slot[(size_t)t * top + k] * width)[i];
+      const float4 p = __ldcs(reinterpret_cast<const float4*>(part + (size_t)pair_slot[(size_t)t * top + k] * width) + i);
       acc.x += p.x;
       acc.y += p.y;
       acc.z += p.z;
@@ -450,17 +453,22 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
   }
 }
 
-template <int EPI>
+template <int EPI, bool W_FIRST>
 static cudaError_t mg_launch(const void* rows, long n_rows, const void* w, const MgArgs& a, cudaStream_t st) {
   CUtensorMap mx, mw;
   if (!make_rows_map(&mx, rows, n_rows, a.K, 64) || !make_rows_map(&mw, w, (long)a.experts * a.N, a.K, 128)) return cudaErrorInvalidValue;
-  auto kern = moe_grouped_gemm_kernel<EPI>;
+  auto kern = moe_grouped_gemm_kernel<EPI, W_FIRST>;
   static std::atomic<uint64_t> smem_set{0};
   if (const cudaError_t e = allow_smem(smem_set, (const void*)kern, kMgSmem); e != cudaSuccess) return e;
   // as many pairs as there can be tiles, one CTA per SM at most
   const long tiles = (n_rows / kMoeTile + (n_rows < a.experts ? n_rows : a.experts)) * ((a.N + 255) / 256);
   const long pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1;
   return launch(kern, dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs))), dim3(kMgThreads), kMgSmem, st, true, mx, mw, a);
+}
+
+template <int EPI>
+static cudaError_t mg_gemm(bool w_first, const void* rows, long n_rows, const void* w, const MgArgs& a, cudaStream_t st) {
+  return w_first ? mg_launch<EPI, true>(rows, n_rows, w, a, st) : mg_launch<EPI, false>(rows, n_rows, w, a, st);
 }
 
 }  // namespace pk
@@ -513,13 +521,17 @@ extern "C" int pk_moe_grouped_act_p(const void* xa, const void* w_up, const void
            slot_pair, pair_slot);
     launch(moe_gather_kernel, dim3((unsigned)pairs), dim3(width >= 2048 ? 256 : 128), 0, st, true, (const bf16*)xa, (const int*)slot_pair, xs, width, top);
   }
+  // From 24 rows an expert on the rows, hidden values and partial sums (100 MB in the call of 2048 tokens) are worth their room in L2, and up to a row tile
+  // an expert the weights are read once: they leave first, where they are too many to be found in L2 again.  B200, 64 experts of 2048 x 1408, top 6, us:
+  // 256 / 512 / 1024 / 2048 tokens 197 207 225 270 -> 188 193 210 264; without the bounds it would be 64 tokens 187 197, 4096 438 445.
+  const bool w_first = pairs >= 24l * experts && pairs <= (kMoeTile - 16l) * experts && (long)experts * width * ff * (act ? 6 : 4) > (256l << 20);
   MgArgs a{hid, meta, slot_pair, weights, experts, max_tiles, act ? 2 * ff : ff, width, p0, p1, wait_err_word()};
-  cudaError_t e = act == 2 ? mg_launch<3>(xs, pairs, w_up, a, st) : act == 1 ? mg_launch<2>(xs, pairs, w_up, a, st) : mg_launch<0>(xs, pairs, w_up, a, st);
+  cudaError_t e = act == 2 ? mg_gemm<3>(w_first, xs, pairs, w_up, a, st) : act == 1 ? mg_gemm<2>(w_first, xs, pairs, w_up, a, st) : mg_gemm<0>(w_first, xs, pairs, w_up, a, st);
   if (e != cudaSuccess) return (int)e;
   a.out = part;
   a.N = width;
   a.K = ff;
-  if ((e = mg_launch<1>(hid, pairs, w_down, a, st)) != cudaSuccess) return (int)e;
+  if ((e = mg_gemm<1>(w_first, hid, pairs, w_down, a, st)) != cudaSuccess) return (int)e;
   launch(moe_combine_kernel, dim3(tokens), dim3(256), 0, st, true, (const float*)part, (const int*)pair_slot, (const bf16*)shared, shared_gate, y, width,
          top);
   return (int)cudaGetLastError();
