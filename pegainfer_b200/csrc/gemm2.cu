@@ -167,6 +167,19 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
       tc_fence_after();
       const int tok = mb * 2 * G2_BM + (int)rank * G2_BM + q * 32 + lane;
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * TN);
+      // 32 columns of the warp's 32 rows, four lanes 64 bytes of a row at a time: a lane that stored its own row would touch a line per 16 bytes, and a tile of
+      // 256 columns would take 4100 clocks to leave -- the last one of a launch, or the only one, with nothing beside it
+      auto store_rows = [&](bf16* base, int ld, const float* r) {
+        uint32_t u[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) u[j] = pack_bf16(r[2 * j], r[2 * j + 1]);
+        transpose4(u, lane);
+        const int tok4 = tok & ~3;
+        bf16* dst = base + (size_t)tok4 * ld + (lane & 3) * 8;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (tok4 + j < N) *reinterpret_cast<uint4*>(dst + (size_t)j * ld) = make_uint4(u[4 * j], u[4 * j + 1], u[4 * j + 2], u[4 * j + 3]);
+      };
       if (a.swiglu) {
         // columns [0, HB) = gate, [HB, BN) = up of features nb*HB + c
 #pragma unroll 1
@@ -175,13 +188,13 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
           tmem_ld32_nowait(t_row + (uint32_t)c, gv);
           tmem_ld32(t_row + (uint32_t)(HB + c), uv);
           const int f0 = nb * HB + c;
-          if (tok < N && f0 < M) {
-            bf16* dst = a.Y + (size_t)tok * a.ldy + f0;
+          if (tok - lane < N && f0 < M) {  // (a warp at a time: the lanes store for one another)
             // one loop per activation and step: a branch per element would leave the elements' long chains one behind the other
             float g[32], u[32], r[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
-              g[j] = round_bf16(__uint_as_float(gv[j]));  // gate_up_out is bf16 in the reference
+              // gate_up_out is bf16 in the reference.  1 behind the last token: a division of zero leaves its fast path (9728 x 2560, 200 tokens: 42 us for 30)
+              g[j] = tok < N ? round_bf16(__uint_as_float(gv[j])) : 1.f;
               u[j] = round_bf16(__uint_as_float(uv[j]));
             }
             if (a.swiglu == 2) {
@@ -197,19 +210,11 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
               for (int j = 0; j < 32; ++j) r[j] = g[j] / r[j] * u[j];
             }
             if (M % 8 == 0 && a.ldy % 8 == 0 && f0 + 32 <= M && (reinterpret_cast<uintptr_t>(a.Y) & 15) == 0) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                uint4 o;
-                o.x = pack_bf16(r[j * 8 + 0], r[j * 8 + 1]);
-                o.y = pack_bf16(r[j * 8 + 2], r[j * 8 + 3]);
-                o.z = pack_bf16(r[j * 8 + 4], r[j * 8 + 5]);
-                o.w = pack_bf16(r[j * 8 + 6], r[j * 8 + 7]);
-                reinterpret_cast<uint4*>(dst)[j] = o;
-              }
-            } else {
+              store_rows(a.Y + f0, a.ldy, r);
+            } else if (tok < N) {
 #pragma unroll
               for (int j = 0; j < 32; ++j)
-                if (f0 + j < M) dst[j] = f2bf(r[j]);
+                if (f0 + j < M) a.Y[(size_t)tok * a.ldy + f0 + j] = f2bf(r[j]);
             }
           }
         }
@@ -219,22 +224,12 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
           uint32_t v[32];
           tmem_ld32(t_row + (uint32_t)c, v);
           const int f0 = nb * TN + c;
-          if (tok < N && f0 < M) {
-            bf16* dst;
-            if (f0 < a.e0) dst = a.Y + (size_t)tok * a.e0 + f0;
-            else if (f0 < a.e1) dst = a.Y1 + (size_t)tok * (a.e1 - a.e0) + (f0 - a.e0);
-            else dst = a.Y2 + (size_t)tok * (M - a.e1) + (f0 - a.e1);
+          if (tok - lane < N && f0 < M) {  // (a warp at a time: the lanes store for one another)
             if (vec_ok && f0 + 32 <= M) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                uint4 o;
-                o.x = pack_bf16(__uint_as_float(v[j * 8 + 0]), __uint_as_float(v[j * 8 + 1]));
-                o.y = pack_bf16(__uint_as_float(v[j * 8 + 2]), __uint_as_float(v[j * 8 + 3]));
-                o.z = pack_bf16(__uint_as_float(v[j * 8 + 4]), __uint_as_float(v[j * 8 + 5]));
-                o.w = pack_bf16(__uint_as_float(v[j * 8 + 6]), __uint_as_float(v[j * 8 + 7]));
-                reinterpret_cast<uint4*>(dst)[j] = o;
-              }
-            } else {
+              if (f0 < a.e0) store_rows(a.Y + f0, a.e0, reinterpret_cast<const float*>(v));
+              else if (f0 < a.e1) store_rows(a.Y1 + (f0 - a.e0), a.e1 - a.e0, reinterpret_cast<const float*>(v));
+              else store_rows(a.Y2 + (f0 - a.e1), M - a.e1, reinterpret_cast<const float*>(v));
+            } else if (tok < N) {
 #pragma unroll
               for (int j = 0; j < 32; ++j) {
                 const int f = f0 + j;

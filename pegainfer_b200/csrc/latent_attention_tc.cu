@@ -87,23 +87,6 @@ __device__ __forceinline__ float lt_exp2(float x) {
   return y;
 }
 
-// v[4 p ..]: piece p (16 bytes) of this lane's row <-> piece `lane & 3` of row p of the four lanes
-__device__ __forceinline__ void lt_transpose4(uint32_t* v, int lane) {
-#pragma unroll
-  for (int d = 1; d <= 2; d *= 2) {
-    const bool up = lane & d;
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      if (p & d) continue;
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        uint32_t &lo = v[4 * p + x], &hi = v[4 * (p + d) + x];
-        const uint32_t other = __shfl_xor_sync(0xffffffffu, up ? lo : hi, d);
-        (up ? lo : hi) = other;
-      }
-    }
-  }
-}
 // The grid's next CTA that has not begun, taken away from the launch: the answer (16 bytes) comes with the barrier's phase
 __device__ __forceinline__ void lt_take_next(void* answer, uint64_t* bar) {
   asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(answer)), "r"(smem_u32(bar))
@@ -429,8 +412,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
           t[4 * x + 2] = u.z;
           t[4 * x + 3] = u.w;
         }
-        lt_transpose4(t, lane);
-        lt_transpose4(t + 16, lane);
+        transpose4(t, lane);
+        transpose4(t + 16, lane);
         tmem_put32(t_lane + 128 + c * 32, t);
       }
       tmem_put_wait();
@@ -538,7 +521,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         if (nb > 0) tmem_ld32(t_o + c, t);  // no visible key at all (a position before the first): O is zero, as the sum is
 #pragma unroll
         for (int x = 0; x < 16; ++x) u[x] = pack_bf16(__uint_as_float(t[2 * x]) * inv, __uint_as_float(t[2 * x + 1]) * inv);
-        lt_transpose4(u, lane);
+        transpose4(u, lane);
 #pragma unroll
         for (int x = 0; x < 4; ++x)
           if (rows >> ((lane & ~3) + x) & 1)

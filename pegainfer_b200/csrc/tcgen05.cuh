@@ -210,6 +210,23 @@ inline EncodeTiledFn encode_fn() {
 }
 
 
+// v[4 p ..]: piece p (16 bytes) of this lane's row <-> piece `lane & 3` of row p of the four lanes
+__device__ __forceinline__ void transpose4(uint32_t* v, int lane) {
+#pragma unroll
+  for (int d = 1; d <= 2; d *= 2) {
+    const bool up = lane & d;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      if (p & d) continue;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        uint32_t &lo = v[4 * p + x], &hi = v[4 * (p + d) + x];
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, up ? lo : hi, d);
+        (up ? lo : hi) = other;
+      }
+    }
+  }
+}
 // TMA load of a tile of a 2-D tensor (c0: element of a row, a multiple of 16 bytes; c1: row); completes on `bar`
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
   asm volatile(
