@@ -172,22 +172,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         uint32_t v[32];
         tmem_ld32(t_row + (uint32_t)c, v);
         const int f0 = nb * BN + c;
-        if (tok < N && f0 < M) {
-          bf16* dst;
-          if (f0 < e0) dst = Y + (size_t)tok * e0 + f0;
-          else if (f0 < e1) dst = Y1 + (size_t)tok * (e1 - e0) + (f0 - e0);
-          else dst = Y2 + (size_t)tok * (M - e1) + (f0 - e1);
-          if (vec_ok && f0 + 32 <= M) {
+        if (tok - lane < N && f0 < M) {
+          if (vec_ok && f0 + 32 <= M) {  // four lanes store 64 bytes of a row at a time (a lane by itself would touch a line per 16 bytes)
+            uint32_t u[16];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint4 o;
-              o.x = pack_bf16(__uint_as_float(v[j * 8 + 0]), __uint_as_float(v[j * 8 + 1]));
-              o.y = pack_bf16(__uint_as_float(v[j * 8 + 2]), __uint_as_float(v[j * 8 + 3]));
-              o.z = pack_bf16(__uint_as_float(v[j * 8 + 4]), __uint_as_float(v[j * 8 + 5]));
-              o.w = pack_bf16(__uint_as_float(v[j * 8 + 6]), __uint_as_float(v[j * 8 + 7]));
-              reinterpret_cast<uint4*>(dst)[j] = o;
-            }
-          } else {
+            for (int j = 0; j < 16; ++j) u[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+            transpose4(u, lane);
+            const int tok4 = tok & ~3, ld = f0 < e0 ? e0 : f0 < e1 ? e1 - e0 : M - e1;
+            bf16* dst = (f0 < e0 ? Y + f0 : f0 < e1 ? Y1 + (f0 - e0) : Y2 + (f0 - e1)) + (size_t)tok4 * ld + (lane & 3) * 8;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (tok4 + j < N) *reinterpret_cast<uint4*>(dst + (size_t)j * ld) = make_uint4(u[4 * j], u[4 * j + 1], u[4 * j + 2], u[4 * j + 3]);
+          } else if (tok < N) {
             for (int j = 0; j < 32 && f0 + j < M; ++j) {
               const int f = f0 + j;
               bf16* d1 = f < e0 ? Y + (size_t)tok * e0 + f
