@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(128 * WG)
 latent_attention_mma_kernel(const bf16* __restrict__ qa, const bf16* __restrict__ cache, const bf16* __restrict__ sink, const int* __restrict__ pos,
                             const int* __restrict__ req, const int* __restrict__ page_off, const int* __restrict__ pages, bf16* __restrict__ out,
                             float* __restrict__ part_o, float* __restrict__ part_ml, long page_stride, int page_size, int tokens, int heads, int rank,
-                            int rot, float scale, int window) {
+                            int rot, float scale, int window, int own) {  // own: rows from one tile to the next, ROWS or fewer
   constexpr int ROWS_G = 16 * MT, ROWS = ROWS_G * WG, NR = 2 * MT;  // NR = rows per thread: rb + g + 8 * i, i < NR
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int D = rank + rot, ldk = D + 8, nv = rank / 32;
@@ -38,7 +38,7 @@ latent_attention_mma_kernel(const bf16* __restrict__ qa, const bf16* __restrict_
   float* wsum = wmax + 4 * ROWS;                           // [4][ROWS]
   const int tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) & 3, rb = (tid >> 7) * ROWS_G, g = lane >> 2, tq = lane & 3;
   const int nthreads = 128 * WG;
-  const int total_rows = tokens * heads, R0 = blockIdx.x * ROWS;
+  const int R0 = blockIdx.x * own, total_rows = min(tokens * heads, R0 + own);
   const int split = blockIdx.y, nsplit = gridDim.y;
   pdl_wait();
   pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
@@ -62,7 +62,7 @@ latent_attention_mma_kernel(const bf16* __restrict__ qa, const bf16* __restrict_
     row_tok[i] = R < total_rows ? R / heads : -1;
     row_pos[i] = row_tok[i] >= 0 ? pos[row_tok[i]] : -1;
   }
-  const int t_first = R0 / heads, t_last = (min(total_rows, R0 + ROWS) - 1) / heads;
+  const int t_first = R0 / heads, t_last = (total_rows - 1) / heads;
   int t = t_first;
   while (t <= t_last) {
     const int rq = req[t];
@@ -259,11 +259,11 @@ latent_attention_mma_kernel(const bf16* __restrict__ qa, const bf16* __restrict_
 
 // one block per query row: combine the splits' (m, l, O) and the sink
 __global__ void latent_attention_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const bf16* __restrict__ sink,
-                                              bf16* __restrict__ out, int nsplit, int heads, int rank, int tile_rows) {
+                                              bf16* __restrict__ out, int nsplit, int heads, int rank, int tile_rows, int own) {
   __shared__ float wgt[64];  // per split: exp(m_s - M) / denominator
   pdl_wait();
   pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
-  const int R = blockIdx.x, tile = R / tile_rows, r = R % tile_rows;
+  const int R = blockIdx.x, tile = R / own, r = R % own;
   const size_t slot0 = (size_t)tile * nsplit * tile_rows + r;  // split s at slot0 + s * tile_rows
   if (threadIdx.x < 32) {
     const float sk = sink ? bf2f(sink[R % heads]) : kNegBig;
@@ -300,14 +300,14 @@ __global__ void latent_attention_merge_kernel(const float* __restrict__ part_o, 
 template <int NV, int MT, int WG>
 static cudaError_t launch_mma(dim3 grid, size_t smem, cudaStream_t st, const bf16* qa, const bf16* cache, const bf16* sink, const int* pos, const int* req,
                               const int* page_off, const int* pages, bf16* out, float* po, float* pml, long page_stride, int page_size, int tokens,
-                              int heads, int rank, int rot, float scale, int window) {
+                              int heads, int rank, int rot, float scale, int window, int own) {
   static bool attr_done = false;
   if (!attr_done) {
     cudaFuncSetAttribute(latent_attention_mma_kernel<NV, MT, WG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     attr_done = true;
   }
   return launch(latent_attention_mma_kernel<NV, MT, WG>, grid, dim3(128 * WG), smem, st, true, qa, cache, sink, pos, req, page_off, pages, out, po, pml,
-                page_stride, page_size, tokens, heads, rank, rot, scale, window);
+                page_stride, page_size, tokens, heads, rank, rot, scale, window, own);
 }
 
 static size_t mma_smem_bytes(int rows, int D) { return (size_t)(rows + 2 * kMmaKeys) * (D + 8) * 2 + (size_t)rows * 72 * 2 + (size_t)8 * rows * 4; }
@@ -327,10 +327,16 @@ int launch_latent_attention_mma(const bf16* qa, const bf16* cache, const bf16* s
   const int wg = (total >= 32 * sm_count() && mma_smem_bytes(32, D) <= 200 * 1024) ? 2 : 1;
   const int rows = 16 * wg;
   const size_t smem = mma_smem_bytes(rows, D);
-  const int tiles = (total + rows - 1) / rows;
+  // Short contexts of few tokens: a tile per token, since a tile that holds several requests walks one's keys after the other's.  B200, us: 6 requests of 78
+  // cached tokens, 8 heads, latent 512 + 64 29 -> 15; 24 of 100, 4 heads, 256 + 32 33 -> 11
+  const int own = max_kv_len <= 2 * kMmaKeys && heads < rows && tokens <= sm_count() ? heads : rows;
+  const int tiles = (total + own - 1) / own;
   int splits = 1;
   ThreadState& ts = tls();
-  if (max_kv_len > 2 * kMmaKeys && tiles < 2 * sm_count() && ts.work()) {
+  // Two blocks of keys are cut for few tiles and latents above 256: there a block takes 6 us, more than the merge of few rows (512 + 64, 16 heads, us: one token
+  // behind 100 16.9 -> 14.8, 24 of them 16.9 -> 15.4, but 70 tokens 16.9 -> 20.3); below 256 it takes 2
+  const bool cut = max_kv_len > 2 * kMmaKeys || (max_kv_len > kMmaKeys && rank > 256 && 4 * tiles <= sm_count());
+  if (cut && tiles < 2 * sm_count() && ts.work()) {
     splits = min(min((2 * sm_count() + tiles - 1) / tiles, (max_kv_len + kMmaKeys - 1) / kMmaKeys), 64);
     while (splits > 1 && (size_t)tiles * splits * rows * (rank + 2) * 4 > ts.work_bytes()) --splits;
   }
@@ -340,7 +346,7 @@ int launch_latent_attention_mma(const bf16* qa, const bf16* cache, const bf16* s
   const int nv = rank / 32;
   cudaError_t e;
 #define PK_LAUNCH_MMA(NVV, WGG) \
-  launch_mma<NVV, 1, WGG>(grid, smem, st, qa, cache, sink, pos, req, page_off, pages, out, po, pml, page_stride, page_size, tokens, heads, rank, rot, scale, window)
+  launch_mma<NVV, 1, WGG>(grid, smem, st, qa, cache, sink, pos, req, page_off, pages, out, po, pml, page_stride, page_size, tokens, heads, rank, rot, scale, window, own)
   if (wg == 2) {
     if (nv <= 2) e = PK_LAUNCH_MMA(2, 2);
     else if (nv <= 4) e = PK_LAUNCH_MMA(4, 2);
@@ -356,7 +362,7 @@ int launch_latent_attention_mma(const bf16* qa, const bf16* cache, const bf16* s
   if (e != cudaSuccess) return (int)e;
   if (splits > 1)
     e = launch(latent_attention_merge_kernel, dim3(total, (rank + 127) / 128), dim3(128), 0, st, true, (const float*)po, (const float*)pml, sink, out, splits, heads, rank,
-               rows);
+               rows, own);
   return (int)e;
 }
 

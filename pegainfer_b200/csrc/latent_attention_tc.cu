@@ -557,10 +557,10 @@ int launch_latent_attention_tc(const bf16* qa, const bf16* cache, const bf16* si
   // keys of the longest context; that one 11 and, for every 16 rows of 64 keys, 0.05 (latent 512), 0.02 (256) or 0.007 (128), so that short contexts cancel
   // out and the number of rows decides.  Up to 512 keys a request that is longer than all others costs little here (140 decoding, one of them
   // at 510, latent 512 + 64, 8 heads, 33.3 31.2), and one CTA in twelve SMs is enough; latents below 128 and unequal halves, which gain less, take one
-  // in six.  One or two blocks of keys are one pass in that kernel.  Us, 16 heads, 512 + 64, that kernel and this one: 200 tokens 51.7 16.8, 150 37.4 14.9,
+  // in six.  One or two blocks of keys are one pass in that kernel while its CTAs, one to an SM above latents of 256, fit at once.  Us, 16 heads, 512 + 64, that kernel and this one: 200 tokens 51.7 16.8, 150 37.4 14.9,
   // 100 behind 400 keys 57.9 23.1, 80 decoding at 480 55.8 39.3; 8 heads, 500 tokens 92.7 23.0; latent 256 + 32, 16 heads, 200 tokens 27.0 14.8.
   const int keys = window > 0 && window + (long)tokens < max_kv_len ? window + tokens : max_kv_len;
-  const bool few_keys = keys > (rank > 256 ? 1 : 2) * LT_KEYS && keys <= 8 * LT_KEYS;
+  const bool few_keys = keys <= 8 * LT_KEYS && (keys > 2 * LT_KEYS || (keys > LT_KEYS && rank > 256 && rows > 16l * sm_count()));
   if (tiles * halves < sm_count() / (!few_keys ? 2 : rank < 128 || v0 != v1 ? 6 : 12)) return -2;
   EncodeTiledFn fn = encode_fn();
   if (!fn) return -2;
