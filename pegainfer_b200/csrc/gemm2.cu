@@ -168,7 +168,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
       const int tok = mb * 2 * G2_BM + (int)rank * G2_BM + q * 32 + lane;
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * TN);
       // 32 columns of the warp's 32 rows, four lanes 64 bytes of a row at a time: a lane that stored its own row would touch a line per 16 bytes, and a tile of
-      // 256 columns would take 4100 clocks to leave -- the last one of a launch, or the only one, with nothing beside it
+      // 256 columns would take 4100 clocks to leave -- the last one of a launch, or the only one, with nothing beside it (2560 x 4096, 2048 tokens: 33.8 -> 31.6 us,
+      // 12288 x 2560, 200 tokens 23.3 -> 18.6)
       auto store_rows = [&](bf16* base, int ld, const float* r) {
         uint32_t u[16];
 #pragma unroll
@@ -286,6 +287,7 @@ cudaError_t g2_launch(const CUtensorMap& mx, const CUtensorMap& mw, const G2Args
 //   2560 x 9728, 3001      111.2   105.2   129.8   112.4   124.0
 //   9728 x 2560,  400       57.9            53.9            53.5    (gated)
 //   4096 x 12288, 4096     305.2   378.3   332.9   336.4   331.9
+// (A launch has since become 1 to 3 us shorter at every width: how the results leave, see store_rows.)
 // Beyond three waves of 256 the last one matters less than what narrower tiles read more often, and 256 columns stand.
 // In the units of gemm.cu's model: a pair tile of 256 tokens on sms/2 pairs costs what a 128-token tile of the same width costs on sms single CTAs.
 // Returns the index into g2_widths, or -2 when the single-CTA kernel of gemm.cu should take the shape.

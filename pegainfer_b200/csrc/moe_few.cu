@@ -179,14 +179,12 @@ __global__ void __launch_bounds__(kMfThreads, 1) moe_few_kernel(const MfArgs a) 
     // Behind a run-out no barrier says when the copies under way have landed: two milliseconds, where a copy takes a thousandth of that
     if (!go)
       for (int i = 0; i < 2000; ++i) __nanosleep(1000);
-    asm volatile("bar.arrive 15, %0;" ::"n"(kMfThreads) : "memory");
-    return;
   }
   const int group = warp >> 2, wg = warp & 3, g = lane >> 2, tq = lane & 3;
   auto bar = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); };
   auto bar_all = [] { asm volatile("bar.sync 14, %0;" ::"n"(32 * kMfWarps) : "memory"); };
   int used = 0;  // stages of this group
-  for (int blk = blk0; blk < blk_end; blk += gridDim.x) {
+  for (int blk = warp < kMfWarps ? blk0 : blk_end; blk < blk_end; blk += gridDim.x) {
     for (int first = 0; first < n_units; first += kMfGroups) {
       const int live = min(kMfGroups, n_units - first);
       if (group < live) {
@@ -297,7 +295,7 @@ __global__ void __launch_bounds__(kMfThreads, 1) moe_few_kernel(const MfArgs a) 
       bar_all();  // (before the next rows' first)
     }
   }
-  asm volatile("bar.sync 15, %0;" ::"n"(kMfThreads) : "memory");  // every role is through with its waits
+  __syncthreads();  // every role is through with its waits
   if (tid == 0) count_run_out(dead, a.err);
 }
 
