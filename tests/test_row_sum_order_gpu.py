@@ -77,3 +77,38 @@ def test_qk_norm_on_eight_byte_boundaries(lib, offset):
                                              nkv, 128, tokens, EPS, None)
     torch.cuda.synchronize()
     assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+
+
+def norm_sum(sq, few):
+    """of rows [n, dim] of squares.  A row by itself: chains of eight elements, by exchange within 32 of them, then so between the warps; many rows: lane l
+    takes its pieces l, l + 32, .. one after the other, then by exchange"""
+    pieces = sq.unflatten(-1, (-1, 8))
+    if few:
+        s = torch.nn.functional.pad(chain(pieces), (0, 1024 - pieces.shape[-2])).unflatten(-1, (32, 32))
+        return halves(halves(s))
+    pieces = torch.nn.functional.pad(pieces, (0, 0, 0, -pieces.shape[-2] % 32)).unflatten(-2, (-1, 32))
+    return halves(chain(pieces.transpose(-3, -2).flatten(-2)))
+
+
+@pytest.mark.parametrize("dim", [8, 1024, 1032, 2560, 2816, 4096])
+@pytest.mark.parametrize("rows", [295, 297, 2051])
+def test_norms(lib, dim, rows):
+    sms, width = torch.cuda.get_device_properties(0).multi_processor_count, torch.full((1,), float(dim), device="cuda")  # (by a number: times its reciprocal)
+    for seed in range(6 if rows < 300 else 1):  # (few sums fall where the order shows in bf16)
+        g = torch.Generator(device="cuda").manual_seed(dim + rows + 7 * seed)
+        x, r, w = rnd(g, rows, dim), rnd(g, rows, dim), rnd(g, dim)
+        out, one, hidden, added = (torch.full_like(x, float("nan")) for _ in range(4))
+        hidden.copy_(x)
+        lib.rms_norm_batched_cuda(x.data_ptr(), w.data_ptr(), out.data_ptr(), dim, rows, EPS, None)
+        lib.rms_norm_batched_offset_cuda(x.data_ptr(), w.data_ptr(), one.data_ptr(), dim, rows, EPS, None)
+        lib.fused_add_rms_norm_batched_cuda(hidden.data_ptr(), r.data_ptr(), w.data_ptr(), added.data_ptr(), dim, rows, EPS, None)
+        torch.cuda.synchronize()
+
+        def scaled(v, weight):
+            return (v * torch.rsqrt(norm_sum(v.square(), rows < 2 * sms) / width + EPS)[:, None] * weight).to(BF16)
+        assert torch.equal(out, scaled(x.to(F32), w.to(F32)))
+        assert torch.equal(one, scaled(x.to(F32), 1 + w.to(F32)))
+        h = x.to(F32) + r.to(F32)
+        assert torch.equal(hidden, h.to(BF16))
+        # (the squares of these sums round: against a fused multiply-add a chain of additions is off by a last bit, which bf16 seldom shows)
+        assert (added != scaled(h, w.to(F32))).float().mean() < 1e-4
