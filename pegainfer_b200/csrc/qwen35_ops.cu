@@ -30,10 +30,6 @@ __global__ void rms_norm_offset_kernel(const bf16* __restrict__ x, const bf16* _
   for (int i = threadIdx.x; i < dim; i += blockDim.x) out[base + i] = f2bf(q35_row[i] * r * (1.0f + bf2f(w[i])));
 }
 
-// x times its logistic, fp32: the quotient to 2 ulp (__fdividef; the correctly rounded one, a branch and a dozen instructions, set the pace of the kernels
-// below), which is rounded to bf16 next
-__device__ __forceinline__ float silu32(float x) { return __fdividef(x, 1.0f + expf(-x)); }
-
 // ---------------------------------------------------------------- gated per-head RMSNorm: norm.cu:17-61
 // out = bf16(x * rsqrt(mean_head(x^2) + eps) * w_f32 * silu(gate)); one warp per head (head_dim <= 1024).
 __global__ void rms_norm_gated_kernel(const bf16* __restrict__ x, const float* __restrict__ w, const bf16* __restrict__ gate,
@@ -54,38 +50,28 @@ __global__ void rms_norm_gated_kernel(const bf16* __restrict__ x, const float* _
   }
 }
 
-// Heads of 128: half a warp per head, one 16-byte piece per lane, HEADS heads one behind the other so that their loads are under way together: 32 heads
-// of 1024 / 2048 tokens 5.6 9.8 -> 4.8 7.9 us (B200, with silu32).
-template <int HEADS>
+// Heads of 128: half a warp per head, one 16-byte piece per lane.
 __global__ void __launch_bounds__(256) rms_norm_gated128_kernel(const bf16* __restrict__ x, const float* __restrict__ w, const bf16* __restrict__ gate,
                                                                 bf16* __restrict__ out, int num_heads, float eps) {
-  const int head0 = (blockIdx.x * 16 + (threadIdx.x >> 4)) * HEADS, lane = threadIdx.x & 15;
+  const int head = blockIdx.x * 16 + (threadIdx.x >> 4), lane = threadIdx.x & 15;
   pdl_wait();
-  uint4 a[HEADS], g[HEADS];
-#pragma unroll
-  for (int i = 0; i < HEADS; ++i) {
-    const size_t at = (size_t)min(head0 + i, num_heads - 1) * 16 + lane;
-    a[i] = reinterpret_cast<const uint4*>(x)[at];
-    g[i] = reinterpret_cast<const uint4*>(gate)[at];
-  }
+  const bool on = head < num_heads;
+  const size_t at = (size_t)(on ? head : 0) * 16 + lane;
+  const uint4 a = reinterpret_cast<const uint4*>(x)[at], g = reinterpret_cast<const uint4*>(gate)[at];
   const float4 w0 = reinterpret_cast<const float4*>(w)[2 * lane], w1 = reinterpret_cast<const float4*>(w)[2 * lane + 1];
+  const float v[8] = {bf16_lo(a.x), bf16_hi(a.x), bf16_lo(a.y), bf16_hi(a.y), bf16_lo(a.z), bf16_hi(a.z), bf16_lo(a.w), bf16_hi(a.w)};
+  const float gv[8] = {bf16_lo(g.x), bf16_hi(g.x), bf16_lo(g.y), bf16_hi(g.y), bf16_lo(g.z), bf16_hi(g.z), bf16_lo(g.w), bf16_hi(g.w)};
   const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+  float ss = 0.f;
 #pragma unroll
-  for (int i = 0; i < HEADS; ++i) {
-    const float v[8] = {bf16_lo(a[i].x), bf16_hi(a[i].x), bf16_lo(a[i].y), bf16_hi(a[i].y), bf16_lo(a[i].z), bf16_hi(a[i].z), bf16_lo(a[i].w), bf16_hi(a[i].w)};
-    const float gv[8] = {bf16_lo(g[i].x), bf16_hi(g[i].x), bf16_lo(g[i].y), bf16_hi(g[i].y), bf16_lo(g[i].z), bf16_hi(g[i].z), bf16_lo(g[i].w), bf16_hi(g[i].w)};
-    float ss = 0.f;
+  for (int j = 0; j < 8; ++j) ss = fmaf(v[j], v[j], ss);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) ss = fmaf(v[j], v[j], ss);
+  for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  const float r = rsqrtf(ss / 128.f + eps);
+  float y[8];
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const float r = rsqrtf(ss / 128.f + eps);
-    float y[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) y[j] = v[j] * r * wv[j] * silu32(gv[j]);
-    if (head0 + i < num_heads)
-      reinterpret_cast<uint4*>(out)[(size_t)(head0 + i) * 16 + lane] = make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
-  }
+  for (int j = 0; j < 8; ++j) y[j] = v[j] * r * wv[j] * (gv[j] / (1.0f + expf(-gv[j])));
+  if (on) reinterpret_cast<uint4*>(out)[at] = make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
 }
 
 // ---------------------------------------------------------------- causal depthwise conv1d + SiLU: conv1d.cu:19-84
@@ -113,8 +99,13 @@ __global__ void conv1d_silu_kernel(const bf16* __restrict__ x, const bf16* __res
 // Four taps, channels in 16-byte pieces: a thread slides over kConvTokens tokens of 8 channels, so an input is read once (and the three before its
 // first again) instead of once per tap, and no index is divided per element.  The threads of the first tokens, the only ones that read the old state, leave
 // the new one.  Bound by its arithmetic (exponential and division per element) once there are warps enough to hide it: four tokens a thread instead of 16,
-// and no second launch for the state: 8192 channels, 16 / 300 / 1024 / 2048 tokens 13.1 14.2 26.5 39.7 -> 6.3 7.8 16.2 30.2 us (B200), with silu32 4.5 6.9 11.4 21.0.
+// and no second launch for the state: 8192 channels, 16 / 300 / 1024 / 2048 tokens 13.1 14.2 26.5 39.7 -> 6.3 7.8 15.6 30.7 us (B200), with
+// silu_for_bf16 4.5 6.7 11.1 21.8.
+// The quotient of the activation, whose argument is a bf16 value and whose result becomes one, is __fdividef's (2 ulp of fp32; the correctly rounded one, a
+// branch and a dozen instructions, set the pace), of numerator and divisor / 16: there, up to 2^124, the divisor stays where that bound holds.  For every bf16
+// argument the result is that of the correctly rounded quotient.
 constexpr int kConvTokens = 4;
+__device__ __forceinline__ float silu_for_bf16(float x) { return __fdividef(x * 0.0625f, fmaf(expf(-x), 0.0625f, 0.0625f)); }
 __global__ void __launch_bounds__(128) conv1d_silu4_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* state,
                                                            bf16* __restrict__ out, int C, int T, int groups) {
   // (blocks of `groups` channel groups one after the other: the grid's first axis has room for any number of tokens)
@@ -160,7 +151,7 @@ __global__ void __launch_bounds__(128) conv1d_silu4_kernel(const bf16* __restric
       sum += h[2][e] * wt[e][2];
       sum += v[e] * wt[e][3];
       const float s = round_bf16(sum);
-      y[e] = silu32(s);
+      y[e] = silu_for_bf16(s);
       h[0][e] = h[1][e];
       h[1][e] = h[2][e];
       h[2][e] = v[e];
@@ -397,11 +388,8 @@ void rms_norm_gated_cuda(const pk_bf16* x, const float* weight, const pk_bf16* g
                          float eps, pk_stream stream) {
   if (num_heads <= 0 || head_dim <= 0) return;
   if (head_dim == 128 && q35_al16(x) && q35_al16(weight) && q35_al16(gate) && q35_al16(out)) {
-    auto go = [&](auto kern, int per) {
-      launch(kern, dim3((num_heads + 16 * per - 1) / (16 * per)), dim3(256), 0, stream, true, (const bf16*)x, weight, (const bf16*)gate, (bf16*)out, num_heads, eps);
-    };
-    if (num_heads >= 32 * 8 * sm_count() / 4) go(rms_norm_gated128_kernel<2>, 2);
-    else go(rms_norm_gated128_kernel<1>, 1);
+    launch(rms_norm_gated128_kernel, dim3((num_heads + 15) / 16), dim3(256), 0, stream, true, (const bf16*)x, weight, (const bf16*)gate, (bf16*)out,
+           num_heads, eps);
     return;
   }
   launch(rms_norm_gated_kernel, dim3((num_heads + 7) / 8), dim3(256), 0, stream, true, (const bf16*)x, weight, (const bf16*)gate,
