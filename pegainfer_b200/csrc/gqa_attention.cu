@@ -883,11 +883,15 @@ static void launch_gqa_mma(const bf16* q, const bf16* cache, const bf16* sink, c
   }
   float* po = ts.work();
   float* pml = po ? po + (size_t)H * splits * T * D : nullptr;
-  // From 64 rows on: as many CTAs of a cluster (8 at most) to a (tile, head) as the GPU holds at once, while each has a few blocks of keys to walk (a context
-  // no longer than the step is a prompt from its start, whose rows see half of it); the exchange takes about 5 us.
-  int cs = 1;
-  if (T >= kAmRows)
-    while (cs < 8 && (long)H * tiles * cs * 2 <= 3 * sm_count() && (span <= 0 || (span > T ? span : span / 2) >= 4 * cs * kAmKeys)) cs *= 2;
+  // From 64 rows on: as many CTAs of a cluster to a (tile, head) as the GPU holds at once, where there are keys enough.  A share's start and the exchange cost
+  // 9 us with two CTAs (each finishes 32 rows), 7 with four or eight, a block of 64 keys 2.7, so eight pay from 4 blocks on, four from 5 and two from 16; counted
+  // are the longest context's, half of them where it is no longer than the step (a prompt from its start), none where the length is unknown.  B200, us, 1 / 2 /
+  // 4 / 8 CTAs, 16 heads of 128 in 4 groups: 64 rows behind 100 13.9 20.8 16.0 15.6, behind 200 19.2 23.8 19.0 16.1, behind 700 37.9 32.7 22.0 19.8; 200
+  // behind 300 27.3 27.1 23.7 31.4; 400 behind 700 51.5 51.0 54.3 65.5; prompts of 512 / 1024 27.4 33.2 37.9 53.4 / 59.3 52.3 73.3 116; 3 of 333 32.4 44.4 58.6 103.
+  // (Of 390 steps of six shapes none is more than 2 % slower than without clusters, the mean 0.727 of it, the best choice each time 0.703.)
+  const int blocks = (span > T ? span : span / 2) / kAmKeys;
+  auto holds = [&](int n) { return (long)H * tiles * n <= 3 * sm_count(); };
+  const int cs = T < kAmRows ? 1 : blocks >= 4 && holds(8) ? 8 : blocks >= 5 && holds(4) ? 4 : blocks >= 16 && holds(2) ? 2 : 1;
   if (cs > 1) {
     static std::atomic<uint64_t> smem_set{0};  // per template instance
     if (allow_smem(smem_set, (const void*)gqa_attention_cluster_kernel<D, D>, smem) == cudaSuccess) {
