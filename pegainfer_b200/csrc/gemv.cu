@@ -732,26 +732,24 @@ static cudaError_t launch_gemv_t(GemvArgs a, cudaStream_t stream) {
 
 template <int NTOK>
 static cudaError_t launch_gemv_rows(GemvArgs a, cudaStream_t stream) {
-  constexpr size_t most = 224 * 1024;
+  constexpr size_t most = 224 * 1024;  // (activations take 96 KB of it at most)
   const size_t x_bytes = (size_t)NTOK * a.K * 2, fixed = kRw * kRwStages * sizeof(uint64_t) + (16 + NTOK * kRwOwn) * sizeof(float);
   const bool glu = a.epi == 1 || a.epi >= 4;
   const int units = glu ? a.M : (a.M + 1) / 2, grid = units < sm_count() ? units : sm_count(), mine = (units + grid - 1) / grid;
-  size_t sums = 0;
-  auto plan = [&](int kc) {  // stages that fit
-    const int chunks = (a.K + kc - 1) / kc, fit = kRwSums / (2 * chunks);
-    a.kc = kc;
-    a.block_rows = mine < fit ? mine : fit > 0 ? fit : 1;
-    a.part_ld = a.block_rows * 2 * chunks;
-    sums = (size_t)NTOK * a.part_ld * sizeof(float);
-    const size_t used = x_bytes + fixed + sums;
-    const size_t n = used < most ? (most - used) / ((size_t)kRw * 4 * kc) : 0;
-    return (int)(n > kRwStages ? kRwStages : n);
-  };
-  // long chunks (fewer waits and sums) while three of them are under way
-  a.stages = plan(a.K >= 1024 ? 1024 : 512);
-  if (a.stages < 3) a.stages = plan(512);
-  if (a.stages < 2) a.stages = plan(256);
-  if (a.stages < 1 || ((a.epi == 2 || a.epi == 3) && 2 * mine > kRwOwn)) return cudaErrorInvalidValue;
+  if ((a.epi == 2 || a.epi == 3) && 2 * mine > kRwOwn) return cudaErrorInvalidValue;
+  // Long chunks (fewer waits and sums) while three of them can be under way beside the sums of a row pair per warp.  By K and the tokens alone: where a row is cut
+  // decides its bits, which are the same in stacked and single calls, gated or not.
+  const size_t left = most - x_bytes - fixed;
+  auto stage_bytes = [](int kc) { return (size_t)kRw * 4 * kc; };
+  auto pair_bytes = [&](int kc) { return (size_t)NTOK * 2 * ((a.K + kc - 1) / kc) * sizeof(float); };
+  a.kc = a.K >= 1024 && left >= 3 * stage_bytes(1024) + kRw * pair_bytes(1024) ? 1024 : 512;
+  // pairs to a block: all, or equal blocks of what three stages leave and kRwSums holds
+  const size_t per = pair_bytes(a.kc), room = left - 3 * stage_bytes(a.kc), most_sums = (size_t)NTOK * kRwSums * sizeof(float);
+  const int fit = (int)((room < most_sums ? room : most_sums) / per), blocks = (mine + fit - 1) / fit;
+  a.block_rows = (mine + blocks - 1) / blocks;
+  a.part_ld = (int)(a.block_rows * per / (NTOK * sizeof(float)));
+  const size_t sums = a.block_rows * per, stages = (left - sums) / stage_bytes(a.kc);
+  a.stages = stages < kRwStages ? (int)stages : kRwStages;
   const size_t smem = (size_t)kRw * a.stages * 4 * a.kc + x_bytes + fixed + sums;
   static std::atomic<uint64_t> smem_set{0};
   if (const cudaError_t e = allow_smem(smem_set, (const void*)gemv_rows_kernel<NTOK>, most); e != cudaSuccess) return e;
