@@ -257,8 +257,9 @@ typedef struct {
 } pk_b200_gemv_args;
 int pk_b200_gemv_fused(const pk_b200_gemv_args* args, pk_stream stream);
 /* Ring depth (2..12 stages of 8 row segments), CTAs per SM and K elements per row segment (multiple of
- * 256) of the streaming GEMV; 0 keeps a value.  Defaults: PK_GEMV_STAGES / PK_GEMV_CTAS_PER_SM /
- * PK_GEMV_KC or the built-in tuning. */
+ * 256) of the streaming GEMV, which takes one token, and 2 to 4 with x_mode 2; 0 keeps a value.  Defaults:
+ * PK_GEMV_STAGES / PK_GEMV_CTAS_PER_SM / PK_GEMV_KC or the built-in tuning.  The kernel of 2 to 4 tokens
+ * derives its own. */
 void pk_b200_set_gemv_tuning(int stages, int ctas_per_sm, int segment_elems);
 
 /* QK-norm + RoPE + KV append + split-KV GQA decode attention + merge in ONE launch.
@@ -299,7 +300,7 @@ int pk_b200_fa2_trace_copy(void* host_out, int bytes);
  * bs-1 decode attention is latency-bound (a few MB of K/V against ~10 us of dependent steps) and leaves HBM
  * idle; extra clusters of the same launch use that window to pull weight rows into the 126 MB L2
  * (cp.async.bulk.prefetch.L2), after the previous kernel has drained.  A span describes one row-major weight
- * block and how the GEMV that will read it cuts it: `slices` = that GEMV's grid (pk_b200_gemv_grid), and the
+ * block and how the GEMV that will read it cuts it: `slices` = that GEMV's grid (pk_b200_gemv_slices), and the
  * first `prefetch_rows` rows of every slice are requested so all of its CTAs gain equally.  Results are
  * identical with or without spans.  At most 4 spans; row_bytes % 16 == 0, base 16-byte aligned (else -1). */
 typedef struct pk_b200_prefetch_span {
@@ -318,8 +319,10 @@ int pk_b200_decode_attention_fused_prefetch(
     int chunk_tokens, int max_chunks, int num_qo_heads, int num_kv_heads, int head_dim,
     int page_size, int batch_size, int64_t stride_page, float sm_scale,
     const pk_b200_prefetch_span* spans, int num_spans, pk_stream stream);
-/* Grid (row slices) pk_b200_gemv_fused / gemm_cuda(N <= 4) uses for M output rows with epilogue `epi`. */
+/* Grid (row slices) of the streaming GEMV for M output rows with epilogue `epi`: of a call of one token, and of 2 to 4 with x_mode 2. */
 int pk_b200_gemv_grid(int M, int epi);
+/* The same for any call of pk_b200_gemv_fused / gemm_cuda with N <= 4 tokens: its CTAs own equal runs of rows (of row pairs, N >= 2). */
+int pk_b200_gemv_slices(int M, int N, int x_mode, int epi);
 
 /* ---- Qwen3.5 hybrid-layer ops (next scope row; ffi.rs:181-226,981-1039) --------
  * Pieces of the gated-delta-net / gated HD-256 attention layers behind the reference's names

@@ -730,12 +730,18 @@ static cudaError_t launch_gemv_t(GemvArgs a, cudaStream_t stream) {
   return launch(kern, dim3(grid), dim3(kConsumerThreads + 32), smem, stream, true, a);
 }
 
+// CTA count of gemv_rows_kernel: a row pair each at least, one CTA per SM at most
+static int gemv_rows_grid(int M, int epi) {
+  const int units = epi == 1 || epi >= 4 ? M : (M + 1) / 2;
+  return units < sm_count() ? units : sm_count();
+}
+
 template <int NTOK>
 static cudaError_t launch_gemv_rows(GemvArgs a, cudaStream_t stream) {
   constexpr size_t most = 224 * 1024;  // (activations take 96 KB of it at most)
   const size_t x_bytes = (size_t)NTOK * a.K * 2, fixed = kRw * kRwStages * sizeof(uint64_t) + (16 + NTOK * kRwOwn) * sizeof(float);
   const bool glu = a.epi == 1 || a.epi >= 4;
-  const int units = glu ? a.M : (a.M + 1) / 2, grid = units < sm_count() ? units : sm_count(), mine = (units + grid - 1) / grid;
+  const int grid = gemv_rows_grid(a.M, a.epi), mine = ((glu ? a.M : (a.M + 1) / 2) + grid - 1) / grid;
   if ((a.epi == 2 || a.epi == 3) && 2 * mine > kRwOwn) return cudaErrorInvalidValue;
   // Long chunks (fewer waits and sums) while three of them can be under way beside the sums of a row pair per warp.  By K and the tokens alone: where a row is cut
   // decides its bits, which are the same in stacked and single calls, gated or not.
@@ -809,9 +815,14 @@ void gemm_graphsafe_cuda(const pk_bf16* W, const pk_bf16* X, pk_bf16* Y, int M, 
   launch_gemv(a, N, stream);
 }
 
-// ring depth (2..12 stages), CTAs per SM and K elements per row segment of the streaming GEMV; 0 keeps a value
 int pk_b200_gemv_grid(int M, int epi) { return M > 0 ? pk::gemv_grid(M, epi) : 0; }
 
+int pk_b200_gemv_slices(int M, int N, int x_mode, int epi) {
+  if (M <= 0 || N < 1 || N > 4) return 0;
+  return N == 1 || x_mode == 2 ? pk::gemv_grid(M, epi) : pk::gemv_rows_grid(M, epi);
+}
+
+// ring depth (2..12 stages), CTAs per SM and K elements per row segment of the streaming GEMV; 0 keeps a value
 void pk_b200_set_gemv_tuning(int stages, int ctas_per_sm, int segment_elems) {
   pk::gemv_set_tuning(stages, ctas_per_sm, segment_elems);
 }

@@ -34,7 +34,7 @@ std::string KernelLib::load(const std::string& p) {
   PQ_OPT(pk_b200_launch_count) PQ_OPT(pk_b200_wait_errors_seen) PQ_OPT(pk_b200_set_pdl) PQ_OPT(pk_b200_gemv_fused) PQ_OPT(pk_b200_gemm_segments)
   PQ_OPT(pk_b200_decode_attention_fused) PQ_OPT(pk_tp_all_reduce_rows)
   PQ_OPT(pk_tp_all_reduce_add_rms_norm) PQ_OPT(pk_tp_max_rows)
-  PQ_OPT(pk_b200_decode_attention_fused_prefetch) PQ_OPT(pk_b200_gemv_grid) PQ_OPT(pk_tp_top1_exchange) PQ_OPT(pk_b200_gemm_swiglu)
+  PQ_OPT(pk_b200_decode_attention_fused_prefetch) PQ_OPT(pk_b200_gemv_slices) PQ_OPT(pk_tp_top1_exchange) PQ_OPT(pk_b200_gemm_swiglu)
 #undef PQ_REQ
 #undef PQ_OPT
   if (!missing.empty()) return "kernel library " + p + " lacks:" + missing;
@@ -857,9 +857,8 @@ bool Qwen3Model::decode_kernels_fused(int bs) {
   // slice to request (0 disables), defaults tuned on B200 (profiles/README.md).
   static const int pf_o_rows = [] { const char* e = getenv("PK_PF_O"); return e ? atoi(e) : 0; }();
   static const int pf_gu_rows = [] { const char* e = getenv("PK_PF_GU"); return e ? atoi(e) : 0; }();
-  const bool can_prefetch = k.pk_b200_decode_attention_fused_prefetch && k.pk_b200_gemv_grid && (pf_o_rows > 0 || pf_gu_rows > 0);
-  const int o_slices = can_prefetch ? k.pk_b200_gemv_grid(H, 0) : 1;
-  const int gu_slices = can_prefetch ? k.pk_b200_gemv_grid(I, 1) : 1;
+  const bool can_prefetch = k.pk_b200_decode_attention_fused_prefetch && k.pk_b200_gemv_slices && (pf_o_rows > 0 || pf_gu_rows > 0);
+  int o_slices = 1, gu_slices = 1;  // how the two GEMVs of this step cut their rows
   auto attention = [&](TransformerBlock& L, int64_t k_off, int64_t v_off) -> bool {
     if (!can_prefetch) {
       if (k.pk_b200_decode_attention_fused(
@@ -911,6 +910,10 @@ bool Qwen3Model::decode_kernels_fused(int bs) {
   const bool tp_fuse = tp_on && tp_mode_env >= 1;
   const int red_mode = (tp_on && !tp_ll) ? 2 : 1;
   const int push_epi = tp_on ? (tp_ll ? 3 : 2) : 0;
+  if (can_prefetch) {
+    o_slices = k.pk_b200_gemv_slices(H, bs, 0, push_epi);
+    gu_slices = k.pk_b200_gemv_slices(I, bs, tp_fuse ? red_mode : 0, 1);
+  }
   const pk_bf16* prev_residual = zero_residual.bf();  // layer 0: hidden + 0
   if (tp_on && !tp_fuse) {
     k.rms_norm_batched_cuda(Ha, layers[0].input_layernorm.data.bf(), normed.data.bf(), H, bs, eps, st);

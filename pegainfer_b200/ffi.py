@@ -93,6 +93,7 @@ EXT_SIGNATURES = {
     "pk_b200_decode_attention_fused_prefetch": (i32, [vp, vp, vp, vp, vp, i64, i64] + [vp] * 8 + [f32, vp, vp] + [i32] * 7
                                                 + [i64, f32, C.POINTER(PrefetchSpan), i32, vp]),
     "pk_b200_gemv_grid": (i32, [i32, i32]),
+    "pk_b200_gemv_slices": (i32, [i32, i32, i32, i32]),
     "pk_b200_prefill_attention_tc": (i32, [vp, vp, vp, i64, i64, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i64, f32, vp]),
     "pk_b200_fa2_trace_copy": (i32, [vp, i32]),
     "pk_b200_gemm_plan": (i32, [i32, i32, i32, i32, i32]),
