@@ -50,7 +50,7 @@ struct GemvArgs {
 };
 
 // 8 bf16 x bf16 products onto `acc`, as two interleaved 4-long FMA chains (ILP: the consumer loop is
-// latency-bound on dependent FMAs otherwise -- profiles/r1_gemv_v1.md)
+// latency-bound on dependent FMAs otherwise)
 __device__ __forceinline__ float dot8(const uint4& w, const uint4& x, float acc) {
   float a = fmaf(bf16_lo(w.x), bf16_lo(x.x), acc);
   float b = bf16_hi(w.x) * bf16_hi(x.x);
@@ -172,6 +172,7 @@ gemv_stream_kernel(const GemvArgs a) {
   const int G = gridDim.x;
   const int M = a.M, K = a.K;
   const bool glu = a.epi == 1 || a.epi >= 4;  // interleaved gate / up row groups
+  const int x_mode = NTOK == 1 ? a.x_mode : 2;  // (the others of 2 to 4 tokens: gemv_rows_kernel)
   const int rows_per_group = glu ? kCW / 2 : kCW;
   const int r0 = (int)(((int64_t)blockIdx.x * M) / G);
   const int r1 = (int)(((int64_t)(blockIdx.x + 1) * M) / G);
@@ -226,7 +227,7 @@ gemv_stream_kernel(const GemvArgs a) {
   pdl_wait();  // activations come from the previous kernel
   {
     const int tid = threadIdx.x;  // 0..255
-    if (a.x_mode == 0) {
+    if (x_mode == 0) {
       const int nv = (NTOK * K) >> 3;
       for (int i = tid; i < nv; i += kConsumerThreads)
         reinterpret_cast<uint4*>(xs)[i] = reinterpret_cast<const uint4*>(a.X)[i];
@@ -239,7 +240,7 @@ gemv_stream_kernel(const GemvArgs a) {
       constexpr int kMaxVec = 5;  // K <= 5 * 256 * 8 = 10240
       const int nv = K >> 3;
       const uint8_t* stage_base = nullptr;
-      if (a.x_mode == 2) {
+      if (x_mode == 2) {
         uint32_t* my_flags = a.tp.flags[a.tp.rank];
         const uint32_t seq = *reinterpret_cast<volatile uint32_t*>(my_flags + 2 * kTpMaxCtas * kTpMaxWorld);
         const int slot = (int)(seq & 1u);
@@ -261,7 +262,7 @@ gemv_stream_kernel(const GemvArgs a) {
           if (i < nv) {
             const uint4 h = h4[i];
             uint4 r;
-            if (a.x_mode == 2) {
+            if (x_mode == 2) {
               float acc8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
               for (int rk = 0; rk < a.tp.world; ++rk) {
                 const uint4 pv = __ldcg(reinterpret_cast<const uint4*>(stage_base + (size_t)rk * a.tp.slot_bytes +
@@ -278,7 +279,7 @@ gemv_stream_kernel(const GemvArgs a) {
             v[j][2] = bf16_lo(h.y) + bf16_lo(r.y); v[j][3] = bf16_hi(h.y) + bf16_hi(r.y);
             v[j][4] = bf16_lo(h.z) + bf16_lo(r.z); v[j][5] = bf16_hi(h.z) + bf16_hi(r.z);
             v[j][6] = bf16_lo(h.w) + bf16_lo(r.w); v[j][7] = bf16_hi(h.w) + bf16_hi(r.w);
-            if (a.x_mode == 3) {  // Qwen3.5: the residual sum is ROUNDED to bf16 before the norm (add_batch then norm)
+            if (x_mode == 3) {  // Qwen3.5: the residual sum is ROUNDED to bf16 before the norm (add_batch then norm)
 #pragma unroll
               for (int e = 0; e < 8; ++e) v[j][e] = round_bf16(v[j][e]);
             }
@@ -300,7 +301,7 @@ gemv_stream_kernel(const GemvArgs a) {
           const int i = tid + j * kConsumerThreads;
           if (i < nv) {
             const uint4 g = g4[i];
-            const float wo = a.x_mode == 3 ? 1.0f : 0.0f;  // (1 + w) RMSNorm of Qwen3.5 (flashinfer_norm.cu:108-133)
+            const float wo = x_mode == 3 ? 1.0f : 0.0f;  // (1 + w) RMSNorm of Qwen3.5 (flashinfer_norm.cu:108-133)
             uint4 o;
             o.x = pack_bf16(v[j][0] * rinv * (wo + bf16_lo(g.x)), v[j][1] * rinv * (wo + bf16_hi(g.x)));
             o.y = pack_bf16(v[j][2] * rinv * (wo + bf16_lo(g.y)), v[j][3] * rinv * (wo + bf16_hi(g.y)));
@@ -670,7 +671,7 @@ static int g_gemv_stages = 0, g_gemv_ctas_per_sm = 0, g_gemv_kc = 0;
 static void gemv_tuning() {
   if (g_gemv_stages == 0) {
     const char* s = getenv("PK_GEMV_STAGES");
-    g_gemv_stages = s ? atoi(s) : 6;  // 4 -> 6: -0.05 ms per Qwen3-4B decode step on B200 (profiles/README.md r2)
+    g_gemv_stages = s ? atoi(s) : 6;  // 4 -> 6: -0.05 ms per Qwen3-4B decode step on B200
     if (g_gemv_stages < 2) g_gemv_stages = 2;
     if (g_gemv_stages > kMaxStages) g_gemv_stages = kMaxStages;
     const char* c = getenv("PK_GEMV_CTAS_PER_SM");
