@@ -1,4 +1,4 @@
-// The two products of moe.cu for a few tokens, bf16: a chosen expert's weight rows are read once for all tokens that chose it, and on the tensor cores.
+// The two products of moe.cu for a few tokens, bf16: a chosen expert's weight rows are read once for up to 16 tokens that chose it, and on the tensor cores.
 //   up    hid[t, k, f] = act(W_up[ids[t, k]] x_t)             down  y[t] = sum_k wts[t, k] W_down[ids[t, k]] hid[t, k] (+ shared expert)
 // The (token, choice) pairs are listed by expert, in entries of at most 16 pairs (every CTA lists them for itself: some hundred ids).  A CTA streams units
 // of up to 16 weight rows of an entry's expert by bulk copies through rings in shared memory, one ring to a group of four warps that share the elements of a
@@ -6,10 +6,12 @@
 // tile would be 1/8 full, and the products are a twentieth of the time that the weights take.)
 //   up    the units of all entries, one behind the other, in equal runs for the CTAs
 //   down  each CTA has the same <= 16 rows of every entry: it holds all of a token's choices, and adds them in the order of k
-// Bound by HBM: the bytes of the distinct experts.  A pair's sums do not depend on the other pairs.
+// Bound by HBM: the bytes of the distinct experts, once per 16 pairs of one (entries are numbered by their first pair: a crowded expert's rows may
+// have left L2 when its next entry asks for them).  A pair's sums do not depend on the other pairs.
 // Both products, us, 64 experts of 2048 x 1408, top 6, relu^2, 1 / 3 / 8 / 16 / 31 tokens (B200; floor 11 29 61 89 107): 44 79 126 228 413 with the warp-per-row
 // kernels of moe.cu, which read an expert's rows once per pair, 24 46 85 117 145 here; gated 54 89 179 314 581 -> 30 63 115 168 200; 16 experts of
-// 1024 x 768, top 2, 1 / 8 / 31 tokens 14 23 46 -> 14 20 28.  On the way there: the copies of a stage by one warp 41 (1 token) and 296 (16), by eight 29 and 181
+// 1024 x 768, top 2, 1 / 8 / 31 tokens 14 23 46 -> 14 20 28.  8 / 16 / 24 / 31 tokens of which every second chooses the same six experts 126 224 323 408 -> 68 121
+// 151 186, of which all do 119 220 320 403 -> 28 43 59 64.  On the way there: the copies of a stage by one warp 41 (1 token) and 296 (16), by eight 29 and 181
 // (a warp's copies are issued one after the other), the pairs' rows out of L2 instead of through the ring 24 and 117 (half the copies, chunks twice as long).
 #include "common.cuh"
 #include "mma.cuh"
@@ -18,7 +20,7 @@ namespace pk {
 
 constexpr int kMfGroups = 3, kMfWarps = 4 * kMfGroups, kMfLoads = 4, kMfThreads = 32 * (kMfWarps + kMfLoads), kMfRows = 16, kMfSlots = 16, kMfKc = 1024, kMfStages = 6, kMfOwn = kMfStages / kMfGroups;  // stages: a ring of its own for each group
 constexpr int kMfStage = kMfRows * kMfKc * 2;             // a chunk of up to kMfKc elements of a unit's rows
-constexpr int kMfPairs = 192;                             // pairs of a call at most
+constexpr int kMfPairs = 192;                             // pairs of a call at most: 31 tokens of 6 choices (a thread each, and 64 bytes of sums; 256 would fit)
 
 static_assert(kMfPairs <= kMfThreads, "a thread per pair");
 
