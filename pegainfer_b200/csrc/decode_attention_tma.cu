@@ -51,6 +51,7 @@ struct TmaAttnArgs {
   const bf16 *qw, *kw, *cosc, *sinc;
   float eps, sm_scale_log2;
   int nq, nkv, nslot;
+  unsigned int* err;  // wait_err_word()
 };
 
 __device__ __forceinline__ uint32_t t_cluster_rank() {
@@ -96,10 +97,6 @@ __device__ __forceinline__ void t_tma_4d(uint32_t dst, const CUtensorMap* map, i
       "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
       : "memory");
 }
-__device__ __forceinline__ void t_wait_or_trap(uint64_t* bar, uint32_t parity) {  // a hung barrier becomes a trap
-  for (uint32_t spins = 0; !mbar_try_wait(bar, parity); ++spins)
-    if (spins > (1u << 26)) __trap();
-}
 // norm + rotation of one head, result to shared memory
 __device__ __forceinline__ void t_norm_rope(const bf16* __restrict__ src, const bf16* __restrict__ w, const bf16* __restrict__ cosc, const bf16* __restrict__ sinc,
                                             int pos, float eps, bf16* dst, int lane) {
@@ -133,8 +130,11 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   const int rank = (int)t_cluster_rank(), cs = (int)t_cluster_size();
   const bool plain = a.k_new == nullptr;
   const int kvh = blockIdx.y;
+  __shared__ int dead_word;
+  volatile int* dead = &dead_word;  // a wait of this CTA has run out
 
   if (threadIdx.x == 0) {
+    *dead = 0;
     for (int s = 0; s < nslot; ++s) mbar_init(full + s, 1);
     // one arrival per (head this CTA leads, source CTA, source warp of the 4 that carry that head's 128 dims)
     const int heads_led = rank < T_GROUP ? (T_GROUP - rank + cs - 1) / cs : 0;
@@ -212,12 +212,14 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   const int k_tok = ((lm_i >> 1) << 3) + lm_r, k_c = lm_i & 1;   // K: matrices {tok 0-7 lo, tok 0-7 hi, tok 8-15 lo, tok 8-15 hi}
   const int v_tok = ((lm_i & 1) << 3) + lm_r, v_c = lm_i >> 1;   // V: {tok 0-7 | tok 8-15} x {dims 8d | 8(d+1)}
 
+  WaitTries tries;
+  bool go = true;  // false behind a run-out: a barrier must not be armed twice in one phase
   // a slot is consumed by ONE warp (slot & 7), in page order: walk the ring passes, then this warp's slots
   for (int base = 0, pass = 0; base < my_pages; base += nslot, ++pass)
   for (int slot = warp; slot < nslot; slot += T_WARPS) {
     const int lp = base + slot;
     if (lp >= my_pages) break;
-    t_wait_or_trap(full + slot, (uint32_t)(pass & 1));
+    go &= mbar_wait_bounded(full + slot, (uint32_t)(pass & 1), dead, tries);
     uint8_t* tile = tiles + (size_t)slot * T_SLOT;
     const int gp = p_lo + lp;
     if (lp == pos_lp) {  // patch the step's own row into the tile (the TMA saw the slot before it was written)
@@ -291,7 +293,7 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     // refill: this warp is the only reader of the slot -> request the page that reuses it
     if (lp + nslot < my_pages) {
       __syncwarp();
-      if (lane == 0) {
+      if (lane == 0 && go) {
         fence_proxy_async_smem();
         issue_page(lp + nslot);
       }
@@ -301,6 +303,7 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
 
   // ---- per-warp states -> shared memory (aliases the page ring: every warp must be done with its tiles) ----
+  if (!go) wait_for_copies();
   __syncthreads();
   if (g < T_GROUP) {
     if (tq == 0) {
@@ -347,11 +350,17 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
       if (lane == 0) t_mbar_arrive_remote(t_map_rank(smem_u32(merged), leader));
     }
   }
-  // Only the head leaders wait (their shared memory is the landing zone); every other CTA is done.
-  if (rank >= T_GROUP || rank >= cs) return;
-  for (uint32_t spins = 0; !t_mbar_try_wait_cluster(merged, 0); ++spins)
-    if (spins > (1u << 26)) __trap();
-  if (threadIdx.x >= T_HD) return;
+  // Only the head leaders wait (their shared memory is the landing zone), longer than any CTA of the cluster can be held by waits of its own: their states come in
+  // any case, and none may land behind this CTA's end.  Every other CTA is done.
+  const bool leads = rank < T_GROUP && rank < cs;
+  if (leads)
+    for (uint32_t spins = 0; !t_mbar_try_wait_cluster(merged, 0); ++spins)
+      if (spins > 8u * kWaitSpins) {
+        *dead = 1;  // (thread 0's own wait here; those for pages lie before the barriers above)
+        break;
+      }
+  if (threadIdx.x == 0) count_run_out(dead, a.err);
+  if (!leads || threadIdx.x >= T_HD) return;
   for (int h = rank; h < T_GROUP; h += cs) {  // this CTA leads heads rank, rank + cs, ...
     const int e0 = (h / cs) * cs;
     float mx = -INFINITY;
@@ -453,6 +462,7 @@ int launch_decode_attention_tma(const ClusterAttnArgs& c, int nkv, int bs, cudaS
   a.qw = c.qw; a.kw = c.kw; a.cosc = c.cosc; a.sinc = c.sinc;
   a.eps = c.eps; a.sm_scale_log2 = c.sm_scale_log2;
   a.nq = c.nq; a.nkv = c.nkv; a.nslot = cfg.nslot;
+  a.err = wait_err_word();
   // cluster size: as many CTAs per (request, kv head) as keeps the grid within ~one wave of the SMs
   int cs = cfg.max_cluster;
   while (cs > 1 && (int64_t)cs * nkv * bs > (int64_t)sm_count() + sm_count() / 8) cs >>= 1;

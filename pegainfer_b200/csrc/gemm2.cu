@@ -24,7 +24,7 @@
 // 6144 x 2560 59.5 -> 48.4, 2560 x 4096 45.6 -> 37.5, 2560 x 9728 88.8 -> 74.3, 4096 x 12288 160.6 -> 144.1.
 // The gated epilogue evaluates its 32 columns side by side, on two warps per lane quarter; one after the other (a branch on the activation per
 // element) a tile's epilogue took 26 us and set the pace: 9728 x 2560 gated 253 -> 154, 12288 x 4096 gated (3001 tokens) 557 -> 433.
-// Every barrier wait is bounded (trap instead of hang).
+// Every barrier wait is bounded (mbar_wait_bounded, common.cuh).
 #include <cuda.h>
 
 #include <cstdlib>
@@ -42,16 +42,13 @@ constexpr int G2_BK = 64;        // K elements per stage (one 128-byte swizzle s
 constexpr int G2_EPI = 8;        // epilogue warps: two for each quarter of the TMEM lanes, taking turns at blocks of 32 columns
 constexpr int G2_THREADS = 64 + 32 * G2_EPI;  // warp 0 TMA, warp 1 MMA, then the epilogue
 
-__device__ __forceinline__ void g2_wait(uint64_t* bar, uint32_t parity) {
-  for (uint32_t spins = 0; !mbar_try_wait(bar, parity); ++spins)
-    if (spins > (1u << 26)) __trap();
-}
 struct G2Args {
   bf16 *Y, *Y1, *Y2;
   int e0, e1;     // output segments (the fused q|k|v projection): features [0,e0) -> Y, [e0,e1) -> Y1, rest -> Y2
   int M, N, K;    // features, tokens, reduction
   int swiglu;     // 1: W = [gate (M rows); up (M rows)], Y[tok][M] = silu(gate) * up; 2: relu(gate) * up; 3: gelu (tanh form) of gate * up
   int ldy;        // gated output: elements from one token's row to the next
+  unsigned int* err;  // wait_err_word()
 };
 
 // A pair tile is 256 tokens x (NSUB * BN) features: NSUB accumulators of BN columns side by side in TMEM, one
@@ -73,7 +70,10 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
   uint64_t* empty = full + STAGES;   // one per CTA (multicast commit)
   uint64_t* tfull = empty + STAGES;  // [2] one per CTA
   uint64_t* tempty = tfull + 2;      // [2] used in the leader (an arrival per epilogue warp of both CTAs)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+  uint64_t* done = tempty + 2;       // behind a run-out: the MMAs under way
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  static_assert((2 * STAGES + 5) * 8 + 8 <= 256, "room behind the stages");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -94,6 +94,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
       mbar_init(tfull + s, 1);
       mbar_init(tempty + s, 2 * G2_EPI);
     }
+    mbar_init(done, 1);
+    *dead = 0;
     mbar_fence_init();
   }
   if (warp == 1) g2_tmem_alloc(tmem_slot, TMEM_COLS);
@@ -109,14 +111,16 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
       int it = 0;
-      for (int tile = pair; tile < num_tiles; tile += num_pairs) {
+      bool go = true;
+      for (int tile = pair; tile < num_tiles && go; tile += num_pairs) {
         const int mb = tile % m_tiles, nb = tile / m_tiles;
         const int tok0 = mb * 2 * G2_BM + (int)rank * G2_BM;
         // this CTA's B rows: its half of the BN features, or (SwiGLU) the gate block (leader) / up block (peer)
         const int wrow0 = a.swiglu ? (int)rank * M + nb * HB : nb * TN + (int)rank * HB;
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
-          g2_wait(empty + s, (uint32_t)(((it / STAGES) & 1) ^ 1));
+          go = mbar_wait_bounded(empty + s, (uint32_t)(((it / STAGES) & 1) ^ 1), dead);
+          if (!go) break;
           const uint32_t fb = g2_map(smem_u32(full + s), 0);
           if (leader) mbar_expect_tx(full + s, 2 * STAGE_BYTES);
           uint8_t* st = smem + (size_t)s * STAGE_BYTES;
@@ -125,6 +129,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
           for (int j = 0; j < NSUB; ++j) g2_tma_2d(st + A_BYTES + j * B_SUB, &map_w, kb * G2_BK, wrow0 + j * BN, fb);
         }
       }
+      if (!go) wait_for_copies();  // (some complete on the leader's barriers)
     }
   } else if (warp == 1) {
     // by elect.sync, not by `lane == 0` (see the head of this file)
@@ -132,14 +137,17 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
       // instruction descriptor: D=f32 [4,6)=1, A=bf16 [7,10)=1, B=bf16 [10,13)=1, K-major both, N>>3 at [17,23), M>>4 at [24,29)
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
       int it = 0, lt = 0;
-      for (int tile = pair; tile < num_tiles; tile += num_pairs, ++lt) {
+      bool go = true;
+      for (int tile = pair; tile < num_tiles && go; tile += num_pairs, ++lt) {
         const int as = lt % NBUF;
-        g2_wait(tempty + as, (uint32_t)(((lt / NBUF) & 1) ^ 1));
+        go = mbar_wait_bounded(tempty + as, (uint32_t)(((lt / NBUF) & 1) ^ 1), dead);
+        if (!go) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(as * TN);
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
-          g2_wait(full + s, (uint32_t)((it / STAGES) & 1));
+          go = mbar_wait_bounded(full + s, (uint32_t)((it / STAGES) & 1), dead);
+          if (!go) break;
           tc_fence_after();
           const uint32_t a_addr = smem_u32(smem + (size_t)s * STAGE_BYTES);
           const uint64_t adesc = make_sw128_desc(a_addr);
@@ -153,6 +161,10 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         }
         g2_commit_both(tfull + as);
       }
+      if (!go) {
+        g2_commit_both(done);
+        mbar_drain(done, 0);
+      }
     }
   } else {
     const int q = warp & 3, c0 = (warp - 2) / 4 * 32;  // TMEM lane quarter this warp may access, its first column
@@ -163,7 +175,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     for (int tile = pair; tile < num_tiles; tile += num_pairs, ++lt) {
       const int mb = tile % m_tiles, nb = tile / m_tiles;
       const int as = lt % NBUF;
-      g2_wait(tfull + as, (uint32_t)((lt / NBUF) & 1));
+      mbar_wait_bounded(tfull + as, (uint32_t)((lt / NBUF) & 1), dead);
+      __syncwarp();
       tc_fence_after();
       const int tok = mb * 2 * G2_BM + (int)rank * G2_BM + q * 32 + lane;
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * TN);
@@ -248,8 +261,10 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
       if (lane == 0) g2_arrive_cluster(tempty_leader0 + (uint32_t)(as * 8));
     }
   }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0) count_run_out(dead, a.err);
   cluster_barrier();  // the peer's MMAs / loads may still target this CTA's shared memory and TMEM
   if (warp == 1) {
     tc_fence_after();
@@ -340,7 +355,7 @@ int launch_gemm_pair(const bf16* W, const bf16* X, bf16* Y, bf16* Y1, bf16* Y2, 
   if (K % 8 != 0 || (reinterpret_cast<uintptr_t>(W) & 15) != 0 || (reinterpret_cast<uintptr_t>(X) & 15) != 0) return -2;
   const int best = g2_plan(M, N, K, swiglu, sm_count());
   if (best < 0) return -2;
-  G2Args a{Y, Y1, Y2, e0, e1, M, N, K, swiglu, ldy};
+  G2Args a{Y, Y1, Y2, e0, e1, M, N, K, swiglu, ldy, wait_err_word()};
   CUtensorMap mx, mw;
   if (!make_rows_map(&mx, X, N, K, G2_BM)) return -2;
   const int rows_w = swiglu ? 2 * M : M;

@@ -51,6 +51,7 @@ struct PrefillTcArgs {
   const int* q_indptr;
   int seq_len, batch_size, nq, nkv;
   float sm_scale_log2;
+  unsigned int* err;  // wait_err_word()
 };
 
 __device__ __forceinline__ float tex2(float x) {
@@ -69,11 +70,6 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
       "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
       "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
       : "memory");
-}
-// A hung barrier becomes a trap (reported as a launch failure) instead of a wedged GPU.
-__device__ __forceinline__ void mbar_wait_or_trap(uint64_t* bar, uint32_t parity) {
-  for (uint32_t spins = 0; !mbar_try_wait(bar, parity); ++spins)
-    if (spins > (1u << 27)) __trap();
 }
 __device__ __forceinline__ void softmax_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 // byte offset of 16-byte chunk `c16` (0..15) of row `r` in a [128 rows x 128 cols] bf16 tile stored as two
@@ -101,6 +97,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   uint64_t* p_full = bars + 10;   // count 256
   uint64_t* pv_full = bars + 11;  // count 1
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+  volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* done = bars + 13;     // behind a run-out: the MMAs under way
   float* xch = reinterpret_cast<float*>(bars + 14);  // [2 parities][2 halves][128 rows] row maxima / denominators
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -143,6 +141,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     }
     mbar_init(p_full, T_SM_THREADS);
     mbar_init(pv_full, 1);
+    mbar_init(done, 1);
+    *dead = 0;
     mbar_fence_init();
   }
   if (warp == T_MMA_WARP) tmem_alloc(tmem_slot, T_TMEM_COLS);
@@ -163,19 +163,22 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  WaitTries tries;
 
   if (warp == T_LOAD_WARP) {
     // =========================== TMA loader ===========================
     if (lane == 0) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
+      bool go = true;  // false behind a run-out: a barrier must not be armed twice in one phase
       for (int j = 0; j < n_blocks; ++j) {
         const int s = j & 1;
         const uint32_t ph = (uint32_t)(((j >> 1) & 1) ^ 1);
         const int p0 = j * (TKV / TPAGE);
         const int npg = min(TKV / TPAGE, np - p0);  // pages of this block that exist
         const uint32_t kdst = smem_u32(KVs + (size_t)s * 2 * TILE_B), vdst = kdst + TILE_B;
-        mbar_wait_or_trap(k_empty + s, ph);
+        go = mbar_wait_bounded(k_empty + s, ph, dead, tries);
+        if (!go) break;
         mbar_expect_tx(k_full + s, (uint32_t)npg * 2 * (64 * TPAGE * 2));
         for (int p = 0; p < npg; ++p) {
           const int page = __ldg(pages + p0 + p);
@@ -183,7 +186,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
           tma_load_4d(kdst + o, &map_k, 0, kvh, 0, page, k_full + s);
           tma_load_4d(kdst + HALF_BYTES + o, &map_k, 64, kvh, 0, page, k_full + s);
         }
-        mbar_wait_or_trap(v_empty + s, ph);
+        go = mbar_wait_bounded(v_empty + s, ph, dead, tries);
+        if (!go) break;
         mbar_expect_tx(v_full + s, (uint32_t)npg * 2 * (64 * TPAGE * 2));
         for (int p = 0; p < npg; ++p) {
           const int page = __ldg(pages + p0 + p);
@@ -192,6 +196,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
           tma_load_4d(vdst + HALF_BYTES + o, &map_v, 64, kvh, 0, page, v_full + s);
         }
       }
+      if (!go) wait_for_copies();
     }
   } else if (warp == T_MMA_WARP) {
     // =========================== MMA issuer ===========================
@@ -201,7 +206,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     const uint32_t q_addr = smem_u32(Qs), p_addr = smem_u32(Ps);
     auto issue_s = [&](int j) {
       const int s = j & 1;
-      mbar_wait_or_trap(k_full + s, (uint32_t)((j >> 1) & 1));
+      mbar_wait_bounded(k_full + s, (uint32_t)((j >> 1) & 1), dead, tries);
       tc_fence_after();
       if (lane == 0) {
         const uint32_t k_addr = smem_u32(KVs + (size_t)s * 2 * TILE_B);
@@ -219,8 +224,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     if (n_blocks > 0) issue_s(0);
     for (int j = 0; j < n_blocks; ++j) {
       if (j + 1 < n_blocks) issue_s(j + 1);  // runs under the softmax of block j
-      mbar_wait_or_trap(p_full, (uint32_t)(j & 1));
-      mbar_wait_or_trap(v_full + (j & 1), (uint32_t)((j >> 1) & 1));
+      mbar_wait_bounded(p_full, (uint32_t)(j & 1), dead, tries);
+      mbar_wait_bounded(v_full + (j & 1), (uint32_t)((j >> 1) & 1), dead, tries);
       tc_fence_after();
       if (lane == 0) {
         const int s = j & 1;
@@ -254,7 +259,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     const uint32_t t_pv = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(2 * TKV + hh * 64);
     // O = O * alpha + P V of block jj (this thread's 64 output columns), 32 columns at a time
     auto fold_pv = [&](int jj, float alpha) {
-      mbar_wait_or_trap(pv_full, (uint32_t)(jj & 1));
+      mbar_wait_bounded(pv_full, (uint32_t)(jj & 1), dead, tries);
       tc_fence_after();
       {
         uint32_t t[64];
@@ -268,7 +273,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     };
     for (int j = 0; j < n_blocks; ++j) {
       const int sb = j & 1;
-      mbar_wait_or_trap(s_full + sb, (uint32_t)((j >> 1) & 1));
+      mbar_wait_bounded(s_full + sb, (uint32_t)((j >> 1) & 1), dead, tries);
       tc_fence_after();
       // Row maximum over all 128 columns, in raw score units (the scale is positive, so max and scale commute
       // exactly): the partner thread's 64 columns are reduced and dropped, ours are kept.  Both threads of a row
@@ -346,8 +351,17 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
                                  pack_bf16(o[c + 4] * inv, o[c + 5] * inv), pack_bf16(o[c + 6] * inv, o[c + 7] * inv));
     }
   }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0) count_run_out(dead, a.err);
+  if (*dead) {  // (for all alike, behind the barrier)
+    if (warp == T_MMA_WARP) {
+      if (lane == 0) umma_commit(done);
+      mbar_drain(done, 0);
+    }
+    __syncthreads();
+  }
   if (warp == T_MMA_WARP) {
     tc_fence_after();
     tmem_dealloc(tmem_base, T_TMEM_COLS);
@@ -383,6 +397,7 @@ int launch_prefill_tc(const bf16* q, bf16* out, const bf16* k_base, const bf16* 
   a.page_indices = page_indices; a.page_indptr = page_indptr; a.last_page_len = last_page_len; a.q_indptr = q_indptr;
   a.seq_len = seq_len; a.batch_size = batch_size; a.nq = nq; a.nkv = nkv;
   a.sm_scale_log2 = sm_scale_log2;
+  a.err = wait_err_word();
   constexpr size_t smem = 6 * TILE_B + 1024 + 256 + 2048;
   static thread_local bool cfg = false;
   if (!cfg) {

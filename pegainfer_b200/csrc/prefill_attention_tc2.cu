@@ -55,6 +55,7 @@ struct Args {
   const int* q_indptr;
   int seq_len, batch_size, nq, nkv;
   float sm_scale_log2;
+  unsigned int* err;  // wait_err_word()
   int dbg;  // PK_FA2_DBG ablation bits (timing experiments only; results are wrong when set): 1 no P V MMAs, 2 no S MMAs, 4 no exponentials, 8 no O rescale, 32 trace, 64 skip the first TMEM read of the max phase
 };
 
@@ -95,11 +96,6 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
       "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
       "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
       : "memory");
-}
-// A hung barrier becomes a trap (reported as a launch failure) instead of a wedged GPU.
-__device__ __forceinline__ void wait_or_trap(uint64_t* bar, uint32_t parity) {
-  for (uint32_t spins = 0; !mbar_try_wait(bar, parity); ++spins)
-    if (spins > (1u << 24)) __trap();
 }
 __device__ __forceinline__ uint32_t sw_off(int r, int c16) {
   return (uint32_t)((c16 >> 3) * HALF_BYTES + r * 128 + (((c16 & 7) ^ (r & 7)) << 4));
@@ -165,6 +161,8 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
   uint64_t* d_ready = bars + 18;      // [tile] final denominators published (128)   softmax -> correction
   uint64_t* p_rest = bars + 20;       // [tile] the k-steps of P(j) from EARLY_STEPS on stored (4 warp arrivals)  softmax -> MMA
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
+  volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* done = bars + 23;         // behind a run-out: the MMAs under way (an arrival per tile)
   float* alpha_s = reinterpret_cast<float*>(bars + 24);  // [tile][128]
   float* denom_s = alpha_s + 2 * TQ;                     // [tile][128]
 
@@ -242,6 +240,8 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
       mbar_init(d_ready + s, 4);
       mbar_init(p_rest + s, 4);
     }
+    mbar_init(done, 2);
+    *dead = 0;
     mbar_fence_init();
   }
   if (warp == W_MMA) tmem_alloc(tmem_slot, TMEM_COLS);
@@ -252,6 +252,7 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
   __syncthreads();  // barriers initialised, TMEM allocated
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  WaitTries tries;
   const bool trace_on = (a.dbg & 32) && blockIdx.x == 0 && blockIdx.y == 0;
 
   if (warp != W_LOAD) {
@@ -274,13 +275,15 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
     if (lane == 0) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
+      bool go = true;  // false behind a run-out: a barrier must not be armed twice in one phase
       for (int j = 0; j < nb; ++j) {
         const int s = j & 1;
         const uint32_t ph = (uint32_t)(((j >> 1) & 1) ^ 1);
         const int p0 = j * (TKV / PAGE);
         const int npg = min(TKV / PAGE, np - p0);
         const uint32_t kdst = smem_u32(KVs + (size_t)s * 2 * TILE_B), vdst = kdst + TILE_B;
-        wait_or_trap(k_empty + s, ph);
+        go = mbar_wait_bounded(k_empty + s, ph, dead, tries);
+        if (!go) break;
         mbar_expect_tx(k_full + s, (uint32_t)npg * 2 * (64 * PAGE * 2));
         for (int p = 0; p < npg; ++p) {
           const int page = __ldg(pages + p0 + p);
@@ -288,7 +291,8 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
           tma_load_4d(kdst + o, &map_k, 0, kvh, 0, page, k_full + s);
           tma_load_4d(kdst + HALF_BYTES + o, &map_k, 64, kvh, 0, page, k_full + s);
         }
-        wait_or_trap(v_empty + s, ph);
+        go = mbar_wait_bounded(v_empty + s, ph, dead, tries);
+        if (!go) break;
         mbar_expect_tx(v_full + s, (uint32_t)npg * 2 * (64 * PAGE * 2));
         for (int p = 0; p < npg; ++p) {
           const int page = __ldg(pages + p0 + p);
@@ -297,6 +301,7 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
           tma_load_4d(vdst + HALF_BYTES + o, &map_v, 64, kvh, 0, page, v_full + s);
         }
       }
+      if (!go) wait_for_copies();
     }
   } else if (warp >= W_MMA) {
     // =========================== MMA issuers: one single-thread pipeline per tile ===========================
@@ -334,18 +339,18 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
         // Stagger the tiles by half a block: tile 1 starts when tile 0 has the first part of its first P, so that one
         // tile's exponentials run under the other's MMAs instead of both contending for the MUFU and then for the
         // tensor pipe (nothing re-synchronises them afterwards; measured with tools/fa2_trace.py).
-        if (i == 1 && !(a.dbg & 128)) wait_or_trap(po_ready + 0, 0);
-        wait_or_trap(k_full, 0);
+        if (i == 1 && !(a.dbg & 128)) mbar_wait_bounded(po_ready + 0, 0, dead, tries);
+        mbar_wait_bounded(k_full, 0, dead, tries);
         tc_fence_after();
         issue_s(0);
       }
       for (int j = 0; j < n_i; ++j) {
         const int s = j & 1;
         // operands first (long since there in steady state), then the hand-over that is on the critical path
-        wait_or_trap(v_full + s, (uint32_t)((j >> 1) & 1));
-        if (j + 1 < n_i) wait_or_trap(k_full + (s ^ 1), (uint32_t)(((j + 1) >> 1) & 1));
+        mbar_wait_bounded(v_full + s, (uint32_t)((j >> 1) & 1), dead, tries);
+        if (j + 1 < n_i) mbar_wait_bounded(k_full + (s ^ 1), (uint32_t)(((j + 1) >> 1) & 1), dead, tries);
         if (i == 0) FA2_TRACE(1, j, 0);
-        wait_or_trap(po_ready + i, (uint32_t)(j & 1));  // the first part of P(j) stored and O scaled by alpha(j)
+        mbar_wait_bounded(po_ready + i, (uint32_t)(j & 1), dead, tries);  // the first part of P(j) stored and O scaled by alpha(j)
         tc_fence_after();
         if (i == 0) FA2_TRACE(1, j, 1);
         const uint64_t v_desc = make_sw128_mn_desc(smem_u32(KVs + (size_t)s * 2 * TILE_B) + TILE_B, HALF_BYTES, 1024);
@@ -356,7 +361,7 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
             if (k < ksteps) umma_bf16_ts(t_o, t_sp + (uint32_t)(k * 8), v_desc + (uint64_t)(k * (2048 >> 4)), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
         }
         __syncwarp();
-        wait_or_trap(p_rest + i, (uint32_t)(j & 1));  // the rest of P(j)
+        mbar_wait_bounded(p_rest + i, (uint32_t)(j & 1), dead, tries);  // the rest of P(j)
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
@@ -380,11 +385,11 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
       for (int i = 0; i < 2; ++i) {
         if (j >= nblk(i)) continue;
         if (j > 0) {
-          wait_or_trap(a_ready + i, (uint32_t)((j - 1) & 1));
+          mbar_wait_bounded(a_ready + i, (uint32_t)((j - 1) & 1), dead, tries);
           if (i == 0 && q4 == 0) FA2_TRACE(2, j, 0);
           const float alpha = alpha_s[i * TQ + r];
           const bool need = !__all_sync(0xffffffffu, alpha == 1.0f);
-          wait_or_trap(pv_done + i, (uint32_t)((j - 1) & 1));  // O holds blocks < j
+          mbar_wait_bounded(pv_done + i, (uint32_t)((j - 1) & 1), dead, tries);  // O holds blocks < j
           tc_fence_after();
           if (i == 0 && q4 == 0) FA2_TRACE(2, j, 1);
           if (need && !(a.dbg & 8)) {
@@ -411,8 +416,8 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
     // epilogue: O / d -> bf16 -> global, one row per thread
     for (int i = 0; i < 2; ++i) {
       if (nblk(i) == 0) continue;
-      wait_or_trap(d_ready + i, 0);
-      wait_or_trap(pv_done + i, (uint32_t)((nblk(i) - 1) & 1));
+      mbar_wait_bounded(d_ready + i, 0, dead, tries);
+      mbar_wait_bounded(pv_done + i, (uint32_t)((nblk(i) - 1) & 1), dead, tries);
       tc_fence_after();
       const int tok = t0 + i * TQ + r;
       const float inv = __fdividef(1.f, denom_s[i * TQ + r]);
@@ -446,7 +451,7 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
     float m = -INFINITY, d = 0.f;
     const int n_i = nblk(i);
     for (int j = 0; j < n_i; ++j) {
-      wait_or_trap(s_full + i, (uint32_t)(j & 1));
+      mbar_wait_bounded(s_full + i, (uint32_t)(j & 1), dead, tries);
       tc_fence_after();
       if (warp == 0) FA2_TRACE(0, j, 0);
       const bool masked = !__all_sync(0xffffffffu, j * TKV + TKV - 1 <= lim);  // warp-uniform
@@ -549,8 +554,17 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
       if (lane == 0) mbar_arrive(d_ready + i);
     }
   }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0) count_run_out(dead, a.err);
+  if (*dead) {  // (for all alike, behind the barrier)
+    if (warp == W_MMA || warp == W_MMA + 1) {
+      if (elect_one()) umma_commit(done);
+      mbar_drain(done, 0);
+    }
+    __syncthreads();
+  }
   if (warp == W_MMA) {
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
@@ -594,6 +608,7 @@ int launch_prefill_tc2(const bf16* q, bf16* out, const bf16* k_base, const bf16*
   a.page_indices = page_indices; a.page_indptr = page_indptr; a.last_page_len = last_page_len; a.q_indptr = q_indptr;
   a.seq_len = seq_len; a.batch_size = batch_size; a.nq = nq; a.nkv = nkv;
   a.sm_scale_log2 = sm_scale_log2;
+  a.err = wait_err_word();
   {
     const char* e = getenv("PK_FA2_DBG");
     a.dbg = e ? atoi(e) : 0;
