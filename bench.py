@@ -1,14 +1,14 @@
 #!/usr/bin/env python
-"""Headline benchmark: Qwen3 greedy decode tok/s (+ TTFT) on B200, BASELINE.json's metric.
+"""Headline benchmark: Qwen3 greedy decode tok/s (+ TTFT) on B200.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 
-N = 1 : BASELINE config[1] -- Qwen3-4B bf16, 2048-token prefill + decode at ctx 2048.., CUDA Graph on,
+N = 1 : Qwen3-4B bf16, 2048-token prefill + decode at ctx 2048.., CUDA Graph on,
         single request.  A "step" is one decode step (one generated token).  The same line also carries
-        BASELINE config[0] (128-token prompt / 64-token decode: `config1`), the Qwen3-8B single-GPU point of
-        config[2] (`tp_base`), BASELINE config[3] (Qwen3.5-4B hybrid, 1024-token prompt: `config4`) and the reference's
+        Qwen3-4B with a 128-token prompt and 64-token decode (`config1`), the Qwen3-8B single-GPU point of
+        the tensor-parallel runs (`tp_base`), the Qwen3.5-4B hybrid with a 1024-token prompt (`config4`) and the reference's
         own CUDA kernels under the same host (`gpu_reference`).
-N > 1 : BASELINE config[2] -- Qwen3-8B bf16, tensor parallel over N ranks (one process per GPU,
+N > 1 : Qwen3-8B bf16, tensor parallel over N ranks (one process per GPU,
         NVLink peer-memory all-reduce), 128-token prompt, decode steps.  scaling = "strong"; the line carries
         `tp1` = the same model / prompt / steps on ONE GPU measured in the same run (rank 0's GPU), so a
         strong-scaling ratio can be formed on one model.
@@ -16,13 +16,13 @@ Checkpoint: random-init weights of the exact architecture generated ON THE CPU (
 pegainfer_b200/synthetic.py) -- the checkpoint the parity tests and the committed oracle fixtures use -- and
 synthetic prompt ids ((i % 1000) + 100, bench_serving.rs:761-763); there is no network for checkpoints.
 
-Keys of the JSON line (see the task contract):
+Keys of the JSON line:
   value     decode tok/s with inputs resident in HBM (per-step metadata pre-staged on the device, token
             fed back on the device, no host sync inside the timed region; CUDA events on the stream)
   e2e       the same metric through the public API with HOST token ids: per step one H2D metadata copy
             from pinned memory, the graph launch, a 4-byte D2H of the sampled token and a stream sync
   parity    the benchmarked model checked against the CPU oracle's committed fixture for this configuration
-            (tests/golden/parity_*.npz: prefill + 8 teacher-forced decode steps, SURVEY 8c rule) BEFORE timing
+            (tests/golden/parity_*.npz: prefill + 8 teacher-forced decode steps) BEFORE timing
   ttft_tensor  TTFT against the tensor roofline: prompt GEMM + causal attention flops / TTFT vs the measured sustained bf16 peak
   roofline  the dominant kernel (the HBM-streaming decode GEMV): algorithmic weight bytes per token /
             CUDA-event time of the token's 145 GEMV launches, vs MEASURED_PEAKS.json hbm_gbs; `traffic` = measured
@@ -73,7 +73,7 @@ PARITY_TOL_ULP = 12  # tests/test_fullsize_gpu.py TOL_ULP
 
 # ------------------------------------------------------------------------------------ helpers
 def weight_bytes_per_token(cfg, world=1, lm_head_rows=None):
-    """SURVEY.md 8d / BASELINE.md 2: decode weight bytes per token per GPU (`lm_head_rows`: the rows of the output
+    """Decode weight bytes per token per GPU (`lm_head_rows`: the rows of the output
     projection this rank streams -- the whole vocabulary unless lm_head is vocab-sharded)."""
     H, I, L, V = cfg.hidden_size, cfg.intermediate_size, cfg.num_hidden_layers, cfg.vocab_size
     per_layer = 2 * (H * (cfg.q_dim + 2 * cfg.kv_dim) + H * cfg.q_dim + 3 * H * I)
@@ -100,7 +100,7 @@ def host_threads():
 
 
 def prefill_tensor_summary(cfg, prompt_len, ttft_ms, world):
-    """TTFT against the tensor roofline (SURVEY 8d): dense GEMM flops of the prompt + causal attention + one lm_head row,
+    """TTFT against the tensor roofline: dense GEMM flops of the prompt + causal attention + one lm_head row,
     per GPU, over the measured TTFT (which also holds the host-side planning and the first sampling)."""
     try:
         h, i, l, v = cfg.hidden_size, cfg.intermediate_size, cfg.num_hidden_layers, cfg.vocab_size
@@ -403,7 +403,7 @@ def make_tp_comm(rank, world, dist, max_tokens, hidden):
 
 # ------------------------------------------------------------------------------------ parity against the fixtures
 def parity_check(model, cfg, prompt_len, world, rank, dist):
-    """Teacher-forced prefill + decode steps of the benchmarked model vs the committed oracle fixture (SURVEY 8c rule).
+    """Teacher-forced prefill + decode steps of the benchmarked model vs the committed oracle fixture.
     Every rank runs the model; rank 0 compares.  Returns a dict for the JSON line (None on other ranks)."""
     import torch
     from pegainfer_b200.synthetic import synthetic_prompt
@@ -537,7 +537,7 @@ def run_ours(args, cfg, rank, world, dist):
     e2e_ms, burst_ms, ttft_ms = max_over_ranks(e2e_ms), max_over_ranks(burst_ms), max_over_ranks(ttft_ms)
     launches_per_step = model.launches_per_step()
 
-    # ---- BASELINE config[0] in the same run: 128-token prompt, 64 generated tokens (1 prefill + 63 decode steps) ----
+    # ---- in the same run: 128-token prompt, 64 generated tokens (1 prefill + 63 decode steps) ----
     config1 = None
     if world == 1:
         p128 = synthetic_prompt(128)
@@ -548,7 +548,7 @@ def run_ours(args, cfg, rank, world, dist):
         tokc = model.sample_greedy(model.prefill([p128], [kvc])[0])
         _, b_ms = model.decode_burst(kvc, tokc, 63)
         model.drop_request(kvc)
-        config1 = {"workload": "Qwen3-4B, 128-token prompt / 64-token greedy decode, bs 1 (BASELINE config 0)",
+        config1 = {"workload": "Qwen3-4B, 128-token prompt / 64-token greedy decode, bs 1",
                    "ttft_ms": statistics.median(t1), "decode_tok_s_e2e": len(gaps) / (sum(gaps) * 1e-3),
                    "decode_tok_s": 63 / (b_ms * 1e-3), "decode_steps": 63, "parity": parity1}
 
@@ -664,10 +664,10 @@ def cpu_baseline_leg(cfg, weights_cpu):
 
 def gpu_reference_leg(cfg, weights_cpu, prompt, pages):
     """The reference's OWN CUDA kernels (cuBLAS GEMV/GEMM + FlashInfer attention/norm/top-1, compiled from
-    /root/reference by oracle/Makefile into oracle/_ref) driven by the same C++ host through the identical C ABI, the
+    the reference tree by oracle/Makefile into oracle/_ref) driven by the same C++ host through the identical C ABI, the
     reference's op sequence, CUDA Graph on: the 'existing kernel to beat' on this box.  Reported baseline only."""
     if not os.path.exists(REF_LIB):
-        return {"available": False, "why": "oracle/_ref/libkernels_ref.so not built (needs /root/reference at build time)"}
+        return {"available": False, "why": "oracle/_ref/libkernels_ref.so not built (needs the reference tree at build time)"}
     from pegainfer_b200.model import ModelRuntimeConfig, Qwen3Model
     try:
         m = Qwen3Model(cfg, weights_cpu, ModelRuntimeConfig(enable_cuda_graph=True, fused=False, num_pages=pages, max_batch=1,
@@ -688,7 +688,7 @@ def gpu_reference_leg(cfg, weights_cpu, prompt, pages):
         ttft128 = statistics.median([m.generate(p128, 1)[1] for _ in range(3)])
         m.close()
         return {"available": True, "decode_tok_s": n / (ms * 1e-3), "ms_per_step": ms / n, "ttft_ms": ttft, "ttft_128_ms": ttft128,
-                "steps": n, "what": "reference kernels (cuBLAS + FlashInfer, sm_100 build of /root/reference/pegainfer-kernels/csrc) "
+                "steps": n, "what": "reference kernels (cuBLAS + FlashInfer, sm_100 build of pegainfer-kernels/csrc) "
                 "under the same host and C ABI, reference op sequence (batch_decode.rs), split-KV decode attention, CUDA Graph; "
                 "timed through the public API (host token in/out per step)"}
     except Exception as e:  # a baseline leg must never take the benchmark down
@@ -696,7 +696,7 @@ def gpu_reference_leg(cfg, weights_cpu, prompt, pages):
 
 
 def config4_leg(device):
-    """BASELINE config 4: Qwen3.5-4B hybrid (24 gated-delta-rule + 8 full-attention layers, head dim 256), 1024-token
+    """Qwen3.5-4B hybrid (24 gated-delta-rule + 8 full-attention layers, head dim 256), 1024-token
     prompt, single request: TTFT and decode tok/s through the C++ hybrid host.  Random-init checkpoint generated on the
     GPU; parity of this path is pinned on the tiny hybrid stack (tests/test_qwen35_model_gpu.py vs the HF-pinned numpy
     oracle) -- the 4B hybrid has no CPU oracle run (the numpy restatement is token-by-token)."""
@@ -713,7 +713,7 @@ def config4_leg(device):
         _, _, gaps = m.generate(prompt, 129)
         tpot = statistics.median(gaps[1:])
         wbytes = sum(int(torch.tensor(s).prod()) * (4 if d == torch.float32 else 2) for s, d in weight_shapes(QWEN35_4B).values())
-        state_bytes = 24 * 32 * 128 * 128 * 4 * 2  # fp32 delta-rule state read + written per token (SURVEY 8d config 4)
+        state_bytes = 24 * 32 * 128 * 128 * 4 * 2  # fp32 delta-rule state read + written per token
         peak, _ = measured_peaks()
         launches = m.launches_per_step()
         m.close()
@@ -727,7 +727,7 @@ def config4_leg(device):
 
 
 def tp_base_leg(cfg8, device):
-    """Qwen3-8B on ONE GPU, 128-token prompt, 256 decode steps: the N=1 point of BASELINE config 2 ('1/2/4/8')."""
+    """Qwen3-8B on ONE GPU, 128-token prompt, 256 decode steps: the N=1 point of the tensor-parallel runs."""
     from pegainfer_b200.model import ModelRuntimeConfig, Qwen3Model
     from pegainfer_b200.synthetic import iter_random_weights, synthetic_prompt
     import torch

@@ -9,7 +9,7 @@
  * (INTEGRATION.md shows the build.rs change).  Section "B200 extensions" adds the
  * fused / tensor-parallel entry points the reference does not have.
  *
- * Conventions (reference: SURVEY.md 8b):
+ * Conventions:
  *  - pk_bf16 = uint16_t bf16 bit pattern (`pub type Half = u16`, ffi.rs:4).
  *  - All pointers are DEVICE pointers unless a comment says host.
  *  - Activations are `HiddenStates[dim, tokens]`: token t occupies elements
@@ -172,7 +172,7 @@ void gpu_sample_flashinfer_cuda(const pk_bf16* logits, float* probs_scratch, uin
 
 /* =============================== B200 extensions ===============================
  * Not in ffi.rs.  The fused decode layer used by the host mirror
- * (pegainfer_b200/csrc/host) and the TP hook north_star asks pegainfer-comm to gain. */
+ * (pegainfer_b200/csrc/host) and the tensor-parallel collectives. */
 
 /* Library / build identification ("pegainfer-kernels-b200 sm_100a ..."). */
 const char* pk_b200_version(void);
@@ -291,7 +291,7 @@ int pk_b200_prefill_attention_tc(const pk_bf16* q, pk_bf16* output, const pk_bf1
 
 /* Measurement aid of prefill_attention_tc2.cu: with PK_FA2_DBG=32 the heaviest CTA of head 0 stamps %clock64 at the
  * hand-over points of its tile 0; this copies the stamps ([role: softmax, MMA issuer, correction][block < 128][8] u64) to
- * the host (tools/fa2_trace.py, profiles/r2_prefill_attention.md).  The other PK_FA2_DBG bits (1 no P V MMAs, 2 no S
+ * the host.  The other PK_FA2_DBG bits (1 no P V MMAs, 2 no S
  * MMAs, 4 no exponentials, 8 no O rescale, 64 skip one TMEM read, 128 no tile stagger) are timing ablations and give
  * wrong results by construction; unset = the product path.  Returns cudaError. */
 int pk_b200_fa2_trace_copy(void* host_out, int bytes);

@@ -1,4 +1,4 @@
-"""CPU restatement of the reference's Qwen3.5 hybrid forward (SURVEY.md section 8(f)-1, BASELINE config 4).
+"""CPU restatement of the reference's Qwen3.5 hybrid forward.
 
 TEST INFRASTRUCTURE ONLY, groundwork for the next scope row: nothing under pegainfer_b200/ may import it.  It restates,
 with the reference's rounding points, the per-token recurrent form of every Qwen3.5 op; the reference's prefill uses
@@ -7,7 +7,7 @@ Pinned against HF transformers' `Qwen3_5ForCausalLM` (the reference's declared e
 scripts/generate_test_data.py) by tests/test_oracle_qwen35.py: tiny random-init hybrid model, logits within a few bf16
 ulps of the row maximum, arg-max identical.
 
-Reference rules followed (paths relative to /root/reference):
+Reference rules followed (paths relative to the reference repo root):
   * (1+w) RMSNorm, one rounding             pegainfer-kernels/csrc/flashinfer_norm.cu:108-133 (FlashInfer GemmaRMSNorm)
   * full attention: q_proj rows per head = [q(hd) | gate(hd)], per-head (1+w) norm -> bf16, partial NeoX RoPE on the
     first rotary_dim dims with bf16 cos/sin, gate = sigmoid in fp32, one rounding each
@@ -152,7 +152,7 @@ class OracleQwen35:
         for h in range(nq):
             s = (K[:, h // grp] @ q[h]).astype(np.float32) * scale
             pr = np.exp(s - s.max(), dtype=np.float32)
-            if prefill:  # FA2 prefill rounds P to bf16 and sums the rounded P; the decode kernel keeps fp32 (a6 / a8)
+            if prefill:  # FA2 prefill rounds P to bf16 and sums the rounded P; the decode kernel keeps fp32
                 pr = rb(pr)
             out[h] = rb((pr @ V[:, h // grp]) / pr.sum(dtype=np.float32))
         out = rb(out * (1.0 / (1.0 + np.exp(-gate, dtype=np.float32))))

@@ -12,7 +12,7 @@
  * noted; all accumulation is fp32 (FMA-contracted, like the GPU).  Reduction
  * ORDER is the oracle's own (the reference's cuBLAS / FlashInfer orders are
  * unspecified), so parity against CUDA is stated with a tolerance of a few
- * bf16 ulps per op, not bit equality -- see DESIGN.md "Parity".
+ * bf16 ulps per op, not bit equality.
  *
  * Pinning: tests/test_oracle_golden.py checks this file against every
  * weight-free known-answer test the reference holds for the path

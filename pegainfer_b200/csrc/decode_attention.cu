@@ -7,7 +7,7 @@
 // fp32; s = (q.k) * sm_scale * log2(e); running max / denominator with ex2.approx; o = sum p*v in
 // fp32; o/d rounded ONCE to bf16.  The ABI split-KV entry keeps the reference's rounding of the
 // per-chunk NORMALISED partial to bf16 (tmp_v) and base-2 LSE (tmp_s); the internal split used by
-// the non-partition / fused entries keeps fp32 partials (documented in DESIGN.md).
+// the non-partition / fused entries keeps fp32 partials.
 //
 // HBM-bound: K+V bytes per (token, kv head) = 512; algorithmic bytes per call = 4096 * kv_len.
 // Layout: one CTA per (kv chunk, kv head, request); the 4 warps stride over the chunk's tokens,

@@ -5,7 +5,7 @@
 // 16-byte rows requested before the current round is reduced), keeps an online-softmax state per half-warp,
 // merges inside the CTA through shared memory, then writes its (max, denominator, 4 x 128 numerators) straight
 // into the LEADER CTA's shared memory over DSMEM (st.shared::cluster), one cluster barrier, and the leader
-// produces the bf16 output.  Compared with the ticket version in decode_attention.cu (profiles/README.md,
+// produces the bf16 output.  Compared with the ticket version in decode_attention.cu (with
 // the kernel before it: 22 us per layer, of which the partial-store -> __threadfence -> atomic ticket -> L2 re-read chain
 // is 3-4 dependent global round trips) there is no global-memory synchronisation at all.
 // The CTA that owns the step's position also appends the normed/roped K and the V row to the paged cache and

@@ -1,7 +1,7 @@
 // Fused decode attention: TMA page tiles + tensor-core (mma.sync) score / PV products.
 //
 // Why: the LDG cluster kernel (decode_attention_cluster.cu) reads K/V with per-lane LDGs and reduces every
-// q.k product with a 4-level shuffle tree -- ncu (profiles/r1_v4_attn_cluster_full_details.txt) shows ~215 issued
+// q.k product with a 4-level shuffle tree -- ncu shows ~215 issued
 // instructions per token row and 2 warps per scheduler: latency-bound on its own instruction stream (6.8 cycles per
 // issue), 6 % of DRAM bandwidth, 64 CTAs on 148 SMs.  Here:
 //   * one thread-block cluster of up to 16 CTAs per (request, kv head) -> 128 CTAs for Qwen3-4B at bs 1; CTA r owns a

@@ -2,7 +2,7 @@
 //
 // Why: the single-CTA kernel (gemm.cu, cta_group::1, M128 x N256 x K16 per instruction) reads 12 KB of operands from
 // shared memory per 128-cycle instruction and TMA writes another 12 KB: ~190 B/clk against a 128 B/clk shared-memory
-// port.  ncu (profiles/r1_v3_gemm_full_details.txt) shows the tensor pipe 61-64 % active and cuBLAS' sm_100 kernels
+// port.  ncu shows the tensor pipe 61-64 % active and cuBLAS' sm_100 kernels
 // 1.27-1.53 PFLOP/s against our 0.77-1.20 on the same shapes.  A CTA pair (two SMs of one TPC) computes a
 // 256-token x BN-feature tile: each CTA stages its OWN 128 tokens of A and only HALF of B (BN/2 features), the
 // pair's tensor cores share the B halves, so per SM the operand traffic is 8 KB read + 8 KB written per instruction.

@@ -1,4 +1,4 @@
-// C++ mirror of the reference's Rust host side for the Qwen3.5 hybrid model (SURVEY 8f-1, BASELINE config 4):
+// C++ mirror of the reference's Rust host side for the Qwen3.5 hybrid model:
 //   config / layer kinds       pegainfer-qwen35-4b/src/config.rs:4-155
 //   weights                    pegainfer-qwen35-4b/src/weights.rs:25-390 (HF `qwen3_5` text-model tensor names)
 //   recurrent state            pegainfer-qwen35-4b/src/recurrent_state.rs:9-55  (per request: conv window + fp32 S per linear layer)

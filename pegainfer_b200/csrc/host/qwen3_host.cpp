@@ -193,7 +193,7 @@ struct Qwen3Model {
   int local_inter() const { return config.intermediate_size / tp.world_size; }
   int local_q_dim() const { return local_heads() * config.head_dim; }
   int local_kv_dim() const { return local_kv_heads() * config.head_dim; }
-  // Vocab-sharded lm_head (SURVEY 8f-4): on the fused TP path every rank streams only rows [rank * V/N, (rank+1) * V/N)
+  // Vocab-sharded lm_head: on the fused TP path every rank streams only rows [rank * V/N, (rank+1) * V/N)
   // of the output projection and the greedy token is agreed on with a (max, index) exchange; the reference keeps
   // lm_head replicated (weights.rs:104-119), which is what mode 0 (its op sequence) still does.
   bool vocab_sharded() const {
@@ -854,7 +854,7 @@ bool Qwen3Model::decode_kernels_fused(int bs) {
   // Fused attention launch; when the kernel library offers it, the launch also prefetches into L2 the weights the
   // next two GEMVs will stream (all of o_proj, the leading rows of every gate_up slice): bs-1 attention is
   // latency-bound and would otherwise leave HBM idle for ~10 us per layer.  PK_PF_O / PK_PF_GU = rows per GEMV
-  // slice to request (0 disables), defaults tuned on B200 (profiles/README.md).
+  // slice to request (0 disables), defaults tuned on B200.
   static const int pf_o_rows = [] { const char* e = getenv("PK_PF_O"); return e ? atoi(e) : 0; }();
   static const int pf_gu_rows = [] { const char* e = getenv("PK_PF_GU"); return e ? atoi(e) : 0; }();
   const bool can_prefetch = k.pk_b200_decode_attention_fused_prefetch && k.pk_b200_gemv_slices && (pf_o_rows > 0 || pf_gu_rows > 0);
@@ -892,7 +892,7 @@ bool Qwen3Model::decode_kernels_fused(int bs) {
   //  * fused: the row-parallel GEMVs (o_proj, down_proj) push their partial rows to every rank
   //    (epi 2) and the following GEMV's prologue reduces them (x_mode 2): 5 launches per layer, the layer's two
   //    all-reduces live inside the GEMVs.
-  //  Measured (Qwen3-8B, bs 1, profiles/README.md): 2 x B200 398 vs 367 tok/s, 8 x B200 411 vs 350 tok/s -- every one
+  //  Measured (Qwen3-8B, bs 1): 2 x B200 398 vs 367 tok/s, 8 x B200 411 vs 350 tok/s -- every one
   //  of the push epilogue's ~300 CTAs pays a system-scope fence after its remote stores and the grid ticket
   //  serialises behind them, which costs more than a single-CTA collective launch.
   //  * ll (default): the row-parallel GEMVs reduce their own rows INSIDE the kernel (epi 3: 8-byte {data, seq} lines

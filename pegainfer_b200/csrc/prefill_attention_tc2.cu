@@ -5,7 +5,7 @@
 // 128-token KV block, P rounded to bf16 for P V, denominator = row sum of the ROUNDED P (flashinfer prefill.cuh:956-985
 // sums the converted fragment on the tensor cores), O / d rounded once to bf16.
 //
-// Why a second design (profiles/r1_v6_prefill_attn_tc_full_details.txt): the first kernel keeps ONE query tile per CTA
+// Why a second design: the first kernel (prefill_attention_tc.cu) keeps ONE query tile per CTA
 // and folds P V into register-resident O in the softmax warps -- ~790 instructions per softmax warp per KV block on
 // 2 warps per scheduler, 68 % of cycles with no eligible warp, tensor pipe 15 % busy.  Here
 //   * each CTA owns 256 query tokens of one head as two tiles; while tile A's softmax runs, the tensor core does tile
@@ -59,7 +59,7 @@ struct Args {
   int dbg;  // PK_FA2_DBG ablation bits (timing experiments only; results are wrong when set): 1 no P V MMAs, 2 no S MMAs, 4 no exponentials, 8 no O rescale, 32 trace, 64 skip the first TMEM read of the max phase
 };
 
-// PK_FA2_DBG bit 32: the heaviest CTA of head 0 records %clock64 at the hand-over points of tile 0 (tools/fa2_trace.py)
+// PK_FA2_DBG bit 32: the heaviest CTA of head 0 records %clock64 at the hand-over points of tile 0 (pk_b200_fa2_trace_copy)
 __device__ unsigned long long g_fa2_trace[3 * 128 * 8];
 #define FA2_TRACE(role, j, slot)                                                                                  \
   do {                                                                                                            \
@@ -305,7 +305,7 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
     }
   } else if (warp >= W_MMA) {
     // =========================== MMA issuers: one single-thread pipeline per tile ===========================
-    // The trace of the one-issuer version (tools/fa2_trace.py) showed the issuing thread busy ~100 % of the time: every
+    // The trace of the one-issuer version showed the issuing thread busy ~100 % of the time: every
     // tcgen05.mma stalls until the tensor queue has room, so issue time ~ execution time, and the waits / commits
     // between the batches (~320 cycles each) left the pipe dry.  Two issuers (disjoint TMEM regions) interleave in the
     // hardware queue, the K / V arrivals are checked before the P hand-over, and the descriptors are precomputed.
@@ -338,7 +338,7 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
       if (n_i > 0) {
         // Stagger the tiles by half a block: tile 1 starts when tile 0 has the first part of its first P, so that one
         // tile's exponentials run under the other's MMAs instead of both contending for the MUFU and then for the
-        // tensor pipe (nothing re-synchronises them afterwards; measured with tools/fa2_trace.py).
+        // tensor pipe (nothing re-synchronises them afterwards; measured with that trace).
         if (i == 1 && !(a.dbg & 128)) mbar_wait_bounded(po_ready + 0, 0, dead, tries);
         mbar_wait_bounded(k_full, 0, dead, tries);
         tc_fence_after();

@@ -227,13 +227,13 @@ extern "C" int pk_top1_rows_f32(const float* logits, int* out, int rows, int voc
 }
 
 // =====================================================================================================
-// Non-greedy sampling (SURVEY.md 8f-3): temperature softmax + top-k / top-p filtering + multinomial draw.
+// Non-greedy sampling: temperature softmax + top-k / top-p filtering + multinomial draw.
 // Replaces csrc/flashinfer_sampling.cu:13-110 (logits_to_probs_kernel + FlashInfer
 // {TopKTopP,TopK,TopP,}SamplingFromProb).  Distribution semantics are the reference's: probs =
 // softmax(bf16 logits * inv_temperature) in fp32; a token is eligible iff it is among the top_k most probable
 // (top_k > 0) AND inside the smallest prefix of the probability-sorted vocabulary whose mass reaches top_p
 // (top_p < 1), both evaluated on the unfiltered probs ("joint" filtering); the draw is from the renormalised
-// eligible set.  The RANDOM STREAM is not FlashInfer's Philox: u = splitmix64(seed) (documented in DESIGN.md);
+// eligible set.  The RANDOM STREAM is not FlashInfer's Philox: u = splitmix64(seed);
 // the reference's own test only pins greedy-equivalent cases and "token in range" (ops/tests.rs:228-305).
 // One CTA; thresholds by bisection on the fp32 bit pattern (probabilities are >= 0, so bits are monotone).
 namespace pk {

@@ -1,6 +1,5 @@
 // Tensor-parallel all-reduce over NVLink peer memory, optionally fused with the residual add +
-// RMSNorm that follows it in the layer.  This is the hook north_star asks pegainfer-comm to gain;
-// it replaces `Qwen3Model::all_reduce_hidden` (pegainfer-qwen3-4b/src/weights.rs:396-405, an
+// RMSNorm that follows it in the layer.  It replaces `Qwen3Model::all_reduce_hidden` (pegainfer-qwen3-4b/src/weights.rs:396-405, an
 // ncclAllReduce on the compute stream) and the fused_add_rms_norm launch after it
 // (batch_decode.rs:266-277,292 / prefill.rs:154-163).
 //

@@ -46,7 +46,7 @@ def _layer_types(n: int, full_every: int = 4) -> tuple:
     return tuple("full_attention" if (i + 1) % full_every == 0 else "linear_attention" for i in range(n))
 
 
-# Qwen3.5-4B text model (docs/models/qwen35/optimization.md:57-77; SURVEY 8d config 4): 24 linear + 8 full-attention layers
+# Qwen3.5-4B text model (docs/models/qwen35/optimization.md:57-77): 24 linear + 8 full-attention layers
 QWEN35_4B = Qwen35Config(2560, 9216, 32, 16, 4, 256, 248320, 16, 32, 128, 128, 4, _layer_types(32), 1e-6, 1e7, 0.25, "qwen3.5-4b")
 # small hybrid stack for parity tests the numpy oracle finishes in seconds (the kernels' head sizes are fixed: 256 / 128 x 128)
 QWEN35_TINY = Qwen35Config(256, 512, 4, 4, 1, 256, 512, 2, 4, 128, 128, 4,

@@ -1,7 +1,7 @@
 """Random-init Qwen3 checkpoints and synthetic prompts (no network, no real weights).
 
 Weights follow HF ``Qwen3ForCausalLM`` default init (Linear / Embedding N(0, 0.02),
-norm weights 1.0 -- SURVEY.md section 8d) under the HF tensor names the reference's
+norm weights 1.0) under the HF tensor names the reference's
 loader reads (pegainfer-qwen3-4b/src/weights.rs:100-291).  Prompt ids follow
 pegainfer-server/src/bin/bench_serving.rs:761-763: ``(i % 1000) + 100``.
 """

@@ -4,7 +4,7 @@
 A fixture is the CPU oracle's output for one (model, tp_world, prompt_len) run on the seed-0 CPU-generated
 random-init checkpoint (pegainfer_b200/synthetic.py), teacher-forced with the oracle's own greedy tokens:
 per step (prefill + n decode steps) the 256 largest logits (index + bf16 bits), every 16th logit of the row,
-the row's max |logit| (the ulp scale of the SURVEY 8c rule) and the top-1/top-2 margin.  ~20 KB per step instead of
+the row's max |logit| (the ulp scale of the parity rule) and the top-1/top-2 margin.  ~20 KB per step instead of
 the 300 KB full row; written by tests/golden/make_parity_fixtures.py (committed generator).
 """
 from __future__ import annotations
@@ -84,7 +84,7 @@ class Fixture:
         return int(self.idx_top[step][0])
 
     def compare(self, step: int, got_bits: np.ndarray, max_ulp_rowmax: float) -> tuple[bool, dict]:
-        """SURVEY 8c rule on the sampled row: |dlogit| <= N bf16 ulps at the row's max magnitude on the top-256 and
+        """Parity rule on the sampled row: |dlogit| <= N bf16 ulps at the row's max magnitude on the top-256 and
         the strided sample, arg-max equal unless the oracle's top-1/top-2 gap is inside the tolerance."""
         g = _f32(np.asarray(got_bits, np.uint16).reshape(-1))
         tol = max_ulp_rowmax * bf16_ulp(self.rowmax[step])

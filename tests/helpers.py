@@ -44,7 +44,7 @@ def assert_bf16_close(got_bits, want_bits, max_ulp, floor=0.0, frac_exact=None, 
 
 
 def logits_agree(got_bits, want_bits, max_ulp_rowmax):
-    """SURVEY 8c parity rule: |dlogit| <= N ulp at the row's max magnitude, and arg-max
+    """Parity rule: |dlogit| <= N ulp at the row's max magnitude, and arg-max
     equality unless the oracle's top-1/top-2 gap is within that tolerance."""
     g, w = f32(got_bits), f32(want_bits)
     tol = max_ulp_rowmax * float(O.bf16_ulp(np.abs(w).max()))

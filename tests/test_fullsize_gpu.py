@@ -1,7 +1,7 @@
-"""Parity at the configurations the benchmark runs (VERDICT r1 row g; BASELINE.json configs 1 and 2).
+"""Parity at the configurations the benchmark runs.
 
 The model under test is the FULL Qwen3-4B (36 layers, V = 151,936) on the seed-0 CPU-generated random-init
-checkpoint -- the same checkpoint bench.py loads -- teacher-forced against the CPU oracle with the SURVEY 8c rule
+checkpoint -- the same checkpoint bench.py loads -- teacher-forced against the CPU oracle with the parity rule
 (every logit within TOL bf16 ulps of the row's max magnitude; arg-max equal unless the oracle's top-1/top-2 gap is
 inside the tolerance), plus the free-running first-divergence index (reported).  The reference's counterpart:
 HF bf16 greedy on the real model (scripts/generate_test_data.py:41-52) and the real-model batch/sequential test
@@ -30,7 +30,7 @@ from tests.helpers import bits, logits_agree, oracle_cfg
 pytestmark = [pytest.mark.gpu,
               pytest.mark.skipif(os.environ.get("PK_SKIP_FULLSIZE") == "1", reason="PK_SKIP_FULLSIZE=1")]
 
-# bf16 ulps at the row's max |logit| after 36 layers.  Measured on B200 (profiles/README.md):
+# bf16 ulps at the row's max |logit| after 36 layers.  Measured on B200:
 # fused 7.4 worst over 65 steps of config 1, 5.4 on config 2; compat 5.9 / 5.0 -- rounding-point flips accumulate as
 # ~sqrt(layers) (the 2-4 layer configs of test_model_gpu.py sit at <= 2 with a bound of 6).  12 = 1.6 x the worst seen.
 TOL_ULP = 12

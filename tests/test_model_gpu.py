@@ -1,7 +1,7 @@
 """Model-level parity on the GPU: the C++ host mirror driving the sm_100a kernels through the C ABI,
 teacher-forced against the CPU oracle on the same random-init weights and synthetic token ids.
 
-Parity rule (SURVEY.md 8c): at every step feed the ORACLE's token; require every logit within
+Parity rule: at every step feed the ORACLE's token; require every logit within
 `TOL_ULP` bf16 ulps of the row's max magnitude and arg-max equality unless the oracle's top-1/top-2
 gap is inside that tolerance.  Runs the B200 fused path, the reference op sequence on our kernels
 (`fused=False`) and -- when oracle/_ref exists -- the reference's own kernels under the same host."""

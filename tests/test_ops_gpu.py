@@ -456,7 +456,7 @@ def test_top1_matches_argmax(lib, n):
             assert float(val[0].float()) == float(xf[want])
 
 
-# ------------------------------------------------------------------ non-greedy sampling (SURVEY 8f-3)
+# ------------------------------------------------------------------ non-greedy sampling
 def _sample(lib, logits, inv_t, top_k, top_p, seed):
     n = logits.numel()
     probs = torch.zeros(n, dtype=torch.float32, device="cuda")
@@ -690,7 +690,7 @@ def test_prefill_attention_tc(starts, lens, nq, nkv, impl, monkeypatch):
     from tests.helpers import ulp_err
     e = ulp_err(bits(out).ravel(), np.asarray(want).ravel(), float(np.abs(f32(want)).max()) / 32)
     print(f"\n[prefill attention {impl}] lens {lens} starts {starts}: max err {e.max():.2f} ulp, {float((e == 0).mean()):.4f} bit-exact")
-    # Measured on B200 (profiles/r2_prefill_attention_parity.txt): 1.1-2.5 ulp on every case but the one whose chunk starts
+    # Measured on B200: 1.1-2.5 ulp on every case but the one whose chunk starts
     # 900 tokens into the request (6.7 ulp): there the kernels' 128-token blocks and the oracle's 64-token tiles advance the
     # running maximum at different KV positions over a long cached prefix, so more P values round differently.
     tol = 8 if max(starts) >= 512 else 4

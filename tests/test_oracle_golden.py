@@ -1,5 +1,5 @@
 """Pin the CPU oracle against every weight-free golden vector the reference holds
-for the hot path (SURVEY.md 8c) and against the committed HF fixture.  CPU only."""
+for the hot path and against the committed HF fixture.  CPU only."""
 import math
 import os
 
@@ -71,7 +71,7 @@ def test_kv_layout_stride_geometry():  # pegainfer-core/src/kv_pool.rs:290-310
     from pegainfer_b200.paged_kv import PagedKvLayout
     l35 = PagedKvLayout.new(8, 4, 256, 16)
     assert (l35.kv_block_len, l35.layer_stride, l35.page_stride) == (16384, 32768, 262144)
-    l4b = PagedKvLayout.new(36, 4, 128, 16)  # SURVEY section 4: page_stride == 589_824
+    l4b = PagedKvLayout.new(36, 4, 128, 16)  # page_stride == 589_824
     assert l4b.page_stride == 589_824
     assert PagedKvLayout.new(36, 8, 128, 16).page_stride == 1_179_648  # 2.25 MiB / page
 

@@ -1,4 +1,4 @@
-"""Pins oracle/qwen35_oracle.py (groundwork for SURVEY 8(f)-1, the Qwen3.5 hybrid layers) to HF transformers through the
+"""Pins oracle/qwen35_oracle.py (the Qwen3.5 hybrid layers) to HF transformers through the
 committed fixture tests/golden/hf_qwen35_tiny.npz (generator: tests/golden/make_hf_qwen35_fixtures.py)."""
 import os
 

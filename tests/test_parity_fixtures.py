@@ -1,5 +1,5 @@
 """The committed full-size oracle fixtures (tests/golden/parity_*.npz) are self-consistent and belong to the checkpoint
-the generator produces: what the GPU parity tests and bench.py's `parity` key compare against (SURVEY 8c)."""
+the generator produces: what the GPU parity tests and bench.py's `parity` key compare against."""
 import glob
 import os
 

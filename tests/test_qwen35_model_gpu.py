@@ -1,4 +1,4 @@
-"""Qwen3.5 hybrid model (BASELINE config 4, SURVEY 8f-1): the C++ host (csrc/host/qwen35_host.cpp) driving the sm_100a
+"""Qwen3.5 hybrid model: the C++ host (csrc/host/qwen35_host.cpp) driving the sm_100a
 kernels through the C ABI, against oracle/qwen35_oracle.py (pinned to HF Qwen3_5ForCausalLM by tests/test_oracle_qwen35.py)
 on a tiny random-init hybrid stack: batched prefill (tensor-core GEMMs, conv1d, delta-rule sequence kernel, HD-256 paged
 prefill attention), chunked prefill, then teacher-forced decode steps through the CUDA graph."""

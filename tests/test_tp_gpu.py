@@ -1,9 +1,9 @@
-"""Tensor-parallel parity on real GPUs (SURVEY 8 row a15 / BASELINE config 3): runs tests/tools/tp_check.py under
+"""Tensor-parallel parity on real GPUs: runs tests/tools/tp_check.py under
 torchrun when the machine has >= 2 GPUs; skipped on one with a single GPU.
 
 * all-reduce kernels (plain, fused with add + RMSNorm) vs torch / the CPU oracle, bit-exact rank-ordered sums
 * Qwen3-small TP-N and the FULL Qwen3-8B TP-N (36 layers, V = 151,936) prefill + decode logits, teacher-forced
-  against the CPU oracle's TP-N model on the seed-0 CPU checkpoint (SURVEY 8c rule).
+  against the CPU oracle's TP-N model on the seed-0 CPU checkpoint (parity rule of tests/helpers.py).
 """
 import os
 import subprocess

@@ -1,8 +1,8 @@
-"""decode GEMV + GQA decode-attention microbench, cold L2, CUDA events.
+"""Decode GEMV + GQA decode-attention microbench, cold L2, CUDA events.
 
 Protocol after the reference's kernel bench (pegainfer-qwen3-4b/src/kernel_bench.rs:236-282,569-586): a streaming
 sweep of a buffer >= 2 x L2 before every timed launch, one untimed pre-launch, N timed launches each bracketed by its
-own event pair.  GEMV: every Qwen3-4B / 8B projection shape (SURVEY.md section 8 row a3), bytes = 2*M*K + 2K + 2M.
+own event pair.  GEMV: every Qwen3-4B / 8B projection shape, bytes = 2*M*K + 2K + 2M.
 Attention: the reference's own case (1 layer, nq 32, nkv 8, hd 128, page 16, bs 1, patterned q / kv), bytes =
 4096*seq + 16 KiB, seq in {1, 128, 1024, 4096}.  When oracle/_ref/libkernels_ref.so is present the reference's own
 kernels (cuBLAS GEMV, FlashInfer decode) are timed beside ours under the same protocol.

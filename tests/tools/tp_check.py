@@ -4,9 +4,9 @@ against torch / the CPU oracle, (2) Qwen3 TP-N prefill + decode logits against t
     python -m torch.distributed.run --nnodes=1 --nproc-per-node 2 --master-addr 127.0.0.1 --master-port 29511 \
         tests/tools/tp_check.py [--model qwen3-small|qwen3-8b] [--prompt 40] [--steps 6]
 
-`--model qwen3-8b` is BASELINE config 3 at full size (36 layers, V = 151,936, untied lm_head): rank 0 generates the
+`--model qwen3-8b` is the full size (36 layers, V = 151,936, untied lm_head): rank 0 generates the
 seed-0 CPU checkpoint (the one bench.py loads), runs the TP-N oracle on the host cores and broadcasts every tensor to
-the other ranks over NCCL; the GPU side is teacher-forced with the oracle's tokens (SURVEY 8c rule).
+the other ranks over NCCL; the GPU side is teacher-forced with the oracle's tokens (parity rule of tests/helpers.py).
 tests/test_tp_gpu.py runs this file under pytest when the box has >= 2 GPUs.
 """
 import argparse
