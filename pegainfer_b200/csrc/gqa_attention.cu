@@ -18,6 +18,7 @@
 //   gqa_attention_kernel        one CTA per (query row, query head): warps stride over the visible keys with an online
 //                               softmax each (lanes split the features), merged with the sink at the end.  Any sizes.
 //   gqa_attention_mma_kernel    bf16 prompt portions on the tensor cores (64 query rows of one head per CTA).
+//   gqa_attention_cluster_kernel  the same where these CTAs leave SMs idle: a cluster shares the keys.
 //   gqa_decode_kernel           bf16, fewer than 64 rows: request by request on the tensor cores, a group's query heads as the rows of a tile.
 #include "common.cuh"
 #include "mma.cuh"
@@ -324,33 +325,22 @@ __global__ void __launch_bounds__(128, 3) gqa_attention_mma_kernel(const bf16* _
                                                                bf16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
                                                                long page_stride, int page_size, int T, int H, int G, float scale, int chunk,
                                                                AttnExtra x) {
-  constexpr int LDK = DQ + 8, LDV = DV + 8;
-  extern __shared__ __align__(16) unsigned char am_smem[];  // two stages of [keys][LDK] K and [keys][LDV] V
-  bf16* const Ks0 = reinterpret_cast<bf16*>(am_smem);
-  bf16* const Vs0 = Ks0 + 2 * kAmKeys * LDK;
-  __shared__ int s_req[kAmRows], s_pos[kAmRows];
-  __shared__ long long s_slot[2][kAmKeys];  // per stage: element offset of every key row's cache slot (-1: not to be read)
+  extern __shared__ __align__(16) unsigned char am_smem[];
   pdl_wait();
   pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
   // grid (head, tile, split): the heads of a tile start together (a group's heads read the same keys), and the tiles run from the
   // end of the step backwards, so that the CTAs that start last are the ones with the fewest visible keys
   const int t0 = (gridDim.y - 1 - blockIdx.y) * kAmRows, h = blockIdx.x, g = h / (H / G);
 #define GQA_T_END T
-#define GQA_CLUSTER 0
 #define GQA_SPLIT blockIdx.z
 #define GQA_SPLITS gridDim.z
 #define GQA_PART_LD nsplit
 #include "gqa_tile.cuh"
-#undef GQA_T_END
-#undef GQA_CLUSTER
-#undef GQA_SPLIT
-#undef GQA_SPLITS
-#undef GQA_PART_LD
 }
 
 // The same for steps whose (tile, head) pairs leave SMs idle: the keys are dealt out to the CTAs of a cluster (the grid's z axis), which combine their states
-// over distributed shared memory.  B200, us, with the append (heads / groups x size): 229 tokens of 6 requests behind 480 (8 / 2 x 128) 91.6 -> 48.6,
-// 100 behind 500 (8 / 4 x 64) 26.9 -> 21.7, 1500 behind 400 (8 / 4 x 64) 80.6 -> 60.7.
+// over distributed shared memory.  B200, us (heads / groups x size): 229 tokens of 6 requests behind 480 (8 / 2 x 128) 74.6 -> 33.8, 100 behind 500 (8 / 4 x 64)
+// 21.3 -> 13.0, 64 behind 2000 (8 / 2 x 128) 93.6 -> 26.9.
 template <int DQ, int DV>
 __global__ void __launch_bounds__(128, 3) gqa_attention_cluster_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache, const bf16* __restrict__ sink,
                                                                const int* __restrict__ pos, const int* __restrict__ req,
@@ -358,12 +348,7 @@ __global__ void __launch_bounds__(128, 3) gqa_attention_cluster_kernel(const bf1
                                                                bf16* __restrict__ out,
                                                                long page_stride, int page_size, int T, int H, int G, float scale, int chunk,
                                                                AttnExtra x) {
-  constexpr int LDK = DQ + 8, LDV = DV + 8;
-  extern __shared__ __align__(16) unsigned char am_smem[];  // two stages of [keys][LDK] K and [keys][LDV] V
-  bf16* const Ks0 = reinterpret_cast<bf16*>(am_smem);
-  bf16* const Vs0 = Ks0 + 2 * kAmKeys * LDK;
-  __shared__ int s_req[kAmRows], s_pos[kAmRows];
-  __shared__ long long s_slot[2][kAmKeys];  // per stage: element offset of every key row's cache slot (-1: not to be read)
+  extern __shared__ __align__(16) unsigned char am_smem[];
   pdl_wait();
   pdl_launch_dependents();  // the next kernel may start its launch; it waits for this grid to finish before it reads
   const int t0 = (gridDim.y - 1 - blockIdx.y) * kAmRows, h = blockIdx.x, g = h / (H / G);
@@ -373,11 +358,6 @@ __global__ void __launch_bounds__(128, 3) gqa_attention_cluster_kernel(const bf1
 #define GQA_SPLITS gridDim.z
 #define GQA_PART_LD nsplit
 #include "gqa_tile.cuh"
-#undef GQA_T_END
-#undef GQA_CLUSTER
-#undef GQA_SPLIT
-#undef GQA_SPLITS
-#undef GQA_PART_LD
 }
 
 // Steps of fewer than 64 rows (below): how a request with several tokens in the step runs.  Launched are cs CTAs for each of its tokens and kv heads; request by
@@ -415,23 +395,12 @@ __device__ __forceinline__ void gqa_tile_of_run(unsigned char* am_smem, const bf
                                                 const int* __restrict__ pages, bf16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
                                                 long page_stride, int page_size, int T, int H, int G, float scale, int chunk, const AttnExtra& x,
                                                 const GdRun run, int h, int share, int most) {
-  constexpr int LDK = DQ + 8, LDV = DV + 8;
-  bf16* const Ks0 = reinterpret_cast<bf16*>(am_smem);
-  bf16* const Vs0 = Ks0 + 2 * kAmKeys * LDK;
-  __shared__ int s_req[kAmRows], s_pos[kAmRows];
-  __shared__ long long s_slot[2][kAmKeys];  // per stage: element offset of every key row's cache slot (-1: not to be read)
   const int t0 = run.start, g = h / (H / G);
 #define GQA_T_END run.start + run.len
-#define GQA_CLUSTER 0
 #define GQA_SPLIT share
 #define GQA_SPLITS run.shares
 #define GQA_PART_LD most
 #include "gqa_tile.cuh"
-#undef GQA_T_END
-#undef GQA_CLUSTER
-#undef GQA_SPLIT
-#undef GQA_SPLITS
-#undef GQA_PART_LD
 }
 
 // one CTA per (row, head): combine the splits' (m, l, O), join the sink, apply the output gate

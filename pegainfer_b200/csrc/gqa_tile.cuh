@@ -1,6 +1,15 @@
 // Body of a CTA that works on 64 rows of one query head (gqa_attention.cu): rows t0 .. t0 + 63 as far as they lie below GQA_T_END, share GQA_SPLIT of GQA_SPLITS of
 // the keys of their requests; several shares leave their states at part_o / part_ml [head][GQA_PART_LD][T].  Included where the kernel of whole steps and
-// the one of few rows need it: as a function that both call, the first was 3 to 5 % slower (registers).
+// the one of few rows need it: as a function that both call, the first was 3 to 5 % slower (registers).  With GQA_CLUSTER the shares are the CTAs of a cluster,
+// and their states meet over distributed shared memory.  am_smem: two stages of [keys][LDK] K and [keys][LDV] V.  The macros end with the file.
+#ifndef GQA_CLUSTER
+#define GQA_CLUSTER 0
+#endif
+  constexpr int LDK = DQ + 8, LDV = DV + 8;
+  bf16* const Ks0 = reinterpret_cast<bf16*>(am_smem);
+  bf16* const Vs0 = Ks0 + 2 * kAmKeys * LDK;
+  __shared__ int s_req[kAmRows], s_pos[kAmRows];
+  __shared__ long long s_slot[2][kAmKeys];  // per stage: element offset of every key row's cache slot (-1: not to be read)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gq = lane >> 2, tq = lane & 3;
   if (tid < kAmRows) {
     const int t = t0 + tid;
@@ -251,3 +260,8 @@
     if (req_b >= 0) *reinterpret_cast<uint32_t*>(out + (size_t)(t0 + rb) * x.out_ld + h * DV + c) = pack_bf16(oa[ni][2] * i_b * g2, oa[ni][3] * i_b * g3);
   }
 #endif
+#undef GQA_T_END
+#undef GQA_CLUSTER
+#undef GQA_SPLIT
+#undef GQA_SPLITS
+#undef GQA_PART_LD

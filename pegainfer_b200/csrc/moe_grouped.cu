@@ -426,6 +426,7 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
   const float g = shared ? (sg ? 1.f / (1.f + expf(-sg[t])) : 1.f) : 0.f;
   for (int i = threadIdx.x; i < nv; i += blockDim.x) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    // two rows under way (four: 0.5 to 1 % of a call more up to 512 tokens, the same beyond), which leave L2 first (2048 tokens 260 -> 256 us)
 #pragma unroll 2
     for (int k = 0; k < top; ++k) {
       const float4 p = __ldcs(reinterpret_cast<const float4*>(part + (size_t)pair_slot[(size_t)t * top + k] * width) + i);
@@ -522,8 +523,9 @@ extern "C" int pk_moe_grouped_act_p(const void* xa, const void* w_up, const void
     launch(moe_gather_kernel, dim3((unsigned)pairs), dim3(width >= 2048 ? 256 : 128), 0, st, true, (const bf16*)xa, (const int*)slot_pair, xs, width, top);
   }
   // From 24 rows an expert on the rows, hidden values and partial sums (100 MB in the call of 2048 tokens) are worth their room in L2, and up to a row tile
-  // an expert the weights are read once: they leave first, where they are too many to be found in L2 again.  B200, 64 experts of 2048 x 1408, top 6, us:
-  // 256 / 512 / 1024 / 2048 tokens 197 207 225 270 -> 188 193 210 264; without the bounds it would be 64 tokens 187 197, 4096 438 445.
+  // an expert the weights are read once: they leave first, where they are too many to be found in L2 again.  B200, 64 experts of 2048 x 1408, top 6, gated, us:
+  // 256 / 512 / 1024 / 2048 tokens 189 199 220 262 -> 181 184 205 257 in a train over other weights each time (a single call with cold caches spreads by as much);
+  // without the bounds it would be 64 tokens 187 197, 4096 438 445.
   const bool w_first = pairs >= 24l * experts && pairs <= (kMoeTile - 16l) * experts && (long)experts * width * ff * (act ? 6 : 4) > (256l << 20);
   MgArgs a{hid, meta, slot_pair, weights, experts, max_tiles, act ? 2 * ff : ff, width, p0, p1, wait_err_word()};
   cudaError_t e = act == 2 ? mg_gemm<3>(w_first, xs, pairs, w_up, a, st) : act == 1 ? mg_gemm<2>(w_first, xs, pairs, w_up, a, st) : mg_gemm<0>(w_first, xs, pairs, w_up, a, st);

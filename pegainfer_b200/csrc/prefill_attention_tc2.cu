@@ -171,7 +171,7 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
   const int kvh = head / (a.nq / a.nkv);
 
   // ---- locate (request, 256-token tile pair): late (heavy) pairs first.  Of many requests one per lane: one after the other every CTA waits for their
-  // loads, twice (B200, 32 heads, us: 60 requests of 40 tokens 128 -> 91, 20 of 100 41 -> 37); 3 of 1111 tokens take 70.8, and a lane each 71.9 ----
+  // loads, twice (B200, 32 heads, us: 60 requests of 40 tokens 128 -> 87, 20 of 100 41 -> 36); 3 of 1111 tokens take 70.8, and a lane each 71.9 ----
   int b = 0, q_start = 0, qo_len = 0, pair = -1;
   {
     if (a.batch_size <= 8) {
