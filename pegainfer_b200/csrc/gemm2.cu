@@ -176,7 +176,6 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
       const int mb = tile % m_tiles, nb = tile / m_tiles;
       const int as = lt % NBUF;
       mbar_wait_bounded(tfull + as, (uint32_t)((lt / NBUF) & 1), dead);
-      __syncwarp();
       tc_fence_after();
       const int tok = mb * 2 * G2_BM + (int)rank * G2_BM + q * 32 + lane;
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * TN);
@@ -261,15 +260,14 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
       if (lane == 0) g2_arrive_cluster(tempty_leader0 + (uint32_t)(as * 8));
     }
   }
-  __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0) count_run_out(dead, a.err);
   cluster_barrier();  // the peer's MMAs / loads may still target this CTA's shared memory and TMEM
   if (warp == 1) {
     tc_fence_after();
     g2_tmem_dealloc(tmem_base, TMEM_COLS);
   }
+  if (threadIdx.x == 0) count_run_out(dead, a.err);
 }
 
 template <int BN, int NSUB, int STAGES>

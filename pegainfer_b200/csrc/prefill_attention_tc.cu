@@ -351,11 +351,10 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
                                  pack_bf16(o[c + 4] * inv, o[c + 5] * inv), pack_bf16(o[c + 6] * inv, o[c + 7] * inv));
     }
   }
-  __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0) count_run_out(dead, a.err);
   if (*dead) {  // (for all alike, behind the barrier)
+    __syncwarp();
     if (warp == T_MMA_WARP) {
       if (lane == 0) umma_commit(done);
       mbar_drain(done, 0);
@@ -366,6 +365,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     tc_fence_after();
     tmem_dealloc(tmem_base, T_TMEM_COLS);
   }
+  if (threadIdx.x == 0) count_run_out(dead, a.err);
 }
 
 // 4-D view of one layer's K (or V) block of the page-first pool: {head dim 128, kv head, slot 16, page};

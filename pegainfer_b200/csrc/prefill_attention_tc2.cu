@@ -554,11 +554,10 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
       if (lane == 0) mbar_arrive(d_ready + i);
     }
   }
-  __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0) count_run_out(dead, a.err);
   if (*dead) {  // (for all alike, behind the barrier)
+    __syncwarp();
     if (warp == W_MMA || warp == W_MMA + 1) {
       if (elect_one()) umma_commit(done);
       mbar_drain(done, 0);
@@ -569,6 +568,7 @@ prefill_attention_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
+  if (threadIdx.x == 0) count_run_out(dead, a.err);
 }
 
 // 4-D view of one layer's K (or V) block of the page-first pool: {head dim 128, kv head, slot 16, page};
