@@ -212,14 +212,13 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   const int k_tok = ((lm_i >> 1) << 3) + lm_r, k_c = lm_i & 1;   // K: matrices {tok 0-7 lo, tok 0-7 hi, tok 8-15 lo, tok 8-15 hi}
   const int v_tok = ((lm_i & 1) << 3) + lm_r, v_c = lm_i >> 1;   // V: {tok 0-7 | tok 8-15} x {dims 8d | 8(d+1)}
 
-  WaitTries tries;
-  bool go = true;  // false behind a run-out: a barrier must not be armed twice in one phase
+  WaitTries tries;  // none left behind a run-out: a barrier must not be armed twice in one phase
   // a slot is consumed by ONE warp (slot & 7), in page order: walk the ring passes, then this warp's slots
   for (int base = 0, pass = 0; base < my_pages; base += nslot, ++pass)
   for (int slot = warp; slot < nslot; slot += T_WARPS) {
     const int lp = base + slot;
     if (lp >= my_pages) break;
-    go &= mbar_wait_bounded(full + slot, (uint32_t)(pass & 1), dead, tries);
+    mbar_wait_bounded(full + slot, (uint32_t)(pass & 1), dead, tries);
     uint8_t* tile = tiles + (size_t)slot * T_SLOT;
     const int gp = p_lo + lp;
     if (lp == pos_lp) {  // patch the step's own row into the tile (the TMA saw the slot before it was written)
@@ -293,7 +292,7 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     // refill: this warp is the only reader of the slot -> request the page that reuses it
     if (lp + nslot < my_pages) {
       __syncwarp();
-      if (lane == 0 && go) {
+      if (lane == 0 && tries.left) {
         fence_proxy_async_smem();
         issue_page(lp + nslot);
       }
@@ -303,7 +302,7 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
 
   // ---- per-warp states -> shared memory (aliases the page ring: every warp must be done with its tiles) ----
-  if (!go) wait_for_copies();
+  if (tries.left == 0) wait_for_copies();
   __syncthreads();
   if (g < T_GROUP) {
     if (tq == 0) {
